@@ -368,3 +368,73 @@ def tolerance(case):
     if kind == "sgd":
         return {"rel": 3e-7}
     return "exact"  # one rank: data movement and casts
+
+
+# ---- what a pass returns, in 64 bits ---------------------------------------------
+
+def _exact_bn(s):
+    bn, x, residual = s["bn"], s["x"], s["residual"]
+    n = x.numel() // x.size(1)
+
+    def column(v):
+        return v.view(1, -1, 1, 1)
+
+    with torch.no_grad():
+        xhat = x.double()
+        var, mean = torch.var_mean(xhat, (0, 2, 3), unbiased=False)
+        xhat.sub_(column(mean)).mul_(column(torch.rsqrt(var + bn.eps)))
+        weight, bias = bn.weight.double(), bn.bias.double()
+        y = (xhat * column(weight)).add_(column(bias))
+        if residual is not None:
+            y.add_(residual)
+        dz = s["dy"].double()
+        if bn.relu:
+            y.relu_()
+            dz.mul_(y > 0)
+        db, dw = dz.sum((0, 2, 3)), (dz * xhat).sum((0, 2, 3))
+        dx = xhat.mul_(column(-dw / n)).add_(dz).sub_(column(db / n))
+        dx.mul_(column(weight * torch.rsqrt(var + bn.eps)))
+        keep = 1.0 - bn.momentum
+        unbiased = var * (n / max(n - 1, 1))
+        running = [bn.running_mean.double() * keep + mean * bn.momentum,
+                   bn.running_var.double() * keep + unbiased * bn.momentum]
+        return [y, *running, dx, dw, db] + ([dz] if residual is not None else [])
+
+
+def _exact_pool(s):
+    x = s["x"].detach().double().requires_grad_(True)
+    y = F.max_pool2d(x, 3, stride=2, padding=1)
+    return y.detach(), torch.autograd.grad(y, x, s["dy"].double())[0]
+
+
+def _exact_sgd(case, s):
+    optimizer = s["optimizer"]
+    weights, momentum = s["weights"].double(), s["momentum"].double()
+    for p in optimizer.param_groups[0]["params"]:
+        m = optimizer.state[p]["momentum_buffer"]
+        w64 = torch.as_strided(weights, p.shape, p.stride(), p.storage_offset())
+        m64 = torch.as_strided(momentum, m.shape, m.stride(), m.storage_offset())
+        g = p.grad.double() + case["weight_decay"] * w64
+        m64.mul_(0.9).add_(g)
+        w64.sub_(0.01 * (g + 0.9 * m64 if case["nesterov"] else m64))
+    return weights.detach(), momentum
+
+
+def exact(case, seed):
+    """What ``run`` returns for these inputs, computed by PyTorch in 64 bits. A
+    training step of the whole model has no such value here."""
+    kind = case["kind"]
+    if kind == "train":
+        return None
+    s = prepare(case, seed)
+    if kind == "bn":
+        return _exact_bn(s)
+    if kind == "pool":
+        return _exact_pool(s)
+    if kind == "sgd":
+        with torch.no_grad():
+            return _exact_sgd(case, s)
+    if kind == "grouped":  # the cast is part of what was asked for
+        sent = {"none": torch.float32, "fp16": torch.float16, "bf16": torch.bfloat16}
+        return [x.to(sent[case["compression"]]).float() for x in s["x"]]
+    return s["x"].clone()  # one rank
