@@ -378,13 +378,13 @@ cudaError_t LaunchBatchNormBackward(const void* dy, const void* y, const void* x
 
 // 3x3 / stride 2 / padding 1 max pooling on channels-last 16-bit activations
 // ([n, h, w, channels], channels a multiple of 8). Forward writes the maxima
-// and one byte per output element naming the winning window position (0..8);
-// backward gathers dy through those bytes into dx (every element written).
+// and one word per 8 channels with the winning window position (0..8) of each in
+// a nibble; backward gathers dy through those into dx (every element written).
 bool MaxPool3s2Supported(int channels);
-cudaError_t LaunchMaxPool3s2Forward(const void* x, void* y, unsigned char* idx, int n, int h,
-                                    int w, int channels, bool bf16, cudaStream_t stream);
-cudaError_t LaunchMaxPool3s2Backward(const void* dy, const unsigned char* idx, void* dx, int n,
-                                     int h, int w, int channels, bool bf16, cudaStream_t stream);
+cudaError_t LaunchMaxPool3s2Forward(const void* x, void* y, uint32_t* idx, int n, int h, int w,
+                                    int channels, bool bf16, cudaStream_t stream);
+cudaError_t LaunchMaxPool3s2Backward(const void* dy, const uint32_t* idx, void* dx, int n, int h,
+                                     int w, int channels, bool bf16, cudaStream_t stream);
 
 // Multi-tensor SGD step in one launch (torch.optim.SGD arithmetic: weight
 // decay added to the gradient, momentum buffer b = momentum * b + (1 -

@@ -144,7 +144,8 @@ void BindModelOps(py::module_& m) {
   m.def("maxpool3s2_supported", [](int64_t channels) {
     return kern::MaxPool3s2Supported(static_cast<int>(channels));
   });
-  // x -> (y, idx): idx holds one byte per output element (winning window position).
+  // x -> (y, idx): idx holds one word per 8 output channels (a nibble for the
+  // winning window position of each).
   m.def("maxpool3s2_forward", [](const at::Tensor& x) {
     CheckActivations(x, "x");
     const int64_t N = x.size(0), C = x.size(1), H = x.size(2), W = x.size(3);
@@ -154,10 +155,10 @@ void BindModelOps(py::module_& m) {
     c10::cuda::CUDAGuard guard(x.device());
     cudaStream_t stream = at::cuda::getCurrentCUDAStream();
     at::Tensor y = at::empty({N, C, Ho, Wo}, x.options(), at::MemoryFormat::ChannelsLast);
-    at::Tensor idx = at::empty({N, Ho, Wo, C}, x.options().dtype(at::kByte));
+    at::Tensor idx = at::empty({N, Ho, Wo, C / 8}, x.options().dtype(at::kInt));
     cudaError_t err = kern::LaunchMaxPool3s2Forward(
-        x.data_ptr(), y.data_ptr(), idx.data_ptr<uint8_t>(), static_cast<int>(N),
-        static_cast<int>(H), static_cast<int>(W), static_cast<int>(C),
+        x.data_ptr(), y.data_ptr(), reinterpret_cast<uint32_t*>(idx.data_ptr<int32_t>()),
+        static_cast<int>(N), static_cast<int>(H), static_cast<int>(W), static_cast<int>(C),
         x.scalar_type() == at::kBFloat16, stream);
     TORCH_CHECK(err == cudaSuccess, "fused max pooling forward: ", cudaGetErrorString(err));
     return std::make_tuple(y, idx);
@@ -167,17 +168,17 @@ void BindModelOps(py::module_& m) {
                                   int64_t W) {
     CheckActivations(dy, "dy");
     const int64_t N = dy.size(0), C = dy.size(1);
-    TORCH_CHECK(idx.is_cuda() && idx.scalar_type() == at::kByte && idx.is_contiguous() &&
-                    idx.numel() == dy.numel(),
-                "idx must be the byte tensor returned by maxpool3s2_forward");
+    TORCH_CHECK(idx.is_cuda() && idx.scalar_type() == at::kInt && idx.is_contiguous() &&
+                    idx.numel() * 8 == dy.numel(),
+                "idx must be the tensor returned by maxpool3s2_forward");
     TORCH_CHECK(dy.size(2) == (H + 2 - 3) / 2 + 1 && dy.size(3) == (W + 2 - 3) / 2 + 1,
                 "dy does not match the pooled size of an input of ", H, " x ", W);
     c10::cuda::CUDAGuard guard(dy.device());
     cudaStream_t stream = at::cuda::getCurrentCUDAStream();
     at::Tensor dx = at::empty({N, C, H, W}, dy.options(), at::MemoryFormat::ChannelsLast);
     cudaError_t err = kern::LaunchMaxPool3s2Backward(
-        dy.data_ptr(), idx.data_ptr<uint8_t>(), dx.data_ptr(), static_cast<int>(N),
-        static_cast<int>(H), static_cast<int>(W), static_cast<int>(C),
+        dy.data_ptr(), reinterpret_cast<const uint32_t*>(idx.data_ptr<int32_t>()), dx.data_ptr(),
+        static_cast<int>(N), static_cast<int>(H), static_cast<int>(W), static_cast<int>(C),
         dy.scalar_type() == at::kBFloat16, stream);
     TORCH_CHECK(err == cudaSuccess, "fused max pooling backward: ", cudaGetErrorString(err));
     return dx;

@@ -5,7 +5,7 @@ PyTorch's ``F.max_pool2d`` everywhere else.
 PyTorch's channels-last max pooling stores an int64 index per output element
 and scatters the gradient with atomics; on the ResNet-50 stem (256 x 64 x 112
 x 112 in bf16) forward plus backward take 2.5 ms per step on a B200. The
-kernels here keep one byte per output element and gather in backward, which
+kernels here keep half a byte per output element and gather in backward, which
 moves a third of the bytes and needs no atomics. Ties and NaN follow PyTorch's
 rule, so outputs and gradients are identical. The reference has no
 counterpart (it takes pooling from the framework).
