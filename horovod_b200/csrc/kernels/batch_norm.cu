@@ -8,12 +8,19 @@
 // consecutive channels of one row (or several rows when C is smaller), so every
 // access is a fully coalesced 512-byte line. Each pass is bound by HBM traffic:
 // the forward reads x twice and writes y once (the PyTorch eager sequence
-// batch_norm + add + relu makes eight passes), the backward reads dy, y, x
-// twice and writes dx (and dres).
+// batch_norm + add + relu makes eight passes), the backward reads dy and x
+// twice and writes dx (and dres). The backward never reads y: without a
+// residual, y > 0 follows from x and the saved scale and shift by the
+// forward's own arithmetic; with one, the forward leaves one bit per element.
 //
-// Per-channel sums are accumulated in fp32 per thread (a few dozen rows), in
-// fp32 across the CTA, and in fp64 across CTAs (atomicAdd on doubles), then
-// mean/variance are formed in fp64.
+// The second kernel of a pair walks the rows from the last to the first, so
+// what the first kernel read last is still in L2 when the second one starts,
+// and is launched while the first one still runs (programmatic dependent
+// launch), which hides its launch latency.
+//
+// Per-channel sums are accumulated in fp32 per thread (a few dozen groups of
+// rows), in fp64 across the warps of a CTA and across CTAs (atomicAdd on
+// doubles), then mean/variance are formed in fp64.
 //
 // The reference has no counterpart: it takes batch normalisation from the
 // framework (horovod/torch/sync_batch_norm.py:98-199 calls
@@ -23,6 +30,7 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <type_traits>
 
 #include "kernels.h"
 
@@ -35,35 +43,64 @@ constexpr int BN_THREADS = 256;
 // Resident CTAs per SM the compiler must leave room for (register budget):
 // these are streaming kernels whose throughput is set by the bytes in flight
 // per SM, i.e. by occupancy.
-constexpr int BN_MIN_BLOCKS_APPLY = 3;   // <= 85 registers per thread
-constexpr int BN_MIN_BLOCKS_REDUCE = 4;  // <= 64 registers per thread
+constexpr int BN_MIN_BLOCKS = 3;        // <= 85 registers per thread
+constexpr int BN_MIN_BLOCKS_STATS = 4;  // <= 64 registers per thread
 constexpr int VEC = 8;  // 16-bit elements per 16-byte access
+constexpr int UNROLL = 4;  // rows in flight per thread
 
-template <typename T> __device__ __forceinline__ float bn_to_float(T v);
-template <> __device__ __forceinline__ float bn_to_float(__nv_bfloat16 v) {
-  return __bfloat162float(v);
-}
-template <> __device__ __forceinline__ float bn_to_float(__half v) { return __half2float(v); }
-template <typename T> __device__ __forceinline__ T bn_from_float(float v);
-template <> __device__ __forceinline__ __nv_bfloat16 bn_from_float(float v) {
-  return __float2bfloat16(v);
-}
-template <> __device__ __forceinline__ __half bn_from_float(float v) { return __float2half(v); }
-
-template <typename T> union Vec8 {
-  uint4 raw;
-  T e[VEC];
+// Two channels per 32-bit word.
+template <typename T> struct Pair;
+template <> struct Pair<__nv_bfloat16> {
+  using type = __nv_bfloat162;
+  static __device__ __forceinline__ float2 widen(type v) { return __bfloat1622float2(v); }
+  static __device__ __forceinline__ type narrow(float a, float b) {
+    return __floats2bfloat162_rn(a, b);
+  }
+};
+template <> struct Pair<__half> {
+  using type = __half2;
+  static __device__ __forceinline__ float2 widen(type v) { return __half22float2(v); }
+  static __device__ __forceinline__ type narrow(float a, float b) { return __floats2half2_rn(a, b); }
 };
 
-__device__ __forceinline__ uint4 ldg16(const void* p) {
-  uint4 v;
+// 8 channels of one row.
+template <typename T> struct Vec8 {
+  using P = typename Pair<T>::type;
+  uint32_t w[VEC / 2];
+  __device__ __forceinline__ P pair(int i) const { return *reinterpret_cast<const P*>(&w[i]); }
+  __device__ __forceinline__ void set(int i, P v) { w[i] = *reinterpret_cast<uint32_t*>(&v); }
+};
+
+template <typename T> __device__ __forceinline__ Vec8<T> ldg16(const T* p) {
+  Vec8<T> v;
   asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
-               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+               : "=r"(v.w[0]), "=r"(v.w[1]), "=r"(v.w[2]), "=r"(v.w[3]) : "l"(p));
   return v;
 }
-__device__ __forceinline__ void stg16(void* p, uint4 v) {
-  asm volatile("st.global.v4.u32 [%0], {%1,%2,%3,%4};" ::"l"(p), "r"(v.x), "r"(v.y),
-               "r"(v.z), "r"(v.w) : "memory");
+template <typename T> __device__ __forceinline__ void stg16(T* p, const Vec8<T>& v) {
+  asm volatile("st.global.v4.u32 [%0], {%1,%2,%3,%4};" ::"l"(p), "r"(v.w[0]), "r"(v.w[1]),
+               "r"(v.w[2]), "r"(v.w[3]) : "memory");
+}
+// The next kernel of the stream may be started; it waits for this one's
+// results with wait_for_previous().
+__device__ __forceinline__ void start_next() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ void wait_for_previous() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+// The signs of 8 outputs in one byte: the even channels in the low nibble, the
+// odd ones in the high nibble. `positive` holds an all-ones half word for each
+// channel whose output is above zero.
+__device__ __forceinline__ uint32_t pack_signs(const uint32_t (&positive)[VEC / 2]) {
+  const uint32_t t = (positive[0] & 0x00010001u) | (positive[1] & 0x00020002u) |
+                     (positive[2] & 0x00040004u) | (positive[3] & 0x00080008u);
+  return (t | (t >> 12)) & 0xffu;
+}
+// Bit i of either half word: the sign of channel 2i or 2i + 1.
+__device__ __forceinline__ uint32_t spread_signs(uint32_t byte) {
+  return (byte & 0xfu) | ((byte & 0xf0u) << 12);
 }
 
 // Thread geometry shared by all four kernels.
@@ -82,283 +119,359 @@ struct Tile {
   }
 };
 
-// Rows [r0, r1) of this CTA.
-__device__ __forceinline__ void cta_rows(int64_t M, int64_t* r0, int64_t* r1) {
+// Rows [r0, r1) of CTA `by`.
+__device__ __forceinline__ void cta_rows(int64_t M, int by, int64_t* r0, int64_t* r1) {
   const int64_t per = (M + gridDim.y - 1) / gridDim.y;
-  *r0 = blockIdx.y * per;
+  *r0 = min(by * per, M);
   *r1 = min(*r0 + per, M);
 }
 
-// Sums `acc` (NV values per thread) over the threads of the CTA that own the
-// same channel group and adds the totals to the fp64 accumulators.
-template <int NV>
-__device__ __forceinline__ void reduce_to_global(const Tile& t, float (&acc)[NV][VEC],
-                                                 double* const (&dst)[NV], int C) {
-  __shared__ float red[BN_THREADS][NV * VEC + 1];
+// Calls rows(U or 1, at): at is the element of the thread's first row, the
+// others lie t.ty rows further on (for_rows) or back (for_rows_back) each.
+template <int U, typename F>
+__device__ __forceinline__ void for_rows(const Tile& t, int64_t r0, int64_t r1, int C, F rows) {
+  const int64_t stride = static_cast<int64_t>(t.ty) * C;
+  int64_t at = (r0 + t.row) * C + t.group * VEC;
+  int64_t left = r1 - r0 - t.row;
+  for (; left > (U - 1) * t.ty; left -= U * t.ty, at += U * stride)
+    rows(std::integral_constant<int, U>(), at);
+  for (; left > 0; left -= t.ty, at += stride) rows(std::integral_constant<int, 1>(), at);
+}
+template <int U, typename F>
+__device__ __forceinline__ void for_rows_back(const Tile& t, int64_t r0, int64_t r1, int C,
+                                              F rows) {
+  const int64_t stride = static_cast<int64_t>(t.ty) * C;
+  int64_t at = (r1 - 1 - t.row) * C + t.group * VEC;
+  int64_t left = r1 - r0 - t.row;
+  for (; left > (U - 1) * t.ty; left -= U * t.ty, at -= U * stride)
+    rows(std::integral_constant<int, U>(), at);
+  for (; left > 0; left -= t.ty, at -= stride) rows(std::integral_constant<int, 1>(), at);
+}
+
+// Sums `acc` (two values per channel of the thread) over the threads of the
+// CTA that own the same channel group and adds the totals to the fp64
+// accumulators: pairwise by shuffles inside a warp, in fp64 across warps.
+__device__ __forceinline__ void reduce_to_global(const Tile& t, float (&acc)[2][VEC], double* dst0,
+                                                 double* dst1) {
+  constexpr int WARPS = BN_THREADS / 32;
+  // Rows of 36 words: the threads of a warp, which read 8 rows of 4 words
+  // below, hit 32 different banks.
+  __shared__ float red[WARPS][2 * VEC][36];
+  for (int lanes = 16; lanes >= t.txg; lanes >>= 1) {
 #pragma unroll
-  for (int k = 0; k < NV; ++k)
+    for (int k = 0; k < 2; ++k)
 #pragma unroll
-    for (int i = 0; i < VEC; ++i) red[threadIdx.x][k * VEC + i] = acc[k][i];
+      for (int i = 0; i < VEC; ++i) acc[k][i] += __shfl_xor_sync(0xffffffffu, acc[k][i], lanes);
+  }
+  const int warp = threadIdx.x / 32;
+  if (static_cast<int>(threadIdx.x % 32) < t.txg) {
+#pragma unroll
+    for (int k = 0; k < 2; ++k)
+#pragma unroll
+      for (int i = 0; i < VEC; ++i) red[warp][k * VEC + i][t.tx] = acc[k][i];
+  }
   __syncthreads();
-  // One thread per (channel group, value): NV * VEC * txg <= 2 * 8 * 32 = 512
-  // sums, two rounds of 256 threads at most.
-  for (int idx = threadIdx.x; idx < t.txg * NV * VEC; idx += BN_THREADS) {
-    const int tx = idx / (NV * VEC), slot = idx % (NV * VEC);
-    float sum = 0.f;
-    for (int r = 0; r < t.ty; ++r) sum += red[r * t.txg + tx][slot];
-    const int64_t ch = (static_cast<int64_t>(blockIdx.x) * t.txg + tx) * VEC + slot % VEC;
-    if (ch < C) atomicAdd(dst[slot / VEC] + ch, static_cast<double>(sum));
+  // 2 * VEC * txg <= 512 totals, two rounds of 256 threads at most.
+  for (int idx = threadIdx.x; idx < t.txg * 2 * VEC; idx += BN_THREADS) {
+    const int i = idx % VEC, tx = idx / VEC % t.txg, k = idx / VEC / t.txg;
+    double sum = 0.0;
+#pragma unroll
+    for (int w = 0; w < WARPS; ++w) sum += static_cast<double>(red[w][k * VEC + i][tx]);
+    atomicAdd((k == 0 ? dst0 : dst1) + (static_cast<int64_t>(blockIdx.x) * t.txg + tx) * VEC + i,
+              sum);
   }
 }
 
 template <typename T>
-__global__ void __launch_bounds__(BN_THREADS, BN_MIN_BLOCKS_REDUCE)
+__global__ void __launch_bounds__(BN_THREADS, BN_MIN_BLOCKS_STATS)
 bn_stats_kernel(const T* __restrict__ x, int64_t M, int C, double* __restrict__ sum,
                 double* __restrict__ sumsq) {
   const Tile t(C);
   int64_t r0, r1;
-  cta_rows(M, &r0, &r1);
+  cta_rows(M, blockIdx.y, &r0, &r1);
   float acc[2][VEC];
 #pragma unroll
   for (int i = 0; i < VEC; ++i) acc[0][i] = acc[1][i] = 0.f;
-  const T* base = x + t.group * VEC;
-  int64_t r = r0 + t.row;
-  for (; r + 3 * t.ty < r1; r += 4 * t.ty) {
-    Vec8<T> v[4];
+  const int64_t stride = static_cast<int64_t>(t.ty) * C;
+  for_rows<UNROLL>(t, r0, r1, C, [&](auto count, int64_t at) {
+    constexpr int U = decltype(count)::value;
+    Vec8<T> v[U];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) v[u].raw = ldg16(base + (r + u * t.ty) * C);
+    for (int u = 0; u < U; ++u) v[u] = ldg16(x + at + u * stride);
+    // The rows of one round are summed among themselves first: a quarter of
+    // the additions into the long-running sums.
 #pragma unroll
-    for (int u = 0; u < 4; ++u)
+    for (int i = 0; i < VEC / 2; ++i) {
+      float2 s = make_float2(0.f, 0.f), q = make_float2(0.f, 0.f);
 #pragma unroll
-      for (int i = 0; i < VEC; ++i) {
-        const float f = bn_to_float(v[u].e[i]);
-        acc[0][i] += f;
-        acc[1][i] += f * f;
+      for (int u = 0; u < U; ++u) {
+        const float2 f = Pair<T>::widen(v[u].pair(i));
+        s.x += f.x;
+        s.y += f.y;
+        q.x = fmaf(f.x, f.x, q.x);
+        q.y = fmaf(f.y, f.y, q.y);
       }
-  }
-  for (; r < r1; r += t.ty) {
-    Vec8<T> v;
-    v.raw = ldg16(base + r * C);
-#pragma unroll
-    for (int i = 0; i < VEC; ++i) {
-      const float f = bn_to_float(v.e[i]);
-      acc[0][i] += f;
-      acc[1][i] += f * f;
+      acc[0][2 * i] += s.x;
+      acc[0][2 * i + 1] += s.y;
+      acc[1][2 * i] += q.x;
+      acc[1][2 * i + 1] += q.y;
     }
-  }
-  double* const dst[2] = {sum, sumsq};
-  reduce_to_global<2>(t, acc, dst, C);
+  });
+  start_next();
+  reduce_to_global(t, acc, sum, sumsq);
 }
 
-// scale/shift of this thread's 8 channels from the fp64 sums.
-__device__ __forceinline__ void channel_affine(const double* sum, const double* sumsq,
-                                               const float* weight, const float* bias,
-                                               int64_t ch0, int64_t M, float eps,
-                                               float (&mean)[VEC], float (&invstd)[VEC],
-                                               float (&scale)[VEC], float (&shift)[VEC]) {
-#pragma unroll
-  for (int i = 0; i < VEC; ++i) {
-    const double m = sum[ch0 + i] / static_cast<double>(M);
-    double var = sumsq[ch0 + i] / static_cast<double>(M) - m * m;
-    if (var < 0.0) var = 0.0;
-    const double is = rsqrt(var + static_cast<double>(eps));
-    mean[i] = static_cast<float>(m);
-    invstd[i] = static_cast<float>(is);
-    const float w = weight ? weight[ch0 + i] : 1.f;
-    const float b = bias ? bias[ch0 + i] : 0.f;
-    scale[i] = w * invstd[i];
-    shift[i] = b - mean[i] * scale[i];
-  }
-}
+// Most channels of a CTA. Their per-channel values are formed by one thread
+// each: in every thread, the fp64 arithmetic would take longer than the rows of
+// a small tensor.
+constexpr int BN_CTA_CHANNELS = 32 * VEC;
 
+// relu(x * scale + shift [+ residual]) of 8 channels.
 template <typename T, bool RELU, bool RES>
-__global__ void __launch_bounds__(BN_THREADS, BN_MIN_BLOCKS_APPLY)
-bn_apply_kernel(const T* __restrict__ x, const T* __restrict__ res, T* __restrict__ y,
-                int64_t M, int C, const double* __restrict__ sum,
-                const double* __restrict__ sumsq, const float* __restrict__ weight,
-                const float* __restrict__ bias, float eps, float momentum,
-                float* __restrict__ save_mean, float* __restrict__ save_invstd,
-                float* __restrict__ running_mean, float* __restrict__ running_var) {
-  const Tile t(C);
-  int64_t r0, r1;
-  cta_rows(M, &r0, &r1);
-  const int64_t ch0 = t.group * VEC;
-  float mean[VEC], invstd[VEC], scale[VEC], shift[VEC];
-  channel_affine(sum, sumsq, weight, bias, ch0, M, eps, mean, invstd, scale, shift);
-  if (blockIdx.y == 0 && t.row == 0) {
+__device__ __forceinline__ Vec8<T> normalise(const Vec8<T>& x, const Vec8<T>& res,
+                                             const float (&scale)[VEC], const float (&shift)[VEC]) {
+  Vec8<T> o;
 #pragma unroll
-    for (int i = 0; i < VEC; ++i) {
-      save_mean[ch0 + i] = mean[i];
-      save_invstd[ch0 + i] = invstd[i];
+  for (int i = 0; i < VEC / 2; ++i) {
+    const float2 a = Pair<T>::widen(x.pair(i));
+    float2 f = make_float2(fmaf(a.x, scale[2 * i], shift[2 * i]),
+                           fmaf(a.y, scale[2 * i + 1], shift[2 * i + 1]));
+    if (RES) {
+      const float2 b = Pair<T>::widen(res.pair(i));
+      f.x += b.x;
+      f.y += b.y;
+    }
+    typename Pair<T>::type v = Pair<T>::narrow(f.x, f.y);
+    if (RELU) v = __hmax2(v, Pair<T>::narrow(0.f, 0.f));
+    o.set(i, v);
+  }
+  return o;
+}
+
+__device__ __forceinline__ void load8(const float* p, float (&v)[VEC]) {
+  const float4 a = *reinterpret_cast<const float4*>(p);
+  const float4 b = *reinterpret_cast<const float4*>(p + 4);
+  v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w;
+  v[4] = b.x, v[5] = b.y, v[6] = b.z, v[7] = b.w;
+}
+
+// saved: rows mean, invstd and shift of [3, C].
+template <typename T, bool RELU, bool RES>
+__global__ void __launch_bounds__(BN_THREADS, BN_MIN_BLOCKS)
+bn_apply_kernel(const T* __restrict__ x, const T* __restrict__ res, T* __restrict__ y,
+                uint8_t* __restrict__ signs, int64_t M, int C, double inv_m,
+                const double* __restrict__ sum, const double* __restrict__ sumsq,
+                const float* __restrict__ weight, const float* __restrict__ bias, float eps,
+                float momentum, float* __restrict__ saved, float* __restrict__ running_mean,
+                float* __restrict__ running_var) {
+  const Tile t(C);
+  const int by = gridDim.y - 1 - blockIdx.y;
+  int64_t r0, r1;
+  cta_rows(M, by, &r0, &r1);
+  __shared__ __align__(16) float s_scale[BN_CTA_CHANNELS];
+  __shared__ __align__(16) float s_shift[BN_CTA_CHANNELS];
+  wait_for_previous();
+  if (static_cast<int>(threadIdx.x) < t.txg * VEC) {
+    const int64_t ch = static_cast<int64_t>(blockIdx.x) * t.txg * VEC + threadIdx.x;
+    const double m = __ldcg(sum + ch) * inv_m;
+    double var = __ldcg(sumsq + ch) * inv_m - m * m;
+    if (var < 0.0) var = 0.0;
+    const float mean = static_cast<float>(m);
+    const float invstd = static_cast<float>(rsqrt(var + static_cast<double>(eps)));
+    const float scale = (weight ? weight[ch] : 1.f) * invstd;
+    const float shift = (bias ? bias[ch] : 0.f) - mean * scale;
+    s_scale[threadIdx.x] = scale;
+    s_shift[threadIdx.x] = shift;
+    if (by == 0) {
+      saved[ch] = mean;
+      saved[C + ch] = invstd;
+      saved[2 * static_cast<int64_t>(C) + ch] = shift;
       if (running_mean != nullptr) {
-        const double m = sum[ch0 + i] / static_cast<double>(M);
-        double var = sumsq[ch0 + i] / static_cast<double>(M) - m * m;
-        if (var < 0.0) var = 0.0;
-        const double unbiased = M > 1 ? var * static_cast<double>(M) / static_cast<double>(M - 1) : var;
-        running_mean[ch0 + i] = (1.f - momentum) * running_mean[ch0 + i] + momentum * mean[i];
-        running_var[ch0 + i] =
-            (1.f - momentum) * running_var[ch0 + i] + momentum * static_cast<float>(unbiased);
+        const double unbiased =
+            M > 1 ? var * static_cast<double>(M) / static_cast<double>(M - 1) : var;
+        running_mean[ch] = (1.f - momentum) * running_mean[ch] + momentum * mean;
+        running_var[ch] =
+            (1.f - momentum) * running_var[ch] + momentum * static_cast<float>(unbiased);
       }
     }
   }
-  const int64_t off = t.group * VEC;
-  auto one = [&](uint4 xv, uint4 rv) {
-    Vec8<T> a, b, o;
-    a.raw = xv;
-    b.raw = rv;
+  __syncthreads();
+  float scale[VEC], shift[VEC];
+  load8(s_scale + t.tx * VEC, scale);
+  load8(s_shift + t.tx * VEC, shift);
+  const int64_t stride = static_cast<int64_t>(t.ty) * C;
+  for_rows_back<UNROLL>(t, r0, r1, C, [&](auto count, int64_t at0) {
+    constexpr int U = decltype(count)::value;
+    Vec8<T> a[U], b[U];
 #pragma unroll
-    for (int i = 0; i < VEC; ++i) {
-      float f = bn_to_float(a.e[i]) * scale[i] + shift[i];
-      if (RES) f += bn_to_float(b.e[i]);
-      if (RELU) f = fmaxf(f, 0.f);
-      o.e[i] = bn_from_float<T>(f);
-    }
-    return o.raw;
-  };
-  int64_t r = r0 + t.row;
-  for (; r + 3 * t.ty < r1; r += 4 * t.ty) {
-    uint4 xv[4], rv[4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      xv[u] = ldg16(x + (r + u * t.ty) * C + off);
-      rv[u] = RES ? ldg16(res + (r + u * t.ty) * C + off) : make_uint4(0, 0, 0, 0);
+    for (int u = 0; u < U; ++u) {
+      a[u] = ldg16(x + at0 - u * stride);
+      if (RES) b[u] = ldg16(res + at0 - u * stride);
     }
 #pragma unroll
-    for (int u = 0; u < 4; ++u) stg16(y + (r + u * t.ty) * C + off, one(xv[u], rv[u]));
-  }
-  for (; r < r1; r += t.ty) {
-    const uint4 xv = ldg16(x + r * C + off);
-    const uint4 rv = RES ? ldg16(res + r * C + off) : make_uint4(0, 0, 0, 0);
-    stg16(y + r * C + off, one(xv, rv));
-  }
+    for (int u = 0; u < U; ++u) {
+      const int64_t at = at0 - u * stride;
+      const Vec8<T> o = normalise<T, RELU, RES>(a[u], b[u], scale, shift);
+      stg16(y + at, o);
+      if (RELU && RES) {
+        uint32_t positive[VEC / 2];
+#pragma unroll
+        for (int i = 0; i < VEC / 2; ++i)
+          positive[i] = __hgt2_mask(o.pair(i), Pair<T>::narrow(0.f, 0.f));
+        signs[at / VEC] = static_cast<uint8_t>(pack_signs(positive));
+      }
+    }
+  });
+}
+
+// Where the backward gets relu's mask from.
+enum Mask : int {
+  MASK_NONE = 0,   // no relu
+  MASK_X = 1,      // x, scale and shift: relu without a residual
+  MASK_SIGNS = 2,  // the forward's bits: relu of a sum with a residual
+};
+
+// dz of channels 2i and 2i + 1: dy where the output was above zero. x: the
+// two inputs; signs: spread_signs() of the forward's byte. MASK_X repeats the
+// forward's arithmetic, rounding included.
+template <typename T, int MASK>
+__device__ __forceinline__ uint32_t masked(int i, uint32_t dy, float2 x, uint32_t signs,
+                                           const float (&scale)[VEC], const float (&shift)[VEC]) {
+  if (MASK == MASK_X)
+    return dy & __hgt2_mask(Pair<T>::narrow(fmaf(x.x, scale[2 * i], shift[2 * i]),
+                                            fmaf(x.y, scale[2 * i + 1], shift[2 * i + 1])),
+                            Pair<T>::narrow(0.f, 0.f));
+  if (MASK == MASK_SIGNS) return dy & (((signs >> i) & 0x00010001u) * 0xffffu);
+  return dy;
 }
 
 // sum(dz) and sum(dz * xhat) per channel.
-template <typename T, bool RELU>
-__global__ void __launch_bounds__(BN_THREADS, BN_MIN_BLOCKS_REDUCE)
-bn_backward_reduce_kernel(const T* __restrict__ dy, const T* __restrict__ y,
+template <typename T, int MASK>
+__global__ void __launch_bounds__(BN_THREADS, BN_MIN_BLOCKS)
+bn_backward_reduce_kernel(const T* __restrict__ dy, const uint8_t* __restrict__ signs,
                           const T* __restrict__ x, int64_t M, int C,
-                          const float* __restrict__ save_mean,
-                          const float* __restrict__ save_invstd, double* __restrict__ sum_dz,
-                          double* __restrict__ sum_dz_xhat) {
+                          const float* __restrict__ weight, const float* __restrict__ saved,
+                          double* __restrict__ sum_dz, double* __restrict__ sum_dz_xhat) {
   const Tile t(C);
   int64_t r0, r1;
-  cta_rows(M, &r0, &r1);
+  cta_rows(M, blockIdx.y, &r0, &r1);
   const int64_t off = t.group * VEC;
-  float mean[VEC], invstd[VEC];
+  float mean[VEC], scale[VEC], shift[VEC];
+  load8(saved + off, mean);
+  if (MASK == MASK_X) {
+    load8(saved + C + off, scale);
+    load8(saved + 2 * static_cast<int64_t>(C) + off, shift);
 #pragma unroll
-  for (int i = 0; i < VEC; ++i) {
-    mean[i] = save_mean[off + i];
-    invstd[i] = save_invstd[off + i];
+    for (int i = 0; i < VEC; ++i) scale[i] *= weight ? weight[off + i] : 1.f;
   }
   float acc[2][VEC];
 #pragma unroll
   for (int i = 0; i < VEC; ++i) acc[0][i] = acc[1][i] = 0.f;
-  auto one = [&](uint4 dv, uint4 yv, uint4 xv) {
-    Vec8<T> d, o, a;
-    d.raw = dv;
-    o.raw = yv;
-    a.raw = xv;
+  const int64_t stride = static_cast<int64_t>(t.ty) * C;
+  // MASK_X keeps 16 more values per thread: four rows would spill.
+  for_rows<MASK == MASK_X ? 3 : UNROLL>(t, r0, r1, C, [&](auto count, int64_t at0) {
+    constexpr int U = decltype(count)::value;
+    Vec8<T> d[U], a[U];
+    uint32_t m[U];
 #pragma unroll
-    for (int i = 0; i < VEC; ++i) {
-      float dz = bn_to_float(d.e[i]);
-      if (RELU && !(bn_to_float(o.e[i]) > 0.f)) dz = 0.f;
-      acc[0][i] += dz;
-      acc[1][i] += dz * (bn_to_float(a.e[i]) - mean[i]) * invstd[i];
-    }
-  };
-  int64_t r = r0 + t.row;
-  for (; r + 1 * t.ty < r1; r += 2 * t.ty) {
-    uint4 dv[2], yv[2], xv[2];
-#pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      const int64_t at = (r + u * t.ty) * C + off;
-      dv[u] = ldg16(dy + at);
-      yv[u] = RELU ? ldg16(y + at) : make_uint4(0, 0, 0, 0);
-      xv[u] = ldg16(x + at);
+    for (int u = 0; u < U; ++u) {
+      const int64_t at = at0 + u * stride;
+      d[u] = ldg16(dy + at);
+      a[u] = ldg16(x + at);
+      m[u] = MASK == MASK_SIGNS ? spread_signs(__ldg(signs + at / VEC)) : 0u;
     }
 #pragma unroll
-    for (int u = 0; u < 2; ++u) one(dv[u], yv[u], xv[u]);
-  }
-  for (; r < r1; r += t.ty) {
-    const int64_t at = r * C + off;
-    one(ldg16(dy + at), RELU ? ldg16(y + at) : make_uint4(0, 0, 0, 0), ldg16(x + at));
-  }
-  double* const dst[2] = {sum_dz, sum_dz_xhat};
-  reduce_to_global<2>(t, acc, dst, C);
+    for (int i = 0; i < VEC / 2; ++i) {
+      float2 s = make_float2(0.f, 0.f), p = make_float2(0.f, 0.f);
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const float2 f = Pair<T>::widen(a[u].pair(i));
+        d[u].w[i] = masked<T, MASK>(i, d[u].w[i], f, m[u], scale, shift);
+        const float2 dz = Pair<T>::widen(d[u].pair(i));
+        s.x += dz.x;
+        s.y += dz.y;
+        p.x = fmaf(dz.x, f.x - mean[2 * i], p.x);
+        p.y = fmaf(dz.y, f.y - mean[2 * i + 1], p.y);
+      }
+      acc[0][2 * i] += s.x;
+      acc[0][2 * i + 1] += s.y;
+      acc[1][2 * i] += p.x;
+      acc[1][2 * i + 1] += p.y;
+    }
+  });
+  start_next();
+  float invstd[VEC];
+  load8(saved + C + off, invstd);
+#pragma unroll
+  for (int i = 0; i < VEC; ++i) acc[1][i] *= invstd[i];
+  reduce_to_global(t, acc, sum_dz, sum_dz_xhat);
 }
 
-template <typename T, bool RELU, bool RES>
-__global__ void __launch_bounds__(BN_THREADS, BN_MIN_BLOCKS_APPLY)
-bn_backward_apply_kernel(const T* __restrict__ dy, const T* __restrict__ y,
+template <typename T, int MASK, bool DRES>
+__global__ void __launch_bounds__(BN_THREADS, BN_MIN_BLOCKS)
+bn_backward_apply_kernel(const T* __restrict__ dy, const uint8_t* __restrict__ signs,
                          const T* __restrict__ x, T* __restrict__ dx, T* __restrict__ dres,
-                         int64_t M, int C, const float* __restrict__ weight,
-                         const float* __restrict__ save_mean,
-                         const float* __restrict__ save_invstd,
-                         const double* __restrict__ sum_dz,
+                         int64_t M, int C, double inv_m, const float* __restrict__ weight,
+                         const float* __restrict__ saved, const double* __restrict__ sum_dz,
                          const double* __restrict__ sum_dz_xhat, float* __restrict__ dweight,
                          float* __restrict__ dbias) {
   const Tile t(C);
+  const int by = gridDim.y - 1 - blockIdx.y;
   int64_t r0, r1;
-  cta_rows(M, &r0, &r1);
-  const int64_t off = t.group * VEC;
-  float mean[VEC], invstd[VEC], scale[VEC], k1[VEC], k2[VEC];
-#pragma unroll
-  for (int i = 0; i < VEC; ++i) {
-    mean[i] = save_mean[off + i];
-    invstd[i] = save_invstd[off + i];
-    scale[i] = (weight ? weight[off + i] : 1.f) * invstd[i];
-    k1[i] = static_cast<float>(sum_dz[off + i] / static_cast<double>(M));
-    k2[i] = static_cast<float>(sum_dz_xhat[off + i] / static_cast<double>(M));
-  }
-  if (blockIdx.y == 0 && t.row == 0) {
-#pragma unroll
-    for (int i = 0; i < VEC; ++i) {
-      if (dweight) dweight[off + i] = static_cast<float>(sum_dz_xhat[off + i]);
-      if (dbias) dbias[off + i] = static_cast<float>(sum_dz[off + i]);
+  cta_rows(M, by, &r0, &r1);
+  __shared__ __align__(16) float s_mean[BN_CTA_CHANNELS], s_scale[BN_CTA_CHANNELS],
+      s_shift[BN_CTA_CHANNELS], s_k1[BN_CTA_CHANNELS], s_k2[BN_CTA_CHANNELS];
+  wait_for_previous();
+  if (static_cast<int>(threadIdx.x) < t.txg * VEC) {
+    const int64_t ch = static_cast<int64_t>(blockIdx.x) * t.txg * VEC + threadIdx.x;
+    const double dz = __ldcg(sum_dz + ch), dz_xhat = __ldcg(sum_dz_xhat + ch);
+    const float invstd = saved[C + ch];
+    s_mean[threadIdx.x] = saved[ch];
+    s_shift[threadIdx.x] = saved[2 * static_cast<int64_t>(C) + ch];
+    s_scale[threadIdx.x] = (weight ? weight[ch] : 1.f) * invstd;
+    s_k1[threadIdx.x] = static_cast<float>(dz * inv_m);
+    s_k2[threadIdx.x] = static_cast<float>(dz_xhat * inv_m) * invstd;
+    if (by == 0) {
+      if (dweight) dweight[ch] = static_cast<float>(dz_xhat);
+      if (dbias) dbias[ch] = static_cast<float>(dz);
     }
   }
-  auto one = [&](uint4 dv, uint4 yv, uint4 xv, uint4* dres_out) {
-    Vec8<T> d, o, a, gx, gr;
-    d.raw = dv;
-    o.raw = yv;
-    a.raw = xv;
+  __syncthreads();
+  float mean[VEC], scale[VEC], shift[VEC], k1[VEC], k2[VEC];
+  load8(s_mean + t.tx * VEC, mean);
+  load8(s_scale + t.tx * VEC, scale);
+  load8(s_k1 + t.tx * VEC, k1);
+  load8(s_k2 + t.tx * VEC, k2);
+  if (MASK == MASK_X) load8(s_shift + t.tx * VEC, shift);
+  const int64_t stride = static_cast<int64_t>(t.ty) * C;
+  for_rows_back<2>(t, r0, r1, C, [&](auto count, int64_t at0) {
+    constexpr int U = decltype(count)::value;
+    Vec8<T> d[U], a[U];
+    uint32_t m[U];
 #pragma unroll
-    for (int i = 0; i < VEC; ++i) {
-      float dz = bn_to_float(d.e[i]);
-      if (RELU && !(bn_to_float(o.e[i]) > 0.f)) dz = 0.f;
-      const float xhat = (bn_to_float(a.e[i]) - mean[i]) * invstd[i];
-      gx.e[i] = bn_from_float<T>(scale[i] * (dz - k1[i] - xhat * k2[i]));
-      gr.e[i] = bn_from_float<T>(dz);
-    }
-    *dres_out = gr.raw;
-    return gx.raw;
-  };
-  int64_t r = r0 + t.row;
-  for (; r + 1 * t.ty < r1; r += 2 * t.ty) {
-    uint4 dv[2], yv[2], xv[2];
-#pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      const int64_t at = (r + u * t.ty) * C + off;
-      dv[u] = ldg16(dy + at);
-      yv[u] = RELU ? ldg16(y + at) : make_uint4(0, 0, 0, 0);
-      xv[u] = ldg16(x + at);
+    for (int u = 0; u < U; ++u) {
+      const int64_t at = at0 - u * stride;
+      d[u] = ldg16(dy + at);
+      a[u] = ldg16(x + at);
+      m[u] = MASK == MASK_SIGNS ? spread_signs(__ldg(signs + at / VEC)) : 0u;
     }
 #pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      const int64_t at = (r + u * t.ty) * C + off;
-      uint4 gr;
-      stg16(dx + at, one(dv[u], yv[u], xv[u], &gr));
-      if (RES) stg16(dres + at, gr);
+    for (int u = 0; u < U; ++u) {
+      const int64_t at = at0 - u * stride;
+      Vec8<T> g;
+#pragma unroll
+      for (int i = 0; i < VEC / 2; ++i) {
+        const float2 f = Pair<T>::widen(a[u].pair(i));
+        d[u].w[i] = masked<T, MASK>(i, d[u].w[i], f, m[u], scale, shift);
+        const float2 z = Pair<T>::widen(d[u].pair(i));
+        const int j = 2 * i, k = 2 * i + 1;
+        g.set(i, Pair<T>::narrow(scale[j] * (z.x - k1[j] - (f.x - mean[j]) * k2[j]),
+                                 scale[k] * (z.y - k1[k] - (f.y - mean[k]) * k2[k])));
+      }
+      stg16(dx + at, g);
+      if (DRES) stg16(dres + at, d[u]);
     }
-  }
-  for (; r < r1; r += t.ty) {
-    const int64_t at = r * C + off;
-    uint4 gr;
-    stg16(dx + at,
-          one(ldg16(dy + at), RELU ? ldg16(y + at) : make_uint4(0, 0, 0, 0), ldg16(x + at), &gr));
-    if (RES) stg16(dres + at, gr);
-  }
+  });
 }
 
 dim3 bn_grid(int64_t M, int C) {
@@ -388,88 +501,102 @@ bool bn_shape_ok(int64_t M, int C) {
 
 bool BatchNormSupported(int64_t rows, int channels) { return bn_shape_ok(rows, channels); }
 
+// Launches the second kernel of a pair so that it may start while the first
+// one is still running (it waits for the results itself).
+template <typename... P, typename... A>
+static cudaError_t LaunchDependent(void (*kernel)(P...), dim3 grid, cudaStream_t stream, A... args) {
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t config = {};
+  config.gridDim = grid;
+  config.blockDim = dim3(BN_THREADS);
+  config.stream = stream;
+  config.attrs = &attr;
+  config.numAttrs = 1;
+  return cudaLaunchKernelEx(&config, kernel, static_cast<P>(args)...);
+}
+
 template <typename T>
-static cudaError_t ForwardTyped(const void* x, const void* res, void* y, int64_t M, int C,
-                                double* sums, const float* weight, const float* bias,
-                                float eps, float momentum, float* save_mean,
-                                float* save_invstd, float* running_mean, float* running_var,
-                                bool relu, cudaStream_t stream) {
+static cudaError_t ForwardTyped(const void* x, const void* res, void* y, uint8_t* signs, int64_t M,
+                                int C, double* sums, const float* weight, const float* bias,
+                                float eps, float momentum, float* saved, float* running_mean,
+                                float* running_var, bool relu, cudaStream_t stream) {
   const dim3 grid = bn_grid(M, C);
   double* sum = sums;
   double* sumsq = sums + C;
   bn_stats_kernel<T><<<grid, BN_THREADS, 0, stream>>>(static_cast<const T*>(x), M, C, sum, sumsq);
-#define HVD_BN_APPLY(RELU, RES)                                                          \
-  bn_apply_kernel<T, RELU, RES><<<grid, BN_THREADS, 0, stream>>>(                         \
-      static_cast<const T*>(x), static_cast<const T*>(res), static_cast<T*>(y), M, C, sum, \
-      sumsq, weight, bias, eps, momentum, save_mean, save_invstd, running_mean, running_var)
-  if (relu && res) HVD_BN_APPLY(true, true);
-  else if (relu) HVD_BN_APPLY(true, false);
-  else if (res) HVD_BN_APPLY(false, true);
-  else HVD_BN_APPLY(false, false);
-#undef HVD_BN_APPLY
-  return cudaGetLastError();
+  cudaError_t err = cudaGetLastError();
+  if (err != cudaSuccess) return err;
+  auto kernel = relu && res ? bn_apply_kernel<T, true, true>
+                : relu      ? bn_apply_kernel<T, true, false>
+                : res       ? bn_apply_kernel<T, false, true>
+                            : bn_apply_kernel<T, false, false>;
+  return LaunchDependent(kernel, grid, stream, static_cast<const T*>(x),
+                         static_cast<const T*>(res), static_cast<T*>(y), signs, M, C,
+                         1.0 / static_cast<double>(M), sum, sumsq, weight, bias, eps, momentum,
+                         saved, running_mean, running_var);
 }
 
 template <typename T>
-static cudaError_t BackwardTyped(const void* dy, const void* y, const void* x, void* dx,
-                                 void* dres, int64_t M, int C, double* sums,
-                                 const float* weight, const float* save_mean,
-                                 const float* save_invstd, float* dweight, float* dbias,
-                                 bool relu, cudaStream_t stream) {
+static cudaError_t BackwardTyped(const void* dy, const uint8_t* signs, const void* x, void* dx,
+                                 void* dres, int64_t M, int C, double* sums, const float* weight,
+                                 const float* saved, float* dweight, float* dbias, bool relu,
+                                 cudaStream_t stream) {
   const dim3 grid = bn_grid(M, C);
   double* sum_dz = sums;
   double* sum_dz_xhat = sums + C;
   const T* dyt = static_cast<const T*>(dy);
-  const T* yt = static_cast<const T*>(y);
   const T* xt = static_cast<const T*>(x);
-  if (relu)
-    bn_backward_reduce_kernel<T, true><<<grid, BN_THREADS, 0, stream>>>(
-        dyt, yt, xt, M, C, save_mean, save_invstd, sum_dz, sum_dz_xhat);
-  else
-    bn_backward_reduce_kernel<T, false><<<grid, BN_THREADS, 0, stream>>>(
-        dyt, yt, xt, M, C, save_mean, save_invstd, sum_dz, sum_dz_xhat);
-#define HVD_BN_BWD(RELU, RES)                                                             \
-  bn_backward_apply_kernel<T, RELU, RES><<<grid, BN_THREADS, 0, stream>>>(                 \
-      dyt, yt, xt, static_cast<T*>(dx), static_cast<T*>(dres), M, C, weight, save_mean,    \
-      save_invstd, sum_dz, sum_dz_xhat, dweight, dbias)
-  if (relu && dres) HVD_BN_BWD(true, true);
-  else if (relu) HVD_BN_BWD(true, false);
-  else if (dres) HVD_BN_BWD(false, true);
-  else HVD_BN_BWD(false, false);
-#undef HVD_BN_BWD
-  return cudaGetLastError();
+  const int mask = !relu ? MASK_NONE : signs == nullptr ? MASK_X : MASK_SIGNS;
+  // A gradient of the residual never comes with MASK_X: that is a layer
+  // without one.
+  if (mask == MASK_X && dres != nullptr) return cudaErrorInvalidValue;
+  auto reduce = mask == MASK_NONE ? bn_backward_reduce_kernel<T, MASK_NONE>
+                : mask == MASK_X  ? bn_backward_reduce_kernel<T, MASK_X>
+                                  : bn_backward_reduce_kernel<T, MASK_SIGNS>;
+  reduce<<<grid, BN_THREADS, 0, stream>>>(dyt, signs, xt, M, C, weight, saved, sum_dz,
+                                          sum_dz_xhat);
+  cudaError_t err = cudaGetLastError();
+  if (err != cudaSuccess) return err;
+  auto apply = mask == MASK_NONE ? (dres ? bn_backward_apply_kernel<T, MASK_NONE, true>
+                                         : bn_backward_apply_kernel<T, MASK_NONE, false>)
+               : mask == MASK_X  ? bn_backward_apply_kernel<T, MASK_X, false>
+                                 : (dres ? bn_backward_apply_kernel<T, MASK_SIGNS, true>
+                                         : bn_backward_apply_kernel<T, MASK_SIGNS, false>);
+  return LaunchDependent(apply, grid, stream, dyt, signs, xt, static_cast<T*>(dx),
+                         static_cast<T*>(dres), M, C, 1.0 / static_cast<double>(M), weight, saved,
+                         sum_dz, sum_dz_xhat, dweight, dbias);
 }
 
-cudaError_t LaunchBatchNormForward(const void* x, const void* residual, void* y, int64_t rows,
-                                   int channels, bool bf16, double* sums_zeroed,
+cudaError_t LaunchBatchNormForward(const void* x, const void* residual, void* y, uint8_t* signs,
+                                   int64_t rows, int channels, bool bf16, double* sums_zeroed,
                                    const float* weight, const float* bias, float eps,
-                                   float momentum, float* save_mean, float* save_invstd,
-                                   float* running_mean, float* running_var, bool relu,
-                                   cudaStream_t stream) {
+                                   float momentum, float* saved, float* running_mean,
+                                   float* running_var, bool relu, cudaStream_t stream) {
   if (!bn_shape_ok(rows, channels)) return cudaErrorInvalidValue;
+  if (relu && residual != nullptr && signs == nullptr) return cudaErrorInvalidValue;
   CountKernelLaunches(2);
-  return bf16 ? ForwardTyped<__nv_bfloat16>(x, residual, y, rows, channels, sums_zeroed, weight,
-                                            bias, eps, momentum, save_mean, save_invstd,
-                                            running_mean, running_var, relu, stream)
-              : ForwardTyped<__half>(x, residual, y, rows, channels, sums_zeroed, weight, bias,
-                                     eps, momentum, save_mean, save_invstd, running_mean,
-                                     running_var, relu, stream);
+  return bf16 ? ForwardTyped<__nv_bfloat16>(x, residual, y, signs, rows, channels, sums_zeroed,
+                                            weight, bias, eps, momentum, saved, running_mean,
+                                            running_var, relu, stream)
+              : ForwardTyped<__half>(x, residual, y, signs, rows, channels, sums_zeroed, weight,
+                                     bias, eps, momentum, saved, running_mean, running_var, relu,
+                                     stream);
 }
 
-cudaError_t LaunchBatchNormBackward(const void* dy, const void* y, const void* x, void* dx,
+cudaError_t LaunchBatchNormBackward(const void* dy, const uint8_t* signs, const void* x, void* dx,
                                     void* dresidual, int64_t rows, int channels, bool bf16,
-                                    double* sums_zeroed, const float* weight,
-                                    const float* save_mean, const float* save_invstd,
+                                    double* sums_zeroed, const float* weight, const float* saved,
                                     float* dweight, float* dbias, bool relu,
                                     cudaStream_t stream) {
   if (!bn_shape_ok(rows, channels)) return cudaErrorInvalidValue;
   CountKernelLaunches(2);
-  return bf16 ? BackwardTyped<__nv_bfloat16>(dy, y, x, dx, dresidual, rows, channels,
-                                             sums_zeroed, weight, save_mean, save_invstd,
-                                             dweight, dbias, relu, stream)
-              : BackwardTyped<__half>(dy, y, x, dx, dresidual, rows, channels, sums_zeroed,
-                                      weight, save_mean, save_invstd, dweight, dbias, relu,
-                                      stream);
+  return bf16 ? BackwardTyped<__nv_bfloat16>(dy, signs, x, dx, dresidual, rows, channels,
+                                             sums_zeroed, weight, saved, dweight, dbias, relu,
+                                             stream)
+              : BackwardTyped<__half>(dy, signs, x, dx, dresidual, rows, channels, sums_zeroed,
+                                      weight, saved, dweight, dbias, relu, stream);
 }
 
 }  // namespace kern

@@ -359,22 +359,22 @@ cudaError_t LaunchScaleBuffer(const void* in, void* out, int64_t count,
 // Training-mode batch normalisation on channels-last 16-bit activations
 // ([rows, channels] row-major), fused with the residual add and the ReLU.
 // `sums_zeroed` is a zero-filled scratch of 2 * channels doubles. Forward:
-// y = act(bn(x) [+ residual]); also writes the batch mean / inverse standard
-// deviation and updates the running statistics (when given). Backward: dx,
-// optionally dresidual (= gradient through the ReLU), dweight, dbias.
+// y = act(bn(x) [+ residual]); also writes `saved` (the rows batch mean, inverse
+// standard deviation and shift of [3, channels]), with a residual and a ReLU
+// `signs` (a byte per 8 channels: which outputs are above zero), and updates
+// the running statistics (when given). Backward: dx, optionally dresidual (=
+// gradient through the ReLU), dweight, dbias; `signs` is null when the forward
+// had no residual.
 bool BatchNormSupported(int64_t rows, int channels);
-cudaError_t LaunchBatchNormForward(const void* x, const void* residual, void* y, int64_t rows,
-                                   int channels, bool bf16, double* sums_zeroed,
+cudaError_t LaunchBatchNormForward(const void* x, const void* residual, void* y, uint8_t* signs,
+                                   int64_t rows, int channels, bool bf16, double* sums_zeroed,
                                    const float* weight, const float* bias, float eps,
-                                   float momentum, float* save_mean, float* save_invstd,
-                                   float* running_mean, float* running_var, bool relu,
-                                   cudaStream_t stream);
-cudaError_t LaunchBatchNormBackward(const void* dy, const void* y, const void* x, void* dx,
+                                   float momentum, float* saved, float* running_mean,
+                                   float* running_var, bool relu, cudaStream_t stream);
+cudaError_t LaunchBatchNormBackward(const void* dy, const uint8_t* signs, const void* x, void* dx,
                                     void* dresidual, int64_t rows, int channels, bool bf16,
-                                    double* sums_zeroed, const float* weight,
-                                    const float* save_mean, const float* save_invstd,
-                                    float* dweight, float* dbias, bool relu,
-                                    cudaStream_t stream);
+                                    double* sums_zeroed, const float* weight, const float* saved,
+                                    float* dweight, float* dbias, bool relu, cudaStream_t stream);
 
 // 3x3 / stride 2 / padding 1 max pooling on channels-last 16-bit activations
 // ([n, h, w, channels], channels a multiple of 8). Forward writes the maxima

@@ -70,7 +70,8 @@ void BindModelOps(py::module_& m) {
     return kern::BatchNormSupported(rows, static_cast<int>(channels));
   });
   // (x, residual?, weight?, bias?, running_mean?, running_var?, momentum, eps, relu)
-  //   -> (y, save_mean, save_invstd)
+  //   -> (y, saved, signs or None): saved holds what the backward needs of the
+  //      statistics, signs (with a residual and a ReLU) which outputs are above zero
   m.def("bn_forward", [](const at::Tensor& x, const c10::optional<at::Tensor>& residual,
                          const c10::optional<at::Tensor>& weight,
                          const c10::optional<at::Tensor>& bias,
@@ -91,8 +92,9 @@ void BindModelOps(py::module_& m) {
     c10::cuda::CUDAGuard guard(x.device());
     cudaStream_t stream = at::cuda::getCurrentCUDAStream();
     at::Tensor y = at::empty_like(x, x.options(), at::MemoryFormat::ChannelsLast);
-    auto fopt = x.options().dtype(at::kFloat);
-    at::Tensor mean = at::empty({C}, fopt), invstd = at::empty({C}, fopt);
+    at::Tensor saved = at::empty({3, C}, x.options().dtype(at::kFloat));
+    at::Tensor signs;
+    if (relu && res != nullptr) signs = at::empty({M, C / 8}, x.options().dtype(at::kByte));
     double* sums = ZeroedDoubles(2 * C, x, stream);
     float* rm = nullptr;
     float* rv = nullptr;
@@ -102,24 +104,35 @@ void BindModelOps(py::module_& m) {
       TORCH_CHECK(rv != nullptr, "running_var must accompany running_mean");
     }
     cudaError_t err = kern::LaunchBatchNormForward(
-        x.data_ptr(), res, y.data_ptr(), M, static_cast<int>(C),
-        x.scalar_type() == at::kBFloat16, sums,
+        x.data_ptr(), res, y.data_ptr(), signs.defined() ? signs.data_ptr<uint8_t>() : nullptr, M,
+        static_cast<int>(C), x.scalar_type() == at::kBFloat16, sums,
         FloatPtrOrNull(weight, C, "weight"), FloatPtrOrNull(bias, C, "bias"),
-        static_cast<float>(eps), static_cast<float>(momentum), mean.data_ptr<float>(),
-        invstd.data_ptr<float>(), rm, rv, relu, stream);
+        static_cast<float>(eps), static_cast<float>(momentum), saved.data_ptr<float>(),
+        rm, rv, relu, stream);
     TORCH_CHECK(err == cudaSuccess, "fused batch norm forward: ", cudaGetErrorString(err));
-    return std::make_tuple(y, mean, invstd);
+    return std::make_tuple(y, saved,
+                           signs.defined() ? c10::optional<at::Tensor>(signs) : c10::nullopt);
   });
-  // (dy, y, x, weight?, save_mean, save_invstd, relu, want_dresidual)
+  // (dy, x, weight?, saved, signs?, relu, want_dresidual)
   //   -> (dx, dresidual or None, dweight, dbias)
-  m.def("bn_backward", [](const at::Tensor& dy, const at::Tensor& y, const at::Tensor& x,
-                          const c10::optional<at::Tensor>& weight, const at::Tensor& save_mean,
-                          const at::Tensor& save_invstd, bool relu, bool want_dresidual) {
+  m.def("bn_backward", [](const at::Tensor& dy, const at::Tensor& x,
+                          const c10::optional<at::Tensor>& weight, const at::Tensor& saved,
+                          const c10::optional<at::Tensor>& signs, bool relu,
+                          bool want_dresidual) {
     CheckActivations(x, "x");
     CheckActivations(dy, "dy");
-    if (relu) CheckActivations(y, "y");
     TORCH_CHECK(dy.sizes() == x.sizes() && dy.scalar_type() == x.scalar_type(), "dy must match x");
     const int64_t C = x.size(1), M = x.numel() / C;
+    TORCH_CHECK(saved.is_cuda() && saved.scalar_type() == at::kFloat && saved.is_contiguous() &&
+                    saved.numel() == 3 * C,
+                "saved must be the tensor returned by bn_forward");
+    const uint8_t* sign_bits = nullptr;
+    if (signs.has_value() && signs->defined()) {
+      TORCH_CHECK(signs->is_cuda() && signs->scalar_type() == at::kByte &&
+                      signs->is_contiguous() && signs->numel() * 8 == x.numel(),
+                  "signs must be the tensor returned by bn_forward");
+      sign_bits = signs->data_ptr<uint8_t>();
+    }
     c10::cuda::CUDAGuard guard(x.device());
     cudaStream_t stream = at::cuda::getCurrentCUDAStream();
     at::Tensor dx = at::empty_like(x, x.options(), at::MemoryFormat::ChannelsLast);
@@ -129,12 +142,11 @@ void BindModelOps(py::module_& m) {
     at::Tensor dweight = at::empty({C}, fopt), dbias = at::empty({C}, fopt);
     double* sums = ZeroedDoubles(2 * C, x, stream);
     cudaError_t err = kern::LaunchBatchNormBackward(
-        dy.data_ptr(), relu ? y.data_ptr() : nullptr, x.data_ptr(), dx.data_ptr(),
+        dy.data_ptr(), sign_bits, x.data_ptr(), dx.data_ptr(),
         want_dresidual ? dres.data_ptr() : nullptr, M, static_cast<int>(C),
         x.scalar_type() == at::kBFloat16, sums,
-        FloatPtrOrNull(weight, C, "weight"), save_mean.data_ptr<float>(),
-        save_invstd.data_ptr<float>(), dweight.data_ptr<float>(), dbias.data_ptr<float>(), relu,
-        stream);
+        FloatPtrOrNull(weight, C, "weight"), saved.data_ptr<float>(), dweight.data_ptr<float>(),
+        dbias.data_ptr<float>(), relu, stream);
     TORCH_CHECK(err == cudaSuccess, "fused batch norm backward: ", cudaGetErrorString(err));
     return std::make_tuple(dx, want_dresidual ? c10::optional<at::Tensor>(dres) : c10::nullopt,
                            dweight, dbias);

@@ -10,7 +10,7 @@ and state_dict keys) whose forward takes an optional residual:
 
 The eager PyTorch sequence batch_norm -> add -> relu makes eight passes over
 the activation in forward and nine in backward; the fused kernels make three
-and seven. The reference has no counterpart (it takes batch normalisation
+or four and five or six. The reference has no counterpart (it takes batch normalisation
 from the framework; horovod/torch/sync_batch_norm.py:98-199 composes
 torch.batch_norm_stats / batch_norm_elemt / batch_norm_backward_reduce).
 """
@@ -41,22 +41,24 @@ def fused_batch_norm_available(x, momentum):
 class _FusedBatchNormAct(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, residual, weight, bias, running_mean, running_var, momentum, eps, relu):
-        y, mean, invstd = _extension().bn_forward(x, residual, weight, bias, running_mean,
+        y, saved, signs = _extension().bn_forward(x, residual, weight, bias, running_mean,
                                                   running_var, momentum, eps, relu)
-        ctx.save_for_backward(x, y if relu else None, weight, mean, invstd)
+        # The kernels do without y; like relu's own backward, this one still
+        # refuses to run when somebody has changed it in place.
+        ctx.save_for_backward(x, y if relu else None, weight, saved, signs)
         ctx.relu = relu
         ctx.has_residual = residual is not None
         return y
 
     @staticmethod
     def backward(ctx, dy):
-        x, y, weight, mean, invstd = ctx.saved_tensors
+        x, _, weight, saved, signs = ctx.saved_tensors
         if dy.dtype != x.dtype:
             dy = dy.to(x.dtype)
         dy = dy.contiguous(memory_format=torch.channels_last)
         want_dres = ctx.has_residual and ctx.needs_input_grad[1]
         dx, dres, dweight, dbias = _extension().bn_backward(
-            dy, y if ctx.relu else dy, x, weight, mean, invstd, ctx.relu, want_dres)
+            dy, x, weight, saved, signs, ctx.relu, want_dres)
         if weight is None:
             dweight = None
         return dx, dres, dweight, dbias if ctx.needs_input_grad[3] else None, None, None, None, \

@@ -36,3 +36,70 @@ def test_max_pool_strips(dtype, shape):
     y.backward(go.contiguous(memory_format=torch.channels_last))
     ref.backward(go.float())
     assert torch.equal(x.grad.float(), ref_x.grad)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("with_res", [False, True])
+@pytest.mark.parametrize("shape", [
+    (1, 8, 1, 3), (3, 8, 31, 33),            # 1 channel group: 256 rows per step of a CTA
+    (2, 64, 9, 7), (1, 256, 5, 5), (5, 512, 7, 7),  # fewer rows than a round, and remainders
+    (37, 32, 53, 51), (8, 2048, 13, 11),     # several rounds per CTA
+])
+def test_batch_norm_mask_without_the_output(shape, with_res, dtype):
+    """The backward finds relu's mask without reading the output. Whole-number
+    gradients have exact sums, so the gradient of the bias must equal the sum
+    over the outputs above zero to the last bit, and the residual's gradient
+    the masked one; tiny scales put outputs where fp16 rounds them to zero."""
+    from horovod_b200.ops.batch_norm import batch_norm_act, fused_batch_norm_available
+    dev, c = _dev(), shape[1]
+    g = torch.Generator(device=dev).manual_seed(3)
+
+    def act():
+        return torch.randn(shape, device=dev, generator=g).to(dtype).contiguous(
+            memory_format=torch.channels_last)
+
+    x = act().requires_grad_(True)
+    res = act().requires_grad_(True) if with_res else None
+    weight = torch.rand(c, device=dev, generator=g) - 0.3
+    weight[::3] *= 1e-7
+    bias = 0.3 * torch.randn(c, device=dev, generator=g)
+    bias[::3] = 0.0
+    weight.requires_grad_(True)
+    bias.requires_grad_(True)
+    assert fused_batch_norm_available(x, 0.1)
+    y = batch_norm_act(x, weight, bias, None, None, residual=res)
+    dy = torch.randint(-4, 5, shape, device=dev, generator=g).to(dtype).contiguous(
+        memory_format=torch.channels_last)
+    y.backward(dy)
+    dz = dy.double() * (y > 0)
+    assert torch.equal(bias.grad.double(), dz.sum((0, 2, 3)))
+    if with_res:
+        assert torch.equal(res.grad.double(), dz)
+    # dx against 64 bits with the same mask: the 16-bit rounding of the result
+    # and of the inputs of a sum of three terms
+    xd = x.detach().double()
+    var, mean = torch.var_mean(xd, (0, 2, 3), unbiased=False, keepdim=True)
+    invstd = torch.rsqrt(var + 1e-5)
+    xhat = (xd - mean) * invstd
+    dx = weight.detach().double().view(1, c, 1, 1) * invstd * (
+        dz - dz.mean((0, 2, 3), keepdim=True) - xhat * (dz * xhat).mean((0, 2, 3), keepdim=True))
+    eps = 2.0 ** (-8 if dtype == torch.bfloat16 else -11)
+    # 1e-5 of the largest: 32-bit terms that cancel; 6e-8: fp16's smallest step
+    bound = eps * dx.abs() + 1e-5 * dx.abs().amax() + 6e-8
+    assert bool(((x.grad.double() - dx).abs() <= bound).all())
+
+
+def test_batch_norm_residual_without_a_gradient():
+    from horovod_b200.ops.batch_norm import batch_norm_act
+    g = torch.Generator(device=_dev()).manual_seed(4)
+    x, res, dy = (torch.randn(3, 16, 5, 5, device=_dev(), generator=g).bfloat16().contiguous(
+        memory_format=torch.channels_last) for _ in range(3))
+    grads = []
+    for wanted in (True, False):
+        xi = x.clone(memory_format=torch.preserve_format).requires_grad_(True)
+        y = batch_norm_act(xi, None, None, None, None,
+                           residual=res.clone(memory_format=torch.preserve_format)
+                           .requires_grad_(wanted))
+        y.backward(dy)
+        grads.append(xi.grad)
+    assert torch.equal(*grads)
