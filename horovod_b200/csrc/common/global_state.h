@@ -73,6 +73,9 @@ struct GlobalState {
   // time: what the caller waits for is negotiated at once (HOROVOD_FLUSH_ON_WAIT).
   std::atomic<int> sync_waiters{0};
   std::mutex wake_mu;
+  // Under wake_mu: waits begun so far, and how many of them a cycle has since
+  // been started for.
+  uint64_t waits_begun = 0, waits_served = 0;
   std::condition_variable wake_cv;
   bool flush_on_wait = true;
   std::string pending_timeline_file;   // non-empty: start; with stop flag: stop

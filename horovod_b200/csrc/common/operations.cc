@@ -133,21 +133,30 @@ bool RunLoopOnce(GlobalState& s,
   if (next > now) {
     if (s.flush_on_wait) {
       // Sleep out the cycle unless somebody blocks in synchronize(): then the
-      // next negotiation starts at once (after a short pause, so that a long
-      // wait does not turn into a busy loop of control-plane rounds). The
-      // cycle time exists to batch tensors for fusion; a caller that is
-      // already waiting has nothing more to add to the batch.
+      // next negotiation starts at once. The cycle time exists to batch
+      // tensors for fusion; a caller that is already waiting has nothing more
+      // to add to the batch. Callers whom a cycle has already been run for
+      // (their peers are late) get the next one after a short pause, so that
+      // a long wait does not turn into a busy loop of control-plane rounds.
+      // The pause must not meet a caller who has only just begun to wait: with
+      // the timer's slack it cost a program that runs one blocking op after
+      // the other 65 of the 100 us per op.
       const auto floor = last_cycle + std::chrono::microseconds(50);
       std::unique_lock<std::mutex> l(s.wake_mu);
       s.wake_cv.wait_until(l, next, [&s] { return s.sync_waiters.load() > 0; });
-      l.unlock();
-      now = std::chrono::steady_clock::now();
-      if (now < floor) std::this_thread::sleep_until(floor);
+      if (s.waits_begun == s.waits_served)
+        s.wake_cv.wait_until(l, floor, [&s] { return s.waits_begun != s.waits_served; });
     } else {
       std::this_thread::sleep_until(next);
     }
   }
   last_cycle = std::chrono::steady_clock::now();
+  {
+    // A caller enqueues its op before it begins to wait: this cycle sees the
+    // ops of everybody counted here.
+    std::lock_guard<std::mutex> l(s.wake_mu);
+    s.waits_served = s.waits_begun;
+  }
 
   {
     std::lock_guard<std::mutex> l(s.ctl_mu);
@@ -384,6 +393,7 @@ void hvd_waiter_enter() {
   {
     std::lock_guard<std::mutex> l(s.wake_mu);
     s.sync_waiters.fetch_add(1);
+    ++s.waits_begun;
   }
   s.wake_cv.notify_all();
 }
