@@ -36,6 +36,63 @@ __device__ __forceinline__ void unpack_range(const TensorList& tl,
                                   [stage](int64_t v) { return ld16(stage + v); });
 }
 
+// One rank: vectors [lo, hi) go straight from the inputs to the outputs, with
+// the arithmetic of the multi-rank variants (prescale, round to the wire type,
+// postscale). Bound by HBM, so what counts is loads in flight: UNROLL vectors
+// per thread with no look-up of the tensor in between.
+template <typename T, typename W, typename S, int UNROLL = 4>
+__device__ __forceinline__ void local_range(const TensorList& tl, int64_t lo, int64_t hi,
+                                            S prescale, bool pre, S postscale, bool post) {
+  constexpr int N = 16 / sizeof(W);
+  constexpr int WORDS = N * sizeof(T) / 16;  // 1, or 2 for fp32 with a 16-bit wire type
+  if (lo >= hi) return;
+  for (int t = find_tensor(tl, lo * N); t < tl.n; ++t) {
+    const int64_t toff = tl.offsets[t];
+    if (toff >= hi * N) break;
+    const int64_t cnt = tl.counts[t];
+    const T* src = static_cast<const T*>(tl.in[t]);
+    T* dst = static_cast<T*>(tl.out[t]);
+    if (dst == nullptr) continue;
+    // Of this tensor: vectors [v0, v1), of which those before vfull are whole.
+    const int64_t v0 = max(lo - toff / N, int64_t(0));
+    const int64_t v1 = min(hi - toff / N, (cnt + N - 1) / N);
+    const bool aligned =
+        ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 15) == 0;
+    const int64_t vfull = src != nullptr && aligned ? max(v0, min(v1, cnt / N)) : v0;
+    const uint4* s4 = reinterpret_cast<const uint4*>(src);
+    uint4* d4 = reinterpret_cast<uint4*>(dst);
+    int64_t v = v0 + threadIdx.x;
+    for (; v + (UNROLL - 1) * THREADS < vfull; v += UNROLL * THREADS) {
+      uint4 raw[UNROLL][WORDS];
+#pragma unroll
+      for (int u = 0; u < UNROLL; ++u)
+#pragma unroll
+        for (int i = 0; i < WORDS; ++i) raw[u][i] = ld16_stream(s4 + (v + u * THREADS) * WORDS + i);
+#pragma unroll
+      for (int u = 0; u < UNROLL; ++u) {
+        uint4 o[WORDS];
+        convert_out<T, W, S>(convert_in<T, W, S>(raw[u], prescale, pre), postscale, post, o);
+#pragma unroll
+        for (int i = 0; i < WORDS; ++i) st16_stream(d4 + (v + u * THREADS) * WORDS + i, o[i]);
+      }
+    }
+    for (; v < vfull; v += THREADS) {
+      uint4 raw[WORDS], o[WORDS];
+#pragma unroll
+      for (int i = 0; i < WORDS; ++i) raw[i] = ld16_stream(s4 + v * WORDS + i);
+      convert_out<T, W, S>(convert_in<T, W, S>(raw, prescale, pre), postscale, post, o);
+#pragma unroll
+      for (int i = 0; i < WORDS; ++i) st16_stream(d4 + v * WORDS + i, o[i]);
+    }
+    // The ragged last vector, or a tensor that is not 16-byte aligned: one
+    // element per thread.
+    const int64_t e1 = min(v1 * N, cnt);
+    for (int64_t e = vfull * N + threadIdx.x; e < e1; e += THREADS)
+      dst[e] = scale_cast<T>(src != nullptr ? scale_cast<W>(src[e], prescale, pre) : W(0.f),
+                             postscale, post);
+  }
+}
+
 // Sum of chunk vectors [lo, hi) over all ranks by peer loads, result stored
 // into every rank's staging buffer. WORLD is a compile-time copy of
 // ctx.world so that the loads of several vectors are all issued before the
@@ -151,18 +208,7 @@ __device__ __forceinline__ void fused_allreduce_body(const InlineTensors& inl,
   if constexpr (ALGO == static_cast<int>(Algo::LOCAL)) {
     const int64_t per = (nvec + G - 1) / G;
     const int64_t lo = b * per, hi = min(lo + per, nvec);
-    // No staging on a single rank: gather (scale, round through the wire
-    // type) and write straight back to the outputs.
-    int cout = lo < hi ? find_tensor(tl, lo * N) : 0;
-    // Same arithmetic as the multi-rank variants: prescale, round to the
-    // wire type, postscale.
-    gather_range<T, W, S, THREADS>(
-        tl, lo, hi, prescale, pre, [&](int64_t v, uint4 x) {
-          // Vectors arrive in increasing order per thread only inside one
-          // tensor; re-seek when the walker moved on to the next tensor.
-          if (v * N < tl.offsets[cout]) cout = find_tensor(tl, v * N);
-          scatter_vec<T, W, S>(tl, cout, v * N, x, postscale, post);
-        });
+    local_range<T, W, S>(tl, lo, hi, prescale, pre, postscale, post);
     return;
   } else if constexpr (ALGO == static_cast<int>(Algo::ONESHOT)) {
     const int64_t per = (nvec + G - 1) / G;

@@ -185,6 +185,7 @@ private:
                         bool skip_end_barrier = false);
   Status CheckKernelStatus();
   int PickCtas(int64_t bytes) const;
+  int LocalCtas(int64_t bytes) const;
   kern::Algo PickAlgo(const SymmSet& set, DataType wire, int64_t bytes) const;
 
   Status SymmAllreduce(std::vector<TensorTableEntry>& entries,

@@ -439,6 +439,13 @@ int GpuOps::PickCtas(int64_t bytes) const {
   return capped(296);  // two CTAs per SM: where the local copy phases peak
 }
 
+int GpuOps::LocalCtas(int64_t bytes) const {
+  // A single rank waits for nobody: the whole GPU copies, at least 16 KB (two
+  // vectors per thread) to a CTA.
+  if (forced_ctas_ > 0) return std::min(forced_ctas_, SYMM_MAX_BLOCKS);
+  return static_cast<int>(std::min<int64_t>(296, std::max<int64_t>(1, bytes >> 14)));
+}
+
 kern::Algo GpuOps::PickAlgo(const SymmSet& set, DataType wire,
                             int64_t bytes) const {
   if (set.world == 1) return kern::Algo::LOCAL;

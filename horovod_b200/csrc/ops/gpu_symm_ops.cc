@@ -183,9 +183,7 @@ Status GpuOps::SymmAllreduce(std::vector<TensorTableEntry>& entries,
     } else {
       kern::Algo algo = PickAlgo(set, wire, bytes);
       int ctas = PickCtas(bytes);
-      // A single rank waits for nobody: use the whole GPU for the copy.
-      if (algo == kern::Algo::LOCAL && forced_ctas_ <= 0)
-        ctas = static_cast<int>(std::min<int64_t>(296, std::max<int64_t>(1, bytes >> 16)));
+      if (algo == kern::Algo::LOCAL) ctas = LocalCtas(bytes);
       int64_t staging_off = 0;
       bool skip_end = false;
       if (algo == kern::Algo::ONESHOT && set.oneshot_bytes >= bytes) {
@@ -498,6 +496,30 @@ Status GpuOps::SymmReducescatter(std::vector<TensorTableEntry>& entries,
         }
       }
       ActEnd(e.name);
+      continue;
+    }
+    if (n == 1) {
+      // A group of one has nobody to exchange shards with: the one-rank
+      // allreduce kernel moves the tensor in one pass (102 MB of fp32: 100 us
+      // through the staging buffer, whose round trip doubles the traffic).
+      // Its arithmetic is the same: prescale, round, postscale.
+      kern::InlineTensors inl;
+      inl.n = 1;
+      inl.offsets[0] = 0;
+      inl.offsets[1] = RoundUp(e.num_elements(), STAGING_ALIGN / es);
+      inl.counts[0] = e.num_elements();
+      inl.in[0] = e.input;
+      inl.out[0] = out;
+      if (e.num_elements() == 0) continue;
+      const kern::TensorList none = {0, nullptr, nullptr, nullptr, nullptr};
+      ActStart(e.name, HVD_ACT_FUSED_KERNEL);
+      cudaError_t err = kern::LaunchFusedAllreduce(
+          none, e.dtype, e.dtype, e.prescale, e.postscale, kern::Algo::LOCAL,
+          LocalCtas(inl.offsets[1] * es), MakeCtx(set, 0), stream_, &inl);
+      ActEnd(e.name);
+      if (err != cudaSuccess)
+        return Status::UnknownError(std::string("reducescatter launch failed: ") +
+                                    cudaGetErrorString(err));
       continue;
     }
     if (sym_off < 0 && staged > static_cast<int64_t>(set.data_bytes))

@@ -103,3 +103,52 @@ def test_batch_norm_residual_without_a_gradient():
         y.backward(dy)
         grads.append(xi.grad)
     assert torch.equal(*grads)
+
+
+@pytest.fixture(scope="module")
+def hvd():
+    import horovod_b200.torch as hvd
+    hvd.init()
+    torch.cuda.set_device(0)
+    yield hvd
+    hvd.shutdown()
+
+
+SIZES = [1, 3, 4, 5, 2047, 2048, 8191, 8192 + 7, (1 << 20) + 1, (3 << 20) + 5]
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float64, torch.int64,
+                                   torch.uint8])
+def test_one_rank_collectives_move_every_element(hvd, dtype):
+    """Sizes around a vector, a round of a CTA and a whole grid, and inputs
+    that do not start on a 16-byte boundary. The results of scaled ones are
+    prescale, round, postscale, round, as with several ranks."""
+    g = torch.Generator(device=_dev()).manual_seed(5)
+    holder = torch.randint(0, 100, (max(SIZES) + 3,), device=_dev(), generator=g).to(dtype)
+    tensors = [holder[:n] for n in SIZES] + [holder[1:1 + n] for n in SIZES]
+    for x, y in zip(tensors, hvd.grouped_allreduce(tensors, op=hvd.Sum, name="edge.%s" % dtype)):
+        assert torch.equal(x, y)
+    for i, x in enumerate(tensors):
+        name = "edge.%s.%d" % (dtype, i)
+        assert torch.equal(hvd.reducescatter(x, op=hvd.Sum, name=name + ".rs"), x)
+        assert torch.equal(hvd.allgather(x, name=name + ".ag"), x)
+        assert torch.equal(hvd.alltoall(x, name=name + ".a2a"), x)
+        if dtype.is_floating_point:
+            wide = torch.float64 if dtype == torch.float64 else torch.float32
+            want = ((x.to(wide) * 0.3).to(dtype).to(wide) * 1.7).to(dtype)
+            for got in (hvd.reducescatter(x, op=hvd.Sum, prescale_factor=0.3, postscale_factor=1.7,
+                                          name=name + ".rss"),
+                        hvd.allreduce(x, op=hvd.Sum, prescale_factor=0.3, postscale_factor=1.7,
+                                      name=name + ".ars")):
+                assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("wire", [torch.float16, torch.bfloat16])
+def test_one_rank_wire_cast_sizes(hvd, wire):
+    g = torch.Generator(device=_dev()).manual_seed(6)
+    holder = torch.randn(max(SIZES) + 3, device=_dev(), generator=g)
+    for i, x in enumerate([holder[:n] for n in SIZES] + [holder[1:1 + n] for n in SIZES]):
+        y = x.clone()
+        hvd.synchronize(hvd.allreduce_async_(y, op=hvd.Sum, wire_dtype=wire,
+                                             name="edge.wire.%s.%d" % (wire, i)))
+        assert torch.equal(y, x.to(wire).float())
