@@ -20,7 +20,9 @@
 //
 // Per-channel sums are accumulated in fp32 per thread (a few dozen groups of
 // rows), in fp64 across the warps of a CTA and across CTAs (atomicAdd on
-// doubles), then mean/variance are formed in fp64.
+// doubles), then mean/variance are formed in fp64. Additions to one address
+// follow each other at about 18 ns, so the CTAs share several copies of the
+// accumulators (bn_copies) and the second kernel adds those up.
 //
 // The reference has no counterpart: it takes batch normalisation from the
 // framework (horovod/torch/sync_batch_norm.py:98-199 calls
@@ -151,8 +153,9 @@ __device__ __forceinline__ void for_rows_back(const Tile& t, int64_t r0, int64_t
 // Sums `acc` (two values per channel of the thread) over the threads of the
 // CTA that own the same channel group and adds the totals to the fp64
 // accumulators: pairwise by shuffles inside a warp, in fp64 across warps.
-__device__ __forceinline__ void reduce_to_global(const Tile& t, float (&acc)[2][VEC], double* dst0,
-                                                 double* dst1) {
+// sums: [copies][2][C]; CTA y adds to copy y % copies.
+__device__ __forceinline__ void reduce_to_global(const Tile& t, float (&acc)[2][VEC], int C,
+                                                 int copies, double* sums) {
   constexpr int WARPS = BN_THREADS / 32;
   // Rows of 36 words: the threads of a warp, which read 8 rows of 4 words
   // below, hit 32 different banks.
@@ -171,21 +174,34 @@ __device__ __forceinline__ void reduce_to_global(const Tile& t, float (&acc)[2][
       for (int i = 0; i < VEC; ++i) red[warp][k * VEC + i][t.tx] = acc[k][i];
   }
   __syncthreads();
+  double* mine = sums + static_cast<int64_t>(blockIdx.y % copies) * 2 * C +
+                 static_cast<int64_t>(blockIdx.x) * t.txg * VEC;
   // 2 * VEC * txg <= 512 totals, two rounds of 256 threads at most.
   for (int idx = threadIdx.x; idx < t.txg * 2 * VEC; idx += BN_THREADS) {
     const int i = idx % VEC, tx = idx / VEC % t.txg, k = idx / VEC / t.txg;
     double sum = 0.0;
 #pragma unroll
     for (int w = 0; w < WARPS; ++w) sum += static_cast<double>(red[w][k * VEC + i][tx]);
-    atomicAdd((k == 0 ? dst0 : dst1) + (static_cast<int64_t>(blockIdx.x) * t.txg + tx) * VEC + i,
-              sum);
+    atomicAdd(mine + static_cast<int64_t>(k) * C + tx * VEC + i, sum);
   }
+}
+
+// The two sums of channel ch over all copies.
+__device__ __forceinline__ double2 total(const double* sums, int C, int copies, int64_t ch) {
+  double2 t = make_double2(0.0, 0.0);
+#pragma unroll 4
+  for (int i = 0; i < copies; ++i) {
+    const double* p = sums + static_cast<int64_t>(i) * 2 * C + ch;
+    t.x += __ldcg(p);
+    t.y += __ldcg(p + C);
+  }
+  return t;
 }
 
 template <typename T>
 __global__ void __launch_bounds__(BN_THREADS, BN_MIN_BLOCKS_STATS)
-bn_stats_kernel(const T* __restrict__ x, int64_t M, int C, double* __restrict__ sum,
-                double* __restrict__ sumsq) {
+bn_stats_kernel(const T* __restrict__ x, int64_t M, int C, int copies,
+                double* __restrict__ sums) {
   const Tile t(C);
   int64_t r0, r1;
   cta_rows(M, blockIdx.y, &r0, &r1);
@@ -218,7 +234,7 @@ bn_stats_kernel(const T* __restrict__ x, int64_t M, int C, double* __restrict__ 
     }
   });
   start_next();
-  reduce_to_global(t, acc, sum, sumsq);
+  reduce_to_global(t, acc, C, copies, sums);
 }
 
 // Most channels of a CTA. Their per-channel values are formed by one thread
@@ -259,9 +275,8 @@ __device__ __forceinline__ void load8(const float* p, float (&v)[VEC]) {
 template <typename T, bool RELU, bool RES>
 __global__ void __launch_bounds__(BN_THREADS, BN_MIN_BLOCKS)
 bn_apply_kernel(const T* __restrict__ x, const T* __restrict__ res, T* __restrict__ y,
-                uint8_t* __restrict__ signs, int64_t M, int C, double inv_m,
-                const double* __restrict__ sum, const double* __restrict__ sumsq,
-                const float* __restrict__ weight, const float* __restrict__ bias, float eps,
+                uint8_t* __restrict__ signs, int64_t M, int C, double inv_m, int copies,
+                const double* __restrict__ sums, const float* __restrict__ weight, const float* __restrict__ bias, float eps,
                 float momentum, float* __restrict__ saved, float* __restrict__ running_mean,
                 float* __restrict__ running_var) {
   const Tile t(C);
@@ -273,8 +288,9 @@ bn_apply_kernel(const T* __restrict__ x, const T* __restrict__ res, T* __restric
   wait_for_previous();
   if (static_cast<int>(threadIdx.x) < t.txg * VEC) {
     const int64_t ch = static_cast<int64_t>(blockIdx.x) * t.txg * VEC + threadIdx.x;
-    const double m = __ldcg(sum + ch) * inv_m;
-    double var = __ldcg(sumsq + ch) * inv_m - m * m;
+    const double2 sum = total(sums, C, copies, ch);
+    const double m = sum.x * inv_m;
+    double var = sum.y * inv_m - m * m;
     if (var < 0.0) var = 0.0;
     const float mean = static_cast<float>(m);
     const float invstd = static_cast<float>(rsqrt(var + static_cast<double>(eps)));
@@ -351,7 +367,7 @@ __global__ void __launch_bounds__(BN_THREADS, BN_MIN_BLOCKS)
 bn_backward_reduce_kernel(const T* __restrict__ dy, const uint8_t* __restrict__ signs,
                           const T* __restrict__ x, int64_t M, int C,
                           const float* __restrict__ weight, const float* __restrict__ saved,
-                          double* __restrict__ sum_dz, double* __restrict__ sum_dz_xhat) {
+                          int copies, double* __restrict__ sums) {
   const Tile t(C);
   int64_t r0, r1;
   cta_rows(M, blockIdx.y, &r0, &r1);
@@ -404,7 +420,7 @@ bn_backward_reduce_kernel(const T* __restrict__ dy, const uint8_t* __restrict__ 
   load8(saved + C + off, invstd);
 #pragma unroll
   for (int i = 0; i < VEC; ++i) acc[1][i] *= invstd[i];
-  reduce_to_global(t, acc, sum_dz, sum_dz_xhat);
+  reduce_to_global(t, acc, C, copies, sums);
 }
 
 template <typename T, int MASK, bool DRES>
@@ -412,8 +428,8 @@ __global__ void __launch_bounds__(BN_THREADS, BN_MIN_BLOCKS)
 bn_backward_apply_kernel(const T* __restrict__ dy, const uint8_t* __restrict__ signs,
                          const T* __restrict__ x, T* __restrict__ dx, T* __restrict__ dres,
                          int64_t M, int C, double inv_m, const float* __restrict__ weight,
-                         const float* __restrict__ saved, const double* __restrict__ sum_dz,
-                         const double* __restrict__ sum_dz_xhat, float* __restrict__ dweight,
+                         const float* __restrict__ saved, int copies,
+                         const double* __restrict__ sums, float* __restrict__ dweight,
                          float* __restrict__ dbias) {
   const Tile t(C);
   const int by = gridDim.y - 1 - blockIdx.y;
@@ -424,7 +440,8 @@ bn_backward_apply_kernel(const T* __restrict__ dy, const uint8_t* __restrict__ s
   wait_for_previous();
   if (static_cast<int>(threadIdx.x) < t.txg * VEC) {
     const int64_t ch = static_cast<int64_t>(blockIdx.x) * t.txg * VEC + threadIdx.x;
-    const double dz = __ldcg(sum_dz + ch), dz_xhat = __ldcg(sum_dz_xhat + ch);
+    const double2 sum = total(sums, C, copies, ch);
+    const double dz = sum.x, dz_xhat = sum.y;
     const float invstd = saved[C + ch];
     s_mean[threadIdx.x] = saved[ch];
     s_shift[threadIdx.x] = saved[2 * static_cast<int64_t>(C) + ch];
@@ -474,13 +491,31 @@ bn_backward_apply_kernel(const T* __restrict__ dy, const uint8_t* __restrict__ s
   });
 }
 
-dim3 bn_grid(int64_t M, int C) {
+// Copies of the per-channel accumulators: 8 up to 256 channels, fewer beyond
+// (more channels are spread over more CTAs, so fewer of them meet at one
+// address). One copy and 1184 CTAs took 23 us for the statistics of 256 x 256 x
+// 14 x 14, 8 copies and 592 CTAs take 7.3; 16 and more cost the second kernel
+// more than they save the first.
+int bn_copies(int C) { return C <= 256 ? 8 : C < 2048 ? 2048 / C : 1; }
+
+// The kernels that sum run as one wave of resident CTAs: each CTA ends with its
+// additions to the accumulators.
+constexpr int BN_CTAS_STATS = 148 * BN_MIN_BLOCKS_STATS;
+constexpr int BN_CTAS_REDUCE = 148 * BN_MIN_BLOCKS;
+// The kernels that write start with reading them, so tensors that fit L2 (126
+// MB) get one wave too: 256 x 256 x 14 x 14 forward 10.7 us, 15.5 with 1184
+// CTAs. Beyond that the time goes to HBM, where more and shorter CTAs even out
+// the SMs: 256 x 256 x 56 x 56 with residual 198 us, 216 with one wave.
+int bn_apply_ctas(int64_t M, int C) { return M * C <= (64 << 20) ? 148 * BN_MIN_BLOCKS : 148 * 8; }
+
+dim3 bn_grid(int64_t M, int C, int ctas) {
   const int cg = C / VEC;
   const int txg = cg < 32 ? cg : 32;
   const int ty = BN_THREADS / txg;
   const int ctiles = cg / txg;
-  // About eight CTAs per SM in total, at least 4 * ty rows each.
-  int64_t by = (148 * 8 + ctiles - 1) / ctiles;
+  // At most `ctas` in total (a few more would be a second wave), at least 4 *
+  // ty rows each.
+  int64_t by = ctas / ctiles;
   const int64_t max_by = (M + 4 * ty - 1) / (4 * ty);
   if (by > max_by) by = max_by;
   if (by < 1) by = 1;
@@ -500,6 +535,10 @@ bool bn_shape_ok(int64_t M, int C) {
 }  // namespace
 
 bool BatchNormSupported(int64_t rows, int channels) { return bn_shape_ok(rows, channels); }
+
+int64_t BatchNormScratchDoubles(int channels) {
+  return static_cast<int64_t>(2) * bn_copies(channels) * channels;
+}
 
 // Launches the second kernel of a pair so that it may start while the first
 // one is still running (it waits for the results itself).
@@ -522,20 +561,19 @@ static cudaError_t ForwardTyped(const void* x, const void* res, void* y, uint8_t
                                 int C, double* sums, const float* weight, const float* bias,
                                 float eps, float momentum, float* saved, float* running_mean,
                                 float* running_var, bool relu, cudaStream_t stream) {
-  const dim3 grid = bn_grid(M, C);
-  double* sum = sums;
-  double* sumsq = sums + C;
-  bn_stats_kernel<T><<<grid, BN_THREADS, 0, stream>>>(static_cast<const T*>(x), M, C, sum, sumsq);
+  const int copies = bn_copies(C);
+  bn_stats_kernel<T><<<bn_grid(M, C, BN_CTAS_STATS), BN_THREADS, 0, stream>>>(
+      static_cast<const T*>(x), M, C, copies, sums);
   cudaError_t err = cudaGetLastError();
   if (err != cudaSuccess) return err;
   auto kernel = relu && res ? bn_apply_kernel<T, true, true>
                 : relu      ? bn_apply_kernel<T, true, false>
                 : res       ? bn_apply_kernel<T, false, true>
                             : bn_apply_kernel<T, false, false>;
-  return LaunchDependent(kernel, grid, stream, static_cast<const T*>(x),
-                         static_cast<const T*>(res), static_cast<T*>(y), signs, M, C,
-                         1.0 / static_cast<double>(M), sum, sumsq, weight, bias, eps, momentum,
-                         saved, running_mean, running_var);
+  return LaunchDependent(kernel, bn_grid(M, C, bn_apply_ctas(M, C)), stream,
+                         static_cast<const T*>(x), static_cast<const T*>(res),
+                         static_cast<T*>(y), signs, M, C, 1.0 / static_cast<double>(M), copies,
+                         sums, weight, bias, eps, momentum, saved, running_mean, running_var);
 }
 
 template <typename T>
@@ -543,9 +581,7 @@ static cudaError_t BackwardTyped(const void* dy, const uint8_t* signs, const voi
                                  void* dres, int64_t M, int C, double* sums, const float* weight,
                                  const float* saved, float* dweight, float* dbias, bool relu,
                                  cudaStream_t stream) {
-  const dim3 grid = bn_grid(M, C);
-  double* sum_dz = sums;
-  double* sum_dz_xhat = sums + C;
+  const int copies = bn_copies(C);
   const T* dyt = static_cast<const T*>(dy);
   const T* xt = static_cast<const T*>(x);
   const int mask = !relu ? MASK_NONE : signs == nullptr ? MASK_X : MASK_SIGNS;
@@ -555,8 +591,8 @@ static cudaError_t BackwardTyped(const void* dy, const uint8_t* signs, const voi
   auto reduce = mask == MASK_NONE ? bn_backward_reduce_kernel<T, MASK_NONE>
                 : mask == MASK_X  ? bn_backward_reduce_kernel<T, MASK_X>
                                   : bn_backward_reduce_kernel<T, MASK_SIGNS>;
-  reduce<<<grid, BN_THREADS, 0, stream>>>(dyt, signs, xt, M, C, weight, saved, sum_dz,
-                                          sum_dz_xhat);
+  reduce<<<bn_grid(M, C, BN_CTAS_REDUCE), BN_THREADS, 0, stream>>>(dyt, signs, xt, M, C, weight,
+                                                                   saved, copies, sums);
   cudaError_t err = cudaGetLastError();
   if (err != cudaSuccess) return err;
   auto apply = mask == MASK_NONE ? (dres ? bn_backward_apply_kernel<T, MASK_NONE, true>
@@ -564,9 +600,10 @@ static cudaError_t BackwardTyped(const void* dy, const uint8_t* signs, const voi
                : mask == MASK_X  ? bn_backward_apply_kernel<T, MASK_X, false>
                                  : (dres ? bn_backward_apply_kernel<T, MASK_SIGNS, true>
                                          : bn_backward_apply_kernel<T, MASK_SIGNS, false>);
-  return LaunchDependent(apply, grid, stream, dyt, signs, xt, static_cast<T*>(dx),
-                         static_cast<T*>(dres), M, C, 1.0 / static_cast<double>(M), weight, saved,
-                         sum_dz, sum_dz_xhat, dweight, dbias);
+  return LaunchDependent(apply, bn_grid(M, C, bn_apply_ctas(M, C)), stream, dyt, signs, xt,
+                         static_cast<T*>(dx), static_cast<T*>(dres), M, C,
+                         1.0 / static_cast<double>(M), weight, saved, copies, sums, dweight,
+                         dbias);
 }
 
 cudaError_t LaunchBatchNormForward(const void* x, const void* residual, void* y, uint8_t* signs,

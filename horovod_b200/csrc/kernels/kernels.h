@@ -358,7 +358,7 @@ cudaError_t LaunchScaleBuffer(const void* in, void* out, int64_t count,
 // Launch* function counts the kernels it enqueues).
 // Training-mode batch normalisation on channels-last 16-bit activations
 // ([rows, channels] row-major), fused with the residual add and the ReLU.
-// `sums_zeroed` is a zero-filled scratch of 2 * channels doubles. Forward:
+// `sums_zeroed` is a zero-filled scratch of BatchNormScratchDoubles(). Forward:
 // y = act(bn(x) [+ residual]); also writes `saved` (the rows batch mean, inverse
 // standard deviation and shift of [3, channels]), with a residual and a ReLU
 // `signs` (a byte per 8 channels: which outputs are above zero), and updates
@@ -366,6 +366,7 @@ cudaError_t LaunchScaleBuffer(const void* in, void* out, int64_t count,
 // gradient through the ReLU), dweight, dbias; `signs` is null when the forward
 // had no residual.
 bool BatchNormSupported(int64_t rows, int channels);
+int64_t BatchNormScratchDoubles(int channels);
 cudaError_t LaunchBatchNormForward(const void* x, const void* residual, void* y, uint8_t* signs,
                                    int64_t rows, int channels, bool bf16, double* sums_zeroed,
                                    const float* weight, const float* bias, float eps,

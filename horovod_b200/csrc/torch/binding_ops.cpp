@@ -95,7 +95,7 @@ void BindModelOps(py::module_& m) {
     at::Tensor saved = at::empty({3, C}, x.options().dtype(at::kFloat));
     at::Tensor signs;
     if (relu && res != nullptr) signs = at::empty({M, C / 8}, x.options().dtype(at::kByte));
-    double* sums = ZeroedDoubles(2 * C, x, stream);
+    double* sums = ZeroedDoubles(kern::BatchNormScratchDoubles(static_cast<int>(C)), x, stream);
     float* rm = nullptr;
     float* rv = nullptr;
     if (running_mean.has_value() && running_mean->defined()) {
@@ -140,7 +140,7 @@ void BindModelOps(py::module_& m) {
     if (want_dresidual) dres = at::empty_like(x, x.options(), at::MemoryFormat::ChannelsLast);
     auto fopt = x.options().dtype(at::kFloat);
     at::Tensor dweight = at::empty({C}, fopt), dbias = at::empty({C}, fopt);
-    double* sums = ZeroedDoubles(2 * C, x, stream);
+    double* sums = ZeroedDoubles(kern::BatchNormScratchDoubles(static_cast<int>(C)), x, stream);
     cudaError_t err = kern::LaunchBatchNormBackward(
         dy.data_ptr(), sign_bits, x.data_ptr(), dx.data_ptr(),
         want_dresidual ? dres.data_ptr() : nullptr, M, static_cast<int>(C),
