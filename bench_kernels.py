@@ -24,8 +24,8 @@ Cases
   max_pool      3x3 / stride 2 / padding 1 max pooling on the ResNet stem
                 activation 256 x 64 x 112 x 112 bf16 (411 MB): forward reads x,
                 writes y (1/4 of x) and one index byte per output element
-                (1/8 of x): 1.375x; backward reads dy and the indices and
-                writes dx: 1.375x. Next to PyTorch's max_pool2d.
+                (1/16 of x): 1.3125x; backward reads dy and the indices and
+                writes dx: 1.3125x. Next to PyTorch's max_pool2d.
   fused_sgd     hvd.FusedSGD step (momentum + weight decay) over 161
                 ResNet-50-shaped fp32 tensors: reads p, g, m, writes p, m
                 (5x bytes). Next to torch.optim.SGD on the same tensors.
@@ -219,8 +219,8 @@ def main():
             y = fwd(x)
             go = torch.randn_like(y)
             t_b = timed_events(lambda: torch.autograd.grad(y, x, go, retain_graph=True), args.iters)
-            report_line(name + "_forward", t_f, 1.375 * xbytes, {"shape": list(x.shape)})
-            report_line(name + "_backward", t_b, 1.375 * xbytes, {"shape": list(x.shape)})
+            report_line(name + "_forward", t_f, 1.3125 * xbytes, {"shape": list(x.shape)})
+            report_line(name + "_backward", t_b, 1.3125 * xbytes, {"shape": list(x.shape)})
             del y
     if "fused_sgd" in cases:
         from horovod_b200.torch.fused_sgd import FusedSGD
@@ -238,12 +238,11 @@ def main():
                          "note": "optimizer.step() as called by a training loop: bounded by "
                                  "its Python work when the GPU is otherwise idle"})
             if cls is FusedSGD:
-                # The kernel alone, through the plan that step() cached.
-                plan, n, n_chunks = next(iter(opt._plans.values()))[1]
+                # The native call alone.
+                bufs = [opt.state[p]["momentum_buffer"] for p in ps]
 
                 def kernel_only():
-                    _C.sgd_step(plan, n, n_chunks, opt.CHUNK, True, 0.01, 0.9, 0.0, 1e-4, False,
-                                False, False)
+                    _C.sgd_step(ps, bufs, 0.01, 0.9, 0.0, 1e-4, False, False, False)
                 us = timed_events(kernel_only, args.iters)
                 report_line("fused_sgd_kernel", us, 5 * total,
                             {"tensors": len(sizes), "payload_mb": total >> 20})

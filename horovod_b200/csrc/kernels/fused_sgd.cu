@@ -4,6 +4,12 @@
 // (or, for tensors whose layout defeats the foreach fast path, one launch per
 // tensor per pass) of the framework's optimizer.
 //
+// Bound by HBM: 20 bytes per element. The tensors are cut into chunks of 4096
+// elements, one per CTA, whose threads have all their loads (12 of 16 bytes
+// with momentum) in flight at once. The list rides in the kernel's parameters,
+// so a step needs no descriptor in device memory, no copy and nothing kept
+// from the step before.
+//
 // The reference has no counterpart (the optimizer is the framework's,
 // horovod/torch/optimizer.py:249-325 only wraps its step()).
 #include "kernels.h"
@@ -14,56 +20,70 @@ namespace kern {
 namespace {
 
 constexpr int SGD_THREADS = 256;
+constexpr int SGD_VECS = SGD_CHUNK_ELEMS / 4 / SGD_THREADS;  // 16-byte vectors per thread
+static_assert(SGD_VECS * SGD_THREADS * 4 == SGD_CHUNK_ELEMS, "whole vectors per thread");
+
+struct SgdRule {
+  float lr, momentum, dampening, weight_decay;
+  bool nesterov, first_step, maximize;
+  // New momentum in *b (read unless first_step); returns the new parameter.
+  __device__ __forceinline__ float operator()(float p, float g, float* b) const {
+    if (maximize) g = -g;
+    if (weight_decay != 0.f) g = fmaf(weight_decay, p, g);
+    if (momentum != 0.f) {
+      *b = first_step ? g : fmaf(momentum, *b, (1.f - dampening) * g);
+      g = nesterov ? fmaf(momentum, *b, g) : *b;
+    }
+    return fmaf(-lr, g, p);
+  }
+};
 
 __global__ void __launch_bounds__(SGD_THREADS)
-fused_sgd_kernel(SgdTensors t, float lr, float momentum, float dampening, float weight_decay,
-                 bool nesterov, bool first_step, bool maximize) {
-  for (int c = blockIdx.x; c < t.n_chunks; c += gridDim.x) {
-    const int ti = t.chunk_tensor[c];
-    const int64_t start = t.chunk_start[c];
-    const int64_t n = min(t.chunk_elems, t.counts[ti] - start);
-    float* p = t.params[ti] + start;
-    const float* g = t.grads[ti] + start;
-    float* b = (t.bufs != nullptr && t.bufs[ti] != nullptr) ? t.bufs[ti] + start : nullptr;
-    auto update = [&](float pv, float gv, float bv, float* b_out) {
-      if (maximize) gv = -gv;
-      if (weight_decay != 0.f) gv = fmaf(weight_decay, pv, gv);
-      if (momentum != 0.f) {
-        bv = first_step ? gv : fmaf(momentum, bv, (1.f - dampening) * gv);
-        *b_out = bv;
-        gv = nesterov ? fmaf(momentum, bv, gv) : bv;
+fused_sgd_kernel(const __grid_constant__ SgdTensors t, const SgdRule rule) {
+  const int c = blockIdx.x;
+  int ti = 0, end = t.n;  // the tensor whose chunks include c
+  while (end - ti > 1) {
+    const int mid = (ti + end) >> 1;
+    if (t.first_chunk[mid] <= c) ti = mid; else end = mid;
+  }
+  const int64_t start = static_cast<int64_t>(c - t.first_chunk[ti]) * SGD_CHUNK_ELEMS;
+  const int n = static_cast<int>(min(static_cast<int64_t>(SGD_CHUNK_ELEMS), t.counts[ti] - start));
+  float* p = t.params[ti] + start;
+  const float* g = t.grads[ti] + start;
+  float* b = rule.momentum != 0.f ? t.bufs[ti] + start : nullptr;
+  const bool read_b = b != nullptr && !rule.first_step;
+  int done = 0;
+  if (((reinterpret_cast<uintptr_t>(p) | reinterpret_cast<uintptr_t>(g) |
+        reinterpret_cast<uintptr_t>(b)) & 15) == 0) {
+    const int nv = n >> 2;
+    float4 pv[SGD_VECS], gv[SGD_VECS], bv[SGD_VECS];
+#pragma unroll
+    for (int u = 0; u < SGD_VECS; ++u) {
+      const int i = threadIdx.x + u * SGD_THREADS;
+      if (i < nv) {
+        pv[u] = reinterpret_cast<const float4*>(p)[i];
+        gv[u] = __ldcs(reinterpret_cast<const float4*>(g) + i);
+        bv[u] = read_b ? reinterpret_cast<const float4*>(b)[i] : make_float4(0.f, 0.f, 0.f, 0.f);
       }
-      return fmaf(-lr, gv, pv);
-    };
-    const bool vec = ((reinterpret_cast<uintptr_t>(p) | reinterpret_cast<uintptr_t>(g) |
-                       reinterpret_cast<uintptr_t>(b)) & 15) == 0;
-    int64_t done = 0;
-    if (vec) {
-      const int64_t nv = n >> 2;
-      float4* p4 = reinterpret_cast<float4*>(p);
-      const float4* g4 = reinterpret_cast<const float4*>(g);
-      float4* b4 = reinterpret_cast<float4*>(b);
-      for (int64_t i = threadIdx.x; i < nv; i += SGD_THREADS) {
-        float4 pv = p4[i];
-        const float4 gv = __ldcs(g4 + i);
-        float4 bv = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (b != nullptr && !first_step) bv = b4[i];
-        float4 bo = bv;
-        pv.x = update(pv.x, gv.x, bv.x, &bo.x);
-        pv.y = update(pv.y, gv.y, bv.y, &bo.y);
-        pv.z = update(pv.z, gv.z, bv.z, &bo.z);
-        pv.w = update(pv.w, gv.w, bv.w, &bo.w);
-        p4[i] = pv;
-        if (b != nullptr && momentum != 0.f) b4[i] = bo;
+    }
+#pragma unroll
+    for (int u = 0; u < SGD_VECS; ++u) {
+      const int i = threadIdx.x + u * SGD_THREADS;
+      if (i < nv) {
+        pv[u].x = rule(pv[u].x, gv[u].x, &bv[u].x);
+        pv[u].y = rule(pv[u].y, gv[u].y, &bv[u].y);
+        pv[u].z = rule(pv[u].z, gv[u].z, &bv[u].z);
+        pv[u].w = rule(pv[u].w, gv[u].w, &bv[u].w);
+        reinterpret_cast<float4*>(p)[i] = pv[u];
+        if (b != nullptr) reinterpret_cast<float4*>(b)[i] = bv[u];
       }
-      done = nv << 2;
     }
-    for (int64_t i = done + threadIdx.x; i < n; i += SGD_THREADS) {
-      float bo = 0.f;
-      const float bv = (b != nullptr && !first_step) ? b[i] : 0.f;
-      p[i] = update(p[i], g[i], bv, &bo);
-      if (b != nullptr && momentum != 0.f) b[i] = bo;
-    }
+    done = nv << 2;
+  }
+  for (int i = done + threadIdx.x; i < n; i += SGD_THREADS) {
+    float bv = read_b ? b[i] : 0.f;
+    p[i] = rule(p[i], g[i], &bv);
+    if (b != nullptr) b[i] = bv;
   }
 }
 
@@ -72,12 +92,12 @@ fused_sgd_kernel(SgdTensors t, float lr, float momentum, float dampening, float 
 cudaError_t LaunchFusedSgd(const SgdTensors& t, float lr, float momentum, float dampening,
                            float weight_decay, bool nesterov, bool first_step, bool maximize,
                            cudaStream_t stream) {
-  if (t.n_chunks <= 0) return cudaSuccess;
-  if (t.chunk_elems <= 0 || (t.chunk_elems & 3) != 0) return cudaErrorInvalidValue;
+  if (t.n < 1 || t.n > SGD_MAX_TENSORS) return cudaErrorInvalidValue;
+  const int chunks = t.first_chunk[t.n];
+  if (chunks <= 0) return cudaSuccess;
   CountKernelLaunches(1);
-  const int grid = t.n_chunks < 148 * 8 ? t.n_chunks : 148 * 8;
-  fused_sgd_kernel<<<grid, SGD_THREADS, 0, stream>>>(t, lr, momentum, dampening, weight_decay,
-                                                     nesterov, first_step, maximize);
+  const SgdRule rule = {lr, momentum, dampening, weight_decay, nesterov, first_step, maximize};
+  fused_sgd_kernel<<<chunks, SGD_THREADS, 0, stream>>>(t, rule);
   return cudaGetLastError();
 }
 

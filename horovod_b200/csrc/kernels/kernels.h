@@ -391,20 +391,18 @@ cudaError_t LaunchMaxPool3s2Backward(const void* dy, const uint32_t* idx, void* 
 // decay added to the gradient, momentum buffer b = momentum * b + (1 -
 // dampening) * g, or b = g on the first step, optional Nesterov, then
 // p -= lr * update). Tensor i has counts[i] fp32 elements at params[i],
-// grads[i], bufs[i] (bufs may be null when momentum == 0); the three arrays of
-// a tensor must share one memory layout. chunk_tensor / chunk_start (device
-// arrays of n_chunks entries) cut the tensors into pieces of at most
-// chunk_elems elements, one per CTA iteration.
+// grads[i], bufs[i] (not read when momentum == 0); the three arrays of a
+// tensor must share one memory layout. Tensor i is cut into the chunks
+// [first_chunk[i], first_chunk[i + 1]) of SGD_CHUNK_ELEMS elements each.
+constexpr int SGD_CHUNK_ELEMS = 4096;
+constexpr int SGD_MAX_TENSORS = 256;  // 9 KB of kernel parameters
 struct SgdTensors {
   int n;
-  float* const* params;
-  const float* const* grads;
-  float* const* bufs;
-  const int64_t* counts;
-  int n_chunks;
-  const int32_t* chunk_tensor;
-  const int64_t* chunk_start;
-  int64_t chunk_elems;
+  int32_t first_chunk[SGD_MAX_TENSORS + 1];
+  float* params[SGD_MAX_TENSORS];
+  const float* grads[SGD_MAX_TENSORS];
+  float* bufs[SGD_MAX_TENSORS];
+  int64_t counts[SGD_MAX_TENSORS];
 };
 cudaError_t LaunchFusedSgd(const SgdTensors& t, float lr, float momentum, float dampening,
                            float weight_decay, bool nesterov, bool first_step, bool maximize,

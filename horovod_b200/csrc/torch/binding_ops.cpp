@@ -4,7 +4,7 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/extension.h>
 
-#include <cstring>
+#include <cstdint>
 #include <map>
 #include <mutex>
 #include <tuple>
@@ -61,6 +61,19 @@ double* ZeroedDoubles(int64_t count, const at::Tensor& like, cudaStream_t stream
   double* out = p.buf.data_ptr<double>() + p.used;
   p.used += need;
   return out;
+}
+
+// Whether t holds fp32 values next to p's, element for element.
+bool SgdLike(const at::Tensor& p, const at::Tensor& t) {
+  return t.defined() && t.layout() == at::kStrided && t.scalar_type() == at::kFloat &&
+         t.device() == p.device() && t.sizes() == p.sizes() && t.strides() == p.strides();
+}
+
+// What the multi-tensor SGD kernel takes: fp32 on a GPU, a gradient of the
+// same memory layout, and no gaps in it.
+bool SgdReady(const at::Tensor& p, const at::Tensor& g) {
+  return p.is_cuda() && p.layout() == at::kStrided && p.scalar_type() == at::kFloat &&
+         SgdLike(p, g) && p.is_non_overlapping_and_dense();
 }
 
 }  // namespace
@@ -197,80 +210,57 @@ void BindModelOps(py::module_& m) {
   });
 
   // ---- multi-tensor SGD ------------------------------------------------------
-  // Builds the device-side tensor list for sgd_step: (descriptor bytes on the
-  // device, number of tensors, number of chunks). Parameters, gradients and
-  // momentum buffers must be fp32 CUDA tensors with one memory layout per
-  // triple; bufs may be empty (no momentum).
-  m.def("sgd_plan", [](const std::vector<at::Tensor>& params,
-                       const std::vector<at::Tensor>& grads,
-                       const std::vector<at::Tensor>& bufs, int64_t chunk_elems) {
-    const size_t n = params.size();
-    TORCH_CHECK(n > 0 && grads.size() == n && (bufs.empty() || bufs.size() == n),
-                "sgd_plan: list lengths differ");
-    TORCH_CHECK(chunk_elems > 0 && chunk_elems % 4 == 0, "chunk_elems must be a multiple of 4");
-    std::vector<int64_t> chunk_start;
-    std::vector<int32_t> chunk_tensor;
-    for (size_t i = 0; i < n; ++i) {
-      const at::Tensor& p = params[i];
-      const at::Tensor& g = grads[i];
-      TORCH_CHECK(p.is_cuda() && p.scalar_type() == at::kFloat && g.is_cuda() &&
-                      g.scalar_type() == at::kFloat && g.device() == p.device(),
-                  "sgd_plan: parameters and gradients must be fp32 tensors on one GPU");
-      TORCH_CHECK(p.is_non_overlapping_and_dense() && g.sizes() == p.sizes() &&
-                      g.strides() == p.strides(),
-                  "sgd_plan: a gradient does not share its parameter's memory layout");
-      if (!bufs.empty())
-        TORCH_CHECK(bufs[i].is_cuda() && bufs[i].scalar_type() == at::kFloat &&
-                        bufs[i].sizes() == p.sizes() && bufs[i].strides() == p.strides(),
-                    "sgd_plan: a momentum buffer does not share its parameter's layout");
-      for (int64_t s = 0; s < p.numel(); s += chunk_elems) {
-        chunk_start.push_back(s);
-        chunk_tensor.push_back(static_cast<int32_t>(i));
-      }
+  // One step over a parameter list, in one launch per 256 tensors. bufs holds
+  // a momentum buffer (or None) per parameter; it is empty when momentum is 0.
+  // Parameters without a gradient are passed over. Returns the positions of
+  // those that the kernel cannot take (see SgdReady), untouched.
+  m.def("sgd_step", [](const std::vector<at::Tensor>& params,
+                       const std::vector<c10::optional<at::Tensor>>& bufs, double lr,
+                       double momentum, double dampening, double weight_decay, bool nesterov,
+                       bool first_step, bool maximize) {
+    const bool with_bufs = momentum != 0.0;
+    TORCH_CHECK(bufs.size() == (with_bufs ? params.size() : 0), "sgd_step: list lengths differ");
+    std::vector<int64_t> rest;
+    std::vector<size_t> ready;
+    for (size_t i = 0; i < params.size(); ++i) {
+      const at::Tensor& g = params[i].grad();
+      if (!g.defined()) continue;
+      if (SgdReady(params[i], g) &&
+          (!with_bufs || (bufs[i].has_value() && SgdLike(params[i], *bufs[i]))))
+        ready.push_back(i);
+      else
+        rest.push_back(static_cast<int64_t>(i));
     }
-    const size_t nc = chunk_start.size();
-    const size_t bytes = n * 32 + nc * 8 + nc * 4;
-    at::Tensor host = at::empty({static_cast<int64_t>(bytes)},
-                                at::TensorOptions().dtype(at::kByte).pinned_memory(true));
-    char* h = static_cast<char*>(host.data_ptr());
-    void** hp = reinterpret_cast<void**>(h);
-    for (size_t i = 0; i < n; ++i) {
-      hp[i] = params[i].data_ptr();
-      hp[n + i] = grads[i].data_ptr();
-      hp[2 * n + i] = bufs.empty() ? nullptr : bufs[i].data_ptr();
-      reinterpret_cast<int64_t*>(h + n * 24)[i] = params[i].numel();
-    }
-    std::memcpy(h + n * 32, chunk_start.data(), nc * 8);
-    std::memcpy(h + n * 32 + nc * 8, chunk_tensor.data(), nc * 4);
-    c10::cuda::CUDAGuard guard(params[0].device());
-    at::Tensor dev = at::empty({static_cast<int64_t>(bytes)},
-                               params[0].options().dtype(at::kByte));
-    dev.copy_(host, /*non_blocking=*/true);
-    return std::make_tuple(dev, static_cast<int64_t>(n), static_cast<int64_t>(nc));
-  });
-  m.def("sgd_step", [](const at::Tensor& plan, int64_t n, int64_t n_chunks, int64_t chunk_elems,
-                       bool has_bufs, double lr, double momentum, double dampening,
-                       double weight_decay, bool nesterov, bool first_step, bool maximize) {
-    TORCH_CHECK(plan.is_cuda() && plan.scalar_type() == at::kByte &&
-                    plan.numel() == n * 32 + n_chunks * 12,
-                "sgd_step: not a plan made by sgd_plan");
-    c10::cuda::CUDAGuard guard(plan.device());
-    cudaStream_t stream = at::cuda::getCurrentCUDAStream();
-    char* d = static_cast<char*>(plan.data_ptr());
     kern::SgdTensors t;
-    t.n = static_cast<int>(n);
-    t.params = reinterpret_cast<float* const*>(d);
-    t.grads = reinterpret_cast<const float* const*>(d + n * 8);
-    t.bufs = has_bufs ? reinterpret_cast<float* const*>(d + n * 16) : nullptr;
-    t.counts = reinterpret_cast<const int64_t*>(d + n * 24);
-    t.n_chunks = static_cast<int>(n_chunks);
-    t.chunk_start = reinterpret_cast<const int64_t*>(d + n * 32);
-    t.chunk_tensor = reinterpret_cast<const int32_t*>(d + n * 32 + n_chunks * 8);
-    t.chunk_elems = chunk_elems;
-    cudaError_t err = kern::LaunchFusedSgd(
-        t, static_cast<float>(lr), static_cast<float>(momentum), static_cast<float>(dampening),
-        static_cast<float>(weight_decay), nesterov, first_step, maximize, stream);
-    TORCH_CHECK(err == cudaSuccess, "fused SGD: ", cudaGetErrorString(err));
+    size_t next = 0;
+    while (next < ready.size()) {
+      // The run of tensors from here on that share a device, as many as fit.
+      const at::Device device = params[ready[next]].device();
+      t.n = 0;
+      int64_t chunks = 0;
+      t.first_chunk[0] = 0;
+      for (; next < ready.size() && t.n < kern::SGD_MAX_TENSORS; ++next) {
+        const at::Tensor& p = params[ready[next]];
+        if (p.device() != device) break;
+        const int64_t more =
+            (p.numel() + kern::SGD_CHUNK_ELEMS - 1) / kern::SGD_CHUNK_ELEMS;
+        if (chunks + more > INT32_MAX) break;
+        chunks += more;
+        t.params[t.n] = p.data_ptr<float>();
+        t.grads[t.n] = p.grad().const_data_ptr<float>();
+        t.bufs[t.n] = with_bufs ? bufs[ready[next]]->data_ptr<float>() : nullptr;
+        t.counts[t.n] = p.numel();
+        t.first_chunk[++t.n] = static_cast<int32_t>(chunks);
+      }
+      TORCH_CHECK(t.n > 0, "sgd_step: a parameter is too large");
+      c10::cuda::CUDAGuard guard(device);
+      cudaError_t err = kern::LaunchFusedSgd(
+          t, static_cast<float>(lr), static_cast<float>(momentum), static_cast<float>(dampening),
+          static_cast<float>(weight_decay), nesterov, first_step, maximize,
+          at::cuda::getCurrentCUDAStream());
+      TORCH_CHECK(err == cudaSuccess, "fused SGD: ", cudaGetErrorString(err));
+    }
+    return rest;
   });
 }
 

@@ -38,8 +38,6 @@ def _dense(t):
 
 
 class FusedSGD(Optimizer):
-    CHUNK = 1 << 16  # elements per CTA iteration
-
     def __init__(self, params, lr=1e-3, momentum=0.0, dampening=0.0, weight_decay=0.0,
                  nesterov=False, maximize=False):
         if lr < 0.0:
@@ -53,7 +51,6 @@ class FusedSGD(Optimizer):
         defaults = dict(lr=lr, momentum=momentum, dampening=dampening,
                         weight_decay=weight_decay, nesterov=nesterov, maximize=maximize)
         super().__init__(params, defaults)
-        self._plans = {}
 
     @staticmethod
     def _kernel_ok(p):
@@ -84,52 +81,45 @@ class FusedSGD(Optimizer):
         if closure is not None:
             with torch.enable_grad():
                 loss = closure()
-        ext = _extension()
-        for gi, group in enumerate(self.param_groups):
-            momentum = group["momentum"]
-            fast = {True: [], False: []}  # keyed by "momentum buffer already exists"
-            for p in group["params"]:
-                if p.grad is None:
-                    continue
-                if not self._kernel_ok(p):
-                    self._torch_update(p, group)
-                    continue
-                has_buf = momentum == 0 or "momentum_buffer" in self.state[p]
-                fast[has_buf].append(p)
-            for has_buf, plist in fast.items():
-                if not plist:
-                    continue
-                first = momentum != 0 and not has_buf
-                bufs = []
-                if momentum != 0:
-                    for p in plist:
-                        state = self.state[p]
-                        if "momentum_buffer" not in state:
-                            state["momentum_buffer"] = torch.empty_like(
-                                p, memory_format=torch.preserve_format)
-                        buf = state["momentum_buffer"]
-                        if buf.stride() != p.stride():  # e.g. loaded from a state_dict
-                            fixed = torch.empty_like(p, memory_format=torch.preserve_format)
-                            fixed.copy_(buf)
-                            buf = state["momentum_buffer"] = fixed
-                        bufs.append(buf)
-                by_device = {}
-                for i, p in enumerate(plist):
-                    by_device.setdefault(p.device, []).append(i)
-                for dev, idxs in by_device.items():
-                    ps = [plist[i] for i in idxs]
-                    gs = [p.grad for p in ps]
-                    bs = [bufs[i] for i in idxs] if bufs else []
-                    key = (gi, has_buf, dev,
-                           tuple(t.data_ptr() for t in ps), tuple(t.data_ptr() for t in gs),
-                           tuple(t.data_ptr() for t in bs))
-                    slot = (gi, has_buf, dev)
-                    cached = self._plans.get(slot)
-                    if cached is None or cached[0] != key:
-                        cached = (key, ext.sgd_plan(ps, gs, bs, self.CHUNK))
-                        self._plans[slot] = cached
-                    plan, n, n_chunks = cached[1]
-                    ext.sgd_step(plan, n, n_chunks, self.CHUNK, bool(bs), group["lr"], momentum,
-                                 group["dampening"], group["weight_decay"], group["nesterov"],
-                                 first, group["maximize"])
+        for group in self.param_groups:
+            params = group["params"]
+            bufs = []
+            if group["momentum"] != 0:
+                get, nothing = self.state.get, {}
+                bufs = [get(p, nothing).get("momentum_buffer") for p in params]
+            rest = self._launch(params, bufs, group, first_step=False)
+            if rest:
+                self._step_rest([params[i] for i in rest], group)
         return loss
+
+    @staticmethod
+    def _launch(params, bufs, group, first_step):
+        """One native call checks, lists and updates all tensors it can; the
+        positions of the others come back."""
+        return _extension().sgd_step(
+            params, bufs, group["lr"], group["momentum"], group["dampening"],
+            group["weight_decay"], group["nesterov"], first_step, group["maximize"])
+
+    def _step_rest(self, params, group):
+        """The parameters that the kernel cannot take as they are: new ones
+        (no momentum yet), a momentum buffer of another layout (e.g. loaded
+        from a state_dict), and those left to PyTorch."""
+        plists = {False: [], True: []}  # keyed by "this is the first step"
+        for p in params:
+            if group["momentum"] == 0 or not self._kernel_ok(p):
+                self._torch_update(p, group)
+                continue
+            state = self.state[p]
+            first = "momentum_buffer" not in state
+            if first:
+                state["momentum_buffer"] = torch.empty_like(
+                    p, memory_format=torch.preserve_format)
+            elif state["momentum_buffer"].stride() != p.stride():
+                fixed = torch.empty_like(p, memory_format=torch.preserve_format)
+                fixed.copy_(state["momentum_buffer"])
+                state["momentum_buffer"] = fixed
+            plists[first].append(p)
+        for first, plist in plists.items():
+            bufs = [self.state[p]["momentum_buffer"] for p in plist]
+            if plist and self._launch(plist, bufs, group, first):
+                raise RuntimeError("FusedSGD: a momentum buffer does not match its parameter")
