@@ -293,18 +293,39 @@ def allreduce_async(tensor, average=None, name=None, op=None, prescale_factor=1.
                             process_set)
 
 
+def _cast_in_kernel(compression, tensors, average, op):
+    """Whether the casts of ``compression`` can happen inside the collective
+    kernel: one pass over the tensors instead of three (cast, reduce, cast
+    back) and no launches and allocations per tensor. The compressors of this
+    library on fp32 CUDA tensors; user-defined ones and everything else run
+    as they are. Depends on nothing that differs between ranks."""
+    return bool((compression is Compression.fp16 or compression is Compression.bf16) and tensors
+            and handle_average_backwards_compatibility(op, average) in (Average, Sum)
+            and all(isinstance(t, torch.Tensor) and t.is_cuda and t.dtype == torch.float32
+                    and not t.is_sparse for t in tensors))
+
+
+def _dense(tensor):
+    """What the cast of a compressor would have made of the tensor's layout."""
+    return tensor if _is_dense(tensor) else tensor.contiguous()
+
+
 class HorovodAllreduce(torch.autograd.Function):
     """Allreduce whose gradient is the allreduce of the incoming gradient."""
 
     @staticmethod
-    def forward(ctx, tensor, average, name, op, prescale_factor, postscale_factor, process_set):
+    def forward(ctx, tensor, average, name, op, prescale_factor, postscale_factor, process_set,
+                compression):
         ctx.average = average
         ctx.op = op
         ctx.prescale_factor = prescale_factor
         ctx.postscale_factor = postscale_factor
         ctx.process_set = process_set
-        handle = allreduce_async(tensor, average, name, op, prescale_factor,
-                                 postscale_factor, process_set)
+        ctx.compression = compression
+        handle = _allreduce_async(tensor, torch.empty_like(tensor), name,
+                                  handle_average_backwards_compatibility(op, average),
+                                  prescale_factor, postscale_factor, process_set,
+                                  compression.wire_dtype)
         return synchronize(handle)
 
     @staticmethod
@@ -312,8 +333,8 @@ class HorovodAllreduce(torch.autograd.Function):
         return (allreduce(grad_output.contiguous(), average=ctx.average, op=ctx.op,
                           prescale_factor=ctx.prescale_factor,
                           postscale_factor=ctx.postscale_factor,
-                          process_set=ctx.process_set),
-                None, None, None, None, None, None)
+                          process_set=ctx.process_set, compression=ctx.compression),
+                None, None, None, None, None, None, None)
 
 
 def allreduce(tensor, average=None, name=None, compression=Compression.none, op=None,
@@ -321,9 +342,12 @@ def allreduce(tensor, average=None, name=None, compression=Compression.none, op=
     """Reduces ``tensor`` over all ranks of the process set and returns the
     result on every rank. Differentiable. ``op`` is Average (default), Sum,
     Adasum, Min, Max or Product."""
+    if _cast_in_kernel(compression, [tensor], average, op):
+        return HorovodAllreduce.apply(_dense(tensor), average, name, op, prescale_factor,
+                                      postscale_factor, process_set, compression)
     tensor_compressed, ctx = compression.compress(tensor)
-    summed = HorovodAllreduce.apply(tensor_compressed, average, name, op,
-                                    prescale_factor, postscale_factor, process_set)
+    summed = HorovodAllreduce.apply(tensor_compressed, average, name, op, prescale_factor,
+                                    postscale_factor, process_set, Compression.none)
     return compression.decompress(summed, ctx)
 
 
@@ -387,14 +411,17 @@ def grouped_allreduce_async(tensors, average=None, name=None, op=None, prescale_
 class HorovodGroupedAllreduce(torch.autograd.Function):
     @staticmethod
     def forward(ctx, average, name, op, prescale_factor, postscale_factor, process_set,
-                *tensors):
+                compression, *tensors):
         ctx.average = average
         ctx.op = op
         ctx.prescale_factor = prescale_factor
         ctx.postscale_factor = postscale_factor
         ctx.process_set = process_set
-        handle = grouped_allreduce_async(list(tensors), average, name, op, prescale_factor,
-                                         postscale_factor, process_set)
+        ctx.compression = compression
+        handle = _grouped_allreduce_async(list(tensors), [torch.empty_like(t) for t in tensors],
+                                          name, handle_average_backwards_compatibility(op, average),
+                                          prescale_factor, postscale_factor, process_set,
+                                          compression.wire_dtype)
         return tuple(synchronize(handle))
 
     @staticmethod
@@ -403,17 +430,22 @@ class HorovodGroupedAllreduce(torch.autograd.Function):
                                   average=ctx.average, op=ctx.op,
                                   prescale_factor=ctx.prescale_factor,
                                   postscale_factor=ctx.postscale_factor,
-                                  process_set=ctx.process_set)
-        return (None, None, None, None, None, None, *grads)
+                                  process_set=ctx.process_set, compression=ctx.compression)
+        return (None, None, None, None, None, None, None, *grads)
 
 
 def grouped_allreduce(tensors, average=None, name=None, compression=Compression.none,
                       op=None, prescale_factor=1.0, postscale_factor=1.0,
                       process_set=global_process_set):
     """Blocking, differentiable grouped allreduce. Returns a list."""
+    tensors = list(tensors)
+    if _cast_in_kernel(compression, tensors, average, op):
+        return list(HorovodGroupedAllreduce.apply(
+            average, name, op, prescale_factor, postscale_factor, process_set, compression,
+            *[_dense(t) for t in tensors]))
     compressed, ctxs = zip(*[compression.compress(t) for t in tensors]) if tensors else ((), ())
-    summed = HorovodGroupedAllreduce.apply(average, name, op, prescale_factor,
-                                           postscale_factor, process_set, *compressed)
+    summed = HorovodGroupedAllreduce.apply(average, name, op, prescale_factor, postscale_factor,
+                                           process_set, Compression.none, *compressed)
     return [compression.decompress(t, c) for t, c in zip(summed, ctxs)]
 
 

@@ -152,3 +152,61 @@ def test_one_rank_wire_cast_sizes(hvd, wire):
         hvd.synchronize(hvd.allreduce_async_(y, op=hvd.Sum, wire_dtype=wire,
                                              name="edge.wire.%s.%d" % (wire, i)))
         assert torch.equal(y, x.to(wire).float())
+
+
+@pytest.mark.parametrize("momentum", [0.0, 0.9])
+def test_fused_sgd_many_tensors(momentum):
+    """More tensors than one launch takes, sizes around a chunk, tensors that
+    are not 16-byte aligned and parameters without a gradient."""
+    from horovod_b200 import _C
+    from horovod_b200.torch.fused_sgd import FusedSGD
+    g = torch.Generator(device=_dev()).manual_seed(7)
+    sizes = [1, 3, 4, 4095, 4096, 4097, 8193, 0] * 40 + [(1 << 20) + 3]
+    holders = [torch.randn(n + 1, device=_dev(), generator=g) for n in sizes]
+    ps = [h[i % 2:i % 2 + n].detach().requires_grad_(True)
+          for i, (h, n) in enumerate(zip(holders, sizes))]
+    qs = [p.detach().clone().requires_grad_(True) for p in ps]
+    kwargs = dict(lr=0.1, momentum=momentum, weight_decay=1e-3)
+    opt, ref = FusedSGD(ps, **kwargs), torch.optim.SGD(qs, foreach=False, **kwargs)
+    for step in range(3):
+        for i, (p, q) in enumerate(zip(ps, qs)):
+            if i % 11 == step:
+                p.grad = q.grad = None
+                continue
+            p.grad = torch.randn(p.shape, device=_dev(), generator=g)
+            q.grad = p.grad.clone()
+        before = _C.kernel_launch_count()
+        opt.step()
+        assert _C.kernel_launch_count() - before >= 2, "321 tensors take two launches"
+        ref.step()
+    for p, q in zip(ps, qs):
+        torch.testing.assert_close(p, q, rtol=1e-5, atol=1e-6)
+    assert len(opt.state) == len(ref.state) or momentum == 0
+
+
+@pytest.mark.parametrize("name", ["fp16", "bf16"])
+def test_compression_inside_the_kernel(hvd, name):
+    """allreduce and grouped_allreduce of fp32 tensors with this library's
+    compressors: values, layouts, dtypes and gradients of the casts around it."""
+    compression = getattr(hvd.Compression, name)
+    g = torch.Generator(device=_dev()).manual_seed(8)
+    base = torch.randn(6, 8, 5, 7, device=_dev(), generator=g)
+    xs = [base, base.contiguous(memory_format=torch.channels_last), base[:, ::2], base[..., 1:],
+          torch.randn((), device=_dev(), generator=g), base.flatten()[1:1 + 4099],
+          torch.empty(0, device=_dev())]
+    leaves = [x.detach().requires_grad_(True) for x in xs]
+    ys = hvd.grouped_allreduce(leaves, name="cmp.%s" % name, compression=compression)
+    for i, (x, y) in enumerate(zip(xs, ys)):
+        want = x.to(compression.wire_dtype).float()
+        assert y.dtype == torch.float32 and y.stride() == want.stride() and torch.equal(y, want)
+        z = hvd.allreduce(x, name="cmp.%s.%d" % (name, i), compression=compression)
+        assert z.stride() == want.stride() and torch.equal(z, want)
+    dys = [torch.randn(y.shape, device=_dev(), generator=g) for y in ys]
+    for dx, dy in zip(torch.autograd.grad(ys, leaves, dys), dys):
+        assert torch.equal(dx, dy.to(compression.wire_dtype).float())
+    # other types keep the casts outside
+    for dtype in (torch.float64, torch.bfloat16, torch.int32):
+        v = torch.arange(9, device=_dev()).to(dtype)
+        out = hvd.allreduce(v, name="cmp.%s.%s" % (name, dtype), compression=compression,
+                            op=hvd.Sum)
+        assert out.dtype == dtype and torch.equal(out, v)
