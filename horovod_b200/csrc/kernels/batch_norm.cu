@@ -278,7 +278,7 @@ bn_apply_kernel(const T* __restrict__ x, const T* __restrict__ res, T* __restric
                 uint8_t* __restrict__ signs, int64_t M, int C, double inv_m, int copies,
                 const double* __restrict__ sums, const float* __restrict__ weight, const float* __restrict__ bias, float eps,
                 float momentum, float* __restrict__ saved, float* __restrict__ running_mean,
-                float* __restrict__ running_var) {
+                float* __restrict__ running_var, int64_t* __restrict__ batches) {
   const Tile t(C);
   const int by = gridDim.y - 1 - blockIdx.y;
   int64_t r0, r1;
@@ -286,6 +286,7 @@ bn_apply_kernel(const T* __restrict__ x, const T* __restrict__ res, T* __restric
   __shared__ __align__(16) float s_scale[BN_CTA_CHANNELS];
   __shared__ __align__(16) float s_shift[BN_CTA_CHANNELS];
   wait_for_previous();
+  if (batches != nullptr && by == 0 && blockIdx.x == 0 && threadIdx.x == 0) *batches += 1;
   if (static_cast<int>(threadIdx.x) < t.txg * VEC) {
     const int64_t ch = static_cast<int64_t>(blockIdx.x) * t.txg * VEC + threadIdx.x;
     const double2 sum = total(sums, C, copies, ch);
@@ -560,7 +561,8 @@ template <typename T>
 static cudaError_t ForwardTyped(const void* x, const void* res, void* y, uint8_t* signs, int64_t M,
                                 int C, double* sums, const float* weight, const float* bias,
                                 float eps, float momentum, float* saved, float* running_mean,
-                                float* running_var, bool relu, cudaStream_t stream) {
+                                float* running_var, int64_t* batches, bool relu,
+                                cudaStream_t stream) {
   const int copies = bn_copies(C);
   bn_stats_kernel<T><<<bn_grid(M, C, BN_CTAS_STATS), BN_THREADS, 0, stream>>>(
       static_cast<const T*>(x), M, C, copies, sums);
@@ -573,7 +575,8 @@ static cudaError_t ForwardTyped(const void* x, const void* res, void* y, uint8_t
   return LaunchDependent(kernel, bn_grid(M, C, bn_apply_ctas(M, C)), stream,
                          static_cast<const T*>(x), static_cast<const T*>(res),
                          static_cast<T*>(y), signs, M, C, 1.0 / static_cast<double>(M), copies,
-                         sums, weight, bias, eps, momentum, saved, running_mean, running_var);
+                         sums, weight, bias, eps, momentum, saved, running_mean, running_var,
+                         batches);
 }
 
 template <typename T>
@@ -610,16 +613,17 @@ cudaError_t LaunchBatchNormForward(const void* x, const void* residual, void* y,
                                    int64_t rows, int channels, bool bf16, double* sums_zeroed,
                                    const float* weight, const float* bias, float eps,
                                    float momentum, float* saved, float* running_mean,
-                                   float* running_var, bool relu, cudaStream_t stream) {
+                                   float* running_var, int64_t* batches, bool relu,
+                                   cudaStream_t stream) {
   if (!bn_shape_ok(rows, channels)) return cudaErrorInvalidValue;
   if (relu && residual != nullptr && signs == nullptr) return cudaErrorInvalidValue;
   CountKernelLaunches(2);
   return bf16 ? ForwardTyped<__nv_bfloat16>(x, residual, y, signs, rows, channels, sums_zeroed,
                                             weight, bias, eps, momentum, saved, running_mean,
-                                            running_var, relu, stream)
+                                            running_var, batches, relu, stream)
               : ForwardTyped<__half>(x, residual, y, signs, rows, channels, sums_zeroed, weight,
-                                     bias, eps, momentum, saved, running_mean, running_var, relu,
-                                     stream);
+                                     bias, eps, momentum, saved, running_mean, running_var,
+                                     batches, relu, stream);
 }
 
 cudaError_t LaunchBatchNormBackward(const void* dy, const uint8_t* signs, const void* x, void* dx,

@@ -362,7 +362,7 @@ cudaError_t LaunchScaleBuffer(const void* in, void* out, int64_t count,
 // y = act(bn(x) [+ residual]); also writes `saved` (the rows batch mean, inverse
 // standard deviation and shift of [3, channels]), with a residual and a ReLU
 // `signs` (a byte per 8 channels: which outputs are above zero), and updates
-// the running statistics (when given). Backward: dx, optionally dresidual (=
+// the running statistics and the count of batches (when given). Backward: dx, optionally dresidual (=
 // gradient through the ReLU), dweight, dbias; `signs` is null when the forward
 // had no residual.
 bool BatchNormSupported(int64_t rows, int channels);
@@ -371,7 +371,8 @@ cudaError_t LaunchBatchNormForward(const void* x, const void* residual, void* y,
                                    int64_t rows, int channels, bool bf16, double* sums_zeroed,
                                    const float* weight, const float* bias, float eps,
                                    float momentum, float* saved, float* running_mean,
-                                   float* running_var, bool relu, cudaStream_t stream);
+                                   float* running_var, int64_t* batches, bool relu,
+                                   cudaStream_t stream);
 cudaError_t LaunchBatchNormBackward(const void* dy, const uint8_t* signs, const void* x, void* dx,
                                     void* dresidual, int64_t rows, int channels, bool bf16,
                                     double* sums_zeroed, const float* weight, const float* saved,

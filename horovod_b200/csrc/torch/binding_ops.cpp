@@ -82,7 +82,8 @@ void BindModelOps(py::module_& m) {
   m.def("bn_supported", [](int64_t rows, int64_t channels) {
     return kern::BatchNormSupported(rows, static_cast<int>(channels));
   });
-  // (x, residual?, weight?, bias?, running_mean?, running_var?, momentum, eps, relu)
+  // (x, residual?, weight?, bias?, running_mean?, running_var?, momentum, eps, relu,
+  //  num_batches_tracked?)
   //   -> (y, saved, signs or None): saved holds what the backward needs of the
   //      statistics, signs (with a residual and a ReLU) which outputs are above zero
   m.def("bn_forward", [](const at::Tensor& x, const c10::optional<at::Tensor>& residual,
@@ -90,7 +91,7 @@ void BindModelOps(py::module_& m) {
                          const c10::optional<at::Tensor>& bias,
                          c10::optional<at::Tensor> running_mean,
                          c10::optional<at::Tensor> running_var, double momentum, double eps,
-                         bool relu) {
+                         bool relu, c10::optional<at::Tensor> batches) {
     CheckActivations(x, "x");
     const int64_t C = x.size(1), M = x.numel() / C;
     TORCH_CHECK(kern::BatchNormSupported(M, static_cast<int>(C)),
@@ -116,12 +117,19 @@ void BindModelOps(py::module_& m) {
       rv = const_cast<float*>(FloatPtrOrNull(running_var, C, "running_var"));
       TORCH_CHECK(rv != nullptr, "running_var must accompany running_mean");
     }
+    int64_t* count = nullptr;
+    if (batches.has_value() && batches->defined()) {
+      TORCH_CHECK(batches->device() == x.device() && batches->scalar_type() == at::kLong &&
+                      batches->numel() == 1,
+                  "num_batches_tracked must be one int64 on the device of x");
+      count = batches->data_ptr<int64_t>();
+    }
     cudaError_t err = kern::LaunchBatchNormForward(
         x.data_ptr(), res, y.data_ptr(), signs.defined() ? signs.data_ptr<uint8_t>() : nullptr, M,
         static_cast<int>(C), x.scalar_type() == at::kBFloat16, sums,
         FloatPtrOrNull(weight, C, "weight"), FloatPtrOrNull(bias, C, "bias"),
         static_cast<float>(eps), static_cast<float>(momentum), saved.data_ptr<float>(),
-        rm, rv, relu, stream);
+        rm, rv, count, relu, stream);
     TORCH_CHECK(err == cudaSuccess, "fused batch norm forward: ", cudaGetErrorString(err));
     return std::make_tuple(y, saved,
                            signs.defined() ? c10::optional<at::Tensor>(signs) : c10::nullopt);

@@ -40,9 +40,10 @@ def fused_batch_norm_available(x, momentum):
 
 class _FusedBatchNormAct(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, x, residual, weight, bias, running_mean, running_var, momentum, eps, relu):
+    def forward(ctx, x, residual, weight, bias, running_mean, running_var, momentum, eps, relu,
+                batches):
         y, saved, signs = _extension().bn_forward(x, residual, weight, bias, running_mean,
-                                                  running_var, momentum, eps, relu)
+                                                  running_var, momentum, eps, relu, batches)
         # The kernels do without y; like relu's own backward, this one still
         # refuses to run when somebody has changed it in place.
         ctx.save_for_backward(x, y if relu else None, weight, saved, signs)
@@ -62,18 +63,26 @@ class _FusedBatchNormAct(torch.autograd.Function):
         if weight is None:
             dweight = None
         return dx, dres, dweight, dbias if ctx.needs_input_grad[3] else None, None, None, None, \
-            None, None
+            None, None, None
 
 
 def batch_norm_act(x, weight, bias, running_mean, running_var, residual=None, training=True,
-                   momentum=0.1, eps=1e-5, relu=True):
-    """relu(batch_norm(x) + residual), fused on the GPU when possible."""
+                   momentum=0.1, eps=1e-5, relu=True, num_batches_tracked=None):
+    """relu(batch_norm(x) + residual), fused on the GPU when possible.
+    ``num_batches_tracked`` (optional, an int64 tensor) is incremented."""
     if training and fused_batch_norm_available(x, momentum) and \
             (residual is None or (residual.shape == x.shape and residual.dtype == x.dtype)):
         if residual is not None:
             residual = residual.contiguous(memory_format=torch.channels_last)
+        if num_batches_tracked is not None and (num_batches_tracked.device != x.device or
+                                                num_batches_tracked.dtype != torch.int64):
+            num_batches_tracked.add_(1)
+            num_batches_tracked = None
         return _FusedBatchNormAct.apply(x, residual, weight, bias, running_mean, running_var,
-                                        float(momentum), float(eps), bool(relu))
+                                        float(momentum), float(eps), bool(relu),
+                                        num_batches_tracked)
+    if num_batches_tracked is not None:
+        num_batches_tracked.add_(1)
     out = F.batch_norm(x, running_mean, running_var, weight, bias, training,
                        0.0 if momentum is None else momentum, eps)
     if residual is not None:
@@ -90,15 +99,17 @@ class BatchNormAct2d(nn.BatchNorm2d):
 
     def forward(self, x, residual=None):
         self._check_input_dim(x)
-        if self.training and self.track_running_stats and self.num_batches_tracked is not None:
-            self.num_batches_tracked.add_(1)
+        batches = self.num_batches_tracked if self.training and self.track_running_stats else None
         training = self.training or (self.running_mean is None and self.running_var is None)
         momentum = self.momentum
         if momentum is None and self.training and self.track_running_stats:
+            if batches is not None:  # counted here: the average needs the count first
+                batches.add_(1)
+                batches = None
             momentum = 1.0 / float(self.num_batches_tracked)
         return batch_norm_act(
             x, self.weight, self.bias,
             self.running_mean if not self.training or self.track_running_stats else None,
             self.running_var if not self.training or self.track_running_stats else None,
             residual=residual, training=training, momentum=momentum, eps=self.eps,
-            relu=self.relu)
+            relu=self.relu, num_batches_tracked=batches)
