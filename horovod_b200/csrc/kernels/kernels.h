@@ -388,6 +388,14 @@ cudaError_t LaunchMaxPool3s2Forward(const void* x, void* y, uint32_t* idx, int n
 cudaError_t LaunchMaxPool3s2Backward(const void* dy, const uint32_t* idx, void* dx, int n, int h,
                                      int w, int channels, bool bf16, cudaStream_t stream);
 
+// 7x7 / stride 2 / padding 3 convolution of 3 channels-last 16-bit channels
+// ([n, h, w, 3]) without bias: y [n, (h - 1) / 2 + 1, (w - 1) / 2 + 1, channels].
+// weight: 16-bit [channels, 3, 7, 7] with the given element strides.
+bool StemConvSupported(int channels);
+cudaError_t LaunchStemConvForward(const void* x, const void* weight, const int64_t* weight_strides,
+                                  void* y, int n, int h, int w, int channels, bool bf16,
+                                  cudaStream_t stream);
+
 // Multi-tensor SGD step in one launch (torch.optim.SGD arithmetic: weight
 // decay added to the gradient, momentum buffer b = momentum * b + (1 -
 // dampening) * g, or b = g on the first step, optional Nesterov, then

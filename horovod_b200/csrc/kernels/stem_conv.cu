@@ -1,0 +1,302 @@
+// The first convolution of a ResNet, 7x7 / stride 2 / padding 3 on 3 channels,
+// forward, channels-last 16-bit, as an implicit GEMM on the 5th-generation
+// tensor cores. cuDNN has no sm_100 kernel for 3 channels and pads them to 4
+// for one of an older architecture.
+//
+// Input pixels are taken in 2 x 2 blocks of 12 values (16 with padding): the
+// convolution is then 4x4 / stride 1 on 16 channels, 16 steps of K = 16, and
+// output (i, j) reads the blocks (i .. i + 3, j .. j + 3). A CTA computes 16
+// rows of 8 output pixels (M = 128) from a patch of 19 x 11 blocks in shared
+// memory, stored without a swizzle as two planes of 16 bytes per block: 8
+// neighbouring blocks of a row are then one 8 x 16-byte core matrix, the rows
+// of the patch are the stride between core matrices, and the operand of every
+// one of the 16 taps is the same descriptor with another start address. No
+// im2col is ever stored. The weights stay in shared memory for all tiles of a
+// CTA; four CTAs per SM take turns with loading, multiplying and storing, and
+// a CTA loads the pixels of its next tile before it waits for the products.
+//
+// Bound by HBM (the output is 5 times the input).
+//
+// The reference has no counterpart (it takes convolutions from the framework).
+#include <cuda_bf16.h>
+#include <cuda_fp16.h>
+
+#include <cstdint>
+#include <mutex>
+
+#include "kernels.h"
+
+namespace hvd {
+namespace kern {
+
+namespace {
+
+constexpr int THREADS = 256;
+constexpr int TILE_H = 16, TILE_W = 8;                      // output pixels: M = 128
+constexpr int PATCH_H = TILE_H + 3, PATCH_W = TILE_W + 3;   // blocks
+constexpr int PATCH = PATCH_H * PATCH_W;
+constexpr int PLANE_BYTES = PATCH * 16;
+constexpr int TAPS = 16, K_CORES = 2 * TAPS;  // 8 values of K each
+static_assert(PATCH <= THREADS, "one block per thread");
+
+__device__ __forceinline__ uint32_t smem_addr(const void* p) {
+  return static_cast<uint32_t>(__cvta_generic_to_shared(p));
+}
+
+// K-major operand without a swizzle: `k_step` bytes between the two core
+// matrices of K = 16, `mn_step` bytes between groups of 8 rows.
+__device__ __forceinline__ uint64_t operand(uint32_t addr, uint32_t k_step, uint32_t mn_step) {
+  return static_cast<uint64_t>((addr >> 4) & 0x3fffu) |
+         (static_cast<uint64_t>((k_step >> 4) & 0x3fffu) << 16) |
+         (static_cast<uint64_t>((mn_step >> 4) & 0x3fffu) << 32) | (1ull << 46);
+}
+
+__device__ __forceinline__ void mma(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, bool add) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+      ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(add ? 1u : 0u) : "memory");
+}
+
+// Waits until phase `parity` of the barrier is complete; false after a second.
+__device__ __forceinline__ bool wait_bounded(uint32_t bar, uint32_t parity) {
+  unsigned long long t0 = 0;
+  for (int i = 0;; ++i) {
+    uint32_t done;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(done) : "r"(bar), "r"(parity), "r"(10000u /* ns */) : "memory");
+    if (done) return true;
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    if (i == 0) t0 = t;
+    if (t - t0 > 1000000000ull) return false;
+  }
+}
+
+template <typename T> __device__ __forceinline__ uint32_t narrow2(float a, float b);
+template <> __device__ __forceinline__ uint32_t narrow2<__nv_bfloat16>(float a, float b) {
+  const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
+  return *reinterpret_cast<const uint32_t*>(&v);
+}
+template <> __device__ __forceinline__ uint32_t narrow2<__half>(float a, float b) {
+  const __half2 v = __floats2half2_rn(a, b);
+  return *reinterpret_cast<const uint32_t*>(&v);
+}
+
+struct StemShape {
+  int n, h, w, ho, wo, channels;  // channels: of the output
+  int64_t tiles;
+  int tiles_h, tiles_w;
+  int64_t ws_o, ws_c, ws_h, ws_w;  // strides of the weights
+};
+
+struct TileAt {
+  int n, i, j;  // image, first output row and column
+};
+__device__ __forceinline__ TileAt tile_at(const StemShape& s, int64_t t) {
+  const int per_image = s.tiles_h * s.tiles_w;
+  const int n = static_cast<int>(t / per_image), r = static_cast<int>(t % per_image);
+  return {n, r / s.tiles_w * TILE_H, r % s.tiles_w * TILE_W};
+}
+
+// The 12 values of this thread's block of the patch (zero outside the image).
+__device__ __forceinline__ void load_block(const uint16_t* __restrict__ x, const StemShape& s,
+                                           const TileAt& t, uint16_t (&v)[12]) {
+#pragma unroll
+  for (int i = 0; i < 12; ++i) v[i] = 0;
+  const int r = threadIdx.x / PATCH_W, c = threadIdx.x % PATCH_W;
+  if (r >= PATCH_H) return;
+  const int row = 2 * (t.i + r - 2), col = 2 * (t.j + c - 2);
+#pragma unroll
+  for (int dr = 0; dr < 2; ++dr)
+#pragma unroll
+    for (int dc = 0; dc < 2; ++dc)
+      if (row + dr >= 0 && row + dr < s.h && col + dc >= 0 && col + dc < s.w) {
+        const uint16_t* p =
+            x + ((static_cast<int64_t>(t.n) * s.h + row + dr) * s.w + col + dc) * 3;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) v[(dr * 2 + dc) * 3 + k] = __ldg(p + k);
+      }
+}
+
+template <typename T>
+__global__ void __launch_bounds__(THREADS, 4)
+stem_conv_forward_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict__ weight,
+                         uint16_t* __restrict__ y, const StemShape s, const uint32_t idesc,
+                         const uint32_t tmem_columns, int* status) {
+  extern __shared__ __align__(128) unsigned char smem[];
+  __shared__ __align__(8) uint64_t s_bar;
+  __shared__ uint32_t s_tmem;
+  const int C = s.channels;
+  unsigned char* patch = smem;                                // [2 planes][PATCH][16 bytes]
+  unsigned char* weights = smem + 2 * PLANE_BYTES;            // [K_CORES][C][16 bytes]
+  unsigned char* staged = weights + K_CORES * C * 16;         // [128 pixels][pitch]
+  const int pitch = C * 2 + 16;  // rows 16 bytes apart modulo 128: no bank conflicts
+  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+
+  int64_t tile = blockIdx.x;
+  uint16_t v[12];
+  load_block(x, s, tile_at(s, tile), v);  // the grid is no larger than the tiles
+  for (int e = threadIdx.x; e < K_CORES * C * 8; e += THREADS) {
+    const int k = e % 8, o = e / 8 % C, core = e / 8 / C;
+    const int c16 = core % 2 * 8 + k, tap = core / 2;
+    const int kh = tap / 4 * 2 + c16 / 6 - 1, kw = tap % 4 * 2 + c16 / 3 % 2 - 1;
+    uint16_t value = 0;
+    if (c16 < 12 && kh >= 0 && kw >= 0)
+      value = __ldg(weight + o * s.ws_o + c16 % 3 * s.ws_c + kh * s.ws_h + kw * s.ws_w);
+    reinterpret_cast<uint16_t*>(weights)[e] = value;
+  }
+  if (threadIdx.x == 0) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&s_bar)) : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
+                 ::"r"(smem_addr(&s_tmem)), "r"(tmem_columns) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = s_tmem;
+
+  uint32_t parity = 0;
+  for (; tile < s.tiles; tile += gridDim.x) {
+    if (threadIdx.x < PATCH) {
+      auto two = [&](int i) {
+        return static_cast<uint32_t>(v[i]) | (static_cast<uint32_t>(v[i + 1]) << 16);
+      };
+      reinterpret_cast<uint4*>(patch)[threadIdx.x] = make_uint4(two(0), two(2), two(4), two(6));
+      reinterpret_cast<uint4*>(patch + PLANE_BYTES)[threadIdx.x] =
+          make_uint4(two(8), two(10), 0u, 0u);
+    }
+    // What the threads wrote is read by the tensor core's proxy.
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+      for (int tap = 0; tap < TAPS; ++tap)
+        mma(tmem,
+            operand(smem_addr(patch) + (tap / 4 * PATCH_W + tap % 4) * 16, PLANE_BYTES,
+                    PATCH_W * 16),
+            operand(smem_addr(weights) + tap * 2 * C * 16, C * 16, 128), idesc, tap > 0);
+      asm volatile(
+          "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
+          ::"r"(smem_addr(&s_bar)) : "memory");
+    }
+    const TileAt at = tile_at(s, tile);
+    if (tile + gridDim.x < s.tiles) load_block(x, s, tile_at(s, tile + gridDim.x), v);
+    const bool ok = wait_bounded(smem_addr(&s_bar), parity);
+    parity ^= 1u;
+    if (__syncthreads_and(ok) == 0) {
+      if (threadIdx.x == 0) *reinterpret_cast<volatile int*>(status) = 1;
+      wait_bounded(smem_addr(&s_bar), parity ^ 1u);  // the products in flight
+      break;
+    }
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    // Warps w and w + 4 read the accumulators of pixels 32 (w % 4) ..., 16
+    // channels at a time in turn.
+    const int pixel = warp % 4 * 32 + lane;
+    for (int c0 = warp / 4 * 16; c0 < C; c0 += 32) {
+      uint32_t r[16];
+      asm volatile(
+          "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+          "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+          : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
+            "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]),
+            "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+          : "r"(tmem + (static_cast<uint32_t>(warp % 4 * 32) << 16) + c0));
+      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+      uint32_t o[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        o[i] = narrow2<T>(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]));
+      uint4* dst = reinterpret_cast<uint4*>(staged + pixel * pitch + c0 * 2);
+      dst[0] = make_uint4(o[0], o[1], o[2], o[3]);
+      dst[1] = make_uint4(o[4], o[5], o[6], o[7]);
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    const int per_pixel = C / 8;  // 16-byte pieces
+    for (int e = threadIdx.x; e < TILE_H * TILE_W * per_pixel; e += THREADS) {
+      const int px = e / per_pixel, piece = e % per_pixel;
+      const int i = at.i + px / TILE_W, j = at.j + px % TILE_W;
+      if (i < s.ho && j < s.wo)
+        reinterpret_cast<uint4*>(y)[((static_cast<int64_t>(at.n) * s.ho + i) * s.wo + j) *
+                                        per_pixel + piece] =
+            *reinterpret_cast<const uint4*>(staged + px * pitch + piece * 16);
+    }
+    // (`staged` is written again only after the next tile's two barriers.)
+  }
+  __syncthreads();
+  if (warp == 0)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;"
+                 ::"r"(tmem), "r"(tmem_columns));
+}
+
+// Host-visible word that a kernel sets when a wait ran out.
+int* StatusWord() {
+  static std::once_flag once;
+  static int* word = nullptr;
+  std::call_once(once, [] {
+    if (cudaHostAlloc(reinterpret_cast<void**>(&word), sizeof(int),
+                      cudaHostAllocMapped | cudaHostAllocPortable) == cudaSuccess)
+      *word = 0;
+    else
+      word = nullptr;
+  });
+  return word;
+}
+
+}  // namespace
+
+bool StemConvSupported(int channels) {
+  return channels >= 16 && channels <= 128 && channels % 16 == 0;
+}
+
+cudaError_t LaunchStemConvForward(const void* x, const void* weight, const int64_t* weight_strides,
+                                  void* y, int n, int h, int w, int channels, bool bf16,
+                                  cudaStream_t stream) {
+  if (!StemConvSupported(channels) || n < 1 || h < 1 || w < 1) return cudaErrorInvalidValue;
+  int* status = StatusWord();
+  if (status == nullptr) return cudaErrorMemoryAllocation;
+  if (*reinterpret_cast<volatile int*>(status) != 0) return cudaErrorLaunchTimeout;
+  StemShape s;
+  s.n = n;
+  s.h = h;
+  s.w = w;
+  s.ho = (h - 1) / 2 + 1;
+  s.wo = (w - 1) / 2 + 1;
+  s.channels = channels;
+  s.tiles_h = (s.ho + TILE_H - 1) / TILE_H;
+  s.tiles_w = (s.wo + TILE_W - 1) / TILE_W;
+  s.tiles = static_cast<int64_t>(n) * s.tiles_h * s.tiles_w;
+  s.ws_o = weight_strides[0];
+  s.ws_c = weight_strides[1];
+  s.ws_h = weight_strides[2];
+  s.ws_w = weight_strides[3];
+  // fp32 accumulators, 16-bit operands, both K-major, M = 128, N = channels.
+  const uint32_t type = bf16 ? 1u : 0u;
+  const uint32_t idesc = (1u << 4) | (type << 7) | (type << 10) |
+                         (static_cast<uint32_t>(channels >> 3) << 17) | ((128u >> 4) << 24);
+  uint32_t columns = 32;  // a power of two; four CTAs share the SM's 512
+  while (columns < static_cast<uint32_t>(channels)) columns *= 2;
+  const int smem = 2 * PLANE_BYTES + K_CORES * channels * 16 +
+                   TILE_H * TILE_W * (channels * 2 + 16);
+  auto kernel = bf16 ? stem_conv_forward_kernel<__nv_bfloat16> : stem_conv_forward_kernel<__half>;
+  cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (err != cudaSuccess) return err;
+  const unsigned grid = static_cast<unsigned>(s.tiles < 148 * 4 ? s.tiles : 148 * 4);
+  CountKernelLaunches(1);
+  kernel<<<grid, THREADS, smem, stream>>>(static_cast<const uint16_t*>(x),
+                                          static_cast<const uint16_t*>(weight),
+                                          static_cast<uint16_t*>(y), s, idesc, columns, status);
+  return cudaGetLastError();
+}
+
+}  // namespace kern
+}  // namespace hvd

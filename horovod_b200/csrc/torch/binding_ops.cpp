@@ -217,6 +217,31 @@ void BindModelOps(py::module_& m) {
     return dx;
   });
 
+  // ---- 7x7 / stride 2 convolution of 3 channels (channels-last, 16-bit) ------
+  m.def("stem_conv_supported", [](int64_t channels) {
+    return kern::StemConvSupported(static_cast<int>(channels));
+  });
+  m.def("stem_conv_forward", [](const at::Tensor& x, const at::Tensor& weight) {
+    CheckActivations(x, "x");
+    const int64_t N = x.size(0), H = x.size(2), W = x.size(3), C = weight.size(0);
+    TORCH_CHECK(weight.is_cuda() && weight.device() == x.device() &&
+                    weight.scalar_type() == x.scalar_type() && weight.dim() == 4 &&
+                    weight.size(1) == 3 && weight.size(2) == 7 && weight.size(3) == 7 &&
+                    x.size(1) == 3,
+                "stem_conv_forward: x must have 3 channels and weight the shape [C, 3, 7, 7]");
+    TORCH_CHECK(kern::StemConvSupported(static_cast<int>(C)),
+                "stem_conv_forward does not support ", C, " channels");
+    c10::cuda::CUDAGuard guard(x.device());
+    at::Tensor y = at::empty({N, C, (H - 1) / 2 + 1, (W - 1) / 2 + 1}, x.options(),
+                             at::MemoryFormat::ChannelsLast);
+    cudaError_t err = kern::LaunchStemConvForward(
+        x.data_ptr(), weight.data_ptr(), weight.strides().data(), y.data_ptr(),
+        static_cast<int>(N), static_cast<int>(H), static_cast<int>(W), static_cast<int>(C),
+        x.scalar_type() == at::kBFloat16, at::cuda::getCurrentCUDAStream());
+    TORCH_CHECK(err == cudaSuccess, "stem convolution: ", cudaGetErrorString(err));
+    return y;
+  });
+
   // ---- multi-tensor SGD ------------------------------------------------------
   // One step over a parameter list, in one launch per 256 tensors. bufs holds
   // a momentum buffer (or None) per parameter; it is empty when momentum is 0.

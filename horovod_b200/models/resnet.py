@@ -9,6 +9,7 @@ import torch.nn as nn
 
 from horovod_b200.ops.batch_norm import BatchNormAct2d
 from horovod_b200.ops.pooling import MaxPool3x3s2
+from horovod_b200.ops.stem_conv import StemConv2d
 
 
 class Bottleneck(nn.Module):
@@ -39,7 +40,7 @@ class ResNet(nn.Module):
     def __init__(self, layers=(3, 4, 6, 3), num_classes=1000, width=64):
         super().__init__()
         self.inplanes = width
-        self.conv1 = nn.Conv2d(3, width, 7, stride=2, padding=3, bias=False)
+        self.conv1 = StemConv2d(3, width, 7, stride=2, padding=3, bias=False)
         self.bn1 = BatchNormAct2d(width, relu=True)
         self.maxpool = MaxPool3x3s2()  # 3x3, stride 2, padding 1
         self.layer1 = self._make_layer(width, layers[0])

@@ -1,0 +1,67 @@
+"""The first convolution of a ResNet (7x7, stride 2, padding 3, 3 channels) for
+channels-last bf16/fp16 inputs on this library's tensor-core kernel
+(csrc/kernels/stem_conv.cu), with PyTorch's convolution everywhere else and
+for the gradients.
+
+``StemConv2d`` is an ``nn.Conv2d`` (same parameters and state_dict keys). The
+reference has no counterpart (it takes convolutions from the framework).
+"""
+import torch
+import torch.nn as nn
+from torch.autograd import forward_ad
+
+
+def _extension():
+    from horovod_b200 import _C
+    return _C
+
+
+class _StemConv(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, x, weight):
+        ctx.save_for_backward(x, weight)
+        return _extension().stem_conv_forward(x, weight)
+
+    @staticmethod
+    def backward(ctx, dy):
+        x, weight = ctx.saved_tensors
+        dx, dw, _ = torch.ops.aten.convolution_backward(
+            dy.to(x.dtype), x, weight, None, [2, 2], [3, 3], [1, 1], False, [0, 0], 1,
+            [ctx.needs_input_grad[0], ctx.needs_input_grad[1], False])
+        return dx, dw
+
+
+class StemConv2d(nn.Conv2d):
+    """``nn.Conv2d`` that runs the kernel where it can."""
+
+    def _kernel_dtype(self, x):
+        """The 16-bit type the convolution runs in, or None for PyTorch's own:
+        another geometry, memory format or type, and what a custom autograd
+        function cannot take part in."""
+        if not (x.is_cuda and x.dim() == 4 and x.size(1) == 3 and x.numel() > 0
+                and self.kernel_size == (7, 7) and self.stride == (2, 2)
+                and self.padding == (3, 3) and self.dilation == (1, 1) and self.groups == 1
+                and self.bias is None and self.padding_mode == "zeros"
+                and self.weight.device == x.device
+                and x.is_contiguous(memory_format=torch.channels_last)):
+            return None
+        if torch.is_autocast_enabled("cuda"):
+            dtype = torch.get_autocast_dtype("cuda")
+        elif x.dtype == self.weight.dtype:
+            dtype = x.dtype
+        else:
+            return None
+        if dtype not in (torch.bfloat16, torch.float16) or \
+                x.dtype not in (torch.float32, torch.bfloat16, torch.float16) or \
+                self.weight.dtype not in (torch.float32, torch.bfloat16, torch.float16):
+            return None
+        if torch.jit.is_tracing() or torch.compiler.is_compiling() or \
+                forward_ad._current_level >= 0 or torch._C._are_functorch_transforms_active():
+            return None
+        return dtype if _extension().stem_conv_supported(self.out_channels) else None
+
+    def forward(self, x):
+        dtype = self._kernel_dtype(x)
+        if dtype is None:
+            return super().forward(x)
+        return _StemConv.apply(x.to(dtype), self.weight.to(dtype))

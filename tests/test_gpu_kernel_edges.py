@@ -210,3 +210,48 @@ def test_compression_inside_the_kernel(hvd, name):
         out = hvd.allreduce(v, name="cmp.%s.%s" % (name, dtype), compression=compression,
                             op=hvd.Sum)
         assert out.dtype == dtype and torch.equal(out, v)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("shape,channels", [
+    ((1, 3, 1, 1), 16), ((2, 3, 33, 17), 64), ((3, 3, 32, 16), 48),  # one past a tile, a tile
+    ((2, 3, 31, 50), 128), ((5, 3, 97, 131), 64), ((40, 3, 224, 224), 64),  # several per CTA
+])
+def test_stem_convolution(shape, channels, dtype):
+    """Against the same convolution in 64 bits: fp32 accumulators, so what is
+    left is the rounding of the result."""
+    from horovod_b200.ops.stem_conv import StemConv2d
+    g = torch.Generator(device=_dev()).manual_seed(9)
+    conv = StemConv2d(3, channels, 7, stride=2, padding=3, bias=False).to(_dev())
+    conv = conv.to(memory_format=torch.channels_last)
+    x = torch.randn(shape, device=_dev(), generator=g).contiguous(
+        memory_format=torch.channels_last)
+    with torch.autocast("cuda", dtype=dtype):
+        assert conv._kernel_dtype(x) == dtype
+        y = conv(x)
+    assert y.dtype == dtype and y.is_contiguous(memory_format=torch.channels_last)
+    xd, wd = x.to(dtype).double(), conv.weight.detach().to(dtype).double()
+    want = F.conv2d(xd, wd, stride=2, padding=3)
+    # 147 products of at most |x| |w| each in fp32, then one rounding
+    size = F.conv2d(xd.abs(), wd.abs(), stride=2, padding=3)
+    eps = 2.0 ** (-8 if dtype == torch.bfloat16 else -11)
+    assert bool(((y.double() - want).abs() <= eps * want.abs() + 2e-5 * size + 6e-8).all())
+    dy = torch.randn(y.shape, device=_dev(), generator=g).to(dtype)
+    y.backward(dy)
+    dw = torch.nn.grad.conv2d_weight(xd, wd.shape, dy.double(), stride=2, padding=3)
+    assert (conv.weight.grad.double() - dw).norm() <= 1e-2 * dw.norm()
+    # fp32 without autocast is PyTorch's
+    assert conv._kernel_dtype(x) is None
+
+
+@pytest.mark.parametrize("momentum", [0.1, None])
+def test_batch_norm_counts_batches_once(momentum):
+    from horovod_b200.ops.batch_norm import BatchNormAct2d
+    bn = BatchNormAct2d(16, momentum=momentum).to(_dev())
+    x = torch.randn(2, 16, 5, 5, device=_dev()).contiguous(memory_format=torch.channels_last)
+    for i, t in enumerate((x.bfloat16(), x, x.half())):  # the kernel, PyTorch, the kernel
+        bn(t)
+        assert int(bn.num_batches_tracked) == i + 1
+    bn.eval()
+    bn(x.bfloat16())
+    assert int(bn.num_batches_tracked) == 3
