@@ -395,6 +395,12 @@ bool StemConvSupported(int channels);
 cudaError_t LaunchStemConvForward(const void* x, const void* weight, const int64_t* weight_strides,
                                   void* y, int n, int h, int w, int channels, bool bf16,
                                   cudaStream_t stream);
+// Gradient of the weights (16-bit, with the given strides) from x and dy.
+// partial: scratch of StemConvWgradCtas() * 256 * channels floats.
+int StemConvWgradCtas(int n, int h, int w, int channels);
+cudaError_t LaunchStemConvWgrad(const void* x, const void* dy, float* partial, void* dw,
+                                const int64_t* weight_strides, int n, int h, int w, int channels,
+                                bool bf16, cudaStream_t stream);
 
 // Multi-tensor SGD step in one launch (torch.optim.SGD arithmetic: weight
 // decay added to the gradient, momentum buffer b = momentum * b + (1 -

@@ -1,6 +1,6 @@
 // The first convolution of a ResNet, 7x7 / stride 2 / padding 3 on 3 channels,
-// forward, channels-last 16-bit, as an implicit GEMM on the 5th-generation
-// tensor cores. cuDNN has no sm_100 kernel for 3 channels and pads them to 4
+// forward and gradient of the weights, channels-last 16-bit, as an implicit
+// GEMM on the 5th-generation tensor cores. cuDNN has no sm_100 kernel for 3 channels and pads them to 4
 // for one of an older architecture.
 //
 // Input pixels are taken in 2 x 2 blocks of 12 values (16 with padding): the
@@ -43,8 +43,8 @@ __device__ __forceinline__ uint32_t smem_addr(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
-// K-major operand without a swizzle: `k_step` bytes between the two core
-// matrices of K = 16, `mn_step` bytes between groups of 8 rows.
+// Operand without a swizzle: `k_step` bytes between the two core matrices of
+// K = 16, `mn_step` bytes between groups of 8 rows (columns).
 __device__ __forceinline__ uint64_t operand(uint32_t addr, uint32_t k_step, uint32_t mn_step) {
   return static_cast<uint64_t>((addr >> 4) & 0x3fffu) |
          (static_cast<uint64_t>((k_step >> 4) & 0x3fffu) << 16) |
@@ -102,27 +102,46 @@ __device__ __forceinline__ TileAt tile_at(const StemShape& s, int64_t t) {
   return {n, r / s.tiles_w * TILE_H, r % s.tiles_w * TILE_W};
 }
 
-// The 12 values of this thread's block of the patch (zero outside the image).
+// The 12 values of this thread's block of the patch, two per word (zero
+// outside the image). PAIRS: the images are an even number of pixels wide and
+// start on a 4-byte boundary, so the six values of a block's row are three
+// words, all of them inside the image or none.
+template <bool PAIRS>
 __device__ __forceinline__ void load_block(const uint16_t* __restrict__ x, const StemShape& s,
-                                           const TileAt& t, uint16_t (&v)[12]) {
+                                           const TileAt& t, uint32_t (&v)[6]) {
 #pragma unroll
-  for (int i = 0; i < 12; ++i) v[i] = 0;
+  for (int i = 0; i < 6; ++i) v[i] = 0u;
   const int r = threadIdx.x / PATCH_W, c = threadIdx.x % PATCH_W;
   if (r >= PATCH_H) return;
   const int row = 2 * (t.i + r - 2), col = 2 * (t.j + c - 2);
 #pragma unroll
-  for (int dr = 0; dr < 2; ++dr)
+  for (int dr = 0; dr < 2; ++dr) {
+    if (row + dr < 0 || row + dr >= s.h) continue;
+    const uint16_t* p = x + ((static_cast<int64_t>(t.n) * s.h + row + dr) * s.w + col) * 3;
+    if (PAIRS) {
+      if (col >= 0 && col < s.w) {
 #pragma unroll
-    for (int dc = 0; dc < 2; ++dc)
-      if (row + dr >= 0 && row + dr < s.h && col + dc >= 0 && col + dc < s.w) {
-        const uint16_t* p =
-            x + ((static_cast<int64_t>(t.n) * s.h + row + dr) * s.w + col + dc) * 3;
-#pragma unroll
-        for (int k = 0; k < 3; ++k) v[(dr * 2 + dc) * 3 + k] = __ldg(p + k);
+        for (int k = 0; k < 3; ++k)
+          v[dr * 3 + k] = __ldg(reinterpret_cast<const uint32_t*>(p) + k);
       }
+    } else {
+      uint32_t e[6] = {0u, 0u, 0u, 0u, 0u, 0u};
+#pragma unroll
+      for (int k = 0; k < 6; ++k)
+        if (col + k / 3 >= 0 && col + k / 3 < s.w) e[k] = __ldg(p + k);
+#pragma unroll
+      for (int k = 0; k < 3; ++k) v[dr * 3 + k] = e[2 * k] | (e[2 * k + 1] << 16);
+    }
+  }
 }
 
-template <typename T>
+__device__ __forceinline__ void store_block(unsigned char* patch, const uint32_t (&v)[6]) {
+  if (threadIdx.x >= PATCH) return;
+  reinterpret_cast<uint4*>(patch)[threadIdx.x] = make_uint4(v[0], v[1], v[2], v[3]);
+  reinterpret_cast<uint4*>(patch + PLANE_BYTES)[threadIdx.x] = make_uint4(v[4], v[5], 0u, 0u);
+}
+
+template <typename T, bool PAIRS>
 __global__ void __launch_bounds__(THREADS, 4)
 stem_conv_forward_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict__ weight,
                          uint16_t* __restrict__ y, const StemShape s, const uint32_t idesc,
@@ -133,13 +152,11 @@ stem_conv_forward_kernel(const uint16_t* __restrict__ x, const uint16_t* __restr
   const int C = s.channels;
   unsigned char* patch = smem;                                // [2 planes][PATCH][16 bytes]
   unsigned char* weights = smem + 2 * PLANE_BYTES;            // [K_CORES][C][16 bytes]
-  unsigned char* staged = weights + K_CORES * C * 16;         // [128 pixels][pitch]
-  const int pitch = C * 2 + 16;  // rows 16 bytes apart modulo 128: no bank conflicts
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
 
   int64_t tile = blockIdx.x;
-  uint16_t v[12];
-  load_block(x, s, tile_at(s, tile), v);  // the grid is no larger than the tiles
+  uint32_t v[6];
+  load_block<PAIRS>(x, s, tile_at(s, tile), v);  // the grid is no larger than the tiles
   for (int e = threadIdx.x; e < K_CORES * C * 8; e += THREADS) {
     const int k = e % 8, o = e / 8 % C, core = e / 8 / C;
     const int c16 = core % 2 * 8 + k, tap = core / 2;
@@ -165,14 +182,7 @@ stem_conv_forward_kernel(const uint16_t* __restrict__ x, const uint16_t* __restr
 
   uint32_t parity = 0;
   for (; tile < s.tiles; tile += gridDim.x) {
-    if (threadIdx.x < PATCH) {
-      auto two = [&](int i) {
-        return static_cast<uint32_t>(v[i]) | (static_cast<uint32_t>(v[i + 1]) << 16);
-      };
-      reinterpret_cast<uint4*>(patch)[threadIdx.x] = make_uint4(two(0), two(2), two(4), two(6));
-      reinterpret_cast<uint4*>(patch + PLANE_BYTES)[threadIdx.x] =
-          make_uint4(two(8), two(10), 0u, 0u);
-    }
+    store_block(patch, v);
     // What the threads wrote is read by the tensor core's proxy.
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncthreads();
@@ -189,7 +199,7 @@ stem_conv_forward_kernel(const uint16_t* __restrict__ x, const uint16_t* __restr
           ::"r"(smem_addr(&s_bar)) : "memory");
     }
     const TileAt at = tile_at(s, tile);
-    if (tile + gridDim.x < s.tiles) load_block(x, s, tile_at(s, tile + gridDim.x), v);
+    if (tile + gridDim.x < s.tiles) load_block<PAIRS>(x, s, tile_at(s, tile + gridDim.x), v);
     const bool ok = wait_bounded(smem_addr(&s_bar), parity);
     parity ^= 1u;
     if (__syncthreads_and(ok) == 0) {
@@ -200,7 +210,10 @@ stem_conv_forward_kernel(const uint16_t* __restrict__ x, const uint16_t* __restr
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     // Warps w and w + 4 read the accumulators of pixels 32 (w % 4) ..., 16
     // channels at a time in turn.
+    // A thread's 16 channels are one 32-byte sector of the output.
     const int pixel = warp % 4 * 32 + lane;
+    const int i = at.i + pixel / TILE_W, j = at.j + pixel % TILE_W;
+    uint16_t* out = y + ((static_cast<int64_t>(at.n) * s.ho + i) * s.wo + j) * C;
     for (int c0 = warp / 4 * 16; c0 < C; c0 += 32) {
       uint32_t r[16];
       asm volatile(
@@ -213,29 +226,181 @@ stem_conv_forward_kernel(const uint16_t* __restrict__ x, const uint16_t* __restr
       asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
       uint32_t o[8];
 #pragma unroll
-      for (int i = 0; i < 8; ++i)
-        o[i] = narrow2<T>(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]));
-      uint4* dst = reinterpret_cast<uint4*>(staged + pixel * pitch + c0 * 2);
-      dst[0] = make_uint4(o[0], o[1], o[2], o[3]);
-      dst[1] = make_uint4(o[4], o[5], o[6], o[7]);
-    }
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    const int per_pixel = C / 8;  // 16-byte pieces
-    for (int e = threadIdx.x; e < TILE_H * TILE_W * per_pixel; e += THREADS) {
-      const int px = e / per_pixel, piece = e % per_pixel;
-      const int i = at.i + px / TILE_W, j = at.j + px % TILE_W;
+      for (int k = 0; k < 8; ++k)
+        o[k] = narrow2<T>(__uint_as_float(r[2 * k]), __uint_as_float(r[2 * k + 1]));
       if (i < s.ho && j < s.wo)
-        reinterpret_cast<uint4*>(y)[((static_cast<int64_t>(at.n) * s.ho + i) * s.wo + j) *
-                                        per_pixel + piece] =
-            *reinterpret_cast<const uint4*>(staged + px * pitch + piece * 16);
+        asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
+                     ::"l"(out + c0), "r"(o[0]), "r"(o[1]), "r"(o[2]), "r"(o[3]), "r"(o[4]),
+                     "r"(o[5]), "r"(o[6]), "r"(o[7]) : "memory");
     }
-    // (`staged` is written again only after the next tile's two barriers.)
+    // The next tile's products wait for these reads (the barrier above).
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   }
   __syncthreads();
   if (warp == 0)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;"
                  ::"r"(tmem), "r"(tmem_columns));
+}
+
+// ---- gradient of the weights ------------------------------------------------
+// D[(tap, channel), o] = sum over output pixels of block value x gradient: the
+// same patch is the M operand (M along channels and taps, K along pixels, both
+// "MN-major"), the gradients of the tile's pixels are the N operand. M groups
+// lie 16 bytes apart, so one M = 128 operand covers 16 consecutive blocks: the
+// four taps of a kernel row (groups 0 .. 3) and of the next one (11 .. 14, a
+// patch row further on); the other groups multiply values that nobody reads.
+// Two pairs of kernel rows x two planes make four accumulators, which stay in
+// tensor memory over all tiles of the CTA; each CTA leaves its sums in
+// `partial` ([CTA][tap][16 channels][o], fp32) and a second kernel adds them
+// up. Two buffers: the next tile is stored while this one is multiplied.
+
+constexpr int DY_PLANE = TILE_H * TILE_W * 16 + 16;  // 16 bytes off: no bank conflicts
+constexpr int PATCH_BYTES = (2 * PLANE_BYTES + 127) / 128 * 128;
+constexpr int DY_PIECES = 8;  // 16-byte pieces per thread at 128 channels
+
+template <bool PAIRS>
+__global__ void __launch_bounds__(THREADS, 2)
+stem_conv_wgrad_kernel(const uint16_t* __restrict__ x, const uint4* __restrict__ dy,
+                       float* __restrict__ partial, const StemShape s, const uint32_t idesc,
+                       const uint32_t tmem_columns, int* status) {
+  extern __shared__ __align__(128) unsigned char smem[];
+  __shared__ __align__(8) uint64_t s_bar[2];
+  __shared__ uint32_t s_tmem;
+  const int C = s.channels, per_pixel = C / 8;
+  const int buffer_bytes = PATCH_BYTES + (per_pixel * DY_PLANE + 127) / 128 * 128;
+  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+
+  uint32_t v[6];
+  uint4 d[DY_PIECES];
+  auto load = [&](int64_t tile) {
+    const TileAt at = tile_at(s, tile);
+    load_block<PAIRS>(x, s, at, v);
+#pragma unroll
+    for (int k = 0; k < DY_PIECES; ++k) {
+      const int e = threadIdx.x + k * THREADS;
+      const int px = e / per_pixel, i = at.i + px / TILE_W, j = at.j + px % TILE_W;
+      d[k] = make_uint4(0u, 0u, 0u, 0u);
+      if (px < TILE_H * TILE_W && i < s.ho && j < s.wo)
+        d[k] = __ldg(dy + ((static_cast<int64_t>(at.n) * s.ho + i) * s.wo + j) * per_pixel +
+                     e % per_pixel);
+    }
+  };
+  int64_t tile = blockIdx.x;
+  load(tile);  // the grid is no larger than the tiles
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < 2; ++i)
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&s_bar[i])) : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
+                 ::"r"(smem_addr(&s_tmem)), "r"(tmem_columns) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = s_tmem;
+
+  bool ok = true;
+  uint32_t issued = 0;  // tiles given to the tensor cores
+  for (; tile < s.tiles; tile += gridDim.x, ++issued) {
+    const uint32_t buffer = issued & 1u, use = issued >> 1;
+    unsigned char* patch = smem + buffer * buffer_bytes;
+    unsigned char* grads = patch + PATCH_BYTES;
+    if (use > 0) ok = wait_bounded(smem_addr(&s_bar[buffer]), (use - 1) & 1u);
+    if (__syncthreads_and(ok) == 0) break;
+    store_block(patch, v);
+#pragma unroll
+    for (int k = 0; k < DY_PIECES; ++k) {
+      const int e = threadIdx.x + k * THREADS;
+      if (e < TILE_H * TILE_W * per_pixel)
+        *reinterpret_cast<uint4*>(grads + e % per_pixel * DY_PLANE + e / per_pixel * 16) = d[k];
+    }
+    if (tile + gridDim.x < s.tiles) load(tile + gridDim.x);
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      for (int k = 0; k < TILE_H / 2; ++k)  // 16 pixels: two rows of the tile
+#pragma unroll
+        for (int acc = 0; acc < 4; ++acc)   // kernel rows 2 (acc / 2) and + 1, plane acc % 2
+          mma(tmem + acc * C,
+              operand(smem_addr(patch) + acc % 2 * PLANE_BYTES +
+                          (k * 2 + acc / 2 * 2) * PATCH_W * 16, PATCH_W * 16, 16),
+              operand(smem_addr(grads) + k * 256, 128, DY_PLANE), idesc, issued > 0 || k > 0);
+      asm volatile(
+          "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
+          ::"r"(smem_addr(&s_bar[buffer])) : "memory");
+    }
+  }
+  // The last tile of each buffer.
+  for (uint32_t b = 0; b < 2; ++b) {
+    const uint32_t uses = (issued + 1 - b) / 2;
+    if (uses > 0 && !wait_bounded(smem_addr(&s_bar[b]), (uses - 1) & 1u)) ok = false;
+  }
+  ok = __syncthreads_and(ok) != 0;
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  if (!ok) {
+    if (threadIdx.x == 0) *reinterpret_cast<volatile int*>(status) = 1;
+  } else {
+    const int m = warp % 4 * 32 + lane, group = m / 8;
+    const bool useful = group < 4 || (group >= 11 && group < 15);
+    for (int c0 = warp / 4 * 16; c0 < 4 * C; c0 += 32) {
+      uint32_t r[16];
+      asm volatile(
+          "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+          "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+          : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
+            "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]),
+            "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+          : "r"(tmem + (static_cast<uint32_t>(warp % 4 * 32) << 16) + c0));
+      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+      const int acc = c0 / C, channel = acc % 2 * 8 + m % 8;
+      const int tap = (acc / 2 * 2 + group / 11) * 4 + group % 11;
+      if (useful && channel < 12) {
+        uint4* out = reinterpret_cast<uint4*>(
+            partial + ((static_cast<int64_t>(blockIdx.x) * TAPS + tap) * 16 + channel) * C +
+            c0 % C);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          out[i] = make_uint4(r[4 * i], r[4 * i + 1], r[4 * i + 2], r[4 * i + 3]);
+      }
+    }
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == 0)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;"
+                 ::"r"(tmem), "r"(tmem_columns));
+}
+
+// dw[o][c][kh][kw] = sum of the CTAs' partial sums, one CTA per (c, kh, kw):
+// threads (o, slice of the CTAs), in fp32 within a slice and in fp64 across.
+template <typename T>
+__global__ void __launch_bounds__(THREADS)
+stem_conv_wgrad_sum_kernel(const float* __restrict__ partial, uint16_t* __restrict__ dw, int ctas,
+                           const StemShape s) {
+  __shared__ double sums[THREADS];
+  const int C = s.channels, slices = THREADS / C;
+  const int c = blockIdx.x % 3, kw = blockIdx.x / 3 % 7, kh = blockIdx.x / 21;
+  const int tap = (kh + 1) / 2 * 4 + (kw + 1) / 2;
+  const int channel = ((kh + 1) % 2 * 2 + (kw + 1) % 2) * 3 + c;
+  const int o = threadIdx.x % C, slice = threadIdx.x / C;
+  float sum = 0.f;
+  if (slice < slices) {
+    const float* p = partial + (static_cast<int64_t>(tap) * 16 + channel) * C + o;
+#pragma unroll 8
+    for (int b = slice; b < ctas; b += slices) sum += __ldg(p + static_cast<int64_t>(b) * 256 * C);
+  }
+  sums[threadIdx.x] = sum;
+  __syncthreads();
+  if (threadIdx.x < C) {
+    double total = 0.0;
+    for (int i = 0; i < slices; ++i) total += sums[i * C + o];
+    const uint32_t v = narrow2<T>(static_cast<float>(total), 0.f);
+    dw[o * s.ws_o + c * s.ws_c + kh * s.ws_h + kw * s.ws_w] = static_cast<uint16_t>(v);
+  }
 }
 
 // Host-visible word that a kernel sets when a wait ran out.
@@ -258,13 +423,7 @@ bool StemConvSupported(int channels) {
   return channels >= 16 && channels <= 128 && channels % 16 == 0;
 }
 
-cudaError_t LaunchStemConvForward(const void* x, const void* weight, const int64_t* weight_strides,
-                                  void* y, int n, int h, int w, int channels, bool bf16,
-                                  cudaStream_t stream) {
-  if (!StemConvSupported(channels) || n < 1 || h < 1 || w < 1) return cudaErrorInvalidValue;
-  int* status = StatusWord();
-  if (status == nullptr) return cudaErrorMemoryAllocation;
-  if (*reinterpret_cast<volatile int*>(status) != 0) return cudaErrorLaunchTimeout;
+static StemShape MakeShape(int n, int h, int w, int channels, const int64_t* weight_strides) {
   StemShape s;
   s.n = n;
   s.h = h;
@@ -279,22 +438,86 @@ cudaError_t LaunchStemConvForward(const void* x, const void* weight, const int64
   s.ws_c = weight_strides[1];
   s.ws_h = weight_strides[2];
   s.ws_w = weight_strides[3];
+  return s;
+}
+
+// cudaSuccess when the kernels may run; *status is where they report to.
+static cudaError_t StemReady(int n, int h, int w, int channels, int** status) {
+  if (!StemConvSupported(channels) || n < 1 || h < 1 || w < 1) return cudaErrorInvalidValue;
+  *status = StatusWord();
+  if (*status == nullptr) return cudaErrorMemoryAllocation;
+  return *static_cast<volatile int*>(*status) != 0 ? cudaErrorLaunchTimeout : cudaSuccess;
+}
+
+cudaError_t LaunchStemConvForward(const void* x, const void* weight, const int64_t* weight_strides,
+                                  void* y, int n, int h, int w, int channels, bool bf16,
+                                  cudaStream_t stream) {
+  int* status = nullptr;
+  cudaError_t err = StemReady(n, h, w, channels, &status);
+  if (err != cudaSuccess) return err;
+  const StemShape s = MakeShape(n, h, w, channels, weight_strides);
   // fp32 accumulators, 16-bit operands, both K-major, M = 128, N = channels.
   const uint32_t type = bf16 ? 1u : 0u;
   const uint32_t idesc = (1u << 4) | (type << 7) | (type << 10) |
                          (static_cast<uint32_t>(channels >> 3) << 17) | ((128u >> 4) << 24);
   uint32_t columns = 32;  // a power of two; four CTAs share the SM's 512
   while (columns < static_cast<uint32_t>(channels)) columns *= 2;
-  const int smem = 2 * PLANE_BYTES + K_CORES * channels * 16 +
-                   TILE_H * TILE_W * (channels * 2 + 16);
-  auto kernel = bf16 ? stem_conv_forward_kernel<__nv_bfloat16> : stem_conv_forward_kernel<__half>;
-  cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  const int smem = 2 * PLANE_BYTES + K_CORES * channels * 16;
+  const bool pairs = w % 2 == 0 && reinterpret_cast<uintptr_t>(x) % 4 == 0;
+  auto kernel = bf16 ? (pairs ? stem_conv_forward_kernel<__nv_bfloat16, true>
+                              : stem_conv_forward_kernel<__nv_bfloat16, false>)
+                     : (pairs ? stem_conv_forward_kernel<__half, true>
+                              : stem_conv_forward_kernel<__half, false>);
+  err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (err != cudaSuccess) return err;
   const unsigned grid = static_cast<unsigned>(s.tiles < 148 * 4 ? s.tiles : 148 * 4);
   CountKernelLaunches(1);
   kernel<<<grid, THREADS, smem, stream>>>(static_cast<const uint16_t*>(x),
                                           static_cast<const uint16_t*>(weight),
                                           static_cast<uint16_t*>(y), s, idesc, columns, status);
+  return cudaGetLastError();
+}
+
+// The four accumulators' columns of tensor memory: a power of two.
+static uint32_t WgradColumns(int channels) {
+  uint32_t columns = 64;
+  while (columns < 4u * static_cast<uint32_t>(channels)) columns *= 2;
+  return columns;
+}
+
+int StemConvWgradCtas(int n, int h, int w, int channels) {
+  const int64_t strides[4] = {0, 0, 0, 0};
+  const int64_t tiles = MakeShape(n, h, w, channels, strides).tiles;
+  // Two per SM, or one where the accumulators take all of the tensor memory.
+  const int64_t most = 148 * (WgradColumns(channels) <= 256 ? 2 : 1);
+  return static_cast<int>(tiles < most ? tiles : most);
+}
+
+cudaError_t LaunchStemConvWgrad(const void* x, const void* dy, float* partial, void* dw,
+                                const int64_t* weight_strides, int n, int h, int w, int channels,
+                                bool bf16, cudaStream_t stream) {
+  int* status = nullptr;
+  cudaError_t err = StemReady(n, h, w, channels, &status);
+  if (err != cudaSuccess) return err;
+  const StemShape s = MakeShape(n, h, w, channels, weight_strides);
+  const int ctas = StemConvWgradCtas(n, h, w, channels);
+  // As above, but both operands MN-major.
+  const uint32_t type = bf16 ? 1u : 0u;
+  const uint32_t idesc = (1u << 4) | (type << 7) | (type << 10) | (1u << 15) | (1u << 16) |
+                         (static_cast<uint32_t>(channels >> 3) << 17) | ((128u >> 4) << 24);
+  const int smem = 2 * (PATCH_BYTES + (channels / 8 * DY_PLANE + 127) / 128 * 128);
+  const bool pairs = w % 2 == 0 && reinterpret_cast<uintptr_t>(x) % 4 == 0;
+  auto kernel = pairs ? stem_conv_wgrad_kernel<true> : stem_conv_wgrad_kernel<false>;
+  auto sum = bf16 ? stem_conv_wgrad_sum_kernel<__nv_bfloat16> : stem_conv_wgrad_sum_kernel<__half>;
+  err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (err != cudaSuccess) return err;
+  CountKernelLaunches(2);
+  kernel<<<ctas, THREADS, smem, stream>>>(static_cast<const uint16_t*>(x),
+                                          static_cast<const uint4*>(dy), partial, s, idesc,
+                                          WgradColumns(channels), status);
+  err = cudaGetLastError();
+  if (err != cudaSuccess) return err;
+  sum<<<3 * 7 * 7, THREADS, 0, stream>>>(partial, static_cast<uint16_t*>(dw), ctas, s);
   return cudaGetLastError();
 }
 

@@ -242,6 +242,36 @@ void BindModelOps(py::module_& m) {
     return y;
   });
 
+  // (x, dy, weight) -> gradient of the weight
+  m.def("stem_conv_wgrad", [](const at::Tensor& x, const at::Tensor& dy, const at::Tensor& weight) {
+    CheckActivations(x, "x");
+    CheckActivations(dy, "dy");
+    const int64_t N = x.size(0), H = x.size(2), W = x.size(3), C = weight.size(0);
+    TORCH_CHECK(weight.scalar_type() == x.scalar_type() && weight.device() == x.device() &&
+                    weight.dim() == 4 && weight.size(1) == 3 && weight.size(2) == 7 &&
+                    weight.size(3) == 7 && weight.is_non_overlapping_and_dense() &&
+                    x.size(1) == 3,
+                "stem_conv_wgrad: x must have 3 channels and weight the shape [C, 3, 7, 7]");
+    TORCH_CHECK(dy.scalar_type() == x.scalar_type() && dy.device() == x.device() &&
+                    dy.size(0) == N && dy.size(1) == C && dy.size(2) == (H - 1) / 2 + 1 &&
+                    dy.size(3) == (W - 1) / 2 + 1,
+                "stem_conv_wgrad: dy does not match x and weight");
+    TORCH_CHECK(kern::StemConvSupported(static_cast<int>(C)),
+                "stem_conv_wgrad does not support ", C, " channels");
+    c10::cuda::CUDAGuard guard(x.device());
+    const int64_t ctas = kern::StemConvWgradCtas(static_cast<int>(N), static_cast<int>(H),
+                                                 static_cast<int>(W), static_cast<int>(C));
+    at::Tensor partial = at::empty({ctas * 256 * C}, x.options().dtype(at::kFloat),
+                                   at::MemoryFormat::Contiguous);
+    at::Tensor dw = at::empty_like(weight);
+    cudaError_t err = kern::LaunchStemConvWgrad(
+        x.data_ptr(), dy.data_ptr(), partial.data_ptr<float>(), dw.data_ptr(),
+        dw.strides().data(), static_cast<int>(N), static_cast<int>(H), static_cast<int>(W),
+        static_cast<int>(C), x.scalar_type() == at::kBFloat16, at::cuda::getCurrentCUDAStream());
+    TORCH_CHECK(err == cudaSuccess, "stem convolution gradient: ", cudaGetErrorString(err));
+    return dw;
+  });
+
   // ---- multi-tensor SGD ------------------------------------------------------
   // One step over a parameter list, in one launch per 256 tensors. bufs holds
   // a momentum buffer (or None) per parameter; it is empty when momentum is 0.

@@ -1,7 +1,7 @@
 """The first convolution of a ResNet (7x7, stride 2, padding 3, 3 channels) for
 channels-last bf16/fp16 inputs on this library's tensor-core kernel
 (csrc/kernels/stem_conv.cu), with PyTorch's convolution everywhere else and
-for the gradients.
+for the gradient of the input.
 
 ``StemConv2d`` is an ``nn.Conv2d`` (same parameters and state_dict keys). The
 reference has no counterpart (it takes convolutions from the framework).
@@ -25,9 +25,17 @@ class _StemConv(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dy):
         x, weight = ctx.saved_tensors
-        dx, dw, _ = torch.ops.aten.convolution_backward(
-            dy.to(x.dtype), x, weight, None, [2, 2], [3, 3], [1, 1], False, [0, 0], 1,
-            [ctx.needs_input_grad[0], ctx.needs_input_grad[1], False])
+        need_x, need_w = ctx.needs_input_grad
+        # A gradient of this gradient is PyTorch's.
+        native = need_w and not torch.is_grad_enabled() and weight.dtype == dy.dtype
+        dx = dw = None
+        if need_x or (need_w and not native):
+            dx, dw, _ = torch.ops.aten.convolution_backward(
+                dy, x, weight, None, [2, 2], [3, 3], [1, 1], False, [0, 0], 1,
+                [need_x, need_w and not native, False])
+        if native:
+            dw = _extension().stem_conv_wgrad(
+                x, dy.contiguous(memory_format=torch.channels_last), weight)
         return dx, dw
 
 
