@@ -13,6 +13,11 @@
 // residual, y > 0 follows from x and the saved scale and shift by the
 // forward's own arithmetic; with one, the forward leaves one bit per element.
 //
+// Of 256 x 256 x 56 x 56 with a residual in bf16 (411 MB a tensor) the four
+// kernels take 70, 204, 138 and 270 us on a B200, 0.92-0.94 of the rate of a
+// plain copy of the bytes they move; with the output read back 78, 204, 194 and
+// 336 us.
+//
 // The second kernel of a pair walks the rows from the last to the first, so
 // what the first kernel read last is still in L2 when the second one starts,
 // and is launched while the first one still runs (programmatic dependent
@@ -436,33 +441,36 @@ bn_backward_apply_kernel(const T* __restrict__ dy, const uint8_t* __restrict__ s
   const int by = gridDim.y - 1 - blockIdx.y;
   int64_t r0, r1;
   cta_rows(M, by, &r0, &r1);
-  __shared__ __align__(16) float s_mean[BN_CTA_CHANNELS], s_scale[BN_CTA_CHANNELS],
-      s_shift[BN_CTA_CHANNELS], s_k1[BN_CTA_CHANNELS], s_k2[BN_CTA_CHANNELS];
+  // dx = scale * dz + kx * x + kc: the terms of the sums folded per channel, in
+  // fp64, which leaves registers for four rows in flight (256 x 64 x 112 x 112:
+  // 221 us, 272 with two rows and five values per channel).
+  __shared__ __align__(16) float s_scale[BN_CTA_CHANNELS], s_shift[BN_CTA_CHANNELS],
+      s_kx[BN_CTA_CHANNELS], s_kc[BN_CTA_CHANNELS];
   wait_for_previous();
   if (static_cast<int>(threadIdx.x) < t.txg * VEC) {
     const int64_t ch = static_cast<int64_t>(blockIdx.x) * t.txg * VEC + threadIdx.x;
     const double2 sum = total(sums, C, copies, ch);
     const double dz = sum.x, dz_xhat = sum.y;
     const float invstd = saved[C + ch];
-    s_mean[threadIdx.x] = saved[ch];
+    const float scale = (weight ? weight[ch] : 1.f) * invstd;
+    s_scale[threadIdx.x] = scale;
     s_shift[threadIdx.x] = saved[2 * static_cast<int64_t>(C) + ch];
-    s_scale[threadIdx.x] = (weight ? weight[ch] : 1.f) * invstd;
-    s_k1[threadIdx.x] = static_cast<float>(dz * inv_m);
-    s_k2[threadIdx.x] = static_cast<float>(dz_xhat * inv_m) * invstd;
+    const double kx = -static_cast<double>(scale) * invstd * dz_xhat * inv_m;
+    s_kx[threadIdx.x] = static_cast<float>(kx);
+    s_kc[threadIdx.x] = static_cast<float>(-scale * dz * inv_m - kx * saved[ch]);
     if (by == 0) {
       if (dweight) dweight[ch] = static_cast<float>(dz_xhat);
       if (dbias) dbias[ch] = static_cast<float>(dz);
     }
   }
   __syncthreads();
-  float mean[VEC], scale[VEC], shift[VEC], k1[VEC], k2[VEC];
-  load8(s_mean + t.tx * VEC, mean);
+  float scale[VEC], shift[VEC], kx[VEC], kc[VEC];
   load8(s_scale + t.tx * VEC, scale);
-  load8(s_k1 + t.tx * VEC, k1);
-  load8(s_k2 + t.tx * VEC, k2);
+  load8(s_kx + t.tx * VEC, kx);
+  load8(s_kc + t.tx * VEC, kc);
   if (MASK == MASK_X) load8(s_shift + t.tx * VEC, shift);
   const int64_t stride = static_cast<int64_t>(t.ty) * C;
-  for_rows_back<2>(t, r0, r1, C, [&](auto count, int64_t at0) {
+  for_rows_back<UNROLL>(t, r0, r1, C, [&](auto count, int64_t at0) {
     constexpr int U = decltype(count)::value;
     Vec8<T> d[U], a[U];
     uint32_t m[U];
@@ -483,8 +491,8 @@ bn_backward_apply_kernel(const T* __restrict__ dy, const uint8_t* __restrict__ s
         d[u].w[i] = masked<T, MASK>(i, d[u].w[i], f, m[u], scale, shift);
         const float2 z = Pair<T>::widen(d[u].pair(i));
         const int j = 2 * i, k = 2 * i + 1;
-        g.set(i, Pair<T>::narrow(scale[j] * (z.x - k1[j] - (f.x - mean[j]) * k2[j]),
-                                 scale[k] * (z.y - k1[k] - (f.y - mean[k]) * k2[k])));
+        g.set(i, Pair<T>::narrow(fmaf(scale[j], z.x, fmaf(kx[j], f.x, kc[j])),
+                                 fmaf(scale[k], z.y, fmaf(kx[k], f.y, kc[k]))));
       }
       stg16(dx + at, g);
       if (DRES) stg16(dres + at, d[u]);
