@@ -458,7 +458,9 @@ cudaError_t LaunchFusedAllreduce(const TensorList& tl, DataType dtype,
                                  double postscale, Algo algo, int num_ctas,
                                  const SymmCtx& ctx, cudaStream_t stream,
                                  const InlineTensors* inline_list) {
-  if (num_ctas < 1 || num_ctas > SYMM_MAX_BLOCKS) return cudaErrorInvalidValue;
+  // (One rank uses no flag words, of which there are SYMM_MAX_BLOCKS.)
+  if (num_ctas < 1 || (algo != Algo::LOCAL && num_ctas > SYMM_MAX_BLOCKS))
+    return cudaErrorInvalidValue;
   CountKernelLaunches(1);
   if (dtype == DataType::FLOAT32 && wire == DataType::BFLOAT16)
     return LaunchTyped<float, __nv_bfloat16>(tl, prescale, postscale, algo, num_ctas, ctx, stream, inline_list);

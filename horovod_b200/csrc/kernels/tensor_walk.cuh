@@ -1,9 +1,9 @@
 // Moving 16-byte vectors between a list of tensors and the linear "fused"
 // index space without ever materialising a separate fusion buffer pass:
-// gather_vec reads one wire vector's worth of elements straight from tensor
-// storage (scaling and casting on the way), scatter_vec writes one back.
-// Tensor starts are 16-byte aligned in the fused space, so a vector never
-// straddles two tensors; elements in the padding read as zero.
+// gather_range reads wire vectors straight from tensor storage (scaling and
+// casting on the way), scatter_range writes them back. Tensor starts are
+// 16-byte aligned in the fused space, so a vector never straddles two tensors;
+// elements in the padding read as zero.
 #pragma once
 
 #include <type_traits>
@@ -44,94 +44,11 @@ __device__ __forceinline__ int find_tensor(const TensorList& tl, int64_t elem) {
   return lo;
 }
 
-// Reads N = 16/sizeof(W) consecutive fused elements starting at `elem`
-// (a multiple of N). `cur` is a cursor into the tensor list that only moves
-// forward; initialise it with find_tensor().
-template <typename T, typename W, typename S>
-__device__ __forceinline__ uint4 gather_vec(const TensorList& tl, int& cur,
-                                            int64_t elem, S scale,
-                                            bool do_scale) {
-  constexpr int N = 16 / sizeof(W);
-  while (cur + 1 < tl.n && elem >= tl.offsets[cur + 1]) ++cur;
-  const int64_t local = elem - tl.offsets[cur];
-  const int64_t cnt = tl.counts[cur];
-  const T* src = static_cast<const T*>(tl.in[cur]);
-  WireVec<W> out;
-  out.raw = make_uint4(0, 0, 0, 0);
-  if (src == nullptr || local >= cnt) return out.raw;
-  src += local;
-  const bool full = local + N <= cnt;
-  if (full && (reinterpret_cast<uintptr_t>(src) & 15) == 0) {
-    constexpr int LOADS = N * sizeof(T) / 16;  // 1, or 2 for fp32 -> 16-bit
-    union {
-      uint4 raw[LOADS];
-      T e[N];
-    } in;
-#pragma unroll
-    for (int i = 0; i < LOADS; ++i)
-      in.raw[i] = ld16_stream(reinterpret_cast<const uint4*>(src) + i);
-    if constexpr (std::is_same<T, W>::value) {
-      if (!do_scale) return in.raw[0];
-    }
-#pragma unroll
-    for (int i = 0; i < N; ++i) out.e[i] = scale_cast<W>(in.e[i], scale, do_scale);
-  } else {
-    const int n = full ? N : static_cast<int>(cnt - local);
-#pragma unroll
-    for (int i = 0; i < N; ++i)
-      if (i < n) out.e[i] = scale_cast<W>(src[i], scale, do_scale);
-  }
-  return out.raw;
-}
-
-// Writes N fused elements starting at `elem` to their tensor (elements in
-// the padding are dropped).
-template <typename T, typename W, typename S>
-__device__ __forceinline__ void scatter_vec(const TensorList& tl, int& cur,
-                                            int64_t elem, uint4 raw, S scale,
-                                            bool do_scale) {
-  constexpr int N = 16 / sizeof(W);
-  while (cur + 1 < tl.n && elem >= tl.offsets[cur + 1]) ++cur;
-  const int64_t local = elem - tl.offsets[cur];
-  const int64_t cnt = tl.counts[cur];
-  T* dst = static_cast<T*>(tl.out[cur]);
-  if (dst == nullptr || local >= cnt) return;
-  dst += local;
-  WireVec<W> in;
-  in.raw = raw;
-  const bool full = local + N <= cnt;
-  if (full && (reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
-    constexpr int STORES = N * sizeof(T) / 16;
-    union {
-      uint4 raw[STORES];
-      T e[N];
-    } out;
-    if constexpr (std::is_same<T, W>::value) {
-      if (!do_scale) {
-        st16_stream(dst, raw);
-        return;
-      }
-    }
-#pragma unroll
-    for (int i = 0; i < N; ++i) out.e[i] = scale_cast<T>(in.e[i], scale, do_scale);
-#pragma unroll
-    for (int i = 0; i < STORES; ++i)
-      st16_stream(reinterpret_cast<uint4*>(dst) + i, out.raw[i]);
-  } else {
-    const int n = full ? N : static_cast<int>(cnt - local);
-#pragma unroll
-    for (int i = 0; i < N; ++i)
-      if (i < n) dst[i] = scale_cast<T>(in.e[i], scale, do_scale);
-  }
-}
-
 // ---- range walkers ---------------------------------------------------------
-// The per-vector functions above look the tensor up for every 16 bytes. The
-// walkers below are what the kernels use for bulk work: the CTA goes through
-// the tensors that overlap its range together, and inside one tensor runs a
-// tight, four-way unrolled vector loop with no per-vector bookkeeping, so
-// many loads are in flight per thread. `sink(v, raw)` receives fused vector
-// index v and its 16 bytes; `source(v)` provides them.
+// The CTA goes through the tensors that overlap its range together, and inside
+// one tensor runs a tight, four-way unrolled vector loop with no per-vector
+// bookkeeping, so many loads are in flight per thread. `sink(v, raw)` receives
+// fused vector index v and its 16 bytes; `source(v)` provides them.
 
 template <typename T, typename W, typename S>
 __device__ __forceinline__ uint4 convert_in(const uint4* raw, S scale, bool do_scale) {
