@@ -12,7 +12,7 @@
 // Backward: one thread owns 8 channels of a 2 x 2 block of input pixels and
 // walks down block rows. Such a block is covered by four windows, two of which
 // the next block down needs again: 2 loads of dy per 4 pixels instead of 9.
-// The ResNet-50 stem at batch 256 (256 x 64 x 112 x 112, bf16) takes 210 us
+// The ResNet-50 stem at batch 256 (256 x 64 x 112 x 112, bf16) takes 204 us
 // forward and backward on a B200; one output or input pixel per thread, with a
 // byte per index, took 521 us. The bytes that have to move (x, y, dy, dx) take
 // 159 us at the rate of a plain copy.
@@ -97,11 +97,12 @@ __device__ __forceinline__ Best row_best(const uint4* __restrict__ row, int w0, 
 // of two channels above.
 __host__ __device__ constexpr int nibble_shift(int i) { return (i >> 1) * 4 + (i & 1) * 16; }
 
+// Five CTAs per SM (48 registers): forward 109 us, 117 with four of 57.
 // I: type of the flat vector index. Tensors of fewer than 2^31 vectors (every
 // practical activation) use 32-bit index arithmetic: the divisions cost several
 // times the pooling itself when done in 64 bits.
 template <typename T, typename I>
-__global__ void __launch_bounds__(POOL_THREADS)
+__global__ void __launch_bounds__(POOL_THREADS, 5)
 maxpool3s2_forward_kernel(const uint4* __restrict__ x, uint4* __restrict__ y,
                           uint32_t* __restrict__ idx, I total, int H, int W, int C8, int Ho,
                           int Wo, int rows) {
