@@ -15,6 +15,11 @@
 // CTA; four CTAs per SM take turns with loading, multiplying and storing, and
 // a CTA loads the pixels of its next tile before it waits for the products.
 //
+// The 4 x 4 blocks of an output are 8 x 8 pixels; the first row and column of
+// them lie outside the 7 x 7 window and are multiplied by zero, which would make
+// NaN of an infinity or a NaN there. A tile whose patch holds one is therefore
+// computed by plain loops over the window (plain_tile).
+//
 // 256 images of 224 x 224 to 64 channels in bf16 on a B200: forward 191 us
 // (cuDNN 1486 us and a padding pass), gradient of the weights 236 us (cuDNN 750
 // us and a padding pass). The bytes of either pass take 75 us at the rate of a
@@ -90,6 +95,24 @@ template <> __device__ __forceinline__ uint32_t narrow2<__half>(float a, float b
   return *reinterpret_cast<const uint32_t*>(&v);
 }
 
+// Exponents of two 16-bit values in a word, and the lowest bit of each.
+template <typename T> struct Exponent;
+template <> struct Exponent<__nv_bfloat16> {
+  static constexpr uint32_t ALL = 0x7f807f80u, LOWEST = 0x00800080u;
+};
+template <> struct Exponent<__half> {
+  static constexpr uint32_t ALL = 0x7c007c00u, LOWEST = 0x04000400u;
+};
+
+// Whether a value of the block is an infinity or a NaN: only an exponent of
+// all ones carries into the sign's place.
+template <typename T> __device__ __forceinline__ bool not_finite(const uint32_t (&v)[6]) {
+  uint32_t carries = 0u;
+#pragma unroll
+  for (int i = 0; i < 6; ++i) carries |= (v[i] & Exponent<T>::ALL) + Exponent<T>::LOWEST;
+  return (carries & 0x80008000u) != 0u;
+}
+
 struct StemShape {
   int n, h, w, ho, wo, channels;  // channels: of the output
   int tiles, tiles_h, tiles_w;
@@ -143,6 +166,39 @@ __device__ __forceinline__ void store_block(unsigned char* patch, const uint32_t
   if (threadIdx.x >= PATCH) return;
   reinterpret_cast<uint4*>(patch)[threadIdx.x] = make_uint4(v[0], v[1], v[2], v[3]);
   reinterpret_cast<uint4*>(patch + PLANE_BYTES)[threadIdx.x] = make_uint4(v[4], v[5], 0u, 0u);
+}
+
+// Output pixels [rows][cols] of a tile from the patch and the weights in shared
+// memory, by loops over the pixels of each window and no others. y: the
+// tile's first pixel.
+template <typename T>
+__device__ __noinline__ void plain_tile(const unsigned char* patch, const unsigned char* weights,
+                                        uint16_t* y, int64_t row_pitch, int rows, int cols,
+                                        int C) {
+  constexpr int PIXELS = TILE_H * TILE_W;
+  const T* p = reinterpret_cast<const T*>(patch);
+  const T* w = reinterpret_cast<const T*>(weights);
+  const int pixel = threadIdx.x % PIXELS, i = pixel / TILE_W, j = pixel % TILE_W;
+  if (i >= rows || j >= cols) return;
+  uint16_t* out = y + i * row_pitch + j * C;
+  for (int c0 = threadIdx.x / PIXELS * 8; c0 < C; c0 += THREADS / PIXELS * 8) {
+    float sum[8] = {};
+#pragma unroll 1
+    for (int tap = 0; tap < TAPS; ++tap) {
+      const int block = (i + tap / 4) * PATCH_W + j + tap % 4;
+#pragma unroll 1
+      for (int c = 0; c < 12; ++c) {  // (row, column) of the pixel in its block, channel
+        if ((tap / 4 == 0 && c / 6 == 0) || (tap % 4 == 0 && c / 3 % 2 == 0)) continue;
+        const float value = static_cast<float>(p[(c / 8 * PATCH + block) * 8 + c % 8]);
+        const T* wc = w + ((tap * 2 + c / 8) * C + c0) * 8 + c % 8;
+#pragma unroll
+        for (int o = 0; o < 8; ++o) sum[o] = fmaf(value, static_cast<float>(wc[o * 8]), sum[o]);
+      }
+    }
+    *reinterpret_cast<uint4*>(out + c0) =
+        make_uint4(narrow2<T>(sum[0], sum[1]), narrow2<T>(sum[2], sum[3]),
+                   narrow2<T>(sum[4], sum[5]), narrow2<T>(sum[6], sum[7]));
+  }
 }
 
 template <typename T, bool PAIRS>
@@ -203,8 +259,8 @@ stem_conv_forward_kernel(const uint16_t* __restrict__ x, const uint16_t* __restr
     store_block(patch, v);
     // What the threads wrote is read by the tensor core's proxy.
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    __syncthreads();
-    if (threadIdx.x == 0) {
+    const bool plain = __syncthreads_or(not_finite<T>(v)) != 0;
+    if (threadIdx.x == 0 && !plain) {
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
       for (int tap = 0; tap < TAPS; ++tap)
@@ -220,6 +276,15 @@ stem_conv_forward_kernel(const uint16_t* __restrict__ x, const uint16_t* __restr
     if (tile + static_cast<int>(gridDim.x) < s.tiles) {
       next = tile_at(s, tile + gridDim.x);
       load_block<PAIRS>(x, s, next, v);
+    }
+    if (plain) {
+      const int64_t row_pitch = static_cast<int64_t>(s.wo) * C;
+      plain_tile<T>(patch, weights,
+                    y + (static_cast<int64_t>(at.n) * s.ho + at.i) * row_pitch + at.j * C,
+                    row_pitch, s.ho - at.i, s.wo - at.j, C);
+      __syncthreads();  // the next tile takes the patch's place
+      at = next;
+      continue;
     }
     const bool ok = wait_bounded(smem_addr(&s_bar), parity);
     parity ^= 1u;

@@ -244,6 +244,54 @@ def test_stem_convolution(shape, channels, dtype):
     assert conv._kernel_dtype(x) is None
 
 
+def _kinds(t):
+    """0 for finite values, 1 for NaN, 2 and 3 for the infinities."""
+    return t.isnan() * 1 + t.isposinf() * 2 + t.isneginf() * 3
+
+
+#: (row, column, channel) of what is not finite in a 67 x 45 image: even and odd
+#: rows and columns, corners, both sides of a tile's edge (rows 31 / 32, columns
+#: 15 / 16) and the last, partial tiles (from row 64 and column 32)
+_SPECIAL_PIXELS = [(8, 8, 0), (9, 8, 1), (8, 9, 2), (9, 9, 0), (0, 0, 1), (66, 44, 2), (31, 15, 0),
+                   (32, 16, 1), (31, 16, 2), (32, 15, 0), (65, 40, 1), (20, 43, 2), (64, 32, 0)]
+
+
+def _special_images(dtype, value):
+    """An image per special pixel, one with all of them and a finite one."""
+    g = torch.Generator().manual_seed(10)
+    x = torch.randn(len(_SPECIAL_PIXELS) + 2, 3, 67, 45, generator=g).to(dtype)
+    for n, (r, c, ch) in enumerate(_SPECIAL_PIXELS):
+        x[n, ch, r, c] = value
+        x[-2, ch, r, c] = value
+    return x.contiguous(memory_format=torch.channels_last)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("value", [float("inf"), float("-inf"), float("nan")])
+@pytest.mark.parametrize("channels", [16, 64])
+def test_stem_convolution_of_special_values(channels, value, dtype):
+    """Infinities and NaN reach the outputs whose 7 x 7 window holds them, and
+    no others."""
+    from horovod_b200 import _C
+    x = _special_images(dtype, value)
+    w = torch.randn(channels, 3, 7, 7, generator=torch.Generator().manual_seed(11)).to(dtype)
+    # five times over: more tiles than CTAs, so that both kinds follow each other
+    many = torch.cat([x] * 5).contiguous(memory_format=torch.channels_last)
+    y = _C.stem_conv_forward(many.to(_dev()), w.to(_dev())).cpu()
+    assert all(torch.equal(y[:len(x)].view(torch.int16), part.view(torch.int16))
+               for part in y.split(len(x)))
+    y = y[:len(x)]
+    want = F.conv2d(x.double(), w.double(), stride=2, padding=3)
+    assert torch.equal(_kinds(y), _kinds(want)) and bool(want[:-1].isfinite().logical_not().any())
+    finite = want.isfinite()
+    # as above: 147 products in fp32, then one rounding
+    size = F.conv2d(torch.nan_to_num(x.double().abs(), 0.0, 0.0, 0.0), w.double().abs(), stride=2,
+                    padding=3)
+    eps = 2.0 ** (-8 if dtype == torch.bfloat16 else -11)
+    bound = eps * want.abs() + 2e-5 * size + 6e-8
+    assert bool(((y.double() - want).abs() <= bound)[finite].all())
+
+
 @pytest.mark.parametrize("momentum", [0.1, None])
 def test_batch_norm_counts_batches_once(momentum):
     from horovod_b200.ops.batch_norm import BatchNormAct2d
