@@ -340,16 +340,72 @@ stem_conv_forward_kernel(const uint16_t* __restrict__ x, const uint16_t* __restr
 // tensor memory over all tiles of the CTA; each CTA leaves its sums in
 // `partial` ([CTA][tap][16 channels][o], fp32) and a second kernel adds them
 // up. Two buffers: the next tile is stored while this one is multiplied.
+//
+// A tile that reaches past the output has gradients of zero there, beside
+// pixels that may exist and make NaN of them where they are not finite. A CTA
+// whose sums hold an infinity or a NaN, in an image with such tiles, therefore
+// computes them again by plain loops over the output pixels that exist
+// (plain_sums). (To look at the pixels instead, inside the main loop, costs every
+// call 4 to 10%.)
 
 constexpr int DY_PLANE = TILE_H * TILE_W * 16 + 16;  // 16 bytes off: no bank conflicts
 constexpr int PATCH_BYTES = (2 * PLANE_BYTES + 127) / 128 * 128;
 constexpr int DY_PIECES = 8;  // 16-byte pieces per thread at 128 channels
 
-template <bool PAIRS>
+// The CTA's sums by plain loops. smem: room for a patch and the gradients of a
+// tile.
+template <typename T, bool PAIRS>
+__device__ __noinline__ void plain_sums(const uint16_t* __restrict__ x,
+                                        const uint4* __restrict__ dy, float* sums,
+                                        const StemShape& s, unsigned char* smem) {
+  const int C = s.channels, per_pixel = C / 8;
+  const T* p = reinterpret_cast<const T*>(smem);
+  uint4* grads = reinterpret_cast<uint4*>(smem + PATCH_BYTES);  // [pixel][C]
+  for (int tile = blockIdx.x; tile < s.tiles; tile += gridDim.x) {
+    const TileAt at = tile_at(s, tile);
+    const int rows = min(s.ho - at.i, TILE_H), cols = min(s.wo - at.j, TILE_W);
+    uint32_t v[6];
+    load_block<PAIRS>(x, s, at, v);
+    __syncthreads();  // the last readers of the buffer
+    store_block(smem, v);
+    for (int e = threadIdx.x; e < rows * cols * per_pixel; e += THREADS) {
+      const int px = e / per_pixel;
+      const int64_t i = static_cast<int64_t>(at.n) * s.ho + at.i + px / cols;
+      grads[e] = __ldg(dy + (i * s.wo + at.j + px % cols) * per_pixel + e % per_pixel);
+    }
+    __syncthreads();
+    // 8 output channels of a tap and an input channel at a time; a thread has
+    // the same ones in every tile.
+#pragma unroll 1
+    for (int e = threadIdx.x; e < TAPS * 12 * per_pixel; e += THREADS) {
+      const int piece = e % per_pixel, c = e / per_pixel % 12, tap = e / per_pixel / 12;
+      float* to = sums + (tap * 16 + c) * C + piece * 8;
+      float sum[8];
+#pragma unroll
+      for (int o = 0; o < 8; ++o) sum[o] = tile == static_cast<int>(blockIdx.x) ? 0.f : to[o];
+      const uint4* g = grads + piece;
+#pragma unroll 1
+      for (int i = 0; i < rows; ++i)
+#pragma unroll 1
+        for (int j = 0; j < cols; ++j, g += per_pixel) {
+          const int block = c / 8 * PATCH + (i + tap / 4) * PATCH_W + j + tap % 4;
+          const float value = static_cast<float>(p[block * 8 + c % 8]);
+          const uint4 raw = *g;
+          const T* d = reinterpret_cast<const T*>(&raw);
+#pragma unroll
+          for (int o = 0; o < 8; ++o) sum[o] = fmaf(value, static_cast<float>(d[o]), sum[o]);
+        }
+#pragma unroll
+      for (int o = 0; o < 8; ++o) to[o] = sum[o];
+    }
+  }
+}
+
+template <typename T, bool PAIRS>
 __global__ void __launch_bounds__(THREADS, 2)
 stem_conv_wgrad_kernel(const uint16_t* __restrict__ x, const uint4* __restrict__ dy,
-                       float* __restrict__ partial, const StemShape s, const uint32_t idesc,
-                       const uint32_t tmem_columns, int* status) {
+                       float* __restrict__ partial, const __grid_constant__ StemShape s,
+                       const uint32_t idesc, const uint32_t tmem_columns, int* status) {
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ __align__(8) uint64_t s_bar[2];
   __shared__ uint32_t s_tmem;
@@ -398,8 +454,9 @@ stem_conv_wgrad_kernel(const uint16_t* __restrict__ x, const uint4* __restrict__
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = s_tmem;
 
-  bool ok = true;
+  bool ok = true, finite = true;  // finite: this thread's sums
   uint32_t issued = 0;  // tiles given to the tensor cores
+  float* const sums = partial + static_cast<int64_t>(blockIdx.x) * TAPS * 16 * C;
   for (; tile < s.tiles; tile += gridDim.x, ++issued) {
     const uint32_t buffer = issued & 1u, use = issued >> 1;
     unsigned char* patch = smem + buffer * buffer_bytes;
@@ -452,20 +509,22 @@ stem_conv_wgrad_kernel(const uint16_t* __restrict__ x, const uint4* __restrict__
       const int acc = c0 / C, channel = acc % 2 * 8 + m % 8;
       const int tap = (acc / 2 * 2 + group / 11) * 4 + group % 11;
       if (useful && channel < 12) {
-        uint4* out = reinterpret_cast<uint4*>(
-            partial + ((static_cast<int64_t>(blockIdx.x) * TAPS + tap) * 16 + channel) * C +
-            c0 % C);
+        uint4* out = reinterpret_cast<uint4*>(sums + (tap * 16 + channel) * C + c0 % C);
 #pragma unroll
         for (int i = 0; i < 4; ++i)
           out[i] = make_uint4(r[4 * i], r[4 * i + 1], r[4 * i + 2], r[4 * i + 3]);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) finite &= (r[i] & 0x7f800000u) != 0x7f800000u;
       }
     }
   }
+  const bool partial_tiles = s.ho % TILE_H != 0 || s.wo % TILE_W != 0;
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  __syncthreads();
+  const bool plain = __syncthreads_or(!finite && partial_tiles && ok) != 0;
   if (warp == 0)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;"
                  ::"r"(tmem), "r"(tmem_columns));
+  if (plain) plain_sums<T, PAIRS>(x, dy, sums, s, smem);
 }
 
 // dw[o][c][kh][kw] = sum of the CTAs' partial sums, one CTA per (c, kh, kw):
@@ -609,7 +668,10 @@ cudaError_t LaunchStemConvWgrad(const void* x, const void* dy, float* partial, v
                          (static_cast<uint32_t>(channels >> 3) << 17) | ((128u >> 4) << 24);
   const int smem = 2 * (PATCH_BYTES + (channels / 8 * DY_PLANE + 127) / 128 * 128);
   const bool pairs = w % 2 == 0 && reinterpret_cast<uintptr_t>(x) % 4 == 0;
-  auto kernel = pairs ? stem_conv_wgrad_kernel<true> : stem_conv_wgrad_kernel<false>;
+  auto kernel = bf16 ? (pairs ? stem_conv_wgrad_kernel<__nv_bfloat16, true>
+                              : stem_conv_wgrad_kernel<__nv_bfloat16, false>)
+                     : (pairs ? stem_conv_wgrad_kernel<__half, true>
+                              : stem_conv_wgrad_kernel<__half, false>);
   auto sum = bf16 ? stem_conv_wgrad_sum_kernel<__nv_bfloat16> : stem_conv_wgrad_sum_kernel<__half>;
   err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (err != cudaSuccess) return err;

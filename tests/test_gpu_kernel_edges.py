@@ -292,6 +292,35 @@ def test_stem_convolution_of_special_values(channels, value, dtype):
     assert bool(((y.double() - want).abs() <= bound)[finite].all())
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("value", [float("inf"), float("-inf"), float("nan")])
+@pytest.mark.parametrize("channels", [16, 64])
+def test_stem_gradient_of_special_values(channels, value, dtype):
+    """Infinities and NaN reach the taps that some output pixel multiplies
+    with them, also where a tile reaches past the output."""
+    from horovod_b200 import _C
+    images = _special_images(dtype, value)
+    w = torch.zeros(channels, 3, 7, 7, dtype=dtype)
+    g = torch.Generator().manual_seed(12)
+    dy = torch.randn(len(images), channels, 34, 23, generator=g).to(dtype)
+    # each image by itself, and many at once (more tiles than CTAs), of which
+    # only one is not finite
+    many = images[-1:].repeat(90, 1, 1, 1)
+    many[-1] = images[5]
+    more = torch.randn(len(many), channels, 34, 23, generator=g).to(dtype)
+    for x, d in [(images[n:n + 1], dy[n:n + 1]) for n in range(len(images))] + [(many, more)]:
+        x, d = (t.contiguous(memory_format=torch.channels_last) for t in (x, d))
+        dw = _C.stem_conv_wgrad(x.to(_dev()), d.to(_dev()), w.to(_dev())).cpu()
+        want = torch.nn.grad.conv2d_weight(x.double(), w.shape, d.double(), stride=2, padding=3)
+        assert torch.equal(_kinds(dw), _kinds(want))
+        # the sum of the products' sizes in fp32, then one rounding
+        size = torch.nn.grad.conv2d_weight(torch.nan_to_num(x.double().abs(), 0.0, 0.0, 0.0),
+                                           w.shape, d.double().abs(), stride=2, padding=3)
+        eps = 2.0 ** (-8 if dtype == torch.bfloat16 else -11)
+        bound = eps * want.abs() + 2e-5 * size + 6e-8
+        assert bool(((dw.double() - want).abs() <= bound)[want.isfinite()].all())
+
+
 @pytest.mark.parametrize("momentum", [0.1, None])
 def test_batch_norm_counts_batches_once(momentum):
     from horovod_b200.ops.batch_norm import BatchNormAct2d
