@@ -391,16 +391,21 @@ cudaError_t LaunchMaxPool3s2Backward(const void* dy, const uint32_t* idx, void* 
 // 7x7 / stride 2 / padding 3 convolution of 3 channels-last 16-bit channels
 // ([n, h, w, 3]) without bias: y [n, (h - 1) / 2 + 1, (w - 1) / 2 + 1, channels].
 // weight: 16-bit [channels, 3, 7, 7] with the given element strides.
+// A kernel waits wait_ns for its products at most; when that is not enough its
+// results are NaN and StemConvFailed(device) is true from then on (until it is
+// called with `clear`).
 bool StemConvSupported(int channels);
+bool StemConvFailed(int device, bool clear);
+constexpr uint32_t STEM_WAIT_NS = 1000000000u;
 cudaError_t LaunchStemConvForward(const void* x, const void* weight, const int64_t* weight_strides,
                                   void* y, int n, int h, int w, int channels, bool bf16,
-                                  cudaStream_t stream);
+                                  cudaStream_t stream, uint32_t wait_ns = STEM_WAIT_NS);
 // Gradient of the weights (16-bit, with the given strides) from x and dy.
 // partial: scratch of StemConvWgradCtas() * 256 * channels floats.
 int StemConvWgradCtas(int n, int h, int w, int channels);
 cudaError_t LaunchStemConvWgrad(const void* x, const void* dy, float* partial, void* dw,
                                 const int64_t* weight_strides, int n, int h, int w, int channels,
-                                bool bf16, cudaStream_t stream);
+                                bool bf16, cudaStream_t stream, uint32_t wait_ns = STEM_WAIT_NS);
 
 // Multi-tensor SGD step in one launch (torch.optim.SGD arithmetic: weight
 // decay added to the gradient, momentum buffer b = momentum * b + (1 -

@@ -26,11 +26,16 @@
 // plain copy; the tensor cores' operand reads from shared memory and the turns
 // between the phases of a tile take the rest.
 //
+// Waits are bounded. When one runs out, what the CTA had not finished becomes NaN
+// (so that the step is seen to have failed), and a host-visible word per device
+// says so (StemConvFailed).
+//
 // The reference has no counterpart (it takes convolutions from the framework).
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
 #include <cstdint>
+#include <cstring>
 #include <mutex>
 
 #include "kernels.h"
@@ -45,6 +50,7 @@ constexpr int TILE_H = 16, TILE_W = 8;                      // output pixels: M 
 constexpr int PATCH_H = TILE_H + 3, PATCH_W = TILE_W + 3;   // blocks
 constexpr int PATCH = PATCH_H * PATCH_W;
 constexpr int PLANE_BYTES = PATCH * 16;
+constexpr uint16_t NAN16 = 0x7fff;  // a NaN of either 16-bit type
 constexpr int TAPS = 16, K_CORES = 2 * TAPS;  // 8 values of K each
 static_assert(PATCH <= THREADS, "one block per thread");
 
@@ -67,9 +73,11 @@ __device__ __forceinline__ void mma(uint32_t d, uint64_t a, uint64_t b, uint32_t
       ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(add ? 1u : 0u) : "memory");
 }
 
-// Waits until phase `parity` of the barrier is complete; false after a second.
-__device__ __forceinline__ bool wait_bounded(uint32_t bar, uint32_t parity) {
+// Waits until phase `parity` of the barrier is complete; false when that takes
+// longer than `limit` nanoseconds (0: at once).
+__device__ __forceinline__ bool wait_bounded(uint32_t bar, uint32_t parity, uint32_t limit) {
   unsigned long long t0 = 0;
+  if (limit == 0) return false;
   for (int i = 0;; ++i) {
     uint32_t done;
     asm volatile(
@@ -81,7 +89,7 @@ __device__ __forceinline__ bool wait_bounded(uint32_t bar, uint32_t parity) {
     unsigned long long t;
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
     if (i == 0) t0 = t;
-    if (t - t0 > 1000000000ull) return false;
+    if (t - t0 > limit) return false;
   }
 }
 
@@ -201,11 +209,23 @@ __device__ __noinline__ void plain_tile(const unsigned char* patch, const unsign
   }
 }
 
+// Fills the outputs of tiles `tile`, `tile` + grid, ... with NaN.
+__device__ __noinline__ void give_up_tiles(uint16_t* y, const StemShape& s, int tile) {
+  for (; tile < s.tiles; tile += gridDim.x) {
+    const TileAt at = tile_at(s, tile);
+    const int rows = min(s.ho - at.i, TILE_H), row_values = min(s.wo - at.j, TILE_W) * s.channels;
+    uint16_t* out = y + ((static_cast<int64_t>(at.n) * s.ho + at.i) * s.wo + at.j) * s.channels;
+    for (int e = threadIdx.x; e < rows * row_values; e += THREADS)
+      out[static_cast<int64_t>(e / row_values) * s.wo * s.channels + e % row_values] = NAN16;
+  }
+}
+
 template <typename T, bool PAIRS>
 __global__ void __launch_bounds__(THREADS, 4)
 stem_conv_forward_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict__ weight,
-                         uint16_t* __restrict__ y, const StemShape s, const uint32_t idesc,
-                         const uint32_t tmem_columns, int* status) {
+                         uint16_t* __restrict__ y, const __grid_constant__ StemShape s,
+                         const uint32_t idesc, const uint32_t tmem_columns, int* status,
+                         const uint32_t wait_ns) {
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ __align__(8) uint64_t s_bar;
   __shared__ uint32_t s_tmem;
@@ -286,11 +306,12 @@ stem_conv_forward_kernel(const uint16_t* __restrict__ x, const uint16_t* __restr
       at = next;
       continue;
     }
-    const bool ok = wait_bounded(smem_addr(&s_bar), parity);
+    const bool ok = wait_bounded(smem_addr(&s_bar), parity, wait_ns);
     parity ^= 1u;
     if (__syncthreads_and(ok) == 0) {
       if (threadIdx.x == 0) *reinterpret_cast<volatile int*>(status) = 1;
-      wait_bounded(smem_addr(&s_bar), parity ^ 1u);  // the products in flight
+      wait_bounded(smem_addr(&s_bar), parity ^ 1u, STEM_WAIT_NS);  // the products in flight
+      give_up_tiles(y, s, tile);
       break;
     }
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -405,7 +426,8 @@ template <typename T, bool PAIRS>
 __global__ void __launch_bounds__(THREADS, 2)
 stem_conv_wgrad_kernel(const uint16_t* __restrict__ x, const uint4* __restrict__ dy,
                        float* __restrict__ partial, const __grid_constant__ StemShape s,
-                       const uint32_t idesc, const uint32_t tmem_columns, int* status) {
+                       const uint32_t idesc, const uint32_t tmem_columns, int* status,
+                       const uint32_t wait_ns) {
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ __align__(8) uint64_t s_bar[2];
   __shared__ uint32_t s_tmem;
@@ -461,7 +483,7 @@ stem_conv_wgrad_kernel(const uint16_t* __restrict__ x, const uint4* __restrict__
     const uint32_t buffer = issued & 1u, use = issued >> 1;
     unsigned char* patch = smem + buffer * buffer_bytes;
     unsigned char* grads = patch + PATCH_BYTES;
-    if (use > 0) ok = wait_bounded(smem_addr(&s_bar[buffer]), (use - 1) & 1u);
+    if (use > 0) ok = wait_bounded(smem_addr(&s_bar[buffer]), (use - 1) & 1u, wait_ns);
     if (__syncthreads_and(ok) == 0) break;
     store_block(patch, v);
 #pragma unroll
@@ -487,12 +509,16 @@ stem_conv_wgrad_kernel(const uint16_t* __restrict__ x, const uint4* __restrict__
   // The last tile of each buffer.
   for (uint32_t b = 0; b < 2; ++b) {
     const uint32_t uses = (issued + 1 - b) / 2;
-    if (uses > 0 && !wait_bounded(smem_addr(&s_bar[b]), (uses - 1) & 1u)) ok = false;
+    if (uses > 0 && !wait_bounded(smem_addr(&s_bar[b]), (uses - 1) & 1u, wait_ns)) {
+      wait_bounded(smem_addr(&s_bar[b]), (uses - 1) & 1u, STEM_WAIT_NS);  // products in flight
+      ok = false;
+    }
   }
   ok = __syncthreads_and(ok) != 0;
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   if (!ok) {
     if (threadIdx.x == 0) *reinterpret_cast<volatile int*>(status) = 1;
+    for (int e = threadIdx.x; e < TAPS * 16 * C; e += THREADS) sums[e] = __int_as_float(0x7fffffff);
   } else {
     const int m = warp % 4 * 32 + lane, group = m / 8;
     const bool useful = group < 4 || (group >= 11 && group < 15);
@@ -558,22 +584,25 @@ stem_conv_wgrad_sum_kernel(const float* __restrict__ partial, uint16_t* __restri
   }
 }
 
-// Host-visible word that a kernel sets when a wait ran out.
-int* StatusWord() {
-  static std::once_flag once;
-  static int* word = nullptr;
-  std::call_once(once, [] {
+// Host-visible word per device that a kernel sets when a wait ran out; null
+// when there is no memory for them or no such device.
+int* StatusWord(int device) {
+  constexpr int DEVICES = 64;
+  static std::mutex mu;
+  static int* words = nullptr;
+  std::lock_guard<std::mutex> lock(mu);
+  if (words == nullptr) {
     // Also when the first call is being captured into a graph.
     cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
     cudaThreadExchangeStreamCaptureMode(&mode);
-    if (cudaHostAlloc(reinterpret_cast<void**>(&word), sizeof(int),
+    if (cudaHostAlloc(reinterpret_cast<void**>(&words), DEVICES * sizeof(int),
                       cudaHostAllocMapped | cudaHostAllocPortable) == cudaSuccess)
-      *word = 0;
+      std::memset(words, 0, DEVICES * sizeof(int));
     else
-      word = nullptr;
+      words = nullptr;
     cudaThreadExchangeStreamCaptureMode(&mode);
-  });
-  return word;
+  }
+  return words != nullptr && device >= 0 && device < DEVICES ? words + device : nullptr;
 }
 
 }  // namespace
@@ -605,14 +634,24 @@ static cudaError_t StemReady(int n, int h, int w, int channels, int** status) {
   if (!StemConvSupported(channels) || n < 1 || h < 1 || w < 1 ||
       static_cast<int64_t>(n) * ((h + 31) / 32) * ((w + 15) / 16) > (1 << 30))
     return cudaErrorInvalidValue;
-  *status = StatusWord();
-  if (*status == nullptr) return cudaErrorMemoryAllocation;
-  return *static_cast<volatile int*>(*status) != 0 ? cudaErrorLaunchTimeout : cudaSuccess;
+  int device = 0;
+  const cudaError_t err = cudaGetDevice(&device);
+  if (err != cudaSuccess) return err;
+  *status = StatusWord(device);
+  return *status != nullptr ? cudaSuccess : cudaErrorMemoryAllocation;
+}
+
+bool StemConvFailed(int device, bool clear) {
+  volatile int* status = StatusWord(device);
+  if (status == nullptr) return true;
+  const bool failed = *status != 0;
+  if (clear) *status = 0;
+  return failed;
 }
 
 cudaError_t LaunchStemConvForward(const void* x, const void* weight, const int64_t* weight_strides,
                                   void* y, int n, int h, int w, int channels, bool bf16,
-                                  cudaStream_t stream) {
+                                  cudaStream_t stream, uint32_t wait_ns) {
   int* status = nullptr;
   cudaError_t err = StemReady(n, h, w, channels, &status);
   if (err != cudaSuccess) return err;
@@ -635,7 +674,8 @@ cudaError_t LaunchStemConvForward(const void* x, const void* weight, const int64
   CountKernelLaunches(1);
   kernel<<<grid, THREADS, smem, stream>>>(static_cast<const uint16_t*>(x),
                                           static_cast<const uint16_t*>(weight),
-                                          static_cast<uint16_t*>(y), s, idesc, columns, status);
+                                          static_cast<uint16_t*>(y), s, idesc, columns, status,
+                                          wait_ns);
   return cudaGetLastError();
 }
 
@@ -656,7 +696,7 @@ int StemConvWgradCtas(int n, int h, int w, int channels) {
 
 cudaError_t LaunchStemConvWgrad(const void* x, const void* dy, float* partial, void* dw,
                                 const int64_t* weight_strides, int n, int h, int w, int channels,
-                                bool bf16, cudaStream_t stream) {
+                                bool bf16, cudaStream_t stream, uint32_t wait_ns) {
   int* status = nullptr;
   cudaError_t err = StemReady(n, h, w, channels, &status);
   if (err != cudaSuccess) return err;
@@ -678,7 +718,7 @@ cudaError_t LaunchStemConvWgrad(const void* x, const void* dy, float* partial, v
   CountKernelLaunches(2);
   kernel<<<ctas, THREADS, smem, stream>>>(static_cast<const uint16_t*>(x),
                                           static_cast<const uint4*>(dy), partial, s, idesc,
-                                          WgradColumns(channels), status);
+                                          WgradColumns(channels), status, wait_ns);
   err = cudaGetLastError();
   if (err != cudaSuccess) return err;
   sum<<<3 * 7 * 7, SUM_THREADS, 0, stream>>>(partial, static_cast<uint16_t*>(dw), ctas, s);

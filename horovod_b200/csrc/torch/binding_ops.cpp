@@ -221,7 +221,9 @@ void BindModelOps(py::module_& m) {
   m.def("stem_conv_supported", [](int64_t channels) {
     return kern::StemConvSupported(static_cast<int>(channels));
   });
-  m.def("stem_conv_forward", [](const at::Tensor& x, const at::Tensor& weight) {
+  // Whether a kernel's wait has run out on this device.
+  m.def("stem_conv_failed", &kern::StemConvFailed, py::arg("device"), py::arg("clear") = false);
+  m.def("stem_conv_forward", [](const at::Tensor& x, const at::Tensor& weight, uint32_t wait_ns) {
     CheckActivations(x, "x");
     const int64_t N = x.size(0), H = x.size(2), W = x.size(3), C = weight.size(0);
     TORCH_CHECK(weight.is_cuda() && weight.device() == x.device() &&
@@ -237,13 +239,14 @@ void BindModelOps(py::module_& m) {
     cudaError_t err = kern::LaunchStemConvForward(
         x.data_ptr(), weight.data_ptr(), weight.strides().data(), y.data_ptr(),
         static_cast<int>(N), static_cast<int>(H), static_cast<int>(W), static_cast<int>(C),
-        x.scalar_type() == at::kBFloat16, at::cuda::getCurrentCUDAStream());
+        x.scalar_type() == at::kBFloat16, at::cuda::getCurrentCUDAStream(), wait_ns);
     TORCH_CHECK(err == cudaSuccess, "stem convolution: ", cudaGetErrorString(err));
     return y;
-  });
+  }, py::arg("x"), py::arg("weight"), py::arg("wait_ns") = kern::STEM_WAIT_NS);
 
   // (x, dy, weight) -> gradient of the weight
-  m.def("stem_conv_wgrad", [](const at::Tensor& x, const at::Tensor& dy, const at::Tensor& weight) {
+  m.def("stem_conv_wgrad", [](const at::Tensor& x, const at::Tensor& dy, const at::Tensor& weight,
+                              uint32_t wait_ns) {
     CheckActivations(x, "x");
     CheckActivations(dy, "dy");
     const int64_t N = x.size(0), H = x.size(2), W = x.size(3), C = weight.size(0);
@@ -267,10 +270,11 @@ void BindModelOps(py::module_& m) {
     cudaError_t err = kern::LaunchStemConvWgrad(
         x.data_ptr(), dy.data_ptr(), partial.data_ptr<float>(), dw.data_ptr(),
         dw.strides().data(), static_cast<int>(N), static_cast<int>(H), static_cast<int>(W),
-        static_cast<int>(C), x.scalar_type() == at::kBFloat16, at::cuda::getCurrentCUDAStream());
+        static_cast<int>(C), x.scalar_type() == at::kBFloat16, at::cuda::getCurrentCUDAStream(),
+        wait_ns);
     TORCH_CHECK(err == cudaSuccess, "stem convolution gradient: ", cudaGetErrorString(err));
     return dw;
-  });
+  }, py::arg("x"), py::arg("dy"), py::arg("weight"), py::arg("wait_ns") = kern::STEM_WAIT_NS);
 
   // ---- multi-tensor SGD ------------------------------------------------------
   // One step over a parameter list, in one launch per 256 tensors. bufs holds

@@ -3,9 +3,16 @@ channels-last bf16/fp16 inputs on this library's tensor-core kernel
 (csrc/kernels/stem_conv.cu), with PyTorch's convolution everywhere else and
 for the gradient of the input.
 
+``HOROVOD_B200_FUSED_STEM=0`` leaves everything to PyTorch, and so does a wait
+that has run out inside the kernel: the results of that call are NaN, later ones
+on the device are PyTorch's.
+
 ``StemConv2d`` is an ``nn.Conv2d`` (same parameters and state_dict keys). The
 reference has no counterpart (it takes convolutions from the framework).
 """
+import os
+import warnings
+
 import torch
 import torch.nn as nn
 from torch.autograd import forward_ad
@@ -14,6 +21,16 @@ from torch.autograd import forward_ad
 def _extension():
     from horovod_b200 import _C
     return _C
+
+
+def _enabled(device):
+    if os.environ.get("HOROVOD_B200_FUSED_STEM", "1") != "1":
+        return False
+    if _extension().stem_conv_failed(device.index):
+        warnings.warn("a wait inside the stem convolution's kernel ran out on %s; the results of "
+                      "that call are NaN, and PyTorch's convolution runs from now on" % device)
+        return False
+    return True
 
 
 class _StemConv(torch.autograd.Function):
@@ -27,7 +44,8 @@ class _StemConv(torch.autograd.Function):
         x, weight = ctx.saved_tensors
         need_x, need_w = ctx.needs_input_grad
         # A gradient of this gradient is PyTorch's.
-        native = need_w and not torch.is_grad_enabled() and weight.dtype == dy.dtype
+        native = need_w and not torch.is_grad_enabled() and weight.dtype == dy.dtype and \
+            _enabled(x.device)
         dx = dw = None
         if need_x or (need_w and not native):
             dx, dw, _ = torch.ops.aten.convolution_backward(
@@ -66,7 +84,9 @@ class StemConv2d(nn.Conv2d):
         if torch.jit.is_tracing() or torch.compiler.is_compiling() or \
                 forward_ad._current_level >= 0 or torch._C._are_functorch_transforms_active():
             return None
-        return dtype if _extension().stem_conv_supported(self.out_channels) else None
+        if not _extension().stem_conv_supported(self.out_channels) or not _enabled(x.device):
+            return None
+        return dtype
 
     def forward(self, x):
         dtype = self._kernel_dtype(x)

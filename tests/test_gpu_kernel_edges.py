@@ -321,6 +321,72 @@ def test_stem_gradient_of_special_values(channels, value, dtype):
         assert bool(((dw.double() - want).abs() <= bound)[want.isfinite()].all())
 
 
+def _fallback_conv(use):
+    """Runs `use` under conditions in which a StemConv2d is PyTorch's."""
+    from horovod_b200 import _C
+    from horovod_b200.ops.stem_conv import StemConv2d
+    conv = StemConv2d(3, 16, 7, stride=2, padding=3, bias=False).to(_dev()).bfloat16()
+    x = torch.randn(2, 3, 20, 20, device=_dev()).bfloat16().contiguous(
+        memory_format=torch.channels_last)
+    assert conv._kernel_dtype(x) == torch.bfloat16
+    with use():
+        assert conv._kernel_dtype(x) is None
+        before = _C.kernel_launch_count()
+        y = conv(x)
+        y.sum().backward()
+        assert _C.kernel_launch_count() == before
+        assert torch.equal(y, F.conv2d(x, conv.weight, stride=2, padding=3))
+    assert conv._kernel_dtype(x) == torch.bfloat16
+
+
+def test_stem_convolution_switch(monkeypatch):
+    import contextlib
+
+    @contextlib.contextmanager
+    def off():
+        with monkeypatch.context() as m:
+            m.setenv("HOROVOD_B200_FUSED_STEM", "0")
+            yield
+    _fallback_conv(off)
+
+
+@pytest.mark.parametrize("channels", [16, 128])
+def test_stem_convolution_whose_waits_run_out(channels):
+    """A limit of 0 makes every wait run out (the kernels then wait for their
+    products in flight all the same): results are NaN, the device is marked, and
+    the module goes on with PyTorch's convolution."""
+    import contextlib
+    from horovod_b200 import _C
+    x = torch.randn(90, 3, 67, 45, device=_dev()).bfloat16().contiguous(
+        memory_format=torch.channels_last)
+    w = torch.randn(channels, 3, 7, 7, device=_dev()).bfloat16()
+    dy = torch.randn(90, channels, 34, 23, device=_dev()).bfloat16().contiguous(
+        memory_format=torch.channels_last)
+    y, dw = _C.stem_conv_forward(x, w), _C.stem_conv_wgrad(x, dy, w)
+    assert not _C.stem_conv_failed(0)
+    try:
+        assert bool(_C.stem_conv_forward(x, w, wait_ns=0).isnan().all())
+        assert _C.stem_conv_failed(0) and _C.stem_conv_failed(0, clear=True)
+        assert not _C.stem_conv_failed(0)
+        assert bool(_C.stem_conv_wgrad(x, dy, w, wait_ns=0).isnan().all())
+        assert _C.stem_conv_failed(0, clear=True)
+
+        @contextlib.contextmanager
+        def failed():
+            _C.stem_conv_forward(x, w, wait_ns=0)
+            torch.cuda.synchronize()
+            with pytest.warns(UserWarning, match="ran out"):
+                yield
+            _C.stem_conv_failed(0, clear=True)
+        _fallback_conv(failed)
+    finally:
+        torch.cuda.synchronize()
+        _C.stem_conv_failed(0, clear=True)
+    # nothing is left behind
+    assert torch.equal(_C.stem_conv_forward(x, w), y)
+    assert torch.equal(_C.stem_conv_wgrad(x, dy, w), dw)
+
+
 @pytest.mark.parametrize("momentum", [0.1, None])
 def test_batch_norm_counts_batches_once(momentum):
     from horovod_b200.ops.batch_norm import BatchNormAct2d
