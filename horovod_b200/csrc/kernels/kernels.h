@@ -394,7 +394,7 @@ cudaError_t LaunchMaxPool3s2Backward(const void* dy, const uint32_t* idx, void* 
 // A kernel waits wait_ns for its products at most; when that is not enough its
 // results are NaN and StemConvFailed(device) is true from then on (until it is
 // called with `clear`).
-bool StemConvSupported(int channels);
+bool StemConvSupported(int64_t n, int64_t h, int64_t w, int64_t channels);
 bool StemConvFailed(int device, bool clear);
 constexpr uint32_t STEM_WAIT_NS = 1000000000u;
 cudaError_t LaunchStemConvForward(const void* x, const void* weight, const int64_t* weight_strides,

@@ -607,8 +607,12 @@ int* StatusWord(int device) {
 
 }  // namespace
 
-bool StemConvSupported(int channels) {
-  return channels >= 16 && channels <= 128 && channels % 16 == 0;
+// Offsets inside a tile are 32-bit, 16 rows of the output at 128 channels being the
+// longest, as is the number of tiles.
+bool StemConvSupported(int64_t n, int64_t h, int64_t w, int64_t channels) {
+  constexpr int64_t MOST = 1 << 24;
+  return channels >= 16 && channels <= 128 && channels % 16 == 0 && n >= 1 && h >= 1 && w >= 1 &&
+         h <= MOST && w <= MOST && n <= (1 << 30) / (((h + 31) / 32) * ((w + 15) / 16));
 }
 
 static StemShape MakeShape(int n, int h, int w, int channels, const int64_t* weight_strides) {
@@ -631,9 +635,7 @@ static StemShape MakeShape(int n, int h, int w, int channels, const int64_t* wei
 
 // cudaSuccess when the kernels may run; *status is where they report to.
 static cudaError_t StemReady(int n, int h, int w, int channels, int** status) {
-  if (!StemConvSupported(channels) || n < 1 || h < 1 || w < 1 ||
-      static_cast<int64_t>(n) * ((h + 31) / 32) * ((w + 15) / 16) > (1 << 30))
-    return cudaErrorInvalidValue;
+  if (!StemConvSupported(n, h, w, channels)) return cudaErrorInvalidValue;
   int device = 0;
   const cudaError_t err = cudaGetDevice(&device);
   if (err != cudaSuccess) return err;

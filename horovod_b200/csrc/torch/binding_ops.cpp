@@ -218,9 +218,7 @@ void BindModelOps(py::module_& m) {
   });
 
   // ---- 7x7 / stride 2 convolution of 3 channels (channels-last, 16-bit) ------
-  m.def("stem_conv_supported", [](int64_t channels) {
-    return kern::StemConvSupported(static_cast<int>(channels));
-  });
+  m.def("stem_conv_supported", &kern::StemConvSupported);  // (n, h, w, channels)
   // Whether a kernel's wait has run out on this device.
   m.def("stem_conv_failed", &kern::StemConvFailed, py::arg("device"), py::arg("clear") = false);
   m.def("stem_conv_forward", [](const at::Tensor& x, const at::Tensor& weight, uint32_t wait_ns) {
@@ -231,8 +229,8 @@ void BindModelOps(py::module_& m) {
                     weight.size(1) == 3 && weight.size(2) == 7 && weight.size(3) == 7 &&
                     x.size(1) == 3,
                 "stem_conv_forward: x must have 3 channels and weight the shape [C, 3, 7, 7]");
-    TORCH_CHECK(kern::StemConvSupported(static_cast<int>(C)),
-                "stem_conv_forward does not support ", C, " channels");
+    TORCH_CHECK(kern::StemConvSupported(N, H, W, C), "stem_conv_forward does not support ", N,
+                " images of ", H, " x ", W, " to ", C, " channels");
     c10::cuda::CUDAGuard guard(x.device());
     at::Tensor y = at::empty({N, C, (H - 1) / 2 + 1, (W - 1) / 2 + 1}, x.options(),
                              at::MemoryFormat::ChannelsLast);
@@ -252,15 +250,14 @@ void BindModelOps(py::module_& m) {
     const int64_t N = x.size(0), H = x.size(2), W = x.size(3), C = weight.size(0);
     TORCH_CHECK(weight.scalar_type() == x.scalar_type() && weight.device() == x.device() &&
                     weight.dim() == 4 && weight.size(1) == 3 && weight.size(2) == 7 &&
-                    weight.size(3) == 7 && weight.is_non_overlapping_and_dense() &&
-                    x.size(1) == 3,
+                    weight.size(3) == 7 && x.size(1) == 3,
                 "stem_conv_wgrad: x must have 3 channels and weight the shape [C, 3, 7, 7]");
     TORCH_CHECK(dy.scalar_type() == x.scalar_type() && dy.device() == x.device() &&
                     dy.size(0) == N && dy.size(1) == C && dy.size(2) == (H - 1) / 2 + 1 &&
                     dy.size(3) == (W - 1) / 2 + 1,
                 "stem_conv_wgrad: dy does not match x and weight");
-    TORCH_CHECK(kern::StemConvSupported(static_cast<int>(C)),
-                "stem_conv_wgrad does not support ", C, " channels");
+    TORCH_CHECK(kern::StemConvSupported(N, H, W, C), "stem_conv_wgrad does not support ", N,
+                " images of ", H, " x ", W, " to ", C, " channels");
     c10::cuda::CUDAGuard guard(x.device());
     const int64_t ctas = kern::StemConvWgradCtas(static_cast<int>(N), static_cast<int>(H),
                                                  static_cast<int>(W), static_cast<int>(C));

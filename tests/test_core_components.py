@@ -303,3 +303,18 @@ def test_response_path_counters_are_readable_without_a_gpu():
     paths = utils.response_paths()
     assert set(paths) == {"symm", "nccl"} and all(isinstance(v, int) and v >= 0
                                                   for v in paths.values())
+
+
+def test_stem_convolution_sizes():
+    """Which images the stem convolution's kernels take: 32-bit offsets inside a
+    tile and a 32-bit number of tiles; the others are left to PyTorch."""
+    from horovod_b200 import _C
+    fits = _C.stem_conv_supported
+    assert fits(256, 224, 224, 64) and fits(1, 1, 1, 16) and fits(1, 1 << 24, 1, 128)
+    # 16 rows of the output, 8 pixels of the last one, in pieces of 8 channels
+    assert fits(1, 33, 1 << 24, 128) and (15 * (1 << 23) + 8) * 16 < 1 << 31
+    assert not fits(1, 33, (1 << 24) + 1, 128) and not fits(1, (1 << 24) + 1, 33, 128)
+    assert fits(1 << 30, 32, 16, 16) and not fits((1 << 30) + 1, 32, 16, 16)
+    assert not fits(1 << 30, 33, 16, 16) and not fits(1 << 40, 1, 1, 16)
+    assert not any(fits(1, 8, 8, c) for c in (0, 8, 24, 144, 1 << 32 | 64))
+    assert not fits(0, 8, 8, 64) and not fits(1, 0, 8, 64) and not fits(1, 8, -1, 64)

@@ -339,6 +339,41 @@ def _fallback_conv(use):
     assert conv._kernel_dtype(x) == torch.bfloat16
 
 
+def test_stem_convolution_left_to_pytorch():
+    """Dispatch modes and tensor subclasses see PyTorch's convolution, as with an
+    nn.Conv2d; a weight with gaps is taken by the kernels."""
+    from torch.utils._python_dispatch import TorchDispatchMode
+    from torch.utils.flop_counter import FlopCounterMode
+    from horovod_b200.ops.stem_conv import StemConv2d
+    _fallback_conv(lambda: FlopCounterMode(display=False))
+
+    class Quiet(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            return func(*args, **(kwargs or {}))
+    _fallback_conv(Quiet)
+
+    class Subclass(torch.Tensor):
+        pass
+    conv = StemConv2d(3, 16, 7, stride=2, padding=3, bias=False).to(_dev()).bfloat16()
+    x = torch.randn(2, 3, 20, 20, device=_dev()).bfloat16().contiguous(
+        memory_format=torch.channels_last)
+    assert conv._kernel_dtype(x.as_subclass(Subclass)) is None
+    assert isinstance(conv(x.as_subclass(Subclass)), Subclass)
+
+    wide = torch.randn(16, 3, 7, 14, device=_dev()).bfloat16()
+    gaps = wide[..., ::2].detach().requires_grad_(True)
+    dense = gaps.detach().clone(memory_format=torch.contiguous_format).requires_grad_(True)
+    grads = []
+    for w in (gaps, dense):
+        conv.weight = torch.nn.Parameter(w.detach())
+        assert conv._kernel_dtype(x) == torch.bfloat16
+        y = conv(x)
+        y.backward(torch.ones_like(y))
+        grads.append((y, conv.weight.grad))
+    assert not gaps.is_contiguous()
+    assert torch.equal(grads[0][0], grads[1][0]) and torch.equal(grads[0][1], grads[1][1])
+
+
 def test_stem_convolution_switch(monkeypatch):
     import contextlib
 
