@@ -25,6 +25,14 @@ void CheckActivations(const at::Tensor& t, const char* what) {
               " must be contiguous in channels_last memory format");
 }
 
+// t, checked, for kernels that access it 16 bytes at a time: a view that starts
+// between two such boundaries (a slice of a flat buffer) is copied.
+at::Tensor Activations(const at::Tensor& t, const char* what) {
+  CheckActivations(t, what);
+  if (reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0) return t;
+  return t.clone(at::MemoryFormat::ChannelsLast);
+}
+
 const float* FloatPtrOrNull(const c10::optional<at::Tensor>& t, int64_t channels, const char* what) {
   if (!t.has_value() || !t->defined()) return nullptr;
   TORCH_CHECK(t->is_cuda() && t->scalar_type() == at::kFloat && t->is_contiguous() &&
@@ -86,19 +94,19 @@ void BindModelOps(py::module_& m) {
   //  num_batches_tracked?)
   //   -> (y, saved, signs or None): saved holds what the backward needs of the
   //      statistics, signs (with a residual and a ReLU) which outputs are above zero
-  m.def("bn_forward", [](const at::Tensor& x, const c10::optional<at::Tensor>& residual,
+  m.def("bn_forward", [](at::Tensor x, c10::optional<at::Tensor> residual,
                          const c10::optional<at::Tensor>& weight,
                          const c10::optional<at::Tensor>& bias,
                          c10::optional<at::Tensor> running_mean,
                          c10::optional<at::Tensor> running_var, double momentum, double eps,
                          bool relu, c10::optional<at::Tensor> batches) {
-    CheckActivations(x, "x");
+    x = Activations(x, "x");
     const int64_t C = x.size(1), M = x.numel() / C;
     TORCH_CHECK(kern::BatchNormSupported(M, static_cast<int>(C)),
                 "fused batch norm does not support ", C, " channels");
     const void* res = nullptr;
     if (residual.has_value() && residual->defined()) {
-      CheckActivations(*residual, "residual");
+      residual = Activations(*residual, "residual");
       TORCH_CHECK(residual->sizes() == x.sizes() && residual->scalar_type() == x.scalar_type(),
                   "residual must match x");
       res = residual->data_ptr();
@@ -136,12 +144,12 @@ void BindModelOps(py::module_& m) {
   });
   // (dy, x, weight?, saved, signs?, relu, want_dresidual)
   //   -> (dx, dresidual or None, dweight, dbias)
-  m.def("bn_backward", [](const at::Tensor& dy, const at::Tensor& x,
+  m.def("bn_backward", [](at::Tensor dy, at::Tensor x,
                           const c10::optional<at::Tensor>& weight, const at::Tensor& saved,
                           const c10::optional<at::Tensor>& signs, bool relu,
                           bool want_dresidual) {
-    CheckActivations(x, "x");
-    CheckActivations(dy, "dy");
+    x = Activations(x, "x");
+    dy = Activations(dy, "dy");
     TORCH_CHECK(dy.sizes() == x.sizes() && dy.scalar_type() == x.scalar_type(), "dy must match x");
     const int64_t C = x.size(1), M = x.numel() / C;
     TORCH_CHECK(saved.is_cuda() && saved.scalar_type() == at::kFloat && saved.is_contiguous() &&
@@ -179,8 +187,8 @@ void BindModelOps(py::module_& m) {
   });
   // x -> (y, idx): idx holds one word per 8 output channels (a nibble for the
   // winning window position of each).
-  m.def("maxpool3s2_forward", [](const at::Tensor& x) {
-    CheckActivations(x, "x");
+  m.def("maxpool3s2_forward", [](at::Tensor x) {
+    x = Activations(x, "x");
     const int64_t N = x.size(0), C = x.size(1), H = x.size(2), W = x.size(3);
     TORCH_CHECK(kern::MaxPool3s2Supported(static_cast<int>(C)),
                 "fused max pooling needs a channel count that is a multiple of 8");
@@ -197,9 +205,8 @@ void BindModelOps(py::module_& m) {
     return std::make_tuple(y, idx);
   });
   // (dy, idx, H, W) -> dx
-  m.def("maxpool3s2_backward", [](const at::Tensor& dy, const at::Tensor& idx, int64_t H,
-                                  int64_t W) {
-    CheckActivations(dy, "dy");
+  m.def("maxpool3s2_backward", [](at::Tensor dy, const at::Tensor& idx, int64_t H, int64_t W) {
+    dy = Activations(dy, "dy");
     const int64_t N = dy.size(0), C = dy.size(1);
     TORCH_CHECK(idx.is_cuda() && idx.scalar_type() == at::kInt && idx.is_contiguous() &&
                     idx.numel() * 8 == dy.numel(),
@@ -243,10 +250,10 @@ void BindModelOps(py::module_& m) {
   }, py::arg("x"), py::arg("weight"), py::arg("wait_ns") = kern::STEM_WAIT_NS);
 
   // (x, dy, weight) -> gradient of the weight
-  m.def("stem_conv_wgrad", [](const at::Tensor& x, const at::Tensor& dy, const at::Tensor& weight,
+  m.def("stem_conv_wgrad", [](const at::Tensor& x, at::Tensor dy, const at::Tensor& weight,
                               uint32_t wait_ns) {
     CheckActivations(x, "x");
-    CheckActivations(dy, "dy");
+    dy = Activations(dy, "dy");
     const int64_t N = x.size(0), H = x.size(2), W = x.size(3), C = weight.size(0);
     TORCH_CHECK(weight.scalar_type() == x.scalar_type() && weight.device() == x.device() &&
                     weight.dim() == 4 && weight.size(1) == 3 && weight.size(2) == 7 &&

@@ -422,6 +422,43 @@ def test_stem_convolution_whose_waits_run_out(channels):
     assert torch.equal(_C.stem_conv_wgrad(x, dy, w), dw)
 
 
+@pytest.mark.parametrize("offset", [1, 2, 4, 7])
+def test_activations_off_a_16_byte_boundary(offset):
+    """Slices of flat buffers as inputs and as gradients: the same results as
+    from tensors of their own."""
+    from horovod_b200.ops.batch_norm import batch_norm_act
+    from horovod_b200.ops.pooling import max_pool_3x3_s2
+    from horovod_b200.ops.stem_conv import StemConv2d
+    g = torch.Generator(device=_dev()).manual_seed(13)
+
+    def pair(n, c, h, w):
+        """The same values at an offset and on a boundary."""
+        flat = torch.randn(n * c * h * w + offset, device=_dev(), generator=g).bfloat16()
+        view = flat[offset:].view(n, h, w, c).permute(0, 3, 1, 2)
+        assert view.data_ptr() % 16 == 2 * offset
+        return view, view.clone(memory_format=torch.channels_last)
+
+    conv = StemConv2d(3, 16, 7, stride=2, padding=3, bias=False).to(_dev()).bfloat16()
+    cases = [
+        (lambda x: batch_norm_act(x, None, None, None, None), [pair(3, 16, 9, 7)]),
+        (lambda x, r: batch_norm_act(x, None, None, None, None, residual=r),
+         [pair(3, 16, 9, 7), pair(3, 16, 9, 7)]),
+        (max_pool_3x3_s2, [pair(3, 16, 9, 7)]),
+        (conv, [pair(3, 3, 18, 20)]), (conv, [pair(3, 3, 17, 19)]),
+    ]
+    for fn, inputs in cases:
+        dy, results = None, []
+        for which in (0, 1):
+            leaves = [p[which].detach().requires_grad_(fn is not conv) for p in inputs]
+            conv.weight.grad = None
+            y = fn(*leaves)
+            dy = dy or pair(*y.shape)
+            y.backward(dy[which])
+            results.append([y] + ([conv.weight.grad] if fn is conv else [t.grad for t in leaves]))
+        for a, b in zip(*results):
+            assert torch.equal(a, b)
+
+
 @pytest.mark.parametrize("momentum", [0.1, None])
 def test_batch_norm_counts_batches_once(momentum):
     from horovod_b200.ops.batch_norm import BatchNormAct2d
