@@ -89,6 +89,43 @@ def test_batch_norm_mask_without_the_output(shape, with_res, dtype):
     assert bool(((x.grad.double() - dx).abs() <= bound).all())
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("ratio", [1, 50, 300, 1000])
+def test_batch_norm_gradient_of_channels_far_from_zero(ratio, dtype):
+    """Means of up to `ratio` times the spread, and a gradient that follows x, so
+    that the terms of dx nearly cancel. Against the same formula in 64 bits with
+    the kernel's own statistics: left are the fp32 terms' roundings (2^-24 each, of
+    the terms' sizes; 2^-19 with those of the sums behind them) and that of the
+    result."""
+    from horovod_b200 import _C
+    dev, shape = _dev(), (4, 64, 31, 33)
+    g = torch.Generator(device=dev).manual_seed(14)
+
+    def column(v):
+        return v.double().view(1, -1, 1, 1)
+
+    mean = ratio * (0.5 + 0.5 * torch.rand(64, device=dev, generator=g))
+    mean[::2] *= -1
+    x = (torch.randn(shape, device=dev, generator=g) + mean.view(1, -1, 1, 1)).to(dtype)
+    x = x.contiguous(memory_format=torch.channels_last)
+    weight = 0.5 + torch.rand(64, device=dev, generator=g)
+    _, saved, _ = _C.bn_forward(x, None, weight, None, None, None, 0.1, 1e-5, False, None)
+    xc = x.double() - column(saved[0])
+    xhat = xc * column(saved[1])
+    # whole numbers: their sums are exact
+    dy = (30 * xhat + torch.randn(shape, device=dev, generator=g)).clamp(-200, 200).round()
+    dy = dy.to(dtype).contiguous(memory_format=torch.channels_last)
+    dx = _C.bn_backward(dy, x, weight, saved, None, False, False)[0].double()
+    dz, dims = dy.double(), (0, 2, 3)
+    scale = column(weight) * column(saved[1])
+    terms = [scale * dz, -scale * dz.mean(dims, keepdim=True),
+             -scale * xhat * (dz * xhat).mean(dims, keepdim=True)]
+    want = sum(terms)
+    eps = 2.0 ** (-8 if dtype == torch.bfloat16 else -11)
+    bound = eps * want.abs() + 2.0 ** -19 * sum(t.abs() for t in terms) + 6e-8
+    assert bool(((dx - want).abs() <= bound).all())
+
+
 def test_batch_norm_residual_without_a_gradient():
     from horovod_b200.ops.batch_norm import batch_norm_act
     g = torch.Generator(device=_dev()).manual_seed(4)
