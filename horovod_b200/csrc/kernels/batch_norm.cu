@@ -520,10 +520,16 @@ int bn_copies(int C) { return C <= 256 ? 8 : C < 2048 ? 2048 / C : 1; }
 // additions to the accumulators.
 constexpr int BN_CTAS_STATS = 148 * BN_MIN_BLOCKS_STATS;
 constexpr int BN_CTAS_REDUCE = 148 * BN_MIN_BLOCKS;
-// The kernels that write start with reading them, so tensors that fit L2 (126
-// MB) get one wave too: 256 x 256 x 14 x 14 forward 10.7 us, 15.5 with 1184
-// CTAs. Beyond that the time goes to HBM, where more and shorter CTAs even out
-// the SMs: 256 x 256 x 56 x 56 with residual 198 us, 216 with one wave.
+// The kernels that write start with reading the sums, which one wave of CTAs does
+// least often: small tensors get one. In large ones more and shorter CTAs even
+// out the SMs. The line lies where the two meet, which differs: with 64 to 1024
+// channels in bf16 both kernels together take, with one wave, against 1184 CTAs,
+//   16 Mi elements  forward 0.89-0.95 of the time  backward 0.92-0.96
+//   32 Mi                   0.96-1.00                       0.94-0.98
+//   64 Mi                   0.99-1.03                       0.96-1.01
+//   96 Mi                   1.02-1.04                       0.98-1.03
+//   192 Mi                  1.03-1.05                       0.98-1.03
+// (the higher figures with a residual).
 int bn_apply_ctas(int64_t M, int C) { return M * C <= (64 << 20) ? 148 * BN_MIN_BLOCKS : 148 * 8; }
 
 dim3 bn_grid(int64_t M, int C, int ctas) {
