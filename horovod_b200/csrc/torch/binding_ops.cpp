@@ -283,8 +283,10 @@ void BindModelOps(py::module_& m) {
   // ---- multi-tensor SGD ------------------------------------------------------
   // One step over a parameter list, in one launch per 256 tensors. bufs holds
   // a momentum buffer (or None) per parameter; it is empty when momentum is 0.
-  // Parameters without a gradient are passed over. Returns the positions of
-  // those that the kernel cannot take (see SgdReady), untouched.
+  // Parameters without a gradient are passed over. Returns whether it launched
+  // and the positions of those that the kernel cannot take (see SgdReady) or that
+  // have no buffer yet, untouched. Where one has a buffer that does not match
+  // it, nothing is launched: a step that fails leaves every parameter as it was.
   m.def("sgd_step", [](const std::vector<at::Tensor>& params,
                        const std::vector<c10::optional<at::Tensor>>& bufs, double lr,
                        double momentum, double dampening, double weight_decay, bool nesterov,
@@ -293,15 +295,22 @@ void BindModelOps(py::module_& m) {
     TORCH_CHECK(bufs.size() == (with_bufs ? params.size() : 0), "sgd_step: list lengths differ");
     std::vector<int64_t> rest;
     std::vector<size_t> ready;
+    bool launch = true;
     for (size_t i = 0; i < params.size(); ++i) {
       const at::Tensor& g = params[i].grad();
       if (!g.defined()) continue;
-      if (SgdReady(params[i], g) &&
-          (!with_bufs || (bufs[i].has_value() && SgdLike(params[i], *bufs[i]))))
+      bool taken = SgdReady(params[i], g);
+      if (taken && with_bufs) {
+        const bool exists = bufs[i].has_value() && bufs[i]->defined();
+        taken = exists && SgdLike(params[i], *bufs[i]);
+        if (exists && !taken) launch = false;
+      }
+      if (taken)
         ready.push_back(i);
       else
         rest.push_back(static_cast<int64_t>(i));
     }
+    if (!launch) return std::make_pair(false, rest);
     kern::SgdTensors t;
     size_t next = 0;
     while (next < ready.size()) {
@@ -331,7 +340,7 @@ void BindModelOps(py::module_& m) {
           at::cuda::getCurrentCUDAStream());
       TORCH_CHECK(err == cudaSuccess, "fused SGD: ", cudaGetErrorString(err));
     }
-    return rest;
+    return std::make_pair(true, rest);
   });
 }
 

@@ -1,12 +1,13 @@
 """``FusedSGD``: torch.optim.SGD arithmetic in one kernel launch per parameter
-group (csrc/kernels/fused_sgd.cu) instead of four to five elementwise passes.
+group (one per 256 tensors; csrc/kernels/fused_sgd.cu) instead of four to five
+elementwise passes.
 
 PyTorch's foreach SGD needs every tensor list to share strides for its
 multi-tensor fast path; with channels-last convolution weights two of its
 passes fall back to one launch per parameter (322 launches, 1.05 ms per step
 on ResNet-50 on a B200). This optimizer walks parameters, gradients and
-momentum buffers of any dense layout in one launch, reading and writing each
-element once. It is an ordinary ``torch.optim.Optimizer``: wrap it in
+momentum buffers of any dense layout together, reading and writing each element
+once. It is an ordinary ``torch.optim.Optimizer``: wrap it in
 ``hvd.DistributedOptimizer`` like any other; ``state_dict`` is compatible with
 ``torch.optim.SGD`` (``momentum_buffer`` per parameter). Parameters the kernel
 cannot take (CPU, non-fp32, sparse gradients, mismatched layouts) are updated
@@ -87,7 +88,15 @@ class FusedSGD(Optimizer):
             if group["momentum"] != 0:
                 get, nothing = self.state.get, {}
                 bufs = [get(p, nothing).get("momentum_buffer") for p in params]
-            rest = self._launch(params, bufs, group, first_step=False)
+            launched, rest = self._launch(params, bufs, group, first_step=False)
+            if not launched:
+                # A momentum buffer does not match its parameter; nothing has
+                # been updated yet.
+                for i in rest:
+                    bufs[i] = self._matching_buffer(params[i], bufs[i])
+                launched, rest = self._launch(params, bufs, group, first_step=False)
+                if not launched:
+                    raise RuntimeError("FusedSGD: a momentum buffer does not match its parameter")
             if rest:
                 self._step_rest([params[i] for i in rest], group)
         return loss
@@ -95,31 +104,34 @@ class FusedSGD(Optimizer):
     @staticmethod
     def _launch(params, bufs, group, first_step):
         """One native call checks, lists and updates all tensors it can; the
-        positions of the others come back."""
+        positions of the others come back, or of all that it would not take if
+        it has done nothing because a momentum buffer does not match."""
         return _extension().sgd_step(
             params, bufs, group["lr"], group["momentum"], group["dampening"],
             group["weight_decay"], group["nesterov"], first_step, group["maximize"])
 
+    def _matching_buffer(self, p, buf):
+        """The momentum buffer in p's memory layout (e.g. after a state_dict was
+        loaded)."""
+        if buf is not None and p.is_cuda and buf.stride() != p.stride():
+            fixed = torch.empty_like(p, memory_format=torch.preserve_format)
+            fixed.copy_(buf)
+            buf = self.state[p]["momentum_buffer"] = fixed
+        return buf
+
     def _step_rest(self, params, group):
-        """The parameters that the kernel cannot take as they are: new ones
-        (no momentum yet), a momentum buffer of another layout (e.g. loaded
-        from a state_dict), and those left to PyTorch."""
-        plists = {False: [], True: []}  # keyed by "this is the first step"
+        """The parameters that the kernel cannot take as they are: new ones (no
+        momentum yet), and those left to PyTorch."""
+        first = []
         for p in params:
             if group["momentum"] == 0 or not self._kernel_ok(p):
                 self._torch_update(p, group)
                 continue
-            state = self.state[p]
-            first = "momentum_buffer" not in state
-            if first:
-                state["momentum_buffer"] = torch.empty_like(
-                    p, memory_format=torch.preserve_format)
-            elif state["momentum_buffer"].stride() != p.stride():
-                fixed = torch.empty_like(p, memory_format=torch.preserve_format)
-                fixed.copy_(state["momentum_buffer"])
-                state["momentum_buffer"] = fixed
-            plists[first].append(p)
-        for first, plist in plists.items():
-            bufs = [self.state[p]["momentum_buffer"] for p in plist]
-            if plist and self._launch(plist, bufs, group, first):
-                raise RuntimeError("FusedSGD: a momentum buffer does not match its parameter")
+            self.state[p]["momentum_buffer"] = torch.empty_like(
+                p, memory_format=torch.preserve_format)
+            first.append(p)
+        if first:
+            bufs = [self.state[p]["momentum_buffer"] for p in first]
+            launched, rest = self._launch(first, bufs, group, first_step=True)
+            if rest or not launched:
+                raise RuntimeError("FusedSGD: the kernel does not take a parameter")

@@ -221,6 +221,51 @@ def test_fused_sgd_many_tensors(momentum):
     assert len(opt.state) == len(ref.state) or momentum == 0
 
 
+def test_fused_sgd_updates_all_or_nothing():
+    """A momentum buffer that the kernel cannot take leaves every parameter as
+    it was; one of another memory layout is put into the right one."""
+    from horovod_b200 import _C
+    from horovod_b200.torch.fused_sgd import FusedSGD
+    g = torch.Generator(device=_dev()).manual_seed(15)
+    shapes = [(5,), (8, 4, 3, 3), (7, 3), (2, 2)]
+    ps = [torch.randn(s, device=_dev(), generator=g) for s in shapes]
+    ps.append(torch.randn(3, device=_dev(), generator=g).double())  # left to PyTorch
+    qs = [p.clone().requires_grad_(True) for p in ps]
+    ps = [p.requires_grad_(True) for p in ps]
+    kwargs = dict(lr=0.1, momentum=0.9, weight_decay=1e-3)
+    opt, ref = FusedSGD(ps, **kwargs), torch.optim.SGD(qs, foreach=False, **kwargs)
+
+    def gradients():
+        for p, q in zip(ps, qs):
+            p.grad = torch.randn(p.shape, device=_dev(), generator=g).to(p.dtype)
+            q.grad = p.grad.clone()
+
+    def compare():
+        for p, q in zip(ps, qs):
+            torch.testing.assert_close(p, q, rtol=1e-5, atol=1e-6)
+
+    gradients()
+    opt.step()
+    ref.step()
+    compare()
+    good = opt.state[ps[2]]["momentum_buffer"]
+    opt.state[ps[1]]["momentum_buffer"] = opt.state[ps[1]]["momentum_buffer"].contiguous(
+        memory_format=torch.channels_last)
+    gradients()
+    for bad in (good.double(), good.cpu(), torch.zeros(6, 3, device=_dev())):
+        opt.state[ps[2]]["momentum_buffer"] = bad
+        before, launches = [p.detach().clone() for p in ps], _C.kernel_launch_count()
+        with pytest.raises(RuntimeError, match="momentum buffer"):
+            opt.step()
+        assert _C.kernel_launch_count() == launches
+        assert all(torch.equal(p, b) for p, b in zip(ps, before))
+    opt.state[ps[2]]["momentum_buffer"] = good
+    opt.step()
+    ref.step()
+    compare()
+    assert opt.state[ps[1]]["momentum_buffer"].stride() == ps[1].stride()
+
+
 @pytest.mark.parametrize("name", ["fp16", "bf16"])
 def test_compression_inside_the_kernel(hvd, name):
     """allreduce and grouped_allreduce of fp32 tensors with this library's
