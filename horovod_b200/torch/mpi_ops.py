@@ -298,7 +298,8 @@ def _cast_in_kernel(compression, tensors, average, op):
     kernel: one pass over the tensors instead of three (cast, reduce, cast
     back) and no launches and allocations per tensor. The compressors of this
     library on fp32 CUDA tensors; user-defined ones and everything else run
-    as they are. Depends on nothing that differs between ranks."""
+    as they are. Depends on the arguments only, and on the type and device of
+    the tensors, which the ranks of an allreduce have in common."""
     return bool((compression is Compression.fp16 or compression is Compression.bf16) and tensors
             and handle_average_backwards_compatibility(op, average) in (Average, Sum)
             and all(isinstance(t, torch.Tensor) and t.is_cuda and t.dtype == torch.float32
@@ -306,8 +307,10 @@ def _cast_in_kernel(compression, tensors, average, op):
 
 
 def _dense(tensor):
-    """What the cast of a compressor would have made of the tensor's layout."""
-    return tensor if _is_dense(tensor) else tensor.contiguous()
+    """The layout that a compressor's cast makes of the tensor's: a copy keeps
+    the strides of a dense tensor (which _check_tensor then refuses if they are
+    a permutation, as without compression) and closes the gaps of others."""
+    return tensor if _is_dense(tensor) else tensor.clone()
 
 
 class HorovodAllreduce(torch.autograd.Function):

@@ -294,6 +294,17 @@ def test_compression_inside_the_kernel(hvd, name):
         assert out.dtype == dtype and torch.equal(out, v)
 
 
+def test_compression_refuses_what_is_refused_without(hvd):
+    """Permuted tensors: with the casts inside the kernel as with those outside."""
+    x = torch.randn(4, 6, device=_dev())
+    for compression in (hvd.Compression.none, hvd.Compression.fp16, hvd.Compression.bf16):
+        for t in (x.t(), x.double().t(), x.cpu().t()):
+            with pytest.raises(ValueError, match="contiguous"):
+                hvd.allreduce(t, name="permuted", compression=compression)
+            with pytest.raises(ValueError, match="contiguous"):
+                hvd.grouped_allreduce([x, t], name="permuted.g", compression=compression)
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("shape,channels", [
     ((1, 3, 1, 1), 16), ((2, 3, 33, 17), 64), ((3, 3, 32, 16), 48),  # one past a tile, a tile

@@ -94,3 +94,32 @@ def test_utils_namespace_without_gpu():
     assert isinstance(u.gpu_backend(), str)
     topo = u.gpu_topology()
     assert "device_count" in topo
+
+
+def test_layouts_of_compressed_tensors():
+    """The copy made for a cast inside the kernel has the strides that the cast
+    outside has, dense or not, and is refused where that one is."""
+    from horovod_b200.torch.compression import Compression
+    from horovod_b200.torch.mpi_ops import _check_tensor, _dense
+    x = torch.randn(6, 8, 5, 7)
+    last = x.contiguous(memory_format=torch.channels_last)
+    forms = [x, last, x[:, ::2], last[:, ::2], last[:, :, 1:], x[..., 1:], last[..., ::3],
+             x.transpose(0, 1), x.permute(3, 0, 2, 1), x.permute(3, 0, 2, 1)[:, ::2],
+             x[0, 0].t(), x[:1].expand(3, 8, 5, 7),
+             torch.randn(1).expand(4), torch.randn(()), torch.empty(0), torch.empty(3, 0).t(),
+             torch.randn(2, 3, 4, 5, 6).contiguous(memory_format=torch.channels_last_3d)[:, 1:]]
+    refused = 0
+    for t in forms:
+        outside = Compression.fp16.compress(t)[0]
+        inside = _dense(t)
+        assert inside.stride() == outside.stride() and torch.equal(inside, t)
+        verdicts = []
+        for c in (inside, outside):
+            try:
+                _check_tensor(c, dense_ok=True)
+                verdicts.append(True)
+            except ValueError:
+                verdicts.append(False)
+        assert verdicts[0] == verdicts[1]
+        refused += not verdicts[0]
+    assert refused > 2
