@@ -1,6 +1,7 @@
 // Python entry points of the model-side kernels (fused batch normalisation).
 // They run on the caller's current CUDA stream like any torch op.
 #include <ATen/cuda/CUDAContext.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/extension.h>
 
@@ -45,8 +46,16 @@ const float* FloatPtrOrNull(const c10::optional<at::Tensor>& t, int64_t channels
 // call: slices are handed out from a per-stream pool that is cleared with one
 // memset whenever it has been used up. Slices are consumed in stream order
 // and the memset is queued behind their consumers, so a slice is zero when
-// the kernel that was given it runs.
-double* ZeroedDoubles(int64_t count, const at::Tensor& like, cudaStream_t stream) {
+// the kernel that was given it runs. A stream that is being captured gets memory
+// of its own, filled inside the graph (`own` keeps it until the launches are
+// queued): every replay has to start from zeros, and slices of the pool would be
+// cleared by none.
+double* ZeroedDoubles(int64_t count, const at::Tensor& like, cudaStream_t stream,
+                      at::Tensor* own) {
+  if (c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None) {
+    *own = at::zeros({count}, like.options().dtype(at::kDouble));
+    return own->data_ptr<double>();
+  }
   struct Pool {
     at::Tensor buf;
     int64_t used = 0;
@@ -117,7 +126,9 @@ void BindModelOps(py::module_& m) {
     at::Tensor saved = at::empty({3, C}, x.options().dtype(at::kFloat));
     at::Tensor signs;
     if (relu && res != nullptr) signs = at::empty({M, C / 8}, x.options().dtype(at::kByte));
-    double* sums = ZeroedDoubles(kern::BatchNormScratchDoubles(static_cast<int>(C)), x, stream);
+    at::Tensor own;
+    double* sums =
+        ZeroedDoubles(kern::BatchNormScratchDoubles(static_cast<int>(C)), x, stream, &own);
     float* rm = nullptr;
     float* rv = nullptr;
     if (running_mean.has_value() && running_mean->defined()) {
@@ -169,7 +180,9 @@ void BindModelOps(py::module_& m) {
     if (want_dresidual) dres = at::empty_like(x, x.options(), at::MemoryFormat::ChannelsLast);
     auto fopt = x.options().dtype(at::kFloat);
     at::Tensor dweight = at::empty({C}, fopt), dbias = at::empty({C}, fopt);
-    double* sums = ZeroedDoubles(kern::BatchNormScratchDoubles(static_cast<int>(C)), x, stream);
+    at::Tensor own;
+    double* sums =
+        ZeroedDoubles(kern::BatchNormScratchDoubles(static_cast<int>(C)), x, stream, &own);
     cudaError_t err = kern::LaunchBatchNormBackward(
         dy.data_ptr(), sign_bits, x.data_ptr(), dx.data_ptr(),
         want_dresidual ? dres.data_ptr() : nullptr, M, static_cast<int>(C),

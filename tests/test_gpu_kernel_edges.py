@@ -552,6 +552,62 @@ def test_activations_off_a_16_byte_boundary(offset):
             assert torch.equal(a, b)
 
 
+def test_model_kernels_in_a_replayed_graph():
+    """Stem convolution, batch norm, pooling and a batch norm with a residual,
+    forward and backward, captured twice (on one stream, as graphs are) and
+    replayed on new inputs, with other calls in between: as without a graph."""
+    import copy
+    from horovod_b200.ops import BatchNormAct2d
+    from horovod_b200.ops.pooling import MaxPool3x3s2
+    from horovod_b200.ops.stem_conv import StemConv2d
+    torch.manual_seed(16)
+
+    class Net(torch.nn.Module):
+        def __init__(self):
+            super().__init__()
+            self.conv = StemConv2d(3, 16, 7, stride=2, padding=3, bias=False)
+            self.bn1, self.bn2 = BatchNormAct2d(16, relu=True), BatchNormAct2d(16, relu=True)
+            self.pool = MaxPool3x3s2()
+
+        def forward(self, x):
+            with torch.autocast("cuda", dtype=torch.bfloat16):
+                y = self.pool(self.bn1(self.conv(x)))
+                return self.bn2(y, y)
+
+    def step(net, x, dy):
+        for p in net.parameters():
+            p.grad = None
+        y = net(x)
+        y.backward(dy)
+        return [y.detach()] + [p.grad for p in net.parameters()]
+
+    net = Net().to(_dev()).to(memory_format=torch.channels_last)
+    twin = copy.deepcopy(net)
+    x = torch.randn(9, 3, 61, 47, device=_dev()).contiguous(memory_format=torch.channels_last)
+    dy = torch.randn(9, 16, 16, 12, device=_dev()).bfloat16().contiguous(
+        memory_format=torch.channels_last)
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        step(net, x, dy)
+        step(twin, x, dy)
+    torch.cuda.current_stream().wait_stream(side)
+    graphs = [torch.cuda.CUDAGraph(), torch.cuda.CUDAGraph()]
+    results = []
+    for graph in graphs:
+        with torch.cuda.graph(graph):
+            results.append(step(net, x, dy))
+    for which in (0, 1, 1, 0, 1):
+        x.copy_(torch.randn_like(x))
+        graphs[which].replay()
+        captured = results[which]
+        for got, want in zip(captured, step(twin, x, dy)):
+            # the sums over CTAs come in any order: 16-bit values may round elsewhere
+            assert (got.double() - want.double()).norm() <= 1e-3 * want.double().norm()
+        for got, want in zip(net.buffers(), twin.buffers()):
+            torch.testing.assert_close(got, want)
+
+
 @pytest.mark.parametrize("momentum", [0.1, None])
 def test_batch_norm_counts_batches_once(momentum):
     from horovod_b200.ops.batch_norm import BatchNormAct2d
