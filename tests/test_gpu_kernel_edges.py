@@ -1,5 +1,7 @@
 """The model-side and single-rank kernels at the sizes where they can go wrong:
-remainders of their tiles and strips, and both sides of each dispatch rule."""
+remainders of their tiles and strips, both sides of each dispatch rule (but for
+pooling's 64-bit indices, which take tensors of 34 GB), and values that are not
+finite."""
 import pytest
 import torch
 import torch.nn.functional as F
@@ -87,6 +89,12 @@ def test_batch_norm_mask_without_the_output(shape, with_res, dtype):
     # 1e-5 of the largest: 32-bit terms that cancel; 6e-8: fp16's smallest step
     bound = eps * dx.abs() + 1e-5 * dx.abs().amax() + 6e-8
     assert bool(((x.grad.double() - dx).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("with_res", [False, True])
+def test_batch_norm_beyond_64_mi_elements(with_res):
+    """The writing kernels' other grid."""
+    test_batch_norm_mask_without_the_output((21, 64, 224, 224), with_res, torch.bfloat16)
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
@@ -178,6 +186,11 @@ def test_one_rank_collectives_move_every_element(hvd, dtype):
                         hvd.allreduce(x, op=hvd.Sum, prescale_factor=0.3, postscale_factor=1.7,
                                       name=name + ".ars")):
                 assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.int32, torch.int8])
+def test_one_rank_collectives_of_the_other_types(hvd, dtype):
+    test_one_rank_collectives_move_every_element(hvd, dtype)
 
 
 @pytest.mark.parametrize("wire", [torch.float16, torch.bfloat16])
@@ -335,6 +348,66 @@ def test_stem_convolution(shape, channels, dtype):
     assert (conv.weight.grad.double() - dw).norm() <= 1e-2 * dw.norm()
     # fp32 without autocast is PyTorch's
     assert conv._kernel_dtype(x) is None
+
+
+@pytest.mark.parametrize("shape,channels", [
+    ((8, 3, 224, 224), 80), ((8, 3, 225, 223), 128), ((40, 3, 97, 131), 64),
+])
+def test_stem_convolution_many_tiles_per_cta(shape, channels):
+    """Accumulators and buffers used again, at widths with one and with two
+    gradient CTAs per SM; every element against 64 bits, weights in PyTorch's own
+    memory format."""
+    from horovod_b200 import _C
+    g = torch.Generator(device=_dev()).manual_seed(17)
+    x = torch.randn(shape, device=_dev(), generator=g).bfloat16().contiguous(
+        memory_format=torch.channels_last)
+    w = torch.randn(channels, 3, 7, 7, device=_dev(), generator=g).bfloat16()
+    y = _C.stem_conv_forward(x, w)
+    dy = torch.randn(y.shape, device=_dev(), generator=g).bfloat16().contiguous(
+        memory_format=torch.channels_last)
+    dw = _C.stem_conv_wgrad(x, dy, w)
+    xd, wd, dyd = x.double(), w.double(), dy.double()
+
+    def wgrad(a, b):
+        return torch.nn.grad.conv2d_weight(a, w.shape, b, stride=2, padding=3)
+
+    for got, want, size in (
+            (y, F.conv2d(xd, wd, stride=2, padding=3),
+             F.conv2d(xd.abs(), wd.abs(), stride=2, padding=3)),
+            (dw, wgrad(xd, dyd), wgrad(xd.abs(), dyd.abs()))):
+        # one rounding to bf16, and the products' fp32 sums
+        bound = 2.0 ** -8 * want.abs() + 2e-5 * size
+        assert bool(((got.double() - want).abs() <= bound).all())
+    assert dw.stride() == w.stride()
+
+
+@pytest.mark.parametrize("width", [20, 21])
+def test_stem_convolution_in_a_16_bit_model(width):
+    """Without autocast, with an input that needs a gradient, and with gradients
+    of gradients, which are PyTorch's: next to an nn.Conv2d in 64 bits."""
+    from horovod_b200.ops.stem_conv import StemConv2d
+    g = torch.Generator(device=_dev()).manual_seed(18)
+    conv = StemConv2d(3, 32, 7, stride=2, padding=3, bias=False).to(_dev()).half()
+    ref = torch.nn.Conv2d(3, 32, 7, stride=2, padding=3, bias=False).to(_dev()).double()
+    ref.load_state_dict(conv.state_dict())
+    x = torch.randn(3, 3, 18, width, device=_dev(), generator=g).half().contiguous(
+        memory_format=torch.channels_last)
+    results = []
+    for module, dtype in ((conv, torch.float16), (ref, torch.float64)):
+        xi = x.to(dtype).requires_grad_(True)
+        y = module(xi)
+        gi = torch.Generator(device=_dev()).manual_seed(19)
+        dy = torch.randn(y.shape, device=_dev(), generator=gi).half().to(dtype)
+        dy.requires_grad_(True)
+        plain = torch.autograd.grad(y, [xi, module.weight], dy, retain_graph=True)
+        first = torch.autograd.grad(y, [xi, module.weight], dy, create_graph=True)
+        second = torch.autograd.grad(sum((t * t).sum() for t in first) * 1e-3,
+                                     [xi, module.weight, dy])
+        results.append([y, *plain, *first, *second])
+    assert conv._kernel_dtype(x) == torch.float16
+    for got, want in zip(*results):
+        # a few roundings to fp16 on the way: 2^-11 each
+        assert (got.double() - want).norm() <= 2e-3 * want.norm()
 
 
 def _kinds(t):
