@@ -441,11 +441,15 @@ int GpuOps::PickCtas(int64_t bytes) const {
 
 int GpuOps::LocalCtas(int64_t bytes) const {
   // A single rank waits for nobody: the whole GPU copies, at least 16 KB (two
-  // vectors per thread) to a CTA, and up to eight waves of CTAs, which even out
-  // the SMs (201 MB of fp32 through fp16: 75 us with 2368 CTAs, 89 with 296;
-  // 102 MB of fp32 37 and 38).
+  // vectors per thread) to a CTA, in one wave of CTAs. Above 80 MB eight waves,
+  // which even out the SMs; below, they cost more than that. fp32 with 296 and
+  // with 2368 CTAs: 32 MB 16.4 and 26.7 us, 64 MB 24.6 and 30.8, 80 MB 29.7 and
+  // 31.6, 100 MB 37.0 and 37.0, 128 MB 49.2 and 47.0, 400 MB 159 and 139; fp32
+  // through 50, 64, 80, 100 and 200 MB of fp16: 43.1 and 47.3, 57.4 and 65.6, 69.7
+  // and 69.8, 87.0 and 82.9, 177 and 141.
   if (forced_ctas_ > 0) return std::min(forced_ctas_, SYMM_MAX_BLOCKS);
-  return static_cast<int>(std::min<int64_t>(148 * 16, std::max<int64_t>(1, bytes >> 14)));
+  const int64_t most = bytes > (80 << 20) ? 148 * 16 : 148 * 2;
+  return static_cast<int>(std::min(most, std::max<int64_t>(1, bytes >> 14)));
 }
 
 kern::Algo GpuOps::PickAlgo(const SymmSet& set, DataType wire,
