@@ -9,21 +9,24 @@ Cases
                 variant): reads 161 ResNet-50-shaped gradient tensors, scales
                 and writes them back in one launch (read + write = 2x bytes).
   fused_fp16    same with float16 tensors.
-  reducescatter reduce-scatter kernel on one rank: stage -> reduce -> write
-                (read + write staging + read staging + write = 4x bytes).
+  reducescatter reduce-scatter of one rank: one pass of the fused allreduce
+                kernel's LOCAL variant (read + write = 2x bytes).
   exchange      allgather of one rank through the exchange kernel: with nobody
                 to send to it is one copy into the output (2x bytes).
   batch_norm    fused batch norm + residual + ReLU on a channels-last bf16
                 activation of 256 x 256 x 56 x 56 (411 MB): forward (statistics
-                pass + apply pass: read x twice, read the residual, write y =
-                4x bytes) and backward (reduce pass reads dy, y, x; apply pass
-                reads them again and writes dx and dres = 8x bytes), timed with
-                CUDA events on the current stream, next to the PyTorch eager
-                composition batch_norm -> add -> relu on the same tensors.
-
+                pass + apply pass: read x twice, read the residual, write y and
+                a bit per element = 4.0625x bytes) and backward (reduce pass
+                reads dy, x and the bits; apply pass reads them again and writes
+                dx and dres = 6.125x bytes), timed with CUDA events on the current
+                stream, next to the PyTorch eager composition batch_norm -> add ->
+                relu on the same tensors, which moves other bytes.
+  stem_conv     7x7 / stride 2 / padding 3 convolution of 256 images of 224 x 224
+                x 3 to 64 channels in bf16: forward reads x and writes y (488 MB),
+                the weights' gradient reads x and dy. Next to PyTorch's.
   max_pool      3x3 / stride 2 / padding 1 max pooling on the ResNet stem
                 activation 256 x 64 x 112 x 112 bf16 (411 MB): forward reads x,
-                writes y (1/4 of x) and one index byte per output element
+                writes y (1/4 of x) and half an index byte per output element
                 (1/16 of x): 1.3125x; backward reads dy and the indices and
                 writes dx: 1.3125x. Next to PyTorch's max_pool2d.
   fused_sgd     hvd.FusedSGD step (momentum + weight decay) over 161
@@ -110,8 +113,8 @@ def main():
                           "hbm_gbs_peak": hbm,
                           "clocks": clock_log.window(t_begin, t_end)}), flush=True)
 
-    cases = ["fused_local", "fused_fp16", "reducescatter", "exchange", "batch_norm", "max_pool",
-             "fused_sgd"] if args.case == "all" else [args.case]
+    cases = ["fused_local", "fused_fp16", "reducescatter", "exchange", "batch_norm", "stem_conv",
+             "max_pool", "fused_sgd"] if args.case == "all" else [args.case]
 
     def timed_events(fn, reps):
         for _ in range(args.warmup):
@@ -128,11 +131,13 @@ def main():
         return statistics.median(ts)
 
     def report_line(name, us, algorithmic, extra=None):
-        gbs = algorithmic / (us * 1e-6) / 1e9
-        print(json.dumps({"case": name, "device_us": round(us, 1),
-                          "algorithmic_gbs": round(gbs, 1),
-                          "frac_of_%s_hbm_copy" % peak_src: round(gbs / hbm, 3),
-                          "hbm_gbs_peak": hbm,
+        # (algorithmic is None for a path that moves other bytes.)
+        rate = {}
+        if algorithmic is not None:
+            gbs = algorithmic / (us * 1e-6) / 1e9
+            rate = {"algorithmic_gbs": round(gbs, 1),
+                    "frac_of_%s_hbm_copy" % peak_src: round(gbs / hbm, 3), "hbm_gbs_peak": hbm}
+        print(json.dumps({"case": name, "device_us": round(us, 1), **rate,
                           "clocks": clock_log.window(time.time() - 1.0, time.time()),
                           **(extra or {})}), flush=True)
     if "fused_local" in cases:
@@ -148,7 +153,7 @@ def main():
     if "reducescatter" in cases:
         n = min(nbytes, 448 << 20) // 4
         x = torch.randn(n, device=dev)
-        run("reducescatter", lambda: hvd.reducescatter(x, op=hvd.Sum, name="k.rs"), 6, 4 * n * 4)
+        run("reducescatter", lambda: hvd.reducescatter(x, op=hvd.Sum, name="k.rs"), 6, 2 * n * 4)
     if "exchange" in cases:
         n = min(nbytes, 192 << 20) // 4
         x = torch.randn(n, device=dev)
@@ -167,29 +172,6 @@ def main():
         rm, rv = torch.zeros(256, device=dev), torch.ones(256, device=dev)
         nbytes_act = x.numel() * 2
 
-        def timed(fn, reps):
-            for _ in range(args.warmup):
-                fn()
-            torch.cuda.synchronize()
-            ts = []
-            for _ in range(reps):
-                e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-                e0.record()
-                fn()
-                e1.record()
-                torch.cuda.synchronize()
-                ts.append(e0.elapsed_time(e1) * 1e3)
-            return statistics.median(ts)
-
-        def report(name, us, algorithmic):
-            gbs = algorithmic / (us * 1e-6) / 1e9
-            print(json.dumps({"case": name, "shape": list(shape), "device_us": round(us, 1),
-                              "algorithmic_gbs": round(gbs, 1),
-                              "frac_of_%s_hbm_copy" % peak_src: round(gbs / hbm, 3),
-                              "hbm_gbs_peak": hbm,
-                              "clocks": clock_log.window(time.time() - 1.0, time.time())}),
-                  flush=True)
-
         def eager_fwd():
             return F.relu(F.batch_norm(x, rm, rv, w, b, True, 0.1, 1e-5) + res)
 
@@ -197,15 +179,39 @@ def main():
             return batch_norm_act(x, w, b, rm, rv, residual=res, training=True, relu=True)
 
         for name, fwd in (("batch_norm_fused", fused_fwd), ("batch_norm_eager", eager_fwd)):
-            t_f = timed(lambda: fwd(), args.iters)
+            t_f = timed_events(fwd, args.iters)
             y = fwd()
 
             def bwd():
                 torch.autograd.grad(y, (x, res, w, b), go, retain_graph=True)
-            t_b = timed(bwd, args.iters)
-            report(name + "_forward", t_f, 4 * nbytes_act)
-            report(name + "_backward", t_b, 8 * nbytes_act)
+            t_b = timed_events(bwd, args.iters)
+            ours = name == "batch_norm_fused"
+            report_line(name + "_forward", t_f, 4.0625 * nbytes_act if ours else None,
+                        {"shape": list(shape)})
+            report_line(name + "_backward", t_b, 6.125 * nbytes_act if ours else None,
+                        {"shape": list(shape)})
             del y
+    if "stem_conv" in cases:
+        n = 256 if args.mb >= 512 else 64
+        x = torch.randn(n, 3, 224, 224, device=dev).bfloat16() \
+            .contiguous(memory_format=torch.channels_last)
+        w = torch.randn(64, 3, 7, 7, device=dev).bfloat16() \
+            .contiguous(memory_format=torch.channels_last)
+        dy = torch.randn_like(_C.stem_conv_forward(x, w))
+        moved = 2 * (x.numel() + dy.numel())
+
+        def torch_wgrad():
+            torch.ops.aten.convolution_backward(dy, x, w, None, [2, 2], [3, 3], [1, 1], False,
+                                                [0, 0], 1, [False, True, False])
+        for name, fwd, wgrad in (
+                ("stem_conv_fused", lambda: _C.stem_conv_forward(x, w),
+                 lambda: _C.stem_conv_wgrad(x, dy, w)),
+                ("stem_conv_torch",
+                 lambda: torch.nn.functional.conv2d(x, w, stride=2, padding=3), torch_wgrad)):
+            for which, fn in (("_forward", fwd), ("_weight_gradient", wgrad)):
+                us = timed_events(fn, args.iters)
+                report_line(name + which, us, moved if name == "stem_conv_fused" else None,
+                            {"shape": list(x.shape)})
     if "max_pool" in cases:
         import torch.nn.functional as F
         from horovod_b200.ops.pooling import max_pool_3x3_s2
@@ -219,8 +225,9 @@ def main():
             y = fwd(x)
             go = torch.randn_like(y)
             t_b = timed_events(lambda: torch.autograd.grad(y, x, go, retain_graph=True), args.iters)
-            report_line(name + "_forward", t_f, 1.3125 * xbytes, {"shape": list(x.shape)})
-            report_line(name + "_backward", t_b, 1.3125 * xbytes, {"shape": list(x.shape)})
+            moved = 1.3125 * xbytes if name == "max_pool_fused" else None
+            report_line(name + "_forward", t_f, moved, {"shape": list(x.shape)})
+            report_line(name + "_backward", t_b, moved, {"shape": list(x.shape)})
             del y
     if "fused_sgd" in cases:
         from horovod_b200.torch.fused_sgd import FusedSGD
