@@ -112,8 +112,8 @@ class FusedSGD(Optimizer):
 
     def _matching_buffer(self, p, buf):
         """The momentum buffer in p's memory layout (e.g. after a state_dict was
-        loaded)."""
-        if buf is not None and p.is_cuda and buf.stride() != p.stride():
+        loaded), if the kernel takes p at all."""
+        if buf is not None and self._kernel_ok(p) and buf.stride() != p.stride():
             fixed = torch.empty_like(p, memory_format=torch.preserve_format)
             fixed.copy_(buf)
             buf = self.state[p]["momentum_buffer"] = fixed

@@ -307,6 +307,24 @@ def test_compression_inside_the_kernel(hvd, name):
         assert out.dtype == dtype and torch.equal(out, v)
 
 
+def test_fused_sgd_leaves_the_buffers_of_other_types():
+    """A buffer that is put into another layout leaves those of parameters that
+    are PyTorch's as they are: fp32 sums of a 16-bit parameter stay fp32."""
+    from horovod_b200.torch.fused_sgd import FusedSGD
+    ps = [torch.zeros(4, 6, device=_dev(), dtype=d).requires_grad_(True)
+          for d in (torch.float32, torch.float16)]
+    opt = FusedSGD(ps, lr=0.5, momentum=0.5)
+    for p in ps:
+        p.grad = torch.ones_like(p)
+        opt.state[p]["momentum_buffer"] = torch.full((6, 4), 2.0 ** -13, device=_dev()).t()
+    opt.step()
+    # 1 + 2^-14 is a number of 24 bits, not of 11
+    assert opt.state[ps[0]]["momentum_buffer"].stride() == ps[0].stride()
+    for p in ps:
+        buf = opt.state[p]["momentum_buffer"]
+        assert buf.dtype == torch.float32 and bool((buf == 1 + 2.0 ** -14).all())
+
+
 def test_compression_refuses_what_is_refused_without(hvd):
     """Permuted tensors: with the casts inside the kernel as with those outside."""
     x = torch.randn(4, 6, device=_dev())
