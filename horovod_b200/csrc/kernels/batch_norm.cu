@@ -67,7 +67,9 @@ template <> struct Pair<__nv_bfloat16> {
 template <> struct Pair<__half> {
   using type = __half2;
   static __device__ __forceinline__ float2 widen(type v) { return __half22float2(v); }
-  static __device__ __forceinline__ type narrow(float a, float b) { return __floats2half2_rn(a, b); }
+  static __device__ __forceinline__ type narrow(float a, float b) {
+    return __floats2half2_rn(a, b);
+  }
 };
 
 // 8 channels of one row.
@@ -281,8 +283,9 @@ template <typename T, bool RELU, bool RES>
 __global__ void __launch_bounds__(BN_THREADS, BN_MIN_BLOCKS)
 bn_apply_kernel(const T* __restrict__ x, const T* __restrict__ res, T* __restrict__ y,
                 uint8_t* __restrict__ signs, int64_t M, int C, double inv_m, int copies,
-                const double* __restrict__ sums, const float* __restrict__ weight, const float* __restrict__ bias, float eps,
-                float momentum, float* __restrict__ saved, float* __restrict__ running_mean,
+                const double* __restrict__ sums, const float* __restrict__ weight,
+                const float* __restrict__ bias, float eps, float momentum,
+                float* __restrict__ saved, float* __restrict__ running_mean,
                 float* __restrict__ running_var, int64_t* __restrict__ batches) {
   const Tile t(C);
   const int by = gridDim.y - 1 - blockIdx.y;
@@ -567,7 +570,8 @@ int64_t BatchNormScratchDoubles(int channels) {
 // Launches the second kernel of a pair so that it may start while the first
 // one is still running (it waits for the results itself).
 template <typename... P, typename... A>
-static cudaError_t LaunchDependent(void (*kernel)(P...), dim3 grid, cudaStream_t stream, A... args) {
+static cudaError_t LaunchDependent(void (*kernel)(P...), dim3 grid, cudaStream_t stream,
+                                   A... args) {
   cudaLaunchAttribute attr;
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr.val.programmaticStreamSerializationAllowed = 1;

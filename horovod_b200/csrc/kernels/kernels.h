@@ -354,17 +354,15 @@ cudaError_t LaunchScaleBuffer(const void* in, void* out, int64_t count,
                               DataType dtype, double scale,
                               cudaStream_t stream);
 
-// Number of kernels of this library launched so far in this process (every
-// Launch* function counts the kernels it enqueues).
 // Training-mode batch normalisation on channels-last 16-bit activations
 // ([rows, channels] row-major), fused with the residual add and the ReLU.
 // `sums_zeroed` is a zero-filled scratch of BatchNormScratchDoubles(). Forward:
 // y = act(bn(x) [+ residual]); also writes `saved` (the rows batch mean, inverse
 // standard deviation and shift of [3, channels]), with a residual and a ReLU
 // `signs` (a byte per 8 channels: which outputs are above zero), and updates
-// the running statistics and the count of batches (when given). Backward: dx, optionally dresidual (=
-// gradient through the ReLU), dweight, dbias; `signs` is null when the forward
-// had no residual.
+// the running statistics and the count of batches (when given). Backward: dx,
+// optionally dresidual (= gradient through the ReLU), dweight, dbias; `signs` is
+// null when the forward had no residual.
 bool BatchNormSupported(int64_t rows, int channels);
 int64_t BatchNormScratchDoubles(int channels);
 cudaError_t LaunchBatchNormForward(const void* x, const void* residual, void* y, uint8_t* signs,
@@ -428,6 +426,8 @@ cudaError_t LaunchFusedSgd(const SgdTensors& t, float lr, float momentum, float 
                            float weight_decay, bool nesterov, bool first_step, bool maximize,
                            cudaStream_t stream);
 
+// Number of kernels of this library launched so far in this process (every
+// Launch* function counts the kernels it enqueues).
 uint64_t KernelLaunchCount();
 void CountKernelLaunches(int n);
 

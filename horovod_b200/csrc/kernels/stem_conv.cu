@@ -1,7 +1,7 @@
 // The first convolution of a ResNet, 7x7 / stride 2 / padding 3 on 3 channels,
 // forward and gradient of the weights, channels-last 16-bit, as an implicit
-// GEMM on the 5th-generation tensor cores. cuDNN has no sm_100 kernel for 3 channels and pads them to 4
-// for one of an older architecture.
+// GEMM on the 5th-generation tensor cores. cuDNN has no sm_100 kernel for 3
+// channels and pads them to 4 for one of an older architecture.
 //
 // Input pixels are taken in 2 x 2 blocks of 12 values (16 with padding): the
 // convolution is then 4x4 / stride 1 on 16 channels, 16 steps of K = 16, and

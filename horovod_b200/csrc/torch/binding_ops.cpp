@@ -34,7 +34,8 @@ at::Tensor Activations(const at::Tensor& t, const char* what) {
   return t.clone(at::MemoryFormat::ChannelsLast);
 }
 
-const float* FloatPtrOrNull(const c10::optional<at::Tensor>& t, int64_t channels, const char* what) {
+const float* FloatPtrOrNull(const c10::optional<at::Tensor>& t, int64_t channels,
+                            const char* what) {
   if (!t.has_value() || !t->defined()) return nullptr;
   TORCH_CHECK(t->is_cuda() && t->scalar_type() == at::kFloat && t->is_contiguous() &&
                   t->numel() == channels,

@@ -68,7 +68,8 @@ class StemConv2d(nn.Conv2d):
         another geometry, memory format or type, and what a custom autograd
         function cannot take part in: tracing, transforms, tensors and modes
         with an __torch_dispatch__ of their own."""
-        if not (type(x) in _PLAIN and type(self.weight) in _PLAIN and x.is_cuda and x.dim() == 4 and x.size(1) == 3 and x.numel() > 0
+        if not (type(x) in _PLAIN and type(self.weight) in _PLAIN
+                and x.is_cuda and x.dim() == 4 and x.size(1) == 3 and x.numel() > 0
                 and self.kernel_size == (7, 7) and self.stride == (2, 2)
                 and self.padding == (3, 3) and self.dilation == (1, 1) and self.groups == 1
                 and self.bias is None and self.padding_mode == "zeros"
