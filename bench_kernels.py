@@ -240,7 +240,7 @@ def main():
             opt = cls(ps, lr=0.01, momentum=0.9, weight_decay=1e-4)
             opt.step()  # creates the momentum buffers
             us = timed_events(opt.step, args.iters)
-            report_line(name + "_step_call", us, 5 * total,
+            report_line(name + "_step_call", us, 5 * total if cls is FusedSGD else None,
                         {"tensors": len(sizes), "payload_mb": total >> 20,
                          "note": "optimizer.step() as called by a training loop: bounded by "
                                  "its Python work when the GPU is otherwise idle"})
