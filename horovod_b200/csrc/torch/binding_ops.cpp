@@ -53,7 +53,10 @@ const float* FloatPtrOrNull(const c10::optional<at::Tensor>& t, int64_t channels
 // cleared by none.
 double* ZeroedDoubles(int64_t count, const at::Tensor& like, cudaStream_t stream,
                       at::Tensor* own) {
-  if (c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None) {
+  // (The default stream cannot be captured. Asking takes 0.2 to 0.4 us on the host,
+  // of 9.4 for a small forward.)
+  if (stream != nullptr &&
+      c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None) {
     *own = at::zeros({count}, like.options().dtype(at::kDouble));
     return own->data_ptr<double>();
   }
