@@ -563,6 +563,8 @@ bool bn_shape_ok(int64_t M, int C) {
 
 bool BatchNormSupported(int64_t rows, int channels) { return bn_shape_ok(rows, channels); }
 
+int BatchNormCopies(int channels) { return bn_copies(channels); }
+
 int64_t BatchNormScratchDoubles(int channels) {
   return static_cast<int64_t>(2) * bn_copies(channels) * channels;
 }
@@ -589,12 +591,15 @@ static cudaError_t ForwardTyped(const void* x, const void* res, void* y, uint8_t
                                 int C, double* sums, const float* weight, const float* bias,
                                 float eps, float momentum, float* saved, float* running_mean,
                                 float* running_var, int64_t* batches, bool relu,
-                                cudaStream_t stream) {
+                                bool summed, cudaStream_t stream) {
   const int copies = bn_copies(C);
-  bn_stats_kernel<T><<<bn_grid(M, C, BN_CTAS_STATS), BN_THREADS, 0, stream>>>(
-      static_cast<const T*>(x), M, C, copies, sums);
-  cudaError_t err = cudaGetLastError();
-  if (err != cudaSuccess) return err;
+  if (!summed) {
+    CountKernelLaunches(1);
+    bn_stats_kernel<T><<<bn_grid(M, C, BN_CTAS_STATS), BN_THREADS, 0, stream>>>(
+        static_cast<const T*>(x), M, C, copies, sums);
+    const cudaError_t err = cudaGetLastError();
+    if (err != cudaSuccess) return err;
+  }
   auto kernel = relu && res ? bn_apply_kernel<T, true, true>
                 : relu      ? bn_apply_kernel<T, true, false>
                 : res       ? bn_apply_kernel<T, false, true>
@@ -637,20 +642,20 @@ static cudaError_t BackwardTyped(const void* dy, const uint8_t* signs, const voi
 }
 
 cudaError_t LaunchBatchNormForward(const void* x, const void* residual, void* y, uint8_t* signs,
-                                   int64_t rows, int channels, bool bf16, double* sums_zeroed,
+                                   int64_t rows, int channels, bool bf16, double* sums,
                                    const float* weight, const float* bias, float eps,
                                    float momentum, float* saved, float* running_mean,
                                    float* running_var, int64_t* batches, bool relu,
-                                   cudaStream_t stream) {
+                                   cudaStream_t stream, bool summed) {
   if (!bn_shape_ok(rows, channels)) return cudaErrorInvalidValue;
   if (relu && residual != nullptr && signs == nullptr) return cudaErrorInvalidValue;
-  CountKernelLaunches(2);
-  return bf16 ? ForwardTyped<__nv_bfloat16>(x, residual, y, signs, rows, channels, sums_zeroed,
-                                            weight, bias, eps, momentum, saved, running_mean,
-                                            running_var, batches, relu, stream)
-              : ForwardTyped<__half>(x, residual, y, signs, rows, channels, sums_zeroed, weight,
-                                     bias, eps, momentum, saved, running_mean, running_var,
-                                     batches, relu, stream);
+  CountKernelLaunches(1);
+  return bf16 ? ForwardTyped<__nv_bfloat16>(x, residual, y, signs, rows, channels, sums, weight,
+                                            bias, eps, momentum, saved, running_mean, running_var,
+                                            batches, relu, summed, stream)
+              : ForwardTyped<__half>(x, residual, y, signs, rows, channels, sums, weight, bias,
+                                     eps, momentum, saved, running_mean, running_var, batches,
+                                     relu, summed, stream);
 }
 
 cudaError_t LaunchBatchNormBackward(const void* dy, const uint8_t* signs, const void* x, void* dx,

@@ -356,7 +356,8 @@ cudaError_t LaunchScaleBuffer(const void* in, void* out, int64_t count,
 
 // Training-mode batch normalisation on channels-last 16-bit activations
 // ([rows, channels] row-major), fused with the residual add and the ReLU.
-// `sums_zeroed` is a zero-filled scratch of BatchNormScratchDoubles(). Forward:
+// `sums` is a zero-filled scratch of BatchNormScratchDoubles(), or, for a forward
+// that is told so (`summed`), already holds the sums of x. Forward:
 // y = act(bn(x) [+ residual]); also writes `saved` (the rows batch mean, inverse
 // standard deviation and shift of [3, channels]), with a residual and a ReLU
 // `signs` (a byte per 8 channels: which outputs are above zero), and updates
@@ -365,12 +366,13 @@ cudaError_t LaunchScaleBuffer(const void* in, void* out, int64_t count,
 // null when the forward had no residual.
 bool BatchNormSupported(int64_t rows, int channels);
 int64_t BatchNormScratchDoubles(int channels);
+int BatchNormCopies(int channels);  // of the sums in it
 cudaError_t LaunchBatchNormForward(const void* x, const void* residual, void* y, uint8_t* signs,
-                                   int64_t rows, int channels, bool bf16, double* sums_zeroed,
+                                   int64_t rows, int channels, bool bf16, double* sums,
                                    const float* weight, const float* bias, float eps,
                                    float momentum, float* saved, float* running_mean,
                                    float* running_var, int64_t* batches, bool relu,
-                                   cudaStream_t stream);
+                                   cudaStream_t stream, bool summed = false);
 cudaError_t LaunchBatchNormBackward(const void* dy, const uint8_t* signs, const void* x, void* dx,
                                     void* dresidual, int64_t rows, int channels, bool bf16,
                                     double* sums_zeroed, const float* weight, const float* saved,
@@ -385,6 +387,20 @@ cudaError_t LaunchMaxPool3s2Forward(const void* x, void* y, uint32_t* idx, int n
                                     int channels, bool bf16, cudaStream_t stream);
 cudaError_t LaunchMaxPool3s2Backward(const void* dy, const uint32_t* idx, void* dx, int n, int h,
                                      int w, int channels, bool bf16, cudaStream_t stream);
+
+// Host-visible word per device that the tensor-core kernels set when a wait ran
+// out (the results of that call are NaN); null when there is none.
+int* TensorCoreStatusWord(int device);
+
+// Up to 4 arrays, each converted between fp32 and a 16-bit type in one launch.
+// Every array starts on a 16-byte boundary.
+struct CastArrays {
+  int n = 0;
+  const void* from[4];
+  void* to[4];
+  int64_t counts[4];
+};
+cudaError_t LaunchCastArrays(const CastArrays& a, bool widen, bool bf16, cudaStream_t stream);
 
 // 7x7 / stride 2 / padding 3 convolution of 3 channels-last 16-bit channels
 // ([n, h, w, 3]) without bias: y [n, (h - 1) / 2 + 1, (w - 1) / 2 + 1, channels].
@@ -404,6 +420,34 @@ int StemConvWgradCtas(int n, int h, int w, int channels);
 cudaError_t LaunchStemConvWgrad(const void* x, const void* dy, float* partial, void* dw,
                                 const int64_t* weight_strides, int n, int h, int w, int channels,
                                 bool bf16, cudaStream_t stream, uint32_t wait_ns = STEM_WAIT_NS);
+
+// 1x1 convolution of channels-last 16-bit activations, as the product
+//   y[rows, n] = x[rows, k] * w (+ add, where signs say so)
+// with w [n, k] (forward) or [k, n] (w_transposed: gradient of the input).
+// sums: also adds up sum(y) and sum(y * y) per channel, as LaunchBatchNormForward
+// does for itself, in `copies` copies of [2][n].
+// add: [rows, n], added in fp32 before y is rounded (y may be the same memory);
+// signs: a byte per 8 channels of it in bn_forward's order, which values count.
+// With a stride of 2, the rows are output pixels [images * height][width], and
+// x (strided_x) or y and add (strided_y) are the pixels of twice the height and
+// width, of which every other one in each direction takes part.
+struct Conv1x1 {
+  const void* x = nullptr;
+  const void* w = nullptr;
+  void* y = nullptr;
+  const void* add = nullptr;
+  const uint8_t* signs = nullptr;
+  double* sums = nullptr;
+  int copies = 0;
+  int64_t rows = 0;
+  int k = 0, n = 0;
+  bool w_transposed = false, strided_x = false, strided_y = false;
+  int width = 0;  // with a stride: of the output
+  bool bf16 = true;
+};
+bool Conv1x1Supported(int64_t rows, int k, int n);
+bool Conv1x1StrideSupported(int64_t rows, int width);
+cudaError_t LaunchConv1x1(const Conv1x1& c, cudaStream_t stream, uint32_t wait_ns = STEM_WAIT_NS);
 
 // Multi-tensor SGD step in one launch (torch.optim.SGD arithmetic: weight
 // decay added to the gradient, momentum buffer b = momentum * b + (1 -

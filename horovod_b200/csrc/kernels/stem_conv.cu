@@ -39,6 +39,7 @@
 #include <mutex>
 
 #include "kernels.h"
+#include "tensor_core.cuh"
 
 namespace hvd {
 namespace kern {
@@ -53,55 +54,6 @@ constexpr int PLANE_BYTES = PATCH * 16;
 constexpr uint16_t NAN16 = 0x7fff;  // a NaN of either 16-bit type
 constexpr int TAPS = 16, K_CORES = 2 * TAPS;  // 8 values of K each
 static_assert(PATCH <= THREADS, "one block per thread");
-
-__device__ __forceinline__ uint32_t smem_addr(const void* p) {
-  return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
-
-// Operand without a swizzle: `k_step` bytes between the two core matrices of
-// K = 16, `mn_step` bytes between groups of 8 rows (columns).
-__device__ __forceinline__ uint64_t operand(uint32_t addr, uint32_t k_step, uint32_t mn_step) {
-  return static_cast<uint64_t>((addr >> 4) & 0x3fffu) |
-         (static_cast<uint64_t>((k_step >> 4) & 0x3fffu) << 16) |
-         (static_cast<uint64_t>((mn_step >> 4) & 0x3fffu) << 32) | (1ull << 46);
-}
-
-__device__ __forceinline__ void mma(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, bool add) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(add ? 1u : 0u) : "memory");
-}
-
-// Waits until phase `parity` of the barrier is complete; false when that takes
-// longer than `limit` nanoseconds (0: at once).
-__device__ __forceinline__ bool wait_bounded(uint32_t bar, uint32_t parity, uint32_t limit) {
-  unsigned long long t0 = 0;
-  if (limit == 0) return false;
-  for (int i = 0;; ++i) {
-    uint32_t done;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(done) : "r"(bar), "r"(parity), "r"(10000u /* ns */) : "memory");
-    if (done) return true;
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    if (i == 0) t0 = t;
-    if (t - t0 > limit) return false;
-  }
-}
-
-template <typename T> __device__ __forceinline__ uint32_t narrow2(float a, float b);
-template <> __device__ __forceinline__ uint32_t narrow2<__nv_bfloat16>(float a, float b) {
-  const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
-  return *reinterpret_cast<const uint32_t*>(&v);
-}
-template <> __device__ __forceinline__ uint32_t narrow2<__half>(float a, float b) {
-  const __half2 v = __floats2half2_rn(a, b);
-  return *reinterpret_cast<const uint32_t*>(&v);
-}
 
 // Exponents of two 16-bit values in a word, and the lowest bit of each.
 template <typename T> struct Exponent;
@@ -288,9 +240,7 @@ stem_conv_forward_kernel(const uint16_t* __restrict__ x, const uint16_t* __restr
             operand(smem_addr(patch) + (tap / 4 * PATCH_W + tap % 4) * 16, PLANE_BYTES,
                     PATCH_W * 16),
             operand(smem_addr(weights) + tap * 2 * C * 16, C * 16, 128), idesc, tap > 0);
-      asm volatile(
-          "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
-          ::"r"(smem_addr(&s_bar)) : "memory");
+      commit(smem_addr(&s_bar));
     }
     TileAt next = at;
     if (tile + static_cast<int>(gridDim.x) < s.tiles) {
@@ -501,9 +451,7 @@ stem_conv_wgrad_kernel(const uint16_t* __restrict__ x, const uint4* __restrict__
               operand(smem_addr(patch) + acc % 2 * PLANE_BYTES +
                           (k * 2 + acc / 2 * 2) * PATCH_W * 16, PATCH_W * 16, 16),
               operand(smem_addr(grads) + k * 256, 128, DY_PLANE), idesc, issued > 0 || k > 0);
-      asm volatile(
-          "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
-          ::"r"(smem_addr(&s_bar[buffer])) : "memory");
+      commit(smem_addr(&s_bar[buffer]));
     }
   }
   // The last tile of each buffer.
@@ -584,9 +532,11 @@ stem_conv_wgrad_sum_kernel(const float* __restrict__ partial, uint16_t* __restri
   }
 }
 
+}  // namespace
+
 // Host-visible word per device that a kernel sets when a wait ran out; null
 // when there is no memory for them or no such device.
-int* StatusWord(int device) {
+int* TensorCoreStatusWord(int device) {
   constexpr int DEVICES = 64;
   static std::mutex mu;
   static int* words = nullptr;
@@ -604,8 +554,6 @@ int* StatusWord(int device) {
   }
   return words != nullptr && device >= 0 && device < DEVICES ? words + device : nullptr;
 }
-
-}  // namespace
 
 // Offsets inside a tile are 32-bit, 16 rows of the output at 128 channels being the
 // longest, as is the number of tiles.
@@ -639,12 +587,12 @@ static cudaError_t StemReady(int n, int h, int w, int channels, int** status) {
   int device = 0;
   const cudaError_t err = cudaGetDevice(&device);
   if (err != cudaSuccess) return err;
-  *status = StatusWord(device);
+  *status = TensorCoreStatusWord(device);
   return *status != nullptr ? cudaSuccess : cudaErrorMemoryAllocation;
 }
 
 bool StemConvFailed(int device, bool clear) {
-  volatile int* status = StatusWord(device);
+  volatile int* status = TensorCoreStatusWord(device);
   if (status == nullptr) return true;
   const bool failed = *status != 0;
   if (clear) *status = 0;
@@ -659,9 +607,7 @@ cudaError_t LaunchStemConvForward(const void* x, const void* weight, const int64
   if (err != cudaSuccess) return err;
   const StemShape s = MakeShape(n, h, w, channels, weight_strides);
   // fp32 accumulators, 16-bit operands, both K-major, M = 128, N = channels.
-  const uint32_t type = bf16 ? 1u : 0u;
-  const uint32_t idesc = (1u << 4) | (type << 7) | (type << 10) |
-                         (static_cast<uint32_t>(channels >> 3) << 17) | ((128u >> 4) << 24);
+  const uint32_t idesc = instruction(bf16, false, false, 128, channels);
   uint32_t columns = 32;  // a power of two; four CTAs share the SM's 512
   while (columns < static_cast<uint32_t>(channels)) columns *= 2;
   const int smem = 2 * PLANE_BYTES + K_CORES * channels * 16;
@@ -705,9 +651,7 @@ cudaError_t LaunchStemConvWgrad(const void* x, const void* dy, float* partial, v
   const StemShape s = MakeShape(n, h, w, channels, weight_strides);
   const int ctas = StemConvWgradCtas(n, h, w, channels);
   // As above, but both operands MN-major.
-  const uint32_t type = bf16 ? 1u : 0u;
-  const uint32_t idesc = (1u << 4) | (type << 7) | (type << 10) | (1u << 15) | (1u << 16) |
-                         (static_cast<uint32_t>(channels >> 3) << 17) | ((128u >> 4) << 24);
+  const uint32_t idesc = instruction(bf16, true, true, 128, channels);
   const int smem = 2 * (PATCH_BYTES + (channels / 8 * DY_PLANE + 127) / 128 * 128);
   const bool pairs = w % 2 == 0 && reinterpret_cast<uintptr_t>(x) % 4 == 0;
   auto kernel = bf16 ? (pairs ? stem_conv_wgrad_kernel<__nv_bfloat16, true>

@@ -33,6 +33,8 @@ void BindGpuDiagnostics(py::module_& m);
 // Defined in binding_testing.cpp.
 void BindTesting(py::module_& m);
 void BindModelOps(py::module_& m);
+void BindBlockOps(py::module_& m);
+void BindBottleneck(py::module_& m);
 void BindEmulation(py::module_& m);
 
 namespace {
@@ -662,5 +664,7 @@ PYBIND11_MODULE(_C, m) {
   BindGpuDiagnostics(m);
   BindTesting(m);
   BindModelOps(m);
+  BindBlockOps(m);
+  BindBottleneck(m);
   BindEmulation(m);
 }

@@ -12,10 +12,9 @@
 #include <vector>
 
 #include "../kernels/kernels.h"
+#include "model_ops.h"
 
 namespace hvd {
-
-namespace {
 
 void CheckActivations(const at::Tensor& t, const char* what) {
   TORCH_CHECK(t.is_cuda(), what, " must be a CUDA tensor");
@@ -83,6 +82,8 @@ double* ZeroedDoubles(int64_t count, const at::Tensor& like, cudaStream_t stream
   p.used += need;
   return out;
 }
+
+namespace {
 
 // Whether t holds fp32 values next to p's, element for element.
 bool SgdLike(const at::Tensor& p, const at::Tensor& t) {

@@ -1,0 +1,424 @@
+// A ResNet bottleneck block (1x1, 3x3, 1x1 convolutions with batch norms, ReLUs
+// and the skip connection) in training as one autograd node. What it saves over
+// the sequence of its layers, per block:
+//   - the statistics of a 1x1 convolution's output come from the convolution;
+//   - the gradient of the skip connection is never stored: the first
+//     convolution's gradient kernel adds dy where the block's output was above
+//     zero, in place of a store and a pass over three tensors;
+//   - the weights are cast in one launch, and so are their gradients.
+// The 3x3 convolution, the gradients of the weights and some 1x1 convolutions are
+// PyTorch's.
+#include <ATen/autocast_mode.h>
+#include <ATen/cuda/CUDAContext.h>
+#include <c10/core/impl/LocalDispatchKeySet.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <torch/extension.h>
+
+#include <array>
+#include <cstdint>
+#include <vector>
+
+#include "../kernels/kernels.h"
+#include "model_ops.h"
+
+namespace hvd {
+
+namespace {
+
+using at::Tensor;
+using torch::autograd::AutogradContext;
+using torch::autograd::Variable;
+using torch::autograd::variable_list;
+
+constexpr auto CL = at::MemoryFormat::ChannelsLast;
+
+// Layers of a block: the three convolutions in order, then the one of the
+// skip connection (its weights are undefined tensors where there is none).
+constexpr int LAYERS = 4, DOWN = 3;
+
+struct Norm {
+  Tensor mean, var, batches;
+  double momentum = 0.0, eps = 0.0;
+};
+
+struct Block {
+  std::array<Norm, LAYERS> norms;
+  int64_t stride = 1;
+  at::ScalarType type = at::kBFloat16;
+};
+
+cudaStream_t Stream() { return at::cuda::getCurrentCUDAStream(); }
+
+void Check(cudaError_t err, const char* what) {
+  TORCH_CHECK(err == cudaSuccess, what, ": ", cudaGetErrorString(err));
+}
+
+int64_t Rows(const Tensor& t) { return t.numel() / t.size(1); }
+int Channels(const Tensor& t) { return static_cast<int>(t.size(1)); }
+
+Tensor NewActivations(const Tensor& like, int64_t channels, int64_t h, int64_t w) {
+  return at::empty({like.size(0), channels, h, w}, like.options(), CL);
+}
+
+// Casts of up to LAYERS tensors in one launch; undefined ones are passed over.
+// The results have the strides of `layouts`, or of `from` where that is dense.
+std::array<Tensor, LAYERS> Cast(const std::array<Tensor, LAYERS>& from, at::ScalarType to,
+                                const std::array<Tensor, LAYERS>* layouts = nullptr) {
+  std::array<Tensor, LAYERS> out;
+  kern::CastArrays a;
+  bool bf16 = true;
+  for (int i = 0; i < LAYERS; ++i) {
+    const Tensor& f = from[i];
+    if (!f.defined()) continue;
+    if (f.scalar_type() == to) {
+      out[i] = f;
+      continue;
+    }
+    const Tensor& layout = layouts ? (*layouts)[i] : f;
+    if (layout.is_non_overlapping_and_dense()) {
+      out[i] = at::empty_strided(layout.sizes(), layout.strides(), f.options().dtype(to));
+      // The order of the elements in memory: strides of dimensions of size 1 do
+      // not matter.
+      bool same = true;
+      for (int64_t d = 0; d < f.dim(); ++d)
+        same = same && (f.size(d) == 1 || f.stride(d) == out[i].stride(d));
+      if (same && reinterpret_cast<uintptr_t>(f.data_ptr()) % 16 == 0) {
+        a.from[a.n] = f.data_ptr();
+        a.to[a.n] = out[i].data_ptr();
+        a.counts[a.n++] = f.numel();
+        bf16 = (to == at::kFloat ? f.scalar_type() : to) == at::kBFloat16;
+        continue;
+      }
+      out[i].copy_(f);
+    } else {
+      out[i] = f.to(to);
+    }
+  }
+  if (a.n > 0) Check(kern::LaunchCastArrays(a, to == at::kFloat, bf16, Stream()), "casts");
+  if (layouts == nullptr)
+    for (Tensor& t : out)  // the kernels' operands: rows of input channels, aligned
+      if (t.defined() && t.size(2) == 1 &&
+          (!t.is_contiguous() || reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 != 0))
+        t = t.clone(at::MemoryFormat::Contiguous);
+  return out;
+}
+
+// Sums of a batch norm's input: scratch, and whether the convolution filled it.
+struct Sums {
+  double* p = nullptr;
+  Tensor own;
+  bool ready = false;
+  Sums(const Tensor& like, int channels) {
+    p = ZeroedDoubles(kern::BatchNormScratchDoubles(channels), like, Stream(), &own);
+  }
+};
+
+// Whether the forward of a 1x1 convolution is this library's. Up to 512 input
+// channels it costs less than PyTorch's and the pass for the statistics; beyond,
+// PyTorch's kernels move the operands between L2 and the SMs less often (1024 to 256
+// channels, 50176 rows: 36 us against 25 and 7 for the statistics).
+bool OwnForward(int64_t rows, int64_t k, int64_t n) {
+  return k <= 512 && kern::Conv1x1Supported(rows, static_cast<int>(k), static_cast<int>(n));
+}
+
+// Whether y of a 1x1 convolution with a stride of 2 lies on every other pixel of x.
+bool EveryOther(const Tensor& x) {
+  return x.size(2) % 2 == 0 && x.size(3) % 2 == 0 &&
+         kern::Conv1x1StrideSupported(Rows(x) / 4, static_cast<int>(x.size(3) / 2));
+}
+
+Tensor ConvForward(const Tensor& x, const Tensor& w, int64_t stride, Sums* sums) {
+  const int64_t kernel = w.size(2), n = w.size(0);
+  const int64_t ho = (x.size(2) - 1) / stride + 1, wo = (x.size(3) - 1) / stride + 1;
+  if (kernel == 1 && OwnForward(x.size(0) * ho * wo, x.size(1), n) &&
+      (stride == 1 || (stride == 2 && EveryOther(x)))) {
+    kern::Conv1x1 c;
+    Tensor y = NewActivations(x, n, ho, wo);
+    c.x = x.data_ptr();
+    c.w = w.data_ptr();
+    c.y = y.data_ptr();
+    c.rows = Rows(y);
+    c.k = Channels(x);
+    c.n = static_cast<int>(n);
+    c.sums = sums->p;
+    c.copies = kern::BatchNormCopies(c.n);
+    c.strided_x = stride == 2;
+    c.width = static_cast<int>(wo);
+    c.bf16 = x.scalar_type() == at::kBFloat16;
+    Check(kern::LaunchConv1x1(c, Stream()), "1x1 convolution");
+    sums->ready = true;
+    return y;
+  }
+  const int64_t pad = kernel / 2;
+  return at::convolution(x, w, {}, {stride, stride}, {pad, pad}, {1, 1}, false, {0, 0}, 1)
+      .contiguous(CL);
+}
+
+// saved: what the backward needs of the statistics; signs: see LaunchBatchNormForward
+// (filled where there is a residual).
+Tensor NormForward(const Tensor& x, const Tensor& residual, const Tensor& weight,
+                   const Tensor& bias, const Norm& norm, bool relu, const Sums& sums,
+                   Tensor* saved, Tensor* signs) {
+  const int C = Channels(x);
+  Tensor y = at::empty_like(x, x.options(), CL);
+  *saved = at::empty({3, C}, x.options().dtype(at::kFloat));
+  if (residual.defined()) *signs = at::empty({Rows(x), C / 8}, x.options().dtype(at::kByte));
+  Check(kern::LaunchBatchNormForward(
+            x.data_ptr(), residual.defined() ? residual.data_ptr() : nullptr, y.data_ptr(),
+            residual.defined() ? signs->data_ptr<uint8_t>() : nullptr, Rows(x), C,
+            x.scalar_type() == at::kBFloat16, sums.p, FloatPtrOrNull(weight, C, "weight"),
+            FloatPtrOrNull(bias, C, "bias"), static_cast<float>(norm.eps),
+            static_cast<float>(norm.momentum), saved->data_ptr<float>(),
+            norm.mean.data_ptr<float>(), norm.var.data_ptr<float>(),
+            norm.batches.defined() ? norm.batches.data_ptr<int64_t>() : nullptr, relu, Stream(),
+            sums.ready),
+        "batch norm forward");
+  return y;
+}
+
+struct NormGradients {
+  Tensor x, residual, weight, bias;
+};
+
+// signs (where defined): dy counts where the block's output was above zero;
+// otherwise relu says whether this layer had a ReLU of its own.
+NormGradients NormBackward(const Tensor& dy, const Tensor& x, const Tensor& weight,
+                           const Tensor& saved, const Tensor& signs, bool relu,
+                           bool want_residual) {
+  const int C = Channels(x);
+  NormGradients g;
+  g.x = at::empty_like(x, x.options(), CL);
+  if (want_residual) g.residual = at::empty_like(x, x.options(), CL);
+  g.weight = at::empty({C}, x.options().dtype(at::kFloat));
+  g.bias = at::empty({C}, x.options().dtype(at::kFloat));
+  Sums sums(x, C);
+  Check(kern::LaunchBatchNormBackward(
+            dy.data_ptr(), signs.defined() ? signs.data_ptr<uint8_t>() : nullptr, x.data_ptr(),
+            g.x.data_ptr(), want_residual ? g.residual.data_ptr() : nullptr, Rows(x), C,
+            x.scalar_type() == at::kBFloat16, sums.p, FloatPtrOrNull(weight, C, "weight"),
+            saved.data_ptr<float>(), g.weight.data_ptr<float>(), g.bias.data_ptr<float>(), relu,
+            Stream()),
+        "batch norm backward");
+  return g;
+}
+
+// PyTorch's gradients of a convolution: of the input (where wanted) and the weight.
+std::pair<Tensor, Tensor> ConvBackward(const Tensor& dy, const Tensor& x, const Tensor& w,
+                                       int64_t stride, bool want_x, bool want_w) {
+  if (!want_x && !want_w) return {};
+  const int64_t pad = w.size(2) / 2;
+  auto g = at::convolution_backward(dy, x, w, c10::nullopt, {stride, stride}, {pad, pad}, {1, 1},
+                                    false, {0, 0}, 1, {want_x, want_w, false});
+  return {want_x ? std::get<0>(g).contiguous(CL) : Tensor(), std::get<1>(g)};
+}
+
+// Gradient of a 1x1 convolution's input, plus `add` (where `signs`, if defined, say
+// so). every_other: the result is `add` itself, changed at every other pixel.
+Tensor ConvInputGradient(const Tensor& dy, const Tensor& w, const Tensor& add, const Tensor& signs,
+                         bool every_other) {
+  kern::Conv1x1 c;
+  Tensor dx = every_other ? add : at::empty_like(add, add.options(), CL);
+  c.x = dy.data_ptr();
+  c.w = w.data_ptr();
+  c.y = dx.data_ptr();
+  c.add = add.data_ptr();
+  if (signs.defined()) c.signs = signs.data_ptr<uint8_t>();
+  c.rows = Rows(dy);
+  c.k = Channels(dy);
+  c.n = Channels(dx);
+  c.w_transposed = true;
+  c.strided_y = every_other;
+  c.width = static_cast<int>(dy.size(3));
+  c.bf16 = dy.scalar_type() == at::kBFloat16;
+  Check(kern::LaunchConv1x1(c, Stream()), "gradient of a 1x1 convolution");
+  return dx;
+}
+
+// The block by PyTorch's operations, for gradients of its gradients.
+Tensor Composition(const Tensor& x, const std::array<Tensor, LAYERS>& w,
+                   const std::array<Tensor, LAYERS>& g, const std::array<Tensor, LAYERS>& b,
+                   const std::vector<double>& eps, int64_t stride) {
+  auto layer = [&](int i, const Tensor& in, int64_t s) {
+    const int64_t pad = w[i].size(2) / 2;
+    const Tensor out = at::convolution(in, w[i].to(in.scalar_type()), {}, {s, s}, {pad, pad},
+                                       {1, 1}, false, {0, 0}, 1);
+    return at::batch_norm(out, g[i], b[i], {}, {}, true, 0.0, eps[i], true);
+  };
+  const Tensor a1 = at::relu(layer(0, x, 1)), a2 = at::relu(layer(1, a1, stride));
+  const Tensor skip = w[DOWN].defined() ? layer(DOWN, x, stride) : x;
+  return at::relu(layer(2, a2, 1) + skip);
+}
+
+class Bottleneck : public torch::autograd::Function<Bottleneck> {
+ public:
+  static Variable forward(AutogradContext* ctx, const Variable& x, const Variable& w0,
+                          const Variable& g0, const Variable& b0, const Variable& w1,
+                          const Variable& g1, const Variable& b1, const Variable& w2,
+                          const Variable& g2, const Variable& b2,
+                          const c10::optional<Tensor>& w3o, const c10::optional<Tensor>& g3o,
+                          const c10::optional<Tensor>& b3o, const Block& block) {
+    const bool down = w3o.has_value();
+    const Tensor w3 = down ? *w3o : Tensor(), g3 = down ? *g3o : Tensor(),
+                 b3 = down ? *b3o : Tensor();
+    c10::impl::ExcludeDispatchKeyGuard no_autocast(c10::DispatchKey::AutocastCUDA);
+    const std::array<Tensor, LAYERS> weights = {w0, w1, w2, w3}, gammas = {g0, g1, g2, g3},
+                                     betas = {b0, b1, b2, b3};
+    c10::cuda::CUDAGuard guard(x.device());
+    const auto w = Cast(weights, block.type);
+    std::array<Tensor, LAYERS> out, saved;  // of the convolutions; of the batch norms
+    Tensor signs;
+    auto layer = [&](int i, const Tensor& in, int64_t stride, const Tensor& residual) {
+      Sums sums(x, static_cast<int>(w[i].size(0)));
+      out[i] = ConvForward(in, w[i], stride, &sums);
+      return NormForward(out[i], residual, gammas[i], betas[i], block.norms[i], i != DOWN, sums,
+                         &saved[i], &signs);
+    };
+    const Tensor a1 = layer(0, x, 1, {});
+    const Tensor a2 = layer(1, a1, block.stride, {});
+    const Tensor skip = down ? layer(DOWN, x, block.stride, {}) : x;
+    const Tensor y = layer(2, a2, 1, skip);
+    // Like relu's own backward, this one refuses to run when somebody has
+    // changed y in place, although it does not read it.
+    variable_list keep = {x, y, a1, a2, signs};
+    for (int i = 0; i < (down ? LAYERS : DOWN); ++i)
+      for (const Tensor& t : {w[i], gammas[i], betas[i], out[i], saved[i]}) keep.push_back(t);
+    ctx->save_for_backward(keep);
+    std::vector<double> eps;
+    for (const Norm& norm : block.norms) eps.push_back(norm.eps);
+    ctx->saved_data["eps"] = eps;
+    ctx->saved_data["stride"] = block.stride;
+    // For gradients of gradients only; a backward of the usual kind works on the
+    // casts, and the weights may have changed since.
+    ctx->saved_data["weights"] =
+        std::vector<Tensor>(weights.begin(), weights.begin() + (down ? LAYERS : DOWN));
+    return y;
+  }
+
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const variable_list keep = ctx->get_saved_variables();
+    const Tensor &x = keep[0], &a1 = keep[2], &a2 = keep[3], &signs = keep[4];
+    const bool down = keep.size() > 5 + 5 * DOWN;
+    const int64_t stride = ctx->saved_data["stride"].toInt();
+    const std::vector<Tensor> leaves = ctx->saved_data["weights"].toTensorVector();
+    std::array<Tensor, LAYERS> w, gammas, betas, out, saved, weights;
+    for (int i = 0; i < (down ? LAYERS : DOWN); ++i) {
+      const size_t at = 5 + 5 * static_cast<size_t>(i);
+      w[i] = keep[at], gammas[i] = keep[at + 1], betas[i] = keep[at + 2], out[i] = keep[at + 3],
+      saved[i] = keep[at + 4], weights[i] = leaves[i];
+    }
+    // Inputs: x, then weight, gamma and beta of each layer.
+    variable_list result(1 + 3 * LAYERS + 1);
+    if (!grads[0].defined()) return result;
+    auto wanted = [&](int input) { return ctx->needs_input_grad(input); };
+    if (at::GradMode::is_enabled()) {
+      variable_list inputs;
+      std::vector<size_t> to;
+      auto add = [&](size_t i, const Tensor& t) {
+        if (t.defined() && wanted(static_cast<int>(i))) inputs.push_back(t), to.push_back(i);
+      };
+      add(0, x);
+      for (int i = 0; i < LAYERS; ++i)
+        add(1 + 3 * i, weights[i]), add(2 + 3 * i, gammas[i]), add(3 + 3 * i, betas[i]);
+      const Tensor y =
+          Composition(x, weights, gammas, betas, ctx->saved_data["eps"].toDoubleVector(), stride);
+      const variable_list g = torch::autograd::grad({y}, inputs, {grads[0]}, true, true, true);
+      for (size_t i = 0; i < to.size(); ++i) result[to[i]] = g[i];
+      return result;
+    }
+    c10::cuda::CUDAGuard guard(x.device());
+    Tensor dy = grads[0];
+    if (dy.scalar_type() != x.scalar_type()) dy = dy.to(x.scalar_type());
+    dy = Activations(dy.contiguous(CL), "dy");
+    std::array<Tensor, LAYERS> dw;
+    auto norm = [&](int i, const Tensor& d, const Tensor& mask, bool want_residual) {
+      NormGradients g = NormBackward(d, out[i], gammas[i], saved[i], mask, true, want_residual);
+      if (wanted(2 + 3 * i)) result[2 + 3 * i] = g.weight;
+      if (wanted(3 + 3 * i)) result[3 + 3 * i] = g.bias;
+      return g;
+    };
+    const bool want_x = wanted(0);
+    // The gradients of x through the first convolution and through the skip
+    // connection meet in a kernel of this library where it takes the shapes.
+    const bool fused = kern::Conv1x1Supported(Rows(x), Channels(out[0]), Channels(x));
+    const NormGradients g3 = norm(2, dy, signs, want_x && !down && !fused);
+    Tensor da2, da1, dx, skip = down ? Tensor() : fused ? dy : g3.residual, mask;
+    if (!down && fused) mask = signs;
+    std::tie(da2, dw[2]) = ConvBackward(g3.x, a2, w[2], 1, true, wanted(7));
+    const Tensor d2 = norm(1, da2, {}, false).x;
+    da2.reset();
+    std::tie(da1, dw[1]) = ConvBackward(d2, a1, w[1], stride, true, wanted(4));
+    const Tensor d1 = norm(0, da1, {}, false).x;
+    da1.reset();
+    if (down) {
+      const Tensor dd = norm(DOWN, dy, signs, false).x;
+      const bool scatter = stride == 2 && EveryOther(x) &&
+                           kern::Conv1x1Supported(Rows(dd), Channels(dd), Channels(x));
+      if (want_x && scatter) {
+        // Its gradient of x is zero but for every fourth pixel: added in place.
+        std::tie(dx, dw[0]) = ConvBackward(d1, x, w[0], 1, true, wanted(1));
+        ConvInputGradient(dd, w[DOWN], dx, {}, true);
+        dw[DOWN] = ConvBackward(dd, x, w[DOWN], stride, false, wanted(10)).second;
+      } else {
+        std::tie(skip, dw[DOWN]) = ConvBackward(dd, x, w[DOWN], stride, want_x, wanted(10));
+      }
+    }
+    if (!dx.defined()) {
+      std::tie(dx, dw[0]) = ConvBackward(d1, x, w[0], 1, want_x && !fused, wanted(1));
+      if (want_x) dx = fused ? ConvInputGradient(d1, w[0], skip, mask, false) : dx.add_(skip);
+    }
+    if (want_x) result[0] = dx;
+    for (int i = 0; i < LAYERS; ++i)
+      if (dw[i].defined() && weights[i].scalar_type() != at::kFloat) {
+        result[1 + 3 * i] = dw[i];
+        dw[i].reset();
+      }
+    const auto wide = Cast(dw, at::kFloat, &weights);
+    for (int i = 0; i < LAYERS; ++i)
+      if (wide[i].defined()) result[1 + 3 * i] = wide[i];
+    return result;
+  }
+};
+
+}  // namespace
+
+void BindBottleneck(py::module_& m) {
+  // (x, [weight, gamma, beta, running mean, running variance, count of batches or
+  //  None] per layer, [(momentum, eps)] per layer, stride)
+  m.def("bottleneck", [](const Tensor& x, const std::vector<std::vector<c10::optional<Tensor>>>& layers,
+                         const std::vector<std::pair<double, double>>& rates, int64_t stride) {
+    TORCH_CHECK(layers.size() >= DOWN && layers.size() <= LAYERS && rates.size() == layers.size(),
+                "bottleneck: three or four layers");
+    CheckActivations(x, "x");
+    Block block;
+    block.stride = stride;
+    block.type = x.scalar_type();
+    std::array<Tensor, 3 * LAYERS> p;
+    for (size_t i = 0; i < layers.size(); ++i) {
+      TORCH_CHECK(layers[i].size() == 6, "bottleneck: six tensors per layer");
+      for (int k = 0; k < 5; ++k)
+        TORCH_CHECK(layers[i][k].has_value() && layers[i][k]->is_cuda(),
+                    "bottleneck: tensors of a layer must be on the GPU");
+      for (int k = 0; k < 3; ++k) p[3 * i + k] = *layers[i][k];
+      TORCH_CHECK(p[3 * i].dim() == 4, "bottleneck: weights of convolutions are 4-D");
+      const int64_t C = p[3 * i].size(0);
+      for (int k = 1; k < 5; ++k) FloatPtrOrNull(layers[i][k], C, "a batch norm's tensor");
+      Norm& n = block.norms[i];
+      n.mean = *layers[i][3];
+      n.var = *layers[i][4];
+      if (layers[i][5].has_value()) n.batches = *layers[i][5];
+      TORCH_CHECK(!n.batches.defined() || (n.batches.is_cuda() && n.batches.numel() == 1 &&
+                                           n.batches.scalar_type() == at::kLong),
+                  "num_batches_tracked must be one int64 on the GPU");
+      n.momentum = rates[i].first;
+      n.eps = rates[i].second;
+    }
+    py::gil_scoped_release unlocked;
+    auto skip = [&](int k) {
+      return p[k].defined() ? c10::optional<Tensor>(p[k]) : c10::nullopt;
+    };
+    return Bottleneck::apply(x, p[0], p[1], p[2], p[3], p[4], p[5], p[6], p[7], p[8], skip(9),
+                             skip(10), skip(11), block);
+  });
+}
+
+}  // namespace hvd

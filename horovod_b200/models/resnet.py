@@ -8,6 +8,7 @@ import torch
 import torch.nn as nn
 
 from horovod_b200.ops.batch_norm import BatchNormAct2d
+from horovod_b200.ops.bottleneck import fused_bottleneck, fused_bottleneck_available
 from horovod_b200.ops.pooling import MaxPool3x3s2
 from horovod_b200.ops.stem_conv import StemConv2d
 
@@ -18,7 +19,8 @@ class Bottleneck(nn.Module):
     def __init__(self, inplanes, planes, stride=1, downsample=None):
         super().__init__()
         # Each batch norm carries its ReLU (and, for the last one, the residual
-        # add): one fused kernel pair on the GPU, plain PyTorch ops elsewhere.
+        # add): one fused kernel pair on the GPU, plain PyTorch ops elsewhere. In
+        # training on the GPU the whole block is one node (ops/bottleneck.py).
         self.conv1 = nn.Conv2d(inplanes, planes, 1, bias=False)
         self.bn1 = BatchNormAct2d(planes, relu=True)
         self.conv2 = nn.Conv2d(planes, planes, 3, stride=stride, padding=1, bias=False)
@@ -28,6 +30,9 @@ class Bottleneck(nn.Module):
         self.downsample = downsample
 
     def forward(self, x):
+        layers = fused_bottleneck_available(self, x)
+        if layers is not None:
+            return fused_bottleneck(x, layers)
         identity = x
         out = self.bn1(self.conv1(x))
         out = self.bn2(self.conv2(out))

@@ -26,14 +26,18 @@ def _extension():
     return _C
 
 
-def _enabled(device):
-    if os.environ.get("HOROVOD_B200_FUSED_STEM", "1") != "1":
-        return False
+def tensor_core_kernels_enabled(device):
+    """False from when a wait inside one of them has run out on the device."""
     if _extension().stem_conv_failed(device.index):
-        warnings.warn("a wait inside the stem convolution's kernel ran out on %s; the results of "
-                      "that call are NaN, and PyTorch's convolution runs from now on" % device)
+        warnings.warn("a wait inside a convolution's kernel ran out on %s; the results of that "
+                      "call are NaN, and PyTorch's convolution runs from now on" % device)
         return False
     return True
+
+
+def _enabled(device):
+    return os.environ.get("HOROVOD_B200_FUSED_STEM", "1") == "1" and \
+        tensor_core_kernels_enabled(device)
 
 
 class _StemConv(torch.autograd.Function):

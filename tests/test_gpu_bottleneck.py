@@ -1,0 +1,396 @@
+"""The ResNet block as one node: the 1x1 convolution kernels at the edges of
+their tiles, the block against its layers and against 64 bits, and what is left to
+the layers."""
+import copy
+
+import pytest
+import torch
+import torch.nn as nn
+
+pytestmark = pytest.mark.gpu
+CL = torch.channels_last
+
+
+def _dev():
+    return torch.device("cuda", 0)
+
+
+def _act(g, n, c, h, w, dtype):
+    return torch.randn(n, h, w, c, device=_dev(), generator=g).to(dtype).permute(0, 3, 1, 2)
+
+
+def _signs(mask):
+    """A byte per 8 channels: even channels in the low nibble, odd ones above."""
+    m = mask.permute(0, 2, 3, 1).reshape(-1, mask.size(1) // 8, 8).int()
+    bits = sum(m[..., c] << i for i, c in enumerate([0, 2, 4, 6, 1, 3, 5, 7]))
+    return bits.to(torch.uint8).contiguous()
+
+
+def _close(got, want, dtype):
+    """One rounding of every value to 16 bits (half a unit in the last place), and
+    the order of the fp32 sums, which is far below it."""
+    half_ulp = {torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -11}[dtype]
+    err = (got.double() - want).abs()
+    lim = half_ulp * want.abs() + 1e-4 * want.abs().max()
+    assert bool((err <= lim).all()), (err - lim).max().item()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("n,k,co,h,w", [
+    (1, 64, 64, 1, 1),        # one row
+    (1, 64, 128, 8, 16),      # exactly one tile
+    (3, 128, 64, 11, 13),     # a ragged second and third one
+    (2, 192, 320, 9, 7),      # channels that are multiples of 64 only
+    (4, 512, 2048, 7, 7),     # a few rows, many columns of tiles
+    (16, 256, 128, 35, 35),   # tiles of 128 columns
+    (32, 64, 256, 29, 28),    # tiles of 256 columns, several per CTA, a ragged last one
+    (1, 64, 64, 128, 2),      # (with a stride) rows of one pixel, of 128
+    (1, 64, 64, 2, 128),
+])
+def test_conv1x1_kernels(dtype, n, k, co, h, w):
+    from horovod_b200 import _C
+    g = torch.Generator(device=_dev()).manual_seed(1)
+    weight = (torch.randn(co, k, device=_dev(), generator=g) / k ** 0.5).to(dtype)
+    x, dy, add = _act(g, n, k, h, w, dtype), _act(g, n, co, h, w, dtype), _act(g, n, k, h, w, dtype)
+    y, sums = _C.conv1x1(x, weight, want_sums=True)
+    _close(y, torch.einsum("nkhw,ok->nohw", x.double(), weight.double()), dtype)
+    rows = y.double().permute(0, 2, 3, 1).reshape(-1, co)
+    # fp32 sums of what was stored: 2^-24 of the terms' magnitudes per addition,
+    # a few hundred additions in a row at most
+    for got, terms in ((sums[0], rows), (sums[1], rows * rows)):
+        assert bool(((got - terms.sum(0)).abs() <= 2e-5 * terms.abs().sum(0) + 1e-12).all())
+    assert torch.equal(_C.conv1x1(x, weight)[0], y)
+    ref = torch.einsum("nohw,ok->nkhw", dy.double(), weight.double())
+    _close(_C.conv1x1(dy, weight, w_transposed=True)[0], ref, dtype)
+    _close(_C.conv1x1(dy, weight, w_transposed=True, add=add)[0], ref + add.double(), dtype)
+    mask = torch.rand(n, k, h, w, device=_dev(), generator=g) > 0.5
+    _close(_C.conv1x1(dy, weight, w_transposed=True, add=add, signs=_signs(mask))[0],
+           ref + add.double() * mask, dtype)
+    # every other pixel of twice the size
+    big = _act(g, n, k, 2 * h, 2 * w, dtype)
+    wide = big.double()
+    wide[:, :, ::2, ::2] += ref
+    _close(_C.conv1x1(dy, weight, w_transposed=True, add=big, scatter=True)[0], wide, dtype)
+    y2, sums2 = _C.conv1x1(big, weight, gather=True, want_sums=True)
+    y3, sums3 = _C.conv1x1(big[:, :, ::2, ::2].contiguous(memory_format=CL), weight,
+                           want_sums=True)
+    assert torch.equal(y2, y3)
+    torch.testing.assert_close(sums2, sums3, rtol=1e-5, atol=1e-3)
+
+
+def test_conv1x1_values_that_are_not_finite():
+    """Infinities and NaN reach the rows that hold them and no others."""
+    from horovod_b200 import _C
+    g = torch.Generator(device=_dev()).manual_seed(2)
+    x = _act(g, 2, 64, 9, 9, torch.bfloat16)
+    weight = torch.randn(64, 64, device=_dev(), generator=g).bfloat16()
+    clean = _C.conv1x1(x, weight)[0]
+    x[0, 3, 2, 1], x[1, 5, 8, 8] = float("inf"), float("nan")
+    y, sums = _C.conv1x1(x, weight, want_sums=True)
+    touched = torch.zeros(2, 1, 9, 9, dtype=torch.bool, device=_dev())
+    touched[0, 0, 2, 1] = touched[1, 0, 8, 8] = True
+    assert torch.equal(torch.where(touched, 0, y), torch.where(touched, 0, clean))
+    assert not bool(y[0, :, 2, 1].isfinite().any()) and bool(y[1, :, 8, 8].isnan().all())
+    assert bool(sums.isnan().all())
+
+
+def test_conv1x1_wait_that_runs_out():
+    """The results are NaN, the device is marked, and nothing is left behind."""
+    from horovod_b200 import _C
+    g = torch.Generator(device=_dev()).manual_seed(3)
+    x, add = _act(g, 8, 64, 30, 30, torch.bfloat16), _act(g, 8, 64, 30, 30, torch.bfloat16)
+    big = _act(g, 8, 64, 60, 60, torch.bfloat16)
+    weight = torch.randn(64, 64, device=_dev(), generator=g).bfloat16()
+    calls = [dict(want_sums=True), dict(w_transposed=True), dict(w_transposed=True, add=add),
+             dict(w_transposed=True, add=big, scatter=True)]
+    try:
+        for kw in calls:
+            before = _C.conv1x1(x, weight, **kw)
+            assert not _C.stem_conv_failed(0)
+            y, sums = _C.conv1x1(x, weight, wait_ns=0, **kw)
+            torch.cuda.synchronize()
+            assert _C.stem_conv_failed(0, clear=True)
+            if "scatter" in kw:
+                assert bool(y[:, :, ::2, ::2].isnan().all())
+                assert torch.equal(y[:, :, 1::2], big[:, :, 1::2])
+            else:
+                assert bool(y.isnan().all())
+            assert sums is None or bool(sums[0].isnan().all())
+            again = _C.conv1x1(x, weight, **kw)
+            assert torch.equal(again[0], before[0])
+        block, x = _block(64, 16, 1, False), _act(g, 2, 64, 8, 8, torch.bfloat16)
+        assert _available(block, x)
+        _C.conv1x1(x, weight, wait_ns=0)
+        torch.cuda.synchronize()
+        with pytest.warns(UserWarning, match="ran out"):
+            assert not _available(block, x)
+    finally:
+        torch.cuda.synchronize()
+        _C.stem_conv_failed(0, clear=True)
+
+
+def _block(inplanes, planes, stride, down, seed=0):
+    from horovod_b200.models.resnet import Bottleneck
+    from horovod_b200.ops.batch_norm import BatchNormAct2d
+    torch.manual_seed(seed)
+    downsample = nn.Sequential(nn.Conv2d(inplanes, planes * 4, 1, stride=stride, bias=False),
+                               BatchNormAct2d(planes * 4, relu=False)) if down else None
+    block = Bottleneck(inplanes, planes, stride, downsample)
+    for m in block.modules():
+        if isinstance(m, nn.BatchNorm2d):
+            nn.init.uniform_(m.weight, 0.5, 1.5)
+            nn.init.normal_(m.bias, std=0.1)
+    return block.to(_dev()).to(memory_format=CL)
+
+
+def _available(block, x):
+    from horovod_b200.ops.bottleneck import fused_bottleneck_available
+    with torch.autocast("cuda", dtype=x.dtype):
+        return fused_bottleneck_available(block, x) is not None
+
+
+def _step(block, x, dy, autocast=True):
+    """y, the gradients of x and of every parameter, and the buffers."""
+    block.zero_grad()
+    x = x.detach().clone(memory_format=CL).requires_grad_(True)
+    with torch.autocast("cuda", dtype=torch.bfloat16 if x.dtype == torch.float64 else x.dtype,
+                        enabled=autocast and x.dtype != torch.float64):
+        y = block(x)
+    y.backward(dy.to(y.dtype))
+    out = {"y": y.detach(), "dx": x.grad}
+    out.update({n: p.grad for n, p in block.named_parameters()})
+    out.update({n: b.clone() for n, b in block.named_buffers()})
+    return out
+
+
+def _rel(a, b):
+    return ((a.double() - b.double()).norm() / (b.double().norm() + 1e-30)).item()
+
+
+SHAPES = [
+    (256, 64, 1, False, 4, 12, 10, torch.bfloat16), (64, 64, 1, True, 4, 12, 10, torch.bfloat16),
+    (256, 128, 2, True, 4, 12, 10, torch.float16),
+    (256, 128, 2, True, 4, 11, 9, torch.bfloat16),    # odd sizes: PyTorch's strided layers
+    (64, 64, 2, True, 1, 2, 260, torch.bfloat16),     # and rows of more than 128 pixels
+    (1024, 256, 1, False, 9, 7, 7, torch.float16),    # the first convolution is PyTorch's
+    (32, 8, 1, False, 4, 9, 9, torch.bfloat16),       # too few channels for the kernels
+    (32, 16, 2, True, 4, 8, 8, torch.bfloat16),
+]
+
+
+@pytest.mark.parametrize("shape", SHAPES)
+def test_block_is_as_close_to_64_bits_as_its_layers(shape, monkeypatch):
+    inplanes, planes, stride, down, n, h, w, dtype = shape
+    block = _block(inplanes, planes, stride, down)
+    g = torch.Generator(device=_dev()).manual_seed(4)
+    x = _act(g, n, inplanes, h, w, dtype).relu_()
+    dy = _act(g, n, planes * 4, (h - 1) // stride + 1, (w - 1) // stride + 1, dtype)
+    assert _available(block, x)
+    fused = _step(copy.deepcopy(block), x, dy)
+    monkeypatch.setenv("HOROVOD_B200_FUSED_BLOCK", "0")
+    assert not _available(block, x)
+    layers = _step(copy.deepcopy(block), x, dy)
+    exact = _step(copy.deepcopy(block).double(), x.double(), dy.double())
+    for name, want in exact.items():
+        if not want.is_floating_point():
+            assert torch.equal(fused[name], want), name
+            continue
+        # Values that pass a ReLU or not by their last bit make most of either
+        # error; which ones do is chance.
+        assert _rel(fused[name], want) <= 1.15 * _rel(layers[name], want) + 2e-3, name
+    for name, p in block.named_parameters():
+        assert fused[name].stride() == p.stride() and fused[name].dtype == p.dtype
+
+
+@pytest.mark.parametrize("change", ["contiguous", "transposed", "flat", "16 bit", "frozen",
+                                    "expanded dy", "strided dy"])
+def test_block_with_other_layouts(change, monkeypatch):
+    """Weights and gradients in layouts other than the usual one: as the layers."""
+    block = _block(256, 64, 2, True)
+    g = torch.Generator(device=_dev()).manual_seed(5)
+    x = _act(g, 4, 256, 12, 10, torch.bfloat16).relu_()
+    dy = _act(g, 4, 256, 6, 5, torch.bfloat16)
+    params = dict(block.named_parameters())
+    if change == "contiguous":
+        block = block.to(memory_format=torch.contiguous_format)
+    elif change == "transposed":
+        for name in ("conv1.weight", "conv3.weight", "downsample.0.weight"):
+            p = params[name]
+            p.data = p.data[:, :, 0, 0].t().contiguous().t()[:, :, None, None]
+    elif change == "flat":  # off a 16-byte boundary
+        for p in params.values():
+            if p.dim() == 4:
+                flat = torch.empty(p.numel() + 1, device=_dev())
+                p.data = torch.as_strided(flat, p.shape, p.stride(), 1).copy_(p.data)
+    elif change == "16 bit":
+        for p in params.values():
+            if p.dim() == 4:
+                p.data = p.data.bfloat16()
+    elif change == "frozen":
+        for name in ("conv1.weight", "bn2.weight", "bn3.bias", "downsample.0.weight"):
+            params[name].requires_grad_(False)
+    elif change == "expanded dy":
+        dy = torch.full((1, 1, 1, 1), 0.5, device=_dev()).bfloat16().expand(4, 256, 6, 5)
+    elif change == "strided dy":
+        dy = dy.contiguous()
+
+    def step(block):
+        xx = x.detach().clone(memory_format=CL).requires_grad_(True)
+        with torch.autocast("cuda", dtype=torch.bfloat16, enabled=change != "16 bit"):
+            y = block(xx)
+        y.backward(dy)
+        return [y.detach(), xx.grad] + [p.grad for p in block.parameters()]
+
+    from horovod_b200.ops.bottleneck import fused_bottleneck_available
+    with torch.autocast("cuda", dtype=torch.bfloat16, enabled=change != "16 bit"):
+        assert fused_bottleneck_available(block, x) is not None
+    fused = step(copy.deepcopy(block))
+    monkeypatch.setenv("HOROVOD_B200_FUSED_BLOCK", "0")
+    layers = step(copy.deepcopy(block))
+    for a, b in zip(fused, layers):
+        assert (a is None) == (b is None)
+        # the two round the same values in the same places but for a few
+        assert a is None or (_rel(a, b) <= 4e-2 and a.dtype == b.dtype)
+
+
+def test_block_leaves_the_rest_to_its_layers():
+    from horovod_b200.ops.bottleneck import fused_bottleneck_available
+    g = torch.Generator(device=_dev()).manual_seed(6)
+    x = _act(g, 2, 256, 8, 8, torch.bfloat16)
+
+    def plain(block, x=x, autocast=torch.bfloat16):
+        with torch.autocast("cuda", dtype=autocast or torch.bfloat16, enabled=autocast is not None):
+            assert fused_bottleneck_available(block, x) is None
+            return block(x)
+
+    def changed(f):
+        block = _block(256, 64, 1, False)
+        f(block)
+        return block
+
+    assert _available(_block(256, 64, 1, False), x)
+    plain(_block(256, 64, 1, False), x.contiguous())
+    plain(_block(256, 64, 1, False), autocast=torch.float16)
+    plain(_block(256, 64, 1, False), x.float())
+    flat = torch.empty(x.numel() + 1, device=_dev(), dtype=x.dtype)
+    plain(_block(256, 64, 1, False), torch.as_strided(flat, x.shape, x.stride(), 1).copy_(x))
+    plain(changed(lambda b: b.eval()))
+    plain(changed(lambda b: b.bn2.eval()))
+    plain(changed(lambda b: setattr(b.bn1, "momentum", None)))
+    plain(changed(lambda b: setattr(b.bn1, "relu", False)))
+    plain(changed(lambda b: setattr(b, "bn1", nn.BatchNorm2d(64).to(_dev()))))
+    plain(changed(lambda b: setattr(b.conv2, "dilation", (2, 2))
+                  or setattr(b.conv2, "padding", (2, 2))))
+    plain(changed(lambda b: nn.utils.parametrizations.weight_norm(b.conv1)))
+    calls = []
+    plain(changed(lambda b: b.conv2.register_forward_hook(lambda *a: calls.append(1))))
+    plain(changed(lambda b: b.bn3.register_full_backward_hook(lambda *a: None)))
+    assert calls == [1]
+    handle = nn.modules.module.register_module_forward_hook(lambda *a: calls.append(2))
+    try:
+        plain(_block(256, 64, 1, False))
+    finally:
+        handle.remove()
+    assert calls.count(2) > 3
+    from torch.autograd import forward_ad
+    with forward_ad.dual_level():
+        plain(_block(256, 64, 1, False))
+    block, seen = _block(256, 64, 1, False), []
+    torch.func.vmap(lambda t: seen.append(fused_bottleneck_available(block, t)) or t)(x[None])
+    assert seen == [None]
+
+
+def test_block_under_autograds_other_uses():
+    """Gradients of gradients, a second backward, saved-tensor hooks, weights that
+    change between forward and backward, an output that does."""
+    block = _block(256, 64, 1, False)
+    g = torch.Generator(device=_dev()).manual_seed(7)
+    x = _act(g, 2, 256, 8, 8, torch.bfloat16).requires_grad_(True)
+    inputs = [x] + list(block.parameters())
+
+    def forward():
+        with torch.autocast("cuda", dtype=torch.bfloat16):
+            return block(x)
+
+    y = forward()
+    dy = torch.ones_like(y)
+    first = torch.autograd.grad(y, inputs, dy, retain_graph=True)
+    again = torch.autograd.grad(y, inputs, dy, retain_graph=True)
+    for a, b in zip(first, again):
+        assert _rel(a, b) <= 1e-3  # sums of the batch norms in another order
+    graph = torch.autograd.grad(y, inputs, dy, create_graph=True)
+    for a, b in zip(graph, first):
+        assert _rel(a, b) <= 0.15  # PyTorch's composition, which rounds elsewhere
+    second = torch.autograd.grad(sum(t.float().square().sum() for t in graph), inputs)
+    assert all(bool(t.isfinite().all()) for t in second)
+    assert second[1].norm().item() > 0
+
+    saved = []
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: saved.append(1) or t.cpu(),
+                                                  lambda t: t.to(_dev())):
+        y = forward()
+    for a, b in zip(torch.autograd.grad(y, inputs, dy), first):
+        assert _rel(a, b) <= 1e-3
+    assert saved
+
+    y = forward()
+    before = block.conv1.weight.detach().clone()
+    with torch.no_grad():
+        block.conv1.weight.zero_()
+    for a, b in zip(torch.autograd.grad(y, inputs, dy), first):
+        assert _rel(a, b) <= 1e-3
+    with torch.no_grad():
+        block.conv1.weight.copy_(before)
+    y = forward()
+    y.detach().add_(1)
+    with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+        torch.autograd.grad(y, inputs, dy)
+
+
+def test_block_in_a_graph():
+    """A captured step replays with new inputs as the same step does eagerly."""
+    block = _block(256, 128, 2, True)
+    g = torch.Generator(device=_dev()).manual_seed(8)
+    x = _act(g, 4, 256, 8, 8, torch.bfloat16).requires_grad_(True)
+    dy = _act(g, 4, 512, 4, 4, torch.bfloat16)
+    inputs = [x] + list(block.parameters())
+
+    def step():
+        with torch.autocast("cuda", dtype=torch.bfloat16, cache_enabled=False):
+            y = block(x)
+        return [y] + list(torch.autograd.grad(y, inputs, dy))
+
+    stream = torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        for _ in range(2):
+            step()
+    stream.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        captured = step()
+    for _ in range(2):
+        with torch.no_grad():
+            x.copy_(_act(g, 4, 256, 8, 8, torch.bfloat16))
+        graph.replay()
+        torch.cuda.synchronize()
+        replayed = [t.clone() for t in captured]
+        for a, b in zip(replayed, step()):
+            assert _rel(a, b) <= 2e-2  # sums in another order
+
+
+def test_block_on_two_streams():
+    """Two streams at once: each has the results of one alone."""
+    g = torch.Generator(device=_dev()).manual_seed(9)
+    blocks = [_block(256, 64, 1, False, seed) for seed in (1, 2)]
+    xs = [_act(g, 16, 256, 28, 28, torch.bfloat16) for _ in blocks]
+    dy = _act(g, 16, 256, 28, 28, torch.bfloat16)
+    alone = [_step(copy.deepcopy(b), x, dy) for b, x in zip(blocks, xs)]
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in blocks]
+    together = []
+    for b, x, s in zip(blocks, xs, streams):
+        with torch.cuda.stream(s):
+            together.append(_step(b, x, dy))
+    torch.cuda.synchronize()
+    for a, b in zip(alone, together):
+        assert max(_rel(b[k], a[k]) for k in a if a[k].is_floating_point()) <= 2e-2
