@@ -98,6 +98,157 @@ bool SgdReady(const at::Tensor& p, const at::Tensor& g) {
          SgdLike(p, g) && p.is_non_overlapping_and_dense();
 }
 
+
+struct NormOutputs {
+  at::Tensor y, saved, signs;
+};
+
+NormOutputs NormForward(at::Tensor x, c10::optional<at::Tensor> residual,
+                        const c10::optional<at::Tensor>& weight,
+                        const c10::optional<at::Tensor>& bias,
+                        const c10::optional<at::Tensor>& running_mean,
+                        const c10::optional<at::Tensor>& running_var, double momentum, double eps,
+                        bool relu, const c10::optional<at::Tensor>& batches) {
+  x = Activations(x, "x");
+  const int64_t C = x.size(1), M = x.numel() / C;
+  TORCH_CHECK(kern::BatchNormSupported(M, static_cast<int>(C)),
+              "fused batch norm does not support ", C, " channels");
+  const void* res = nullptr;
+  if (residual.has_value() && residual->defined()) {
+    residual = Activations(*residual, "residual");
+    TORCH_CHECK(residual->sizes() == x.sizes() && residual->scalar_type() == x.scalar_type(),
+                "residual must match x");
+    res = residual->data_ptr();
+  }
+  c10::cuda::CUDAGuard guard(x.device());
+  cudaStream_t stream = at::cuda::getCurrentCUDAStream();
+  at::Tensor y = at::empty_like(x, x.options(), at::MemoryFormat::ChannelsLast);
+  at::Tensor saved = at::empty({3, C}, x.options().dtype(at::kFloat));
+  at::Tensor signs;
+  if (relu && res != nullptr) signs = at::empty({M, C / 8}, x.options().dtype(at::kByte));
+  at::Tensor own;
+  double* sums =
+      ZeroedDoubles(kern::BatchNormScratchDoubles(static_cast<int>(C)), x, stream, &own);
+  float* rm = nullptr;
+  float* rv = nullptr;
+  if (running_mean.has_value() && running_mean->defined()) {
+    rm = const_cast<float*>(FloatPtrOrNull(running_mean, C, "running_mean"));
+    rv = const_cast<float*>(FloatPtrOrNull(running_var, C, "running_var"));
+    TORCH_CHECK(rv != nullptr, "running_var must accompany running_mean");
+  }
+  int64_t* count = nullptr;
+  if (batches.has_value() && batches->defined()) {
+    TORCH_CHECK(batches->device() == x.device() && batches->scalar_type() == at::kLong &&
+                    batches->numel() == 1,
+                "num_batches_tracked must be one int64 on the device of x");
+    count = batches->data_ptr<int64_t>();
+  }
+  cudaError_t err = kern::LaunchBatchNormForward(
+      x.data_ptr(), res, y.data_ptr(), signs.defined() ? signs.data_ptr<uint8_t>() : nullptr, M,
+      static_cast<int>(C), x.scalar_type() == at::kBFloat16, sums,
+      FloatPtrOrNull(weight, C, "weight"), FloatPtrOrNull(bias, C, "bias"),
+      static_cast<float>(eps), static_cast<float>(momentum), saved.data_ptr<float>(),
+      rm, rv, count, relu, stream);
+  TORCH_CHECK(err == cudaSuccess, "fused batch norm forward: ", cudaGetErrorString(err));
+  return {y, saved, signs};
+}
+
+struct NormGradients {
+  at::Tensor x, residual, weight, bias;
+};
+
+NormGradients NormBackward(at::Tensor dy, at::Tensor x, const c10::optional<at::Tensor>& weight,
+                           const at::Tensor& saved, const c10::optional<at::Tensor>& signs,
+                           bool relu, bool want_dresidual) {
+  x = Activations(x, "x");
+  dy = Activations(dy, "dy");
+  TORCH_CHECK(dy.sizes() == x.sizes() && dy.scalar_type() == x.scalar_type(), "dy must match x");
+  const int64_t C = x.size(1), M = x.numel() / C;
+  TORCH_CHECK(saved.is_cuda() && saved.scalar_type() == at::kFloat && saved.is_contiguous() &&
+                  saved.numel() == 3 * C,
+              "saved must be the tensor returned by bn_forward");
+  const uint8_t* sign_bits = nullptr;
+  if (signs.has_value() && signs->defined()) {
+    TORCH_CHECK(signs->is_cuda() && signs->scalar_type() == at::kByte &&
+                    signs->is_contiguous() && signs->numel() * 8 == x.numel(),
+                "signs must be the tensor returned by bn_forward");
+    sign_bits = signs->data_ptr<uint8_t>();
+  }
+  c10::cuda::CUDAGuard guard(x.device());
+  cudaStream_t stream = at::cuda::getCurrentCUDAStream();
+  at::Tensor dx = at::empty_like(x, x.options(), at::MemoryFormat::ChannelsLast);
+  at::Tensor dres;
+  if (want_dresidual) dres = at::empty_like(x, x.options(), at::MemoryFormat::ChannelsLast);
+  auto fopt = x.options().dtype(at::kFloat);
+  at::Tensor dweight = at::empty({C}, fopt), dbias = at::empty({C}, fopt);
+  at::Tensor own;
+  double* sums =
+      ZeroedDoubles(kern::BatchNormScratchDoubles(static_cast<int>(C)), x, stream, &own);
+  cudaError_t err = kern::LaunchBatchNormBackward(
+      dy.data_ptr(), sign_bits, x.data_ptr(), dx.data_ptr(),
+      want_dresidual ? dres.data_ptr() : nullptr, M, static_cast<int>(C),
+      x.scalar_type() == at::kBFloat16, sums,
+      FloatPtrOrNull(weight, C, "weight"), saved.data_ptr<float>(), dweight.data_ptr<float>(),
+      dbias.data_ptr<float>(), relu, stream);
+  TORCH_CHECK(err == cudaSuccess, "fused batch norm backward: ", cudaGetErrorString(err));
+  return {dx, dres, dweight, dbias};
+}
+
+c10::optional<at::Tensor> OrNone(const at::Tensor& t) {
+  return t.defined() ? c10::optional<at::Tensor>(t) : c10::nullopt;
+}
+
+// The layer as an autograd node. In Python (horovod_b200/ops/batch_norm.py keeps
+// such a node for what this one cannot take part in), the node's own work took
+// 45 us of a forward and backward of 110 on the host.
+class NormNode : public torch::autograd::Function<NormNode> {
+ public:
+  static at::Tensor forward(torch::autograd::AutogradContext* ctx, const at::Tensor& x,
+                            c10::optional<at::Tensor> residual,
+                            const c10::optional<at::Tensor>& weight,
+                            const c10::optional<at::Tensor>& bias,
+                            const c10::optional<at::Tensor>& running_mean,
+                            const c10::optional<at::Tensor>& running_var, double momentum,
+                            double eps, bool relu, c10::optional<at::Tensor> batches) {
+    if (residual.has_value()) residual = residual->contiguous(at::MemoryFormat::ChannelsLast);
+    if (batches.has_value() &&
+        (batches->device() != x.device() || batches->scalar_type() != at::kLong)) {
+      batches->add_(1);
+      batches = c10::nullopt;
+    }
+    const NormOutputs o = NormForward(x, residual, weight, bias, running_mean, running_var,
+                                      momentum, eps, relu, batches);
+    // The kernels do without y; like relu's own backward, this one still
+    // refuses to run when somebody has changed it in place.
+    ctx->save_for_backward({x, relu ? o.y : at::Tensor(), weight.value_or(at::Tensor()), o.saved,
+                            o.signs});
+    ctx->saved_data["flags"] = static_cast<int64_t>((relu ? 1 : 0) | (residual.has_value() ? 2 : 0) |
+                                                    (weight.has_value() ? 4 : 0) |
+                                                    (bias.has_value() ? 8 : 0));
+    return o.y;
+  }
+
+  static torch::autograd::variable_list backward(torch::autograd::AutogradContext* ctx,
+                                                 torch::autograd::variable_list grads) {
+    torch::autograd::variable_list result(10);
+    if (!grads[0].defined()) return result;
+    const auto keep = ctx->get_saved_variables();
+    const at::Tensor &x = keep[0], &weight = keep[2], &saved = keep[3], &signs = keep[4];
+    const int64_t flags = ctx->saved_data["flags"].toInt();
+    at::Tensor dy = grads[0];
+    if (dy.scalar_type() != x.scalar_type()) dy = dy.to(x.scalar_type());
+    dy = dy.contiguous(at::MemoryFormat::ChannelsLast);
+    // The edges of the node are those of the tensors that were given.
+    const NormGradients g = NormBackward(dy, x, OrNone(weight), saved, OrNone(signs), flags & 1,
+                                         (flags & 2) != 0 && ctx->needs_input_grad(1));
+    result[0] = g.x;
+    result[1] = g.residual;
+    if (flags & 4) result[2] = g.weight;
+    if (flags & 8) result[3] = g.bias;
+    return result;
+  }
+};
+
 }  // namespace
 
 void BindModelOps(py::module_& m) {
@@ -108,95 +259,44 @@ void BindModelOps(py::module_& m) {
   //  num_batches_tracked?)
   //   -> (y, saved, signs or None): saved holds what the backward needs of the
   //      statistics, signs (with a residual and a ReLU) which outputs are above zero
-  m.def("bn_forward", [](at::Tensor x, c10::optional<at::Tensor> residual,
+  m.def("bn_forward", [](const at::Tensor& x, const c10::optional<at::Tensor>& residual,
                          const c10::optional<at::Tensor>& weight,
                          const c10::optional<at::Tensor>& bias,
-                         c10::optional<at::Tensor> running_mean,
-                         c10::optional<at::Tensor> running_var, double momentum, double eps,
-                         bool relu, c10::optional<at::Tensor> batches) {
-    x = Activations(x, "x");
-    const int64_t C = x.size(1), M = x.numel() / C;
-    TORCH_CHECK(kern::BatchNormSupported(M, static_cast<int>(C)),
-                "fused batch norm does not support ", C, " channels");
-    const void* res = nullptr;
-    if (residual.has_value() && residual->defined()) {
-      residual = Activations(*residual, "residual");
-      TORCH_CHECK(residual->sizes() == x.sizes() && residual->scalar_type() == x.scalar_type(),
-                  "residual must match x");
-      res = residual->data_ptr();
-    }
-    c10::cuda::CUDAGuard guard(x.device());
-    cudaStream_t stream = at::cuda::getCurrentCUDAStream();
-    at::Tensor y = at::empty_like(x, x.options(), at::MemoryFormat::ChannelsLast);
-    at::Tensor saved = at::empty({3, C}, x.options().dtype(at::kFloat));
-    at::Tensor signs;
-    if (relu && res != nullptr) signs = at::empty({M, C / 8}, x.options().dtype(at::kByte));
-    at::Tensor own;
-    double* sums =
-        ZeroedDoubles(kern::BatchNormScratchDoubles(static_cast<int>(C)), x, stream, &own);
-    float* rm = nullptr;
-    float* rv = nullptr;
-    if (running_mean.has_value() && running_mean->defined()) {
-      rm = const_cast<float*>(FloatPtrOrNull(running_mean, C, "running_mean"));
-      rv = const_cast<float*>(FloatPtrOrNull(running_var, C, "running_var"));
-      TORCH_CHECK(rv != nullptr, "running_var must accompany running_mean");
-    }
-    int64_t* count = nullptr;
-    if (batches.has_value() && batches->defined()) {
-      TORCH_CHECK(batches->device() == x.device() && batches->scalar_type() == at::kLong &&
-                      batches->numel() == 1,
-                  "num_batches_tracked must be one int64 on the device of x");
-      count = batches->data_ptr<int64_t>();
-    }
-    cudaError_t err = kern::LaunchBatchNormForward(
-        x.data_ptr(), res, y.data_ptr(), signs.defined() ? signs.data_ptr<uint8_t>() : nullptr, M,
-        static_cast<int>(C), x.scalar_type() == at::kBFloat16, sums,
-        FloatPtrOrNull(weight, C, "weight"), FloatPtrOrNull(bias, C, "bias"),
-        static_cast<float>(eps), static_cast<float>(momentum), saved.data_ptr<float>(),
-        rm, rv, count, relu, stream);
-    TORCH_CHECK(err == cudaSuccess, "fused batch norm forward: ", cudaGetErrorString(err));
-    return std::make_tuple(y, saved,
-                           signs.defined() ? c10::optional<at::Tensor>(signs) : c10::nullopt);
+                         const c10::optional<at::Tensor>& running_mean,
+                         const c10::optional<at::Tensor>& running_var, double momentum, double eps,
+                         bool relu, const c10::optional<at::Tensor>& batches) {
+    const NormOutputs o = NormForward(x, residual, weight, bias, running_mean, running_var,
+                                      momentum, eps, relu, batches);
+    return std::make_tuple(o.y, o.saved, OrNone(o.signs));
   });
   // (dy, x, weight?, saved, signs?, relu, want_dresidual)
   //   -> (dx, dresidual or None, dweight, dbias)
-  m.def("bn_backward", [](at::Tensor dy, at::Tensor x,
+  m.def("bn_backward", [](const at::Tensor& dy, const at::Tensor& x,
                           const c10::optional<at::Tensor>& weight, const at::Tensor& saved,
                           const c10::optional<at::Tensor>& signs, bool relu,
                           bool want_dresidual) {
-    x = Activations(x, "x");
-    dy = Activations(dy, "dy");
-    TORCH_CHECK(dy.sizes() == x.sizes() && dy.scalar_type() == x.scalar_type(), "dy must match x");
-    const int64_t C = x.size(1), M = x.numel() / C;
-    TORCH_CHECK(saved.is_cuda() && saved.scalar_type() == at::kFloat && saved.is_contiguous() &&
-                    saved.numel() == 3 * C,
-                "saved must be the tensor returned by bn_forward");
-    const uint8_t* sign_bits = nullptr;
-    if (signs.has_value() && signs->defined()) {
-      TORCH_CHECK(signs->is_cuda() && signs->scalar_type() == at::kByte &&
-                      signs->is_contiguous() && signs->numel() * 8 == x.numel(),
-                  "signs must be the tensor returned by bn_forward");
-      sign_bits = signs->data_ptr<uint8_t>();
-    }
-    c10::cuda::CUDAGuard guard(x.device());
-    cudaStream_t stream = at::cuda::getCurrentCUDAStream();
-    at::Tensor dx = at::empty_like(x, x.options(), at::MemoryFormat::ChannelsLast);
-    at::Tensor dres;
-    if (want_dresidual) dres = at::empty_like(x, x.options(), at::MemoryFormat::ChannelsLast);
-    auto fopt = x.options().dtype(at::kFloat);
-    at::Tensor dweight = at::empty({C}, fopt), dbias = at::empty({C}, fopt);
-    at::Tensor own;
-    double* sums =
-        ZeroedDoubles(kern::BatchNormScratchDoubles(static_cast<int>(C)), x, stream, &own);
-    cudaError_t err = kern::LaunchBatchNormBackward(
-        dy.data_ptr(), sign_bits, x.data_ptr(), dx.data_ptr(),
-        want_dresidual ? dres.data_ptr() : nullptr, M, static_cast<int>(C),
-        x.scalar_type() == at::kBFloat16, sums,
-        FloatPtrOrNull(weight, C, "weight"), saved.data_ptr<float>(), dweight.data_ptr<float>(),
-        dbias.data_ptr<float>(), relu, stream);
-    TORCH_CHECK(err == cudaSuccess, "fused batch norm backward: ", cudaGetErrorString(err));
-    return std::make_tuple(dx, want_dresidual ? c10::optional<at::Tensor>(dres) : c10::nullopt,
-                           dweight, dbias);
+    const NormGradients g = NormBackward(dy, x, weight, saved, signs, relu, want_dresidual);
+    return std::make_tuple(g.x, OrNone(g.residual), g.weight, g.bias);
+  });
+  // The whole layer, differentiable: y, or None where the kernels cannot take the
+  // call (the caller then composes PyTorch's operations).
+  m.def("bn_act", [](const at::Tensor& x, const c10::optional<at::Tensor>& residual,
+                     const c10::optional<at::Tensor>& weight,
+                     const c10::optional<at::Tensor>& bias,
+                     const c10::optional<at::Tensor>& running_mean,
+                     const c10::optional<at::Tensor>& running_var, double momentum, double eps,
+                     bool relu,
+                     const c10::optional<at::Tensor>& batches) -> c10::optional<at::Tensor> {
+    if (!x.is_cuda() || x.dim() != 4 ||
+        (x.scalar_type() != at::kBFloat16 && x.scalar_type() != at::kHalf) ||
+        !x.is_contiguous(at::MemoryFormat::ChannelsLast) || x.numel() == 0 ||
+        !kern::BatchNormSupported(x.numel() / x.size(1), static_cast<int>(x.size(1))))
+      return c10::nullopt;
+    if (residual.has_value() &&
+        (residual->sizes() != x.sizes() || residual->scalar_type() != x.scalar_type()))
+      return c10::nullopt;
+    return NormNode::apply(x, residual, weight, bias, running_mean, running_var, momentum, eps,
+                           relu, batches);
   });
 
   // ---- max pooling 3x3 / stride 2 / padding 1 (channels-last, 16-bit) -------

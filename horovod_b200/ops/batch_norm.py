@@ -20,6 +20,8 @@ import torch
 import torch.nn as nn
 import torch.nn.functional as F
 
+from horovod_b200.ops._native import PLAIN, plain_autograd
+
 
 def _extension():
     from horovod_b200 import _C
@@ -38,7 +40,14 @@ def fused_batch_norm_available(x, momentum):
     return _extension().bn_supported(x.numel() // channels, channels)
 
 
+def _native(*tensors):
+    """Whether the layer may run as its native autograd node."""
+    return plain_autograd() and all(t is None or type(t) in PLAIN for t in tensors)
+
+
 class _FusedBatchNormAct(torch.autograd.Function):
+    """The layer where its native node (bn_act) cannot be used."""
+
     @staticmethod
     def forward(ctx, x, residual, weight, bias, running_mean, running_var, momentum, eps, relu,
                 batches):
@@ -70,7 +79,14 @@ def batch_norm_act(x, weight, bias, running_mean, running_var, residual=None, tr
                    momentum=0.1, eps=1e-5, relu=True, num_batches_tracked=None):
     """relu(batch_norm(x) + residual), fused on the GPU when possible.
     ``num_batches_tracked`` (optional, an int64 tensor) is incremented."""
-    if training and fused_batch_norm_available(x, momentum) and \
+    if training and momentum is not None and x.is_cuda and \
+            os.environ.get("HOROVOD_B200_FUSED_BN", "1") == "1" and \
+            _native(x, residual, weight, bias, running_mean, running_var):
+        y = _extension().bn_act(x, residual, weight, bias, running_mean, running_var, momentum,
+                                eps, relu, num_batches_tracked)
+        if y is not None:
+            return y
+    elif training and fused_batch_norm_available(x, momentum) and \
             (residual is None or (residual.shape == x.shape and residual.dtype == x.dtype)):
         if residual is not None:
             residual = residual.contiguous(memory_format=torch.channels_last)

@@ -15,12 +15,11 @@ import os
 
 import torch
 import torch.nn as nn
-from torch.autograd import forward_ad
 from torch.nn.modules.module import _has_any_global_hook
-from torch.utils._python_dispatch import is_in_torch_dispatch_mode
 
+from horovod_b200.ops._native import PLAIN, plain_autograd
 from horovod_b200.ops.batch_norm import BatchNormAct2d, fused_batch_norm_available
-from horovod_b200.ops.stem_conv import _PLAIN, tensor_core_kernels_enabled
+from horovod_b200.ops.stem_conv import tensor_core_kernels_enabled
 
 
 def _extension():
@@ -40,7 +39,7 @@ def _plain_conv(conv, kernel, stride, dtypes, device):
             and conv.stride == (stride, stride)
             and conv.padding == (kernel // 2, kernel // 2) and conv.dilation == (1, 1)
             and conv.groups == 1 and conv.bias is None and conv.padding_mode == "zeros"
-            and type(weight) in _PLAIN and weight.dtype in dtypes and weight.device == device
+            and type(weight) in PLAIN and weight.dtype in dtypes and weight.device == device
             and not _observed(conv))
 
 
@@ -53,10 +52,10 @@ def _plain_norm(norm, relu, conv, device):
     mean, var = norm._buffers["running_mean"], norm._buffers["running_var"]
     batches = norm._buffers["num_batches_tracked"]
     for t in (weight, bias, mean, var):
-        if not (type(t) in _PLAIN and t.dtype == torch.float32 and t.device == device
+        if not (type(t) in PLAIN and t.dtype == torch.float32 and t.device == device
                 and t.is_contiguous()):
             return False
-    return type(batches) in _PLAIN and batches.dtype == torch.int64 and batches.device == device
+    return type(batches) in PLAIN and batches.dtype == torch.int64 and batches.device == device
 
 
 def _layers(block):
@@ -75,14 +74,11 @@ def _layers(block):
 
 def fused_bottleneck_available(block, x):
     """The layers of the block for ``fused_bottleneck``, or None."""
-    if not (type(x) in _PLAIN and x.is_cuda and x.dim() == 4 and x.numel() > 0
+    if not (type(x) in PLAIN and x.is_cuda and x.dim() == 4 and x.numel() > 0
             and x.dtype in (torch.bfloat16, torch.float16)):
         return None
-    if os.environ.get("HOROVOD_B200_FUSED_BLOCK", "1") != "1" or _has_any_global_hook():
-        return None
-    if torch.jit.is_tracing() or torch.compiler.is_compiling() or \
-            forward_ad._current_level >= 0 or torch._C._are_functorch_transforms_active() or \
-            is_in_torch_dispatch_mode():
+    if os.environ.get("HOROVOD_B200_FUSED_BLOCK", "1") != "1" or _has_any_global_hook() or \
+            not plain_autograd():
         return None
     if not x.is_contiguous(memory_format=torch.channels_last) or x.data_ptr() % 16 != 0:
         return None

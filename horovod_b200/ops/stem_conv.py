@@ -15,10 +15,8 @@ import warnings
 
 import torch
 import torch.nn as nn
-from torch.autograd import forward_ad
-from torch.utils._python_dispatch import is_in_torch_dispatch_mode
 
-_PLAIN = (torch.Tensor, nn.Parameter)
+from horovod_b200.ops._native import PLAIN, plain_autograd
 
 
 def _extension():
@@ -72,7 +70,7 @@ class StemConv2d(nn.Conv2d):
         another geometry, memory format or type, and what a custom autograd
         function cannot take part in: tracing, transforms, tensors and modes
         with an __torch_dispatch__ of their own."""
-        if not (type(x) in _PLAIN and type(self.weight) in _PLAIN
+        if not (type(x) in PLAIN and type(self.weight) in PLAIN
                 and x.is_cuda and x.dim() == 4 and x.size(1) == 3 and x.numel() > 0
                 and self.kernel_size == (7, 7) and self.stride == (2, 2)
                 and self.padding == (3, 3) and self.dilation == (1, 1) and self.groups == 1
@@ -90,9 +88,7 @@ class StemConv2d(nn.Conv2d):
                 x.dtype not in (torch.float32, torch.bfloat16, torch.float16) or \
                 self.weight.dtype not in (torch.float32, torch.bfloat16, torch.float16):
             return None
-        if torch.jit.is_tracing() or torch.compiler.is_compiling() or \
-                forward_ad._current_level >= 0 or torch._C._are_functorch_transforms_active() or \
-                is_in_torch_dispatch_mode():
+        if not plain_autograd():
             return None
         n, _, h, w = x.shape
         if not _extension().stem_conv_supported(n, h, w, self.out_channels) or \

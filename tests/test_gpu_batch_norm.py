@@ -119,3 +119,62 @@ def test_resnet_blocks_match_unfused_composition(monkeypatch):
             torch.testing.assert_close(b_fused[n], b_ref[n], rtol=5e-2, atol=5e-2)
         else:
             assert torch.equal(b_fused[n], b_ref[n]), n
+
+
+@pytest.mark.parametrize("with_res,relu,affine", [(True, True, True), (False, True, False),
+                                                  (False, False, True)])
+def test_native_node_and_the_one_in_python_agree(with_res, relu, affine, monkeypatch):
+    """The same bits from both nodes, for inputs that want gradients and for some
+    that do not; a changed output is refused by both."""
+    from horovod_b200.ops import batch_norm as bn
+    dev = torch.device("cuda", 0)
+    g = torch.Generator(device=dev).manual_seed(3)
+
+    def act():
+        return torch.randn(2, 5, 6, 64, device=dev, generator=g).bfloat16().permute(0, 3, 1, 2)
+
+    x, res, dy = act(), act() if with_res else None, act().contiguous()  # dy: NCHW
+
+    def run(native, frozen):
+        monkeypatch.setattr(bn, "_native", lambda *t: native)
+        layer = bn.BatchNormAct2d(64, relu=relu, affine=affine).to(dev)
+        a = x.clone(memory_format=torch.channels_last).requires_grad_(True)
+        r = None if res is None else res.clone(
+            memory_format=torch.channels_last).requires_grad_(not frozen)
+        if affine:
+            layer.bias.requires_grad_(not frozen)
+        y = layer(a, r)
+        wanted = [a] + ([r] if r is not None and not frozen else [])
+        if affine:
+            wanted += [layer.weight] + ([] if frozen else [layer.bias])
+        grads = torch.autograd.grad(y, wanted, dy, retain_graph=True)
+        if relu:
+            y.detach().add_(1)
+            with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+                torch.autograd.grad(y, wanted, dy)
+        return [*grads, layer.running_mean, layer.running_var, layer.num_batches_tracked]
+
+    for frozen in (False, True):
+        for p, q in zip(run(True, frozen), run(False, frozen)):
+            assert torch.equal(p, q)
+
+
+def test_calls_that_stay_with_the_node_in_python():
+    from torch.autograd import forward_ad
+    from torch.utils._python_dispatch import TorchDispatchMode
+    from horovod_b200.ops import batch_norm as bn
+
+    class Mode(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            return func(*args, **(kwargs or {}))
+
+    x = torch.randn(2, 64, 4, 4, device="cuda").bfloat16()
+    assert bn._native(x, None, torch.nn.Parameter(x))
+    assert not bn._native(x.as_subclass(type("Sub", (torch.Tensor,), {})))
+    with Mode():
+        assert not bn._native(x)
+    with forward_ad.dual_level():
+        assert not bn._native(x)
+    seen = []
+    torch.func.vmap(lambda t: seen.append(bn._native(t)) or t)(x)
+    assert seen == [False]
