@@ -39,6 +39,7 @@
 #include <cstdint>
 #include <type_traits>
 
+#include "batch_norm.cuh"
 #include "kernels.h"
 
 namespace hvd {
@@ -52,7 +53,6 @@ constexpr int BN_THREADS = 256;
 // per SM, i.e. by occupancy.
 constexpr int BN_MIN_BLOCKS = 3;        // <= 85 registers per thread
 constexpr int BN_MIN_BLOCKS_STATS = 4;  // <= 64 registers per thread
-constexpr int VEC = 8;  // 16-bit elements per 16-byte access
 constexpr int UNROLL = 4;  // rows in flight per thread
 
 // Two channels per 32-bit word.
@@ -90,15 +90,6 @@ template <typename T> __device__ __forceinline__ void stg16(T* p, const Vec8<T>&
   asm volatile("st.global.v4.u32 [%0], {%1,%2,%3,%4};" ::"l"(p), "r"(v.w[0]), "r"(v.w[1]),
                "r"(v.w[2]), "r"(v.w[3]) : "memory");
 }
-// The next kernel of the stream may be started; it waits for this one's
-// results with wait_for_previous().
-__device__ __forceinline__ void start_next() {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
-__device__ __forceinline__ void wait_for_previous() {
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-}
-
 // The signs of 8 outputs in one byte: the even channels in the low nibble, the
 // odd ones in the high nibble. `positive` holds an all-ones half word for each
 // channel whose output is above zero.
@@ -107,11 +98,6 @@ __device__ __forceinline__ uint32_t pack_signs(const uint32_t (&positive)[VEC / 
                      (positive[2] & 0x00040004u) | (positive[3] & 0x00080008u);
   return (t | (t >> 12)) & 0xffu;
 }
-// Bit i of either half word: the sign of channel 2i or 2i + 1.
-__device__ __forceinline__ uint32_t spread_signs(uint32_t byte) {
-  return (byte & 0xfu) | ((byte & 0xf0u) << 12);
-}
-
 // Thread geometry shared by all four kernels.
 struct Tile {
   int txg;        // channel groups (of 8 channels) per CTA along x: min(C/8, 32)
@@ -191,18 +177,6 @@ __device__ __forceinline__ void reduce_to_global(const Tile& t, float (&acc)[2][
     for (int w = 0; w < WARPS; ++w) sum += static_cast<double>(red[w][k * VEC + i][tx]);
     atomicAdd(mine + static_cast<int64_t>(k) * C + tx * VEC + i, sum);
   }
-}
-
-// The two sums of channel ch over all copies.
-__device__ __forceinline__ double2 total(const double* sums, int C, int copies, int64_t ch) {
-  double2 t = make_double2(0.0, 0.0);
-#pragma unroll 4
-  for (int i = 0; i < copies; ++i) {
-    const double* p = sums + static_cast<int64_t>(i) * 2 * C + ch;
-    t.x += __ldcg(p);
-    t.y += __ldcg(p + C);
-  }
-  return t;
 }
 
 template <typename T>
@@ -444,34 +418,22 @@ bn_backward_apply_kernel(const T* __restrict__ dy, const uint8_t* __restrict__ s
   const int by = gridDim.y - 1 - blockIdx.y;
   int64_t r0, r1;
   cta_rows(M, by, &r0, &r1);
-  // dx = scale * dz + kx * (x - centre) + kc: the terms of the sums folded per
-  // channel, in fp64, which leaves registers for four rows in flight. centre is
-  // the mean rounded to the type of x: the difference of the two is exact in fp32
-  // (but for values that the other one dwarfs), so channels whose mean is many
-  // times their spread lose nothing. 256 x 64 x 112 x 112, both kernels: 359 us,
-  // 357 without the centre, 380 with two centres to a register.
+  // The centre costs 2 us of 359 (256 x 64 x 112 x 112, both kernels); two of them to a
+  // register, 23.
   __shared__ __align__(16) float s_scale[BN_CTA_CHANNELS], s_shift[BN_CTA_CHANNELS],
       s_kx[BN_CTA_CHANNELS], s_kc[BN_CTA_CHANNELS], s_centre[BN_CTA_CHANNELS];
   wait_for_previous();
   if (static_cast<int>(threadIdx.x) < t.txg * VEC) {
     const int64_t ch = static_cast<int64_t>(blockIdx.x) * t.txg * VEC + threadIdx.x;
-    const double2 sum = total(sums, C, copies, ch);
-    const double dz = sum.x, dz_xhat = sum.y;
-    const float invstd = saved[C + ch];
-    const float scale = (weight ? weight[ch] : 1.f) * invstd;
-    s_scale[threadIdx.x] = scale;
+    const BackwardTerms b = backward_terms<T>(sums, C, copies, ch, inv_m, weight, saved);
+    s_scale[threadIdx.x] = b.scale;
     s_shift[threadIdx.x] = saved[2 * static_cast<int64_t>(C) + ch];
-    const float mean = saved[ch];
-    const float centre = static_cast<float>(static_cast<T>(mean));
-    const float kx = static_cast<float>(-static_cast<double>(scale) * invstd * dz_xhat * inv_m);
-    s_centre[threadIdx.x] = centre;
-    s_kx[threadIdx.x] = kx;
-    s_kc[threadIdx.x] = static_cast<float>(
-        -scale * dz * inv_m -
-        static_cast<double>(kx) * (static_cast<double>(mean) - centre));
+    s_centre[threadIdx.x] = b.centre;
+    s_kx[threadIdx.x] = b.kx;
+    s_kc[threadIdx.x] = b.kc;
     if (by == 0) {
-      if (dweight) dweight[ch] = static_cast<float>(dz_xhat);
-      if (dbias) dbias[ch] = static_cast<float>(dz);
+      if (dweight) dweight[ch] = static_cast<float>(b.dz_xhat);
+      if (dbias) dbias[ch] = static_cast<float>(b.dz);
     }
   }
   __syncthreads();
@@ -656,6 +618,25 @@ cudaError_t LaunchBatchNormForward(const void* x, const void* residual, void* y,
               : ForwardTyped<__half>(x, residual, y, signs, rows, channels, sums, weight, bias,
                                      eps, momentum, saved, running_mean, running_var, batches,
                                      relu, summed, stream);
+}
+
+cudaError_t LaunchBatchNormBackwardSums(const void* dy, const uint8_t* signs, const void* x,
+                                        int64_t rows, int channels, bool bf16,
+                                        double* sums_zeroed, const float* weight,
+                                        const float* saved, cudaStream_t stream) {
+  if (!bn_shape_ok(rows, channels) || signs == nullptr) return cudaErrorInvalidValue;
+  CountKernelLaunches(1);
+  const dim3 grid = bn_grid(rows, channels, BN_CTAS_REDUCE);
+  const int copies = bn_copies(channels);
+  if (bf16)
+    bn_backward_reduce_kernel<__nv_bfloat16, MASK_SIGNS><<<grid, BN_THREADS, 0, stream>>>(
+        static_cast<const __nv_bfloat16*>(dy), signs, static_cast<const __nv_bfloat16*>(x), rows,
+        channels, weight, saved, copies, sums_zeroed);
+  else
+    bn_backward_reduce_kernel<__half, MASK_SIGNS><<<grid, BN_THREADS, 0, stream>>>(
+        static_cast<const __half*>(dy), signs, static_cast<const __half*>(x), rows, channels,
+        weight, saved, copies, sums_zeroed);
+  return cudaGetLastError();
 }
 
 cudaError_t LaunchBatchNormBackward(const void* dy, const uint8_t* signs, const void* x, void* dx,

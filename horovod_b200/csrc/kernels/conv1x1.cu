@@ -30,7 +30,6 @@
 // NaN, its sums too, and TensorCoreStatusWord() of the device is set.
 //
 // The reference has no counterpart (it takes convolutions from the framework).
-#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -38,6 +37,7 @@
 
 #include "kernels.h"
 #include "tensor_core.cuh"
+#include "tma.cuh"
 
 namespace hvd {
 namespace kern {
@@ -46,9 +46,8 @@ namespace {
 
 constexpr int THREADS = 384;
 constexpr int EPILOGUE_WARP = 4, EPILOGUE_THREADS = 256;
-constexpr int TILE_M = 128, SLICE_K = 64;
-constexpr int BOX_BYTES = TILE_M * 128;  // 64 channels of 128 rows
-constexpr uint16_t NAN16 = 0x7fff;       // a NaN of either 16-bit type
+constexpr int SLICE_K = 64;
+constexpr uint16_t NAN16 = 0x7fff;  // a NaN of either 16-bit type
 
 enum Epilogue : int { STORE = 0, STORE_SUMS = 1, ADD = 2, ADD_MASKED = 3 };
 
@@ -79,42 +78,6 @@ struct Shape {
   int copies;
 };
 
-__device__ __forceinline__ bool wait_or_stop(uint32_t bar, uint32_t parity, uint32_t limit,
-                                             volatile int* stop) {
-  unsigned long long t0 = 0;
-  if (limit == 0) return false;
-  for (int i = 0;; ++i) {
-    if (phase_done(bar, parity)) return true;
-    if (*stop) return false;
-    const unsigned long long t = nanoseconds();
-    if (i == 0) t0 = t;
-    if (t - t0 > limit) return false;
-  }
-}
-
-__device__ __forceinline__ void expect_bytes(uint32_t bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;"
-               ::"r"(bar), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void arrive(uint32_t bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ void load_box(uint32_t to, const CUtensorMap* map, int c0, int c1,
-                                         int c2, uint32_t bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.3d.shared::cta.global.mbarrier::complete_tx::bytes "
-      "[%0], [%1, {%2, %3, %4}], [%5];"
-      ::"r"(to), "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(bar) : "memory");
-}
-__device__ __forceinline__ void store_box(const CUtensorMap* map, int c0, int c1, int c2,
-                                          uint32_t from) {
-  asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%1, %2, %3}], [%4];"
-               ::"l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(from) : "memory");
-}
-template <int N> __device__ __forceinline__ void stores_read() {
-  asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory");
-}
-
 // Barriers among the epilogue's threads; the second form also says whether
 // `ok` holds for all of them.
 __device__ __forceinline__ void epilogue_sync() {
@@ -127,35 +90,6 @@ __device__ __forceinline__ bool epilogue_all(bool ok) {
       "barrier.cta.red.and.pred q, 2, %2, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
       : "=r"(all) : "r"(ok ? 1u : 0u), "n"(EPILOGUE_THREADS) : "memory");
   return all != 0;
-}
-
-// Where 8 channels (`piece`) of a row lie in a tile of shared memory.
-__device__ __forceinline__ uint32_t piece_at(int row, int piece) {
-  return piece / 8 * BOX_BYTES + row * 128 + ((piece ^ row) & 7) * 16;
-}
-__device__ __forceinline__ uint4 load_piece(uint32_t at) {
-  uint4 v;
-  asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];"
-               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(at) : "memory");
-  return v;
-}
-__device__ __forceinline__ void store_piece(uint32_t at, uint4 v) {
-  asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};"
-               ::"r"(at), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
-}
-
-__device__ __forceinline__ void load_accumulators(uint32_t at, uint32_t (&r)[32]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-      "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
-      "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
-        "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]),
-        "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]),
-        "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-      : "r"(at));
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
 // First element of row `row` of y.
@@ -449,43 +383,6 @@ conv1x1_kernel(const __grid_constant__ Maps maps, const __grid_constant__ Shape 
                  ::"r"(tmem), "n"(2 * BN));
 }
 
-using EncodeFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*,
-                              const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
-                              const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                              CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-EncodeFn Encode() {
-  static const EncodeFn fn = [] {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) !=
-            cudaSuccess ||
-        q != cudaDriverEntryPointSuccess) {
-      cudaGetLastError();
-      p = nullptr;
-    }
-    return reinterpret_cast<EncodeFn>(p);
-  }();
-  return fn;
-}
-
-// A matrix [rows][channels] as the TMA sees it: [rows2][rows1][channels], with
-// boxes of 64 channels x box1 x box2 rows.
-bool MakeMap(CUtensorMap* map, const void* p, bool bf16, int64_t channels, int64_t rows1,
-             int64_t rows2, int64_t pitch1, int64_t pitch2, int box1, int box2) {
-  const cuuint64_t sizes[3] = {static_cast<cuuint64_t>(channels), static_cast<cuuint64_t>(rows1),
-                               static_cast<cuuint64_t>(rows2)};
-  const cuuint64_t pitches[2] = {static_cast<cuuint64_t>(pitch1) * 2,
-                                 static_cast<cuuint64_t>(pitch2) * 2};
-  const cuuint32_t box[3] = {64, static_cast<cuuint32_t>(box1), static_cast<cuuint32_t>(box2)};
-  const cuuint32_t steps[3] = {1, 1, 1};
-  return Encode()(map, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16,
-                  3, const_cast<void*>(p), sizes, pitches, box, steps,
-                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
 template <typename T, int BN, bool W_MN, int EPI>
 cudaError_t LaunchTyped(const Conv1x1& c, Shape s, cudaStream_t stream, int* status,
                         uint32_t wait_ns) {
@@ -567,7 +464,7 @@ cudaError_t LaunchConv1x1(const Conv1x1& c, cudaStream_t stream, uint32_t wait_n
   if ((c.strided_x || c.strided_y) && !Conv1x1StrideSupported(c.rows, c.width))
     return cudaErrorInvalidValue;
   if ((c.strided_x && c.strided_y) || (c.signs != nullptr && (c.add == nullptr || c.strided_y)) ||
-      (c.sums != nullptr && c.copies < 1) || Encode() == nullptr)
+      (c.sums != nullptr && c.copies < 1) || !TmaAvailable())
     return cudaErrorInvalidValue;
   int device = 0;
   const cudaError_t err = cudaGetDevice(&device);

@@ -378,6 +378,13 @@ cudaError_t LaunchBatchNormBackward(const void* dy, const uint8_t* signs, const 
                                     double* sums_zeroed, const float* weight, const float* saved,
                                     float* dweight, float* dbias, bool relu, cudaStream_t stream);
 
+// The first kernel of the backward alone (relu behind a residual): sum(dz) and
+// sum(dz * xhat) per channel into `sums`.
+cudaError_t LaunchBatchNormBackwardSums(const void* dy, const uint8_t* signs, const void* x,
+                                        int64_t rows, int channels, bool bf16,
+                                        double* sums_zeroed, const float* weight,
+                                        const float* saved, cudaStream_t stream);
+
 // 3x3 / stride 2 / padding 1 max pooling on channels-last 16-bit activations
 // ([n, h, w, channels], channels a multiple of 8). Forward writes the maxima
 // and one word per 8 channels with the winning window position (0..8) of each in
@@ -448,6 +455,30 @@ struct Conv1x1 {
 bool Conv1x1Supported(int64_t rows, int k, int n);
 bool Conv1x1StrideSupported(int64_t rows, int width);
 cudaError_t LaunchConv1x1(const Conv1x1& c, cudaStream_t stream, uint32_t wait_ns = STEM_WAIT_NS);
+
+// Backward of a batch norm over cout channels, whose ReLU (behind a residual) left
+// `signs`, and of the 1x1 convolution from cin channels before it, including the
+// batch norm's sums: da (unless null), dw, dgamma, dbeta. x: the convolution's output,
+// a: its input, w: [cout, cin] 16-bit, saved: the forward's, sums: zeroed as above,
+// partial: scratch of NormConvBackwardParts() * cout * cin floats. dw is fp32 or of the
+// activations' type, with the given element strides.
+struct NormConvBackward {
+  const void *dy, *x, *a, *w;
+  const uint8_t* signs;
+  void *da, *dw;
+  bool dw_fp32;
+  int64_t dw_stride_o, dw_stride_i;
+  double* sums;
+  const float *gamma, *saved;
+  float *dgamma, *dbeta, *partial;
+  int64_t rows;
+  int cout, cin;
+  bool bf16;
+};
+bool NormConvBackwardSupported(int64_t rows, int cout, int cin);
+int NormConvBackwardParts(int64_t rows);
+cudaError_t LaunchNormConvBackward(const NormConvBackward& n, cudaStream_t stream,
+                                   uint32_t wait_ns = STEM_WAIT_NS);
 
 // Multi-tensor SGD step in one launch (torch.optim.SGD arithmetic: weight
 // decay added to the gradient, momentum buffer b = momentum * b + (1 -

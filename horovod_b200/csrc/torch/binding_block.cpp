@@ -8,6 +8,7 @@
 #include <tuple>
 
 #include "../kernels/kernels.h"
+#include "model_ops.h"
 
 namespace hvd {
 
@@ -78,6 +79,64 @@ void BindBlockOps(py::module_& m) {
   }, py::arg("x"), py::arg("w"), py::arg("w_transposed") = false, py::arg("add") = c10::nullopt,
      py::arg("signs") = c10::nullopt, py::arg("want_sums") = false, py::arg("gather") = false,
      py::arg("scatter") = false, py::arg("wait_ns") = kern::STEM_WAIT_NS);
+
+  m.def("norm_conv_backward_supported", &kern::NormConvBackwardSupported);  // (rows, cout, cin)
+  // (dy, signs, x, a, w, gamma, saved) -> (da, dw, dgamma, dbeta): see kernels.h.
+  m.def("norm_conv_backward", [](const at::Tensor& dy, const at::Tensor& signs,
+                                 const at::Tensor& x, const at::Tensor& a, const at::Tensor& w,
+                                 const at::Tensor& gamma, const at::Tensor& saved,
+                                 uint32_t wait_ns) {
+    CheckActivations(dy, "dy");
+    CheckActivations(x, "x");
+    CheckActivations(a, "a");
+    const int64_t cout = x.size(1), cin = a.size(1), rows = x.numel() / cout;
+    TORCH_CHECK(kern::NormConvBackwardSupported(rows, static_cast<int>(cout),
+                                                static_cast<int>(cin)),
+                "norm_conv_backward does not support ", rows, " rows of ", cin, " to ", cout,
+                " channels");
+    TORCH_CHECK(dy.sizes() == x.sizes() && a.numel() / cin == rows && w.is_contiguous() &&
+                    w.is_cuda() && w.size(0) == cout && w.numel() == cout * cin &&
+                    dy.scalar_type() == x.scalar_type() && a.scalar_type() == x.scalar_type() &&
+                    w.scalar_type() == x.scalar_type() && signs.is_contiguous() &&
+                    signs.is_cuda() && signs.scalar_type() == at::kByte &&
+                    signs.numel() * 8 == x.numel() && saved.is_contiguous() && saved.is_cuda() &&
+                    saved.scalar_type() == at::kFloat && saved.numel() == 3 * cout,
+                "norm_conv_backward: tensors do not match");
+    c10::cuda::CUDAGuard guard(x.device());
+    const auto fp32 = x.options().dtype(at::kFloat);
+    at::Tensor da = at::empty_like(a, a.options(), at::MemoryFormat::ChannelsLast);
+    at::Tensor dw = at::empty({cout, cin}, fp32, at::MemoryFormat::Contiguous);
+    at::Tensor dgamma = at::empty({cout}, fp32), dbeta = at::empty({cout}, fp32), own;
+    at::Tensor partial = at::empty({kern::NormConvBackwardParts(rows) * cout * cin}, fp32,
+                                   at::MemoryFormat::Contiguous);
+    kern::NormConvBackward n;
+    n.dy = dy.data_ptr();
+    n.x = x.data_ptr();
+    n.a = a.data_ptr();
+    n.w = w.data_ptr();
+    n.signs = signs.data_ptr<uint8_t>();
+    n.da = da.data_ptr();
+    n.dw = dw.data_ptr();
+    n.dw_fp32 = true;
+    n.dw_stride_o = cin;
+    n.dw_stride_i = 1;
+    cudaStream_t stream = at::cuda::getCurrentCUDAStream();
+    n.sums = ZeroedDoubles(kern::BatchNormScratchDoubles(static_cast<int>(cout)), x, stream, &own);
+    n.gamma = FloatPtrOrNull(gamma, cout, "gamma");
+    n.saved = saved.data_ptr<float>();
+    n.dgamma = dgamma.data_ptr<float>();
+    n.dbeta = dbeta.data_ptr<float>();
+    n.partial = partial.data_ptr<float>();
+    n.rows = rows;
+    n.cout = static_cast<int>(cout);
+    n.cin = static_cast<int>(cin);
+    n.bf16 = x.scalar_type() == at::kBFloat16;
+    const cudaError_t err = kern::LaunchNormConvBackward(n, stream, wait_ns);
+    TORCH_CHECK(err == cudaSuccess, "batch norm and convolution backward: ",
+                cudaGetErrorString(err));
+    return std::make_tuple(da, dw, dgamma, dbeta);
+  }, py::arg("dy"), py::arg("signs"), py::arg("x"), py::arg("a"), py::arg("w"), py::arg("gamma"),
+     py::arg("saved"), py::arg("wait_ns") = kern::STEM_WAIT_NS);
 }
 
 }  // namespace hvd

@@ -5,6 +5,8 @@
 //   - the gradient of the skip connection is never stored: the first
 //     convolution's gradient kernel adds dy where the block's output was above
 //     zero, in place of a store and a pass over three tensors;
+//   - the backward of the last batch norm and convolution (of the first stage's
+//     sizes) is one kernel, which stores no gradient of the batch norm's input;
 //   - the weights are cast in one launch, and so are their gradients.
 // The 3x3 convolution, the gradients of the weights and some 1x1 convolutions are
 // PyTorch's.
@@ -202,6 +204,57 @@ NormGradients NormBackward(const Tensor& dy, const Tensor& x, const Tensor& weig
   return g;
 }
 
+// Gradients of a batch norm behind a 1x1 convolution and of that convolution, together.
+struct TailGradients {
+  Tensor a, w, weight, bias;  // of the convolution's input and weight, of the batch norm
+};
+
+bool OwnTail(const Tensor& out, const Tensor& w, int64_t stride) {
+  return stride == 1 && w.size(2) == 1 &&
+         kern::NormConvBackwardSupported(Rows(out), Channels(out), static_cast<int>(w.size(1)));
+}
+
+// a: the convolution's input; leaf: its weight as the user has it.
+TailGradients TailBackward(const Tensor& dy, const Tensor& signs, const Tensor& x, const Tensor& a,
+                           const Tensor& w, const Tensor& weight, const Tensor& saved,
+                           const Tensor& leaf, bool want_a) {
+  kern::NormConvBackward n;
+  const auto fp32 = x.options().dtype(at::kFloat);
+  TailGradients g;
+  n.rows = Rows(x);
+  n.cout = Channels(x);
+  n.cin = Channels(a);
+  n.bf16 = x.scalar_type() == at::kBFloat16;
+  if (want_a) g.a = at::empty_like(a, a.options(), CL);
+  g.w = leaf.is_non_overlapping_and_dense()
+            ? at::empty_strided(leaf.sizes(), leaf.strides(), leaf.options())
+            : at::empty(leaf.sizes(), leaf.options());
+  g.weight = at::empty({n.cout}, fp32);
+  g.bias = at::empty({n.cout}, fp32);
+  const Tensor partial =
+      at::empty({kern::NormConvBackwardParts(n.rows), n.cout, n.cin}, fp32,
+                at::MemoryFormat::Contiguous);
+  Sums sums(x, n.cout);
+  n.dy = dy.data_ptr();
+  n.x = x.data_ptr();
+  n.a = a.data_ptr();
+  n.w = w.data_ptr();
+  n.signs = signs.data_ptr<uint8_t>();
+  n.da = want_a ? g.a.data_ptr() : nullptr;
+  n.dw = g.w.data_ptr();
+  n.dw_fp32 = g.w.scalar_type() == at::kFloat;
+  n.dw_stride_o = g.w.stride(0);
+  n.dw_stride_i = g.w.stride(1);
+  n.sums = sums.p;
+  n.gamma = FloatPtrOrNull(weight, n.cout, "weight");
+  n.saved = saved.data_ptr<float>();
+  n.dgamma = g.weight.data_ptr<float>();
+  n.dbeta = g.bias.data_ptr<float>();
+  n.partial = partial.data_ptr<float>();
+  Check(kern::LaunchNormConvBackward(n, Stream()), "batch norm and convolution backward");
+  return g;
+}
+
 // PyTorch's gradients of a convolution: of the input (where wanted) and the weight.
 std::pair<Tensor, Tensor> ConvBackward(const Tensor& dy, const Tensor& x, const Tensor& w,
                                        int64_t stride, bool want_x, bool want_w) {
@@ -340,26 +393,43 @@ class Bottleneck : public torch::autograd::Function<Bottleneck> {
     // The gradients of x through the first convolution and through the skip
     // connection meet in a kernel of this library where it takes the shapes.
     const bool fused = kern::Conv1x1Supported(Rows(x), Channels(out[0]), Channels(x));
-    const NormGradients g3 = norm(2, dy, signs, want_x && !down && !fused);
-    Tensor da2, da1, dx, skip = down ? Tensor() : fused ? dy : g3.residual, mask;
-    if (!down && fused) mask = signs;
-    std::tie(da2, dw[2]) = ConvBackward(g3.x, a2, w[2], 1, true, wanted(7));
+    Tensor da2, da1, dx, skip, mask;
+    if (!down && fused) skip = dy, mask = signs;
+    // The end of the block and its skip convolution: `in`'s gradient (where
+    // wanted), the weight's goes to dw, the batch norm's to result.
+    auto tail = [&](int i, const Tensor& in, int64_t s, bool want_in) {
+      if (OwnTail(out[i], w[i], s)) {
+        const TailGradients g = TailBackward(dy, signs, out[i], in, w[i], gammas[i], saved[i],
+                                             weights[i], want_in);
+        if (wanted(2 + 3 * i)) result[2 + 3 * i] = g.weight;
+        if (wanted(3 + 3 * i)) result[3 + 3 * i] = g.bias;
+        if (wanted(1 + 3 * i)) result[1 + 3 * i] = g.w;
+        return g.a;
+      }
+      const bool want_skip = i == 2 && want_x && !down && !fused;
+      const NormGradients g = norm(i, dy, signs, want_skip);
+      if (want_skip) skip = g.residual;
+      Tensor d_in;
+      std::tie(d_in, dw[i]) = ConvBackward(g.x, in, w[i], s, want_in, wanted(1 + 3 * i));
+      return d_in;
+    };
+    da2 = tail(2, a2, 1, true);
     const Tensor d2 = norm(1, da2, {}, false).x;
     da2.reset();
     std::tie(da1, dw[1]) = ConvBackward(d2, a1, w[1], stride, true, wanted(4));
     const Tensor d1 = norm(0, da1, {}, false).x;
     da1.reset();
     if (down) {
-      const Tensor dd = norm(DOWN, dy, signs, false).x;
       const bool scatter = stride == 2 && EveryOther(x) &&
-                           kern::Conv1x1Supported(Rows(dd), Channels(dd), Channels(x));
+                           kern::Conv1x1Supported(Rows(dy), Channels(dy), Channels(x));
       if (want_x && scatter) {
         // Its gradient of x is zero but for every fourth pixel: added in place.
+        const Tensor dd = norm(DOWN, dy, signs, false).x;
         std::tie(dx, dw[0]) = ConvBackward(d1, x, w[0], 1, true, wanted(1));
         ConvInputGradient(dd, w[DOWN], dx, {}, true);
         dw[DOWN] = ConvBackward(dd, x, w[DOWN], stride, false, wanted(10)).second;
       } else {
-        std::tie(skip, dw[DOWN]) = ConvBackward(dd, x, w[DOWN], stride, want_x, wanted(10));
+        skip = tail(DOWN, x, stride, want_x);
       }
     }
     if (!dx.defined()) {
@@ -367,6 +437,7 @@ class Bottleneck : public torch::autograd::Function<Bottleneck> {
       if (want_x) dx = fused ? ConvInputGradient(d1, w[0], skip, mask, false) : dx.add_(skip);
     }
     if (want_x) result[0] = dx;
+    // (Weights whose gradients are there already have no dw.)
     for (int i = 0; i < LAYERS; ++i)
       if (dw[i].defined() && weights[i].scalar_type() != at::kFloat) {
         result[1 + 3 * i] = dw[i];

@@ -129,6 +129,78 @@ def test_conv1x1_wait_that_runs_out():
         _C.stem_conv_failed(0, clear=True)
 
 
+def _tail(g, n, cout, h, w, dtype):
+    """What the backward of a batch norm behind a 1x1 convolution of 64 channels gets:
+    dy, signs, x, a, weight, gamma, saved."""
+    from horovod_b200 import _C
+    x, res, dy = (_act(g, n, cout, h, w, dtype) for _ in range(3))
+    a = _act(g, n, 64, h, w, dtype).relu_()
+    weight = (torch.randn(cout, 64, device=_dev(), generator=g) / 8).to(dtype)
+    gamma = torch.rand(cout, device=_dev(), generator=g) + 0.5
+    _, saved, signs = _C.bn_forward(x, res, gamma, torch.zeros_like(gamma), None, None, 0.1, 1e-5,
+                                    True, None)
+    return dy, signs, x, a, weight, gamma, saved
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("n,cout,h,w", [
+    (1, 256, 1, 2), (1, 128, 1, 17),                   # a few rows: one slot of the ring
+    (1, 256, 8, 16), (1, 128, 8, 16),                  # exactly one tile
+    (3, 256, 9, 11), (2, 128, 13, 10),                 # a ragged last one
+    (64, 256, 29, 23), (64, 128, 29, 23),              # several per CTA
+])
+def test_norm_conv_backward(dtype, n, cout, h, w):
+    """dx is formed as by the batch norm's own kernel, bit for bit; da is its product
+    with the weight, rounded once; dW sums in fp32 (and fp64 across CTAs)."""
+    from horovod_b200 import _C
+    g = torch.Generator(device=_dev()).manual_seed(11)
+    dy, signs, x, a, weight, gamma, saved = _tail(g, n, cout, h, w, dtype)
+    da, dw, dgamma, dbeta = _C.norm_conv_backward(dy, signs, x, a, weight, gamma, saved)
+    dx, _, dgamma_ref, dbeta_ref = _C.bn_backward(dy, x, gamma, saved, signs, True, False)
+    _close(da, torch.einsum("nohw,ok->nkhw", dx.double(), weight.double()), dtype)
+    want = torch.einsum("nohw,nkhw->ok", dx.double(), a.double())
+    terms = torch.einsum("nohw,nkhw->ok", dx.double().abs(), a.double().abs())
+    assert bool(((dw - want).abs() <= 1e-5 * terms + 1e-12).all())
+    # the sums' atomics come in any order
+    torch.testing.assert_close(dgamma, dgamma_ref, rtol=1e-6, atol=1e-6)
+    torch.testing.assert_close(dbeta, dbeta_ref, rtol=1e-6, atol=1e-6)
+
+
+def test_norm_conv_backward_values_that_are_not_finite():
+    """A NaN in an activation reaches its column of dW and nothing else; one in the
+    batch norm's input reaches all of its channel."""
+    from horovod_b200 import _C
+    g = torch.Generator(device=_dev()).manual_seed(12)
+    dy, signs, x, a, weight, gamma, saved = _tail(g, 3, 256, 9, 11, torch.bfloat16)
+    da, dw, _, _ = _C.norm_conv_backward(dy, signs, x, a, weight, gamma, saved)
+    a[2, 7, 8, 10] = float("nan")  # of the last, ragged tile
+    da2, dw2, _, _ = _C.norm_conv_backward(dy, signs, x, a, weight, gamma, saved)
+    assert torch.equal(da, da2) and bool(dw2[:, 7].isnan().all())
+    assert torch.equal(dw2[:, :7], dw[:, :7]) and torch.equal(dw2[:, 8:], dw[:, 8:])
+    x[1, 200, 3, 3] = float("inf")
+    da3, dw3, dgamma, _ = _C.norm_conv_backward(dy, signs, x, a, weight, gamma, saved)
+    assert bool(da3.isnan().all()) and bool(dgamma[200].isfinite().logical_not())
+    assert bool(dw3[200].isfinite().logical_not().all())
+    assert torch.equal(dw3[:200, :7], dw[:200, :7])
+
+
+def test_norm_conv_backward_wait_that_runs_out():
+    from horovod_b200 import _C
+    g = torch.Generator(device=_dev()).manual_seed(13)
+    args = _tail(g, 40, 256, 28, 28, torch.bfloat16)
+    before = _C.norm_conv_backward(*args)
+    try:
+        da, dw, _, _ = _C.norm_conv_backward(*args, wait_ns=0)
+        torch.cuda.synchronize()
+        assert _C.stem_conv_failed(0, clear=True)
+        assert bool(da.isnan().all()) and bool(dw.isnan().all())
+    finally:
+        torch.cuda.synchronize()
+        _C.stem_conv_failed(0, clear=True)
+    again = _C.norm_conv_backward(*args)
+    assert all(_rel(p, q) <= 1e-6 for p, q in zip(again, before))
+
+
 def _block(inplanes, planes, stride, down, seed=0):
     from horovod_b200.models.resnet import Bottleneck
     from horovod_b200.ops.batch_norm import BatchNormAct2d
