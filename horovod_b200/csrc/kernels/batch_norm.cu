@@ -143,39 +143,44 @@ __device__ __forceinline__ void for_rows_back(const Tile& t, int64_t r0, int64_t
   for (; left > 0; left -= t.ty, at -= stride) rows(std::integral_constant<int, 1>(), at);
 }
 
-// Sums `acc` (two values per channel of the thread) over the threads of the
+// Sums `acc` (N values per channel of the thread) over the threads of the
 // CTA that own the same channel group and adds the totals to the fp64
 // accumulators: pairwise by shuffles inside a warp, in fp64 across warps.
-// sums: [copies][2][C]; CTA y adds to copy y % copies.
-__device__ __forceinline__ void reduce_to_global(const Tile& t, float (&acc)[2][VEC], int C,
-                                                 int copies, double* sums) {
+// sums: [copies][2][C]; CTA y adds to copy y % copies. Of three values, the first and
+// the third go to `more`.
+template <int N>
+__device__ __forceinline__ void reduce_to_global(const Tile& t, float (&acc)[N][VEC], int C,
+                                                 int copies, double* sums,
+                                                 double* more = nullptr) {
   constexpr int WARPS = BN_THREADS / 32;
   // Rows of 36 words: the threads of a warp, which read 8 rows of 4 words
   // below, hit 32 different banks.
-  __shared__ float red[WARPS][2 * VEC][36];
+  __shared__ float red[WARPS][N * VEC][36];
   for (int lanes = 16; lanes >= t.txg; lanes >>= 1) {
 #pragma unroll
-    for (int k = 0; k < 2; ++k)
+    for (int k = 0; k < N; ++k)
 #pragma unroll
       for (int i = 0; i < VEC; ++i) acc[k][i] += __shfl_xor_sync(0xffffffffu, acc[k][i], lanes);
   }
   const int warp = threadIdx.x / 32;
   if (static_cast<int>(threadIdx.x % 32) < t.txg) {
 #pragma unroll
-    for (int k = 0; k < 2; ++k)
+    for (int k = 0; k < N; ++k)
 #pragma unroll
       for (int i = 0; i < VEC; ++i) red[warp][k * VEC + i][t.tx] = acc[k][i];
   }
   __syncthreads();
-  double* mine = sums + static_cast<int64_t>(blockIdx.y % copies) * 2 * C +
-                 static_cast<int64_t>(blockIdx.x) * t.txg * VEC;
-  // 2 * VEC * txg <= 512 totals, two rounds of 256 threads at most.
-  for (int idx = threadIdx.x; idx < t.txg * 2 * VEC; idx += BN_THREADS) {
+  const int64_t mine = static_cast<int64_t>(blockIdx.y % copies) * 2 * C +
+                       static_cast<int64_t>(blockIdx.x) * t.txg * VEC;
+  // N * VEC * txg <= 256 N totals, N rounds of 256 threads at most.
+  for (int idx = threadIdx.x; idx < t.txg * N * VEC; idx += BN_THREADS) {
     const int i = idx % VEC, tx = idx / VEC % t.txg, k = idx / VEC / t.txg;
     double sum = 0.0;
 #pragma unroll
     for (int w = 0; w < WARPS; ++w) sum += static_cast<double>(red[w][k * VEC + i][tx]);
-    atomicAdd(mine + static_cast<int64_t>(k) * C + tx * VEC + i, sum);
+    const int64_t at = mine + tx * VEC + i;
+    if (k < 2) atomicAdd(sums + at + static_cast<int64_t>(k) * C, sum);
+    if (N == 3 && k != 1) atomicAdd(more + at + (k == 2 ? C : 0), sum);
   }
 }
 
@@ -252,15 +257,43 @@ __device__ __forceinline__ void load8(const float* p, float (&v)[VEC]) {
   v[4] = b.x, v[5] = b.y, v[6] = b.z, v[7] = b.w;
 }
 
-// saved: rows mean, invstd and shift of [3, C].
+// What a channel of x is multiplied with, and what is added. The first CTA of a
+// column also writes `saved` (rows mean, invstd and shift of [3, C]) and the running
+// statistics.
+struct ForwardTerms {
+  float scale, shift;
+};
+__device__ __forceinline__ ForwardTerms forward_terms(const BatchNormForward& n, int64_t M, int C,
+                                                      double inv_m, int copies, int64_t ch,
+                                                      bool first) {
+  const double2 sum = total(n.sums, C, copies, ch);
+  const double m = sum.x * inv_m;
+  double var = sum.y * inv_m - m * m;
+  if (var < 0.0) var = 0.0;
+  const float mean = static_cast<float>(m);
+  const float invstd = static_cast<float>(rsqrt(var + static_cast<double>(n.eps)));
+  const float scale = (n.weight ? n.weight[ch] : 1.f) * invstd;
+  const float shift = (n.bias ? n.bias[ch] : 0.f) - mean * scale;
+  if (first) {
+    n.saved[ch] = mean;
+    n.saved[C + ch] = invstd;
+    n.saved[2 * static_cast<int64_t>(C) + ch] = shift;
+    if (n.running_mean != nullptr) {
+      const double unbiased =
+          M > 1 ? var * static_cast<double>(M) / static_cast<double>(M - 1) : var;
+      n.running_mean[ch] = (1.f - n.momentum) * n.running_mean[ch] + n.momentum * mean;
+      n.running_var[ch] =
+          (1.f - n.momentum) * n.running_var[ch] + n.momentum * static_cast<float>(unbiased);
+    }
+  }
+  return {scale, shift};
+}
+
 template <typename T, bool RELU, bool RES>
 __global__ void __launch_bounds__(BN_THREADS, BN_MIN_BLOCKS)
 bn_apply_kernel(const T* __restrict__ x, const T* __restrict__ res, T* __restrict__ y,
                 uint8_t* __restrict__ signs, int64_t M, int C, double inv_m, int copies,
-                const double* __restrict__ sums, const float* __restrict__ weight,
-                const float* __restrict__ bias, float eps, float momentum,
-                float* __restrict__ saved, float* __restrict__ running_mean,
-                float* __restrict__ running_var, int64_t* __restrict__ batches) {
+                const BatchNormForward n) {
   const Tile t(C);
   const int by = gridDim.y - 1 - blockIdx.y;
   int64_t r0, r1;
@@ -268,31 +301,12 @@ bn_apply_kernel(const T* __restrict__ x, const T* __restrict__ res, T* __restric
   __shared__ __align__(16) float s_scale[BN_CTA_CHANNELS];
   __shared__ __align__(16) float s_shift[BN_CTA_CHANNELS];
   wait_for_previous();
-  if (batches != nullptr && by == 0 && blockIdx.x == 0 && threadIdx.x == 0) *batches += 1;
+  if (n.batches != nullptr && by == 0 && blockIdx.x == 0 && threadIdx.x == 0) *n.batches += 1;
   if (static_cast<int>(threadIdx.x) < t.txg * VEC) {
     const int64_t ch = static_cast<int64_t>(blockIdx.x) * t.txg * VEC + threadIdx.x;
-    const double2 sum = total(sums, C, copies, ch);
-    const double m = sum.x * inv_m;
-    double var = sum.y * inv_m - m * m;
-    if (var < 0.0) var = 0.0;
-    const float mean = static_cast<float>(m);
-    const float invstd = static_cast<float>(rsqrt(var + static_cast<double>(eps)));
-    const float scale = (weight ? weight[ch] : 1.f) * invstd;
-    const float shift = (bias ? bias[ch] : 0.f) - mean * scale;
-    s_scale[threadIdx.x] = scale;
-    s_shift[threadIdx.x] = shift;
-    if (by == 0) {
-      saved[ch] = mean;
-      saved[C + ch] = invstd;
-      saved[2 * static_cast<int64_t>(C) + ch] = shift;
-      if (running_mean != nullptr) {
-        const double unbiased =
-            M > 1 ? var * static_cast<double>(M) / static_cast<double>(M - 1) : var;
-        running_mean[ch] = (1.f - momentum) * running_mean[ch] + momentum * mean;
-        running_var[ch] =
-            (1.f - momentum) * running_var[ch] + momentum * static_cast<float>(unbiased);
-      }
-    }
+    const ForwardTerms f = forward_terms(n, M, C, inv_m, copies, ch, by == 0);
+    s_scale[threadIdx.x] = f.scale;
+    s_shift[threadIdx.x] = f.shift;
   }
   __syncthreads();
   float scale[VEC], shift[VEC];
@@ -319,6 +333,70 @@ bn_apply_kernel(const T* __restrict__ x, const T* __restrict__ res, T* __restric
           positive[i] = __hgt2_mask(o.pair(i), Pair<T>::narrow(0.f, 0.f));
         signs[at / VEC] = static_cast<uint8_t>(pack_signs(positive));
       }
+    }
+  });
+}
+
+// relu(batch norm of x + batch norm of r) and its signs: the end of a residual block
+// whose skip connection has a convolution and a batch norm of its own, which is then
+// neither stored nor read. The four of a ResNet-50 step at batch 256 take 416 us, 676
+// with a pass for the skip connection's batch norm. Bound by HBM.
+template <typename T>
+__global__ void __launch_bounds__(BN_THREADS, BN_MIN_BLOCKS)
+bn_apply_pair_kernel(const T* __restrict__ x, const T* __restrict__ r, T* __restrict__ y,
+                     uint8_t* __restrict__ signs, int64_t M, int C, double inv_m, int copies,
+                     const BatchNormForward nx, const BatchNormForward nr) {
+  const Tile t(C);
+  const int by = gridDim.y - 1 - blockIdx.y;
+  int64_t r0, r1;
+  cta_rows(M, by, &r0, &r1);
+  __shared__ __align__(16) float s_x[BN_CTA_CHANNELS], s_r[BN_CTA_CHANNELS],
+      s_shift[BN_CTA_CHANNELS];
+  wait_for_previous();
+  if (by == 0 && blockIdx.x == 0 && threadIdx.x == 0) {
+    if (nx.batches != nullptr) *nx.batches += 1;
+    if (nr.batches != nullptr) *nr.batches += 1;
+  }
+  if (static_cast<int>(threadIdx.x) < t.txg * VEC) {
+    const int64_t ch = static_cast<int64_t>(blockIdx.x) * t.txg * VEC + threadIdx.x;
+    const ForwardTerms fx = forward_terms(nx, M, C, inv_m, copies, ch, by == 0);
+    const ForwardTerms fr = forward_terms(nr, M, C, inv_m, copies, ch, by == 0);
+    s_x[threadIdx.x] = fx.scale;
+    s_r[threadIdx.x] = fr.scale;
+    s_shift[threadIdx.x] = fx.shift + fr.shift;
+  }
+  __syncthreads();
+  float sx[VEC], sr[VEC], shift[VEC];
+  load8(s_x + t.tx * VEC, sx);
+  load8(s_r + t.tx * VEC, sr);
+  load8(s_shift + t.tx * VEC, shift);
+  const int64_t stride = static_cast<int64_t>(t.ty) * C;
+  for_rows_back<UNROLL>(t, r0, r1, C, [&](auto count, int64_t at0) {
+    constexpr int U = decltype(count)::value;
+    Vec8<T> a[U], b[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      a[u] = ldg16(x + at0 - u * stride);
+      b[u] = ldg16(r + at0 - u * stride);
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int64_t at = at0 - u * stride;
+      Vec8<T> o;
+      uint32_t positive[VEC / 2];
+#pragma unroll
+      for (int i = 0; i < VEC / 2; ++i) {
+        const float2 f = Pair<T>::widen(a[u].pair(i)), g = Pair<T>::widen(b[u].pair(i));
+        const int j = 2 * i, k = 2 * i + 1;
+        const typename Pair<T>::type zero = Pair<T>::narrow(0.f, 0.f);
+        const typename Pair<T>::type v =
+            __hmax2(Pair<T>::narrow(fmaf(f.x, sx[j], fmaf(g.x, sr[j], shift[j])),
+                                    fmaf(f.y, sx[k], fmaf(g.y, sr[k], shift[k]))), zero);
+        positive[i] = __hgt2_mask(v, zero);
+        o.set(i, v);
+      }
+      stg16(y + at, o);
+      signs[at / VEC] = static_cast<uint8_t>(pack_signs(positive));
     }
   });
 }
@@ -406,6 +484,74 @@ bn_backward_reduce_kernel(const T* __restrict__ dy, const uint8_t* __restrict__ 
   reduce_to_global(t, acc, C, copies, sums);
 }
 
+// The same for two batch norms whose sum went through the ReLU: dz is one for both.
+// The four of a ResNet-50 step at batch 256 take 389 us, 533 one after the other.
+template <typename T>
+__global__ void __launch_bounds__(BN_THREADS, BN_MIN_BLOCKS)
+bn_backward_reduce_pair_kernel(const T* __restrict__ dy, const uint8_t* __restrict__ signs,
+                               const T* __restrict__ x, const T* __restrict__ r, int64_t M, int C,
+                               const float* __restrict__ saved_x,
+                               const float* __restrict__ saved_r, int copies,
+                               double* __restrict__ sums_x, double* __restrict__ sums_r) {
+  const Tile t(C);
+  int64_t r0, r1;
+  cta_rows(M, blockIdx.y, &r0, &r1);
+  const int64_t off = t.group * VEC;
+  float mean_x[VEC], mean_r[VEC], acc[3][VEC];
+  load8(saved_x + off, mean_x);
+  load8(saved_r + off, mean_r);
+#pragma unroll
+  for (int i = 0; i < VEC; ++i) acc[0][i] = acc[1][i] = acc[2][i] = 0.f;
+  const int64_t stride = static_cast<int64_t>(t.ty) * C;
+  // (Three rows would spill.)
+  for_rows<2>(t, r0, r1, C, [&](auto count, int64_t at0) {
+    constexpr int U = decltype(count)::value;
+    Vec8<T> d[U], a[U], b[U];
+    uint32_t m[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int64_t at = at0 + u * stride;
+      d[u] = ldg16(dy + at);
+      a[u] = ldg16(x + at);
+      b[u] = ldg16(r + at);
+      m[u] = spread_signs(__ldg(signs + at / VEC));
+    }
+#pragma unroll
+    for (int i = 0; i < VEC / 2; ++i) {
+      const int j = 2 * i, k = 2 * i + 1;
+      float2 s = make_float2(0.f, 0.f), p = s, q = s;
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const float2 f = Pair<T>::widen(a[u].pair(i)), g = Pair<T>::widen(b[u].pair(i));
+        d[u].w[i] &= ((m[u] >> i) & 0x00010001u) * 0xffffu;
+        const float2 dz = Pair<T>::widen(d[u].pair(i));
+        s.x += dz.x;
+        s.y += dz.y;
+        p.x = fmaf(dz.x, f.x - mean_x[j], p.x);
+        p.y = fmaf(dz.y, f.y - mean_x[k], p.y);
+        q.x = fmaf(dz.x, g.x - mean_r[j], q.x);
+        q.y = fmaf(dz.y, g.y - mean_r[k], q.y);
+      }
+      acc[0][j] += s.x;
+      acc[0][k] += s.y;
+      acc[1][j] += p.x;
+      acc[1][k] += p.y;
+      acc[2][j] += q.x;
+      acc[2][k] += q.y;
+    }
+  });
+  start_next();
+  float invstd_x[VEC], invstd_r[VEC];
+  load8(saved_x + C + off, invstd_x);
+  load8(saved_r + C + off, invstd_r);
+#pragma unroll
+  for (int i = 0; i < VEC; ++i) {
+    acc[1][i] *= invstd_x[i];
+    acc[2][i] *= invstd_r[i];
+  }
+  reduce_to_global(t, acc, C, copies, sums_x, sums_r);
+}
+
 template <typename T, int MASK, bool DRES>
 __global__ void __launch_bounds__(BN_THREADS, BN_MIN_BLOCKS)
 bn_backward_apply_kernel(const T* __restrict__ dy, const uint8_t* __restrict__ signs,
@@ -470,6 +616,83 @@ bn_backward_apply_kernel(const T* __restrict__ dy, const uint8_t* __restrict__ s
       }
       stg16(dx + at, g);
       if (DRES) stg16(dres + at, d[u]);
+    }
+  });
+}
+
+// The gradients of both inputs of such a pair. 64 values per channel group stay in
+// registers, hence two CTAs per SM. The three of a ResNet-50 step at batch 256 that take
+// this path: 319 us, 341 one after the other.
+template <typename T>
+__global__ void __launch_bounds__(BN_THREADS, 2)
+bn_backward_apply_pair_kernel(const T* __restrict__ dy, const uint8_t* __restrict__ signs,
+                              const T* __restrict__ x, const T* __restrict__ r,
+                              T* __restrict__ dx, T* __restrict__ dr, int64_t M, int C,
+                              double inv_m, int copies, const BatchNormBackward nx,
+                              const BatchNormBackward nr) {
+  const Tile t(C);
+  const int by = gridDim.y - 1 - blockIdx.y;
+  int64_t r0, r1;
+  cta_rows(M, by, &r0, &r1);
+  __shared__ __align__(16) float s_terms[2][4][BN_CTA_CHANNELS];
+  wait_for_previous();
+  if (static_cast<int>(threadIdx.x) < t.txg * VEC) {
+    const int64_t ch = static_cast<int64_t>(blockIdx.x) * t.txg * VEC + threadIdx.x;
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const BatchNormBackward& n = k == 0 ? nx : nr;
+      const BackwardTerms b = backward_terms<T>(n.sums, C, copies, ch, inv_m, n.weight, n.saved);
+      s_terms[k][0][threadIdx.x] = b.scale;
+      s_terms[k][1][threadIdx.x] = b.kx;
+      s_terms[k][2][threadIdx.x] = b.kc;
+      s_terms[k][3][threadIdx.x] = b.centre;
+      if (by == 0) {
+        n.dweight[ch] = static_cast<float>(b.dz_xhat);
+        n.dbias[ch] = static_cast<float>(b.dz);
+      }
+    }
+  }
+  __syncthreads();
+  float scale[2][VEC], kx[2][VEC], kc[2][VEC], centre[2][VEC];
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    load8(s_terms[k][0] + t.tx * VEC, scale[k]);
+    load8(s_terms[k][1] + t.tx * VEC, kx[k]);
+    load8(s_terms[k][2] + t.tx * VEC, kc[k]);
+    load8(s_terms[k][3] + t.tx * VEC, centre[k]);
+  }
+  const int64_t stride = static_cast<int64_t>(t.ty) * C;
+  for_rows_back<3>(t, r0, r1, C, [&](auto count, int64_t at0) {
+    constexpr int U = decltype(count)::value;
+    Vec8<T> d[U], in[2][U];
+    uint32_t m[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int64_t at = at0 - u * stride;
+      d[u] = ldg16(dy + at);
+      in[0][u] = ldg16(x + at);
+      in[1][u] = ldg16(r + at);
+      m[u] = spread_signs(__ldg(signs + at / VEC));
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int64_t at = at0 - u * stride;
+      Vec8<T> g[2];
+#pragma unroll
+      for (int i = 0; i < VEC / 2; ++i) {
+        d[u].w[i] &= ((m[u] >> i) & 0x00010001u) * 0xffffu;
+        const float2 z = Pair<T>::widen(d[u].pair(i));
+        const int j = 2 * i, l = 2 * i + 1;
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+          const float2 f = Pair<T>::widen(in[k][u].pair(i));
+          g[k].set(i, Pair<T>::narrow(
+              fmaf(scale[k][j], z.x, fmaf(kx[k][j], f.x - centre[k][j], kc[k][j])),
+              fmaf(scale[k][l], z.y, fmaf(kx[k][l], f.y - centre[k][l], kc[k][l]))));
+        }
+      }
+      stg16(dx + at, g[0]);
+      stg16(dr + at, g[1]);
     }
   });
 }
@@ -549,28 +772,66 @@ static cudaError_t LaunchDependent(void (*kernel)(P...), dim3 grid, cudaStream_t
 }
 
 template <typename T>
+static cudaError_t SumsTyped(const void* x, int64_t M, int C, const BatchNormForward& n,
+                             cudaStream_t stream) {
+  if (n.summed) return cudaSuccess;
+  CountKernelLaunches(1);
+  bn_stats_kernel<T><<<bn_grid(M, C, BN_CTAS_STATS), BN_THREADS, 0, stream>>>(
+      static_cast<const T*>(x), M, C, bn_copies(C), n.sums);
+  return cudaGetLastError();
+}
+
+template <typename T>
 static cudaError_t ForwardTyped(const void* x, const void* res, void* y, uint8_t* signs, int64_t M,
-                                int C, double* sums, const float* weight, const float* bias,
-                                float eps, float momentum, float* saved, float* running_mean,
-                                float* running_var, int64_t* batches, bool relu,
-                                bool summed, cudaStream_t stream) {
-  const int copies = bn_copies(C);
-  if (!summed) {
-    CountKernelLaunches(1);
-    bn_stats_kernel<T><<<bn_grid(M, C, BN_CTAS_STATS), BN_THREADS, 0, stream>>>(
-        static_cast<const T*>(x), M, C, copies, sums);
-    const cudaError_t err = cudaGetLastError();
-    if (err != cudaSuccess) return err;
-  }
+                                int C, const BatchNormForward& n, bool relu,
+                                cudaStream_t stream) {
+  const cudaError_t err = SumsTyped<T>(x, M, C, n, stream);
+  if (err != cudaSuccess) return err;
   auto kernel = relu && res ? bn_apply_kernel<T, true, true>
                 : relu      ? bn_apply_kernel<T, true, false>
                 : res       ? bn_apply_kernel<T, false, true>
                             : bn_apply_kernel<T, false, false>;
   return LaunchDependent(kernel, bn_grid(M, C, bn_apply_ctas(M, C)), stream,
                          static_cast<const T*>(x), static_cast<const T*>(res),
-                         static_cast<T*>(y), signs, M, C, 1.0 / static_cast<double>(M), copies,
-                         sums, weight, bias, eps, momentum, saved, running_mean, running_var,
-                         batches);
+                         static_cast<T*>(y), signs, M, C, 1.0 / static_cast<double>(M),
+                         bn_copies(C), n);
+}
+
+template <typename T>
+static cudaError_t PairForwardTyped(const void* x, const void* r, void* y, uint8_t* signs,
+                                    int64_t M, int C, const BatchNormForward& nx,
+                                    const BatchNormForward& nr, cudaStream_t stream) {
+  cudaError_t err = SumsTyped<T>(r, M, C, nr, stream);
+  if (err == cudaSuccess) err = SumsTyped<T>(x, M, C, nx, stream);
+  if (err != cudaSuccess) return err;
+  return LaunchDependent(bn_apply_pair_kernel<T>, bn_grid(M, C, bn_apply_ctas(M, C)), stream,
+                         static_cast<const T*>(x), static_cast<const T*>(r), static_cast<T*>(y),
+                         signs, M, C, 1.0 / static_cast<double>(M), bn_copies(C), nx, nr);
+}
+
+template <typename T>
+static cudaError_t PairSumsTyped(const void* dy, const uint8_t* signs, const void* x,
+                                 const void* r, int64_t M, int C, const BatchNormBackward& nx,
+                                 const BatchNormBackward& nr, cudaStream_t stream) {
+  CountKernelLaunches(1);
+  bn_backward_reduce_pair_kernel<T><<<bn_grid(M, C, BN_CTAS_REDUCE), BN_THREADS, 0, stream>>>(
+      static_cast<const T*>(dy), signs, static_cast<const T*>(x), static_cast<const T*>(r), M, C,
+      nx.saved, nr.saved, bn_copies(C), nx.sums, nr.sums);
+  return cudaGetLastError();
+}
+
+template <typename T>
+static cudaError_t PairBackwardTyped(const void* dy, const uint8_t* signs, const void* x,
+                                     const void* r, void* dx, void* dr, int64_t M, int C,
+                                     const BatchNormBackward& nx, const BatchNormBackward& nr,
+                                     cudaStream_t stream) {
+  const cudaError_t err = PairSumsTyped<T>(dy, signs, x, r, M, C, nx, nr, stream);
+  if (err != cudaSuccess) return err;
+  CountKernelLaunches(1);
+  return LaunchDependent(bn_backward_apply_pair_kernel<T>, bn_grid(M, C, 148 * 2), stream,
+                         static_cast<const T*>(dy), signs, static_cast<const T*>(x),
+                         static_cast<const T*>(r), static_cast<T*>(dx), static_cast<T*>(dr), M, C,
+                         1.0 / static_cast<double>(M), bn_copies(C), nx, nr);
 }
 
 template <typename T>
@@ -604,20 +865,43 @@ static cudaError_t BackwardTyped(const void* dy, const uint8_t* signs, const voi
 }
 
 cudaError_t LaunchBatchNormForward(const void* x, const void* residual, void* y, uint8_t* signs,
-                                   int64_t rows, int channels, bool bf16, double* sums,
-                                   const float* weight, const float* bias, float eps,
-                                   float momentum, float* saved, float* running_mean,
-                                   float* running_var, int64_t* batches, bool relu,
-                                   cudaStream_t stream, bool summed) {
+                                   int64_t rows, int channels, bool bf16,
+                                   const BatchNormForward& n, bool relu, cudaStream_t stream) {
   if (!bn_shape_ok(rows, channels)) return cudaErrorInvalidValue;
   if (relu && residual != nullptr && signs == nullptr) return cudaErrorInvalidValue;
   CountKernelLaunches(1);
-  return bf16 ? ForwardTyped<__nv_bfloat16>(x, residual, y, signs, rows, channels, sums, weight,
-                                            bias, eps, momentum, saved, running_mean, running_var,
-                                            batches, relu, summed, stream)
-              : ForwardTyped<__half>(x, residual, y, signs, rows, channels, sums, weight, bias,
-                                     eps, momentum, saved, running_mean, running_var, batches,
-                                     relu, summed, stream);
+  return bf16 ? ForwardTyped<__nv_bfloat16>(x, residual, y, signs, rows, channels, n, relu, stream)
+              : ForwardTyped<__half>(x, residual, y, signs, rows, channels, n, relu, stream);
+}
+
+cudaError_t LaunchBatchNormPairForward(const void* x, const void* r, void* y, uint8_t* signs,
+                                       int64_t rows, int channels, bool bf16,
+                                       const BatchNormForward& nx, const BatchNormForward& nr,
+                                       cudaStream_t stream) {
+  if (!bn_shape_ok(rows, channels)) return cudaErrorInvalidValue;
+  CountKernelLaunches(1);
+  return bf16 ? PairForwardTyped<__nv_bfloat16>(x, r, y, signs, rows, channels, nx, nr, stream)
+              : PairForwardTyped<__half>(x, r, y, signs, rows, channels, nx, nr, stream);
+}
+
+cudaError_t LaunchBatchNormPairSums(const void* dy, const uint8_t* signs, const void* x,
+                                    const void* r, int64_t rows, int channels, bool bf16,
+                                    const BatchNormBackward& nx, const BatchNormBackward& nr,
+                                    cudaStream_t stream) {
+  if (!bn_shape_ok(rows, channels)) return cudaErrorInvalidValue;
+  return bf16 ? PairSumsTyped<__nv_bfloat16>(dy, signs, x, r, rows, channels, nx, nr, stream)
+              : PairSumsTyped<__half>(dy, signs, x, r, rows, channels, nx, nr, stream);
+}
+
+cudaError_t LaunchBatchNormPairBackward(const void* dy, const uint8_t* signs, const void* x,
+                                        const void* r, void* dx, void* dr, int64_t rows,
+                                        int channels, bool bf16, const BatchNormBackward& nx,
+                                        const BatchNormBackward& nr, cudaStream_t stream) {
+  if (!bn_shape_ok(rows, channels)) return cudaErrorInvalidValue;
+  return bf16 ? PairBackwardTyped<__nv_bfloat16>(dy, signs, x, r, dx, dr, rows, channels, nx, nr,
+                                                 stream)
+              : PairBackwardTyped<__half>(dy, signs, x, r, dx, dr, rows, channels, nx, nr,
+                                          stream);
 }
 
 cudaError_t LaunchBatchNormBackwardSums(const void* dy, const uint8_t* signs, const void* x,

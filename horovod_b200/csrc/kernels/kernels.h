@@ -356,23 +356,27 @@ cudaError_t LaunchScaleBuffer(const void* in, void* out, int64_t count,
 
 // Training-mode batch normalisation on channels-last 16-bit activations
 // ([rows, channels] row-major), fused with the residual add and the ReLU.
-// `sums` is a zero-filled scratch of BatchNormScratchDoubles(), or, for a forward
-// that is told so (`summed`), already holds the sums of x. Forward:
-// y = act(bn(x) [+ residual]); also writes `saved` (the rows batch mean, inverse
-// standard deviation and shift of [3, channels]), with a residual and a ReLU
+// Forward: y = act(bn(x) [+ residual]); also writes n.saved (the rows batch mean,
+// inverse standard deviation and shift of [3, channels]), with a residual and a ReLU
 // `signs` (a byte per 8 channels: which outputs are above zero), and updates
-// the running statistics and the count of batches (when given). Backward: dx,
+// the running statistics and the count of batches (where given). Backward: dx,
 // optionally dresidual (= gradient through the ReLU), dweight, dbias; `signs` is
-// null when the forward had no residual.
+// null when the forward had no residual. sums: scratch of BatchNormScratchDoubles(),
+// zero-filled or, where `summed`, with the sums of x (and of its squares) in it.
+struct BatchNormForward {
+  double* sums = nullptr;
+  bool summed = false;
+  const float *weight = nullptr, *bias = nullptr;
+  float eps = 0.f, momentum = 0.f;
+  float *saved = nullptr, *running_mean = nullptr, *running_var = nullptr;
+  int64_t* batches = nullptr;
+};
 bool BatchNormSupported(int64_t rows, int channels);
 int64_t BatchNormScratchDoubles(int channels);
 int BatchNormCopies(int channels);  // of the sums in it
 cudaError_t LaunchBatchNormForward(const void* x, const void* residual, void* y, uint8_t* signs,
-                                   int64_t rows, int channels, bool bf16, double* sums,
-                                   const float* weight, const float* bias, float eps,
-                                   float momentum, float* saved, float* running_mean,
-                                   float* running_var, int64_t* batches, bool relu,
-                                   cudaStream_t stream, bool summed = false);
+                                   int64_t rows, int channels, bool bf16,
+                                   const BatchNormForward& n, bool relu, cudaStream_t stream);
 cudaError_t LaunchBatchNormBackward(const void* dy, const uint8_t* signs, const void* x, void* dx,
                                     void* dresidual, int64_t rows, int channels, bool bf16,
                                     double* sums_zeroed, const float* weight, const float* saved,
@@ -384,6 +388,26 @@ cudaError_t LaunchBatchNormBackwardSums(const void* dy, const uint8_t* signs, co
                                         int64_t rows, int channels, bool bf16,
                                         double* sums_zeroed, const float* weight,
                                         const float* saved, cudaStream_t stream);
+
+// relu(bn(x) + bn(r)), each with a batch norm of its own, and the gradients of both
+// inputs. Sums: of the backward alone, into both scratches.
+struct BatchNormBackward {
+  double* sums = nullptr;  // zero-filled
+  const float *weight = nullptr, *saved = nullptr;
+  float *dweight = nullptr, *dbias = nullptr;
+};
+cudaError_t LaunchBatchNormPairForward(const void* x, const void* r, void* y, uint8_t* signs,
+                                       int64_t rows, int channels, bool bf16,
+                                       const BatchNormForward& nx, const BatchNormForward& nr,
+                                       cudaStream_t stream);
+cudaError_t LaunchBatchNormPairSums(const void* dy, const uint8_t* signs, const void* x,
+                                    const void* r, int64_t rows, int channels, bool bf16,
+                                    const BatchNormBackward& nx, const BatchNormBackward& nr,
+                                    cudaStream_t stream);
+cudaError_t LaunchBatchNormPairBackward(const void* dy, const uint8_t* signs, const void* x,
+                                        const void* r, void* dx, void* dr, int64_t rows,
+                                        int channels, bool bf16, const BatchNormBackward& nx,
+                                        const BatchNormBackward& nr, cudaStream_t stream);
 
 // 3x3 / stride 2 / padding 1 max pooling on channels-last 16-bit activations
 // ([n, h, w, channels], channels a multiple of 8). Forward writes the maxima
@@ -458,7 +482,7 @@ cudaError_t LaunchConv1x1(const Conv1x1& c, cudaStream_t stream, uint32_t wait_n
 
 // Backward of a batch norm over cout channels, whose ReLU (behind a residual) left
 // `signs`, and of the 1x1 convolution from cin channels before it, including the
-// batch norm's sums: da (unless null), dw, dgamma, dbeta. x: the convolution's output,
+// batch norm's sums (unless `summed`): da (unless null), dw, dgamma, dbeta. x: the convolution's output,
 // a: its input, w: [cout, cin] 16-bit, saved: the forward's, sums: zeroed as above,
 // partial: scratch of NormConvBackwardParts() * cout * cin floats. dw is fp32 or of the
 // activations' type, with the given element strides.
@@ -469,6 +493,7 @@ struct NormConvBackward {
   bool dw_fp32;
   int64_t dw_stride_o, dw_stride_i;
   double* sums;
+  bool summed;
   const float *gamma, *saved;
   float *dgamma, *dbeta, *partial;
   int64_t rows;

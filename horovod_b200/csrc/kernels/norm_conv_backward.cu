@@ -470,8 +470,9 @@ cudaError_t LaunchNormConvBackward(const NormConvBackward& n, cudaStream_t strea
   if (err != cudaSuccess) return err;
   int* status = TensorCoreStatusWord(device);
   if (status == nullptr) return cudaErrorMemoryAllocation;
-  err = LaunchBatchNormBackwardSums(n.dy, n.signs, n.x, n.rows, n.cout, n.bf16, n.sums, n.gamma,
-                                    n.saved, stream);
+  if (!n.summed)
+    err = LaunchBatchNormBackwardSums(n.dy, n.signs, n.x, n.rows, n.cout, n.bf16, n.sums, n.gamma,
+                                      n.saved, stream);
   if (err != cudaSuccess) return err;
   if (n.bf16)
     return n.cout == 256 ? LaunchTyped<__nv_bfloat16, 256>(n, stream, status, wait_ns)

@@ -122,6 +122,7 @@ void BindBlockOps(py::module_& m) {
     n.dw_stride_i = 1;
     cudaStream_t stream = at::cuda::getCurrentCUDAStream();
     n.sums = ZeroedDoubles(kern::BatchNormScratchDoubles(static_cast<int>(cout)), x, stream, &own);
+    n.summed = false;
     n.gamma = FloatPtrOrNull(gamma, cout, "gamma");
     n.saved = saved.data_ptr<float>();
     n.dgamma = dgamma.data_ptr<float>();

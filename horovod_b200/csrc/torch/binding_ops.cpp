@@ -143,12 +143,19 @@ NormOutputs NormForward(at::Tensor x, c10::optional<at::Tensor> residual,
                 "num_batches_tracked must be one int64 on the device of x");
     count = batches->data_ptr<int64_t>();
   }
-  cudaError_t err = kern::LaunchBatchNormForward(
+  kern::BatchNormForward n;
+  n.sums = sums;
+  n.weight = FloatPtrOrNull(weight, C, "weight");
+  n.bias = FloatPtrOrNull(bias, C, "bias");
+  n.eps = static_cast<float>(eps);
+  n.momentum = static_cast<float>(momentum);
+  n.saved = saved.data_ptr<float>();
+  n.running_mean = rm;
+  n.running_var = rv;
+  n.batches = count;
+  const cudaError_t err = kern::LaunchBatchNormForward(
       x.data_ptr(), res, y.data_ptr(), signs.defined() ? signs.data_ptr<uint8_t>() : nullptr, M,
-      static_cast<int>(C), x.scalar_type() == at::kBFloat16, sums,
-      FloatPtrOrNull(weight, C, "weight"), FloatPtrOrNull(bias, C, "bias"),
-      static_cast<float>(eps), static_cast<float>(momentum), saved.data_ptr<float>(),
-      rm, rv, count, relu, stream);
+      static_cast<int>(C), x.scalar_type() == at::kBFloat16, n, relu, stream);
   TORCH_CHECK(err == cudaSuccess, "fused batch norm forward: ", cudaGetErrorString(err));
   return {y, saved, signs};
 }

@@ -7,6 +7,8 @@
 //     zero, in place of a store and a pass over three tensors;
 //   - the backward of the last batch norm and convolution (of the first stage's
 //     sizes) is one kernel, which stores no gradient of the batch norm's input;
+//   - the batch norm of the skip connection is formed where it is added, and the two
+//     batch norms' backwards read dy once;
 //   - the weights are cast in one launch, and so are their gradients.
 // The 3x3 convolution, the gradients of the weights and some 1x1 convolutions are
 // PyTorch's.
@@ -110,6 +112,7 @@ struct Sums {
   double* p = nullptr;
   Tensor own;
   bool ready = false;
+  Sums() = default;
   Sums(const Tensor& like, int channels) {
     p = ZeroedDoubles(kern::BatchNormScratchDoubles(channels), like, Stream(), &own);
   }
@@ -156,24 +159,38 @@ Tensor ConvForward(const Tensor& x, const Tensor& w, int64_t stride, Sums* sums)
       .contiguous(CL);
 }
 
-// saved: what the backward needs of the statistics; signs: see LaunchBatchNormForward
-// (filled where there is a residual).
-Tensor NormForward(const Tensor& x, const Tensor& residual, const Tensor& weight,
-                   const Tensor& bias, const Norm& norm, bool relu, const Sums& sums,
-                   Tensor* saved, Tensor* signs) {
+// The batch norm's arguments; *saved: what the backward needs of the statistics.
+kern::BatchNormForward Describe(const Tensor& weight, const Tensor& bias, const Norm& norm,
+                                const Sums& sums, Tensor* saved) {
+  const int64_t C = weight.numel();
+  *saved = at::empty({3, C}, weight.options());
+  kern::BatchNormForward n;
+  n.sums = sums.p;
+  n.summed = sums.ready;
+  n.weight = FloatPtrOrNull(weight, C, "weight");
+  n.bias = FloatPtrOrNull(bias, C, "bias");
+  n.eps = static_cast<float>(norm.eps);
+  n.momentum = static_cast<float>(norm.momentum);
+  n.saved = saved->data_ptr<float>();
+  n.running_mean = norm.mean.data_ptr<float>();
+  n.running_var = norm.var.data_ptr<float>();
+  n.batches = norm.batches.defined() ? norm.batches.data_ptr<int64_t>() : nullptr;
+  return n;
+}
+
+// relu(batch norm of x [+ residual, or batch norm of it]); signs are for the latter two.
+Tensor NormForward(const Tensor& x, const kern::BatchNormForward& n, const Tensor& residual,
+                   const kern::BatchNormForward* of_residual, Tensor* signs) {
   const int C = Channels(x);
+  const bool bf16 = x.scalar_type() == at::kBFloat16;
   Tensor y = at::empty_like(x, x.options(), CL);
-  *saved = at::empty({3, C}, x.options().dtype(at::kFloat));
   if (residual.defined()) *signs = at::empty({Rows(x), C / 8}, x.options().dtype(at::kByte));
-  Check(kern::LaunchBatchNormForward(
-            x.data_ptr(), residual.defined() ? residual.data_ptr() : nullptr, y.data_ptr(),
-            residual.defined() ? signs->data_ptr<uint8_t>() : nullptr, Rows(x), C,
-            x.scalar_type() == at::kBFloat16, sums.p, FloatPtrOrNull(weight, C, "weight"),
-            FloatPtrOrNull(bias, C, "bias"), static_cast<float>(norm.eps),
-            static_cast<float>(norm.momentum), saved->data_ptr<float>(),
-            norm.mean.data_ptr<float>(), norm.var.data_ptr<float>(),
-            norm.batches.defined() ? norm.batches.data_ptr<int64_t>() : nullptr, relu, Stream(),
-            sums.ready),
+  uint8_t* bits = residual.defined() ? signs->data_ptr<uint8_t>() : nullptr;
+  const void* r = residual.defined() ? residual.data_ptr() : nullptr;
+  Check(of_residual ? kern::LaunchBatchNormPairForward(x.data_ptr(), r, y.data_ptr(), bits, Rows(x),
+                                                       C, bf16, n, *of_residual, Stream())
+                    : kern::LaunchBatchNormForward(x.data_ptr(), r, y.data_ptr(), bits, Rows(x), C,
+                                                   bf16, n, true, Stream()),
         "batch norm forward");
   return y;
 }
@@ -181,6 +198,23 @@ Tensor NormForward(const Tensor& x, const Tensor& residual, const Tensor& weight
 struct NormGradients {
   Tensor x, residual, weight, bias;
 };
+
+// Of the two batch norms whose sum is the block's output: their sums alone, or the
+// gradients too.
+kern::BatchNormBackward Describe(const Tensor& weight, const Tensor& saved, const Sums& sums,
+                                 NormGradients* g) {
+  kern::BatchNormBackward n;
+  n.sums = sums.p;
+  n.weight = FloatPtrOrNull(weight, weight.numel(), "weight");
+  n.saved = saved.data_ptr<float>();
+  if (g != nullptr) {
+    g->weight = at::empty_like(weight);
+    g->bias = at::empty_like(weight);
+    n.dweight = g->weight.data_ptr<float>();
+    n.dbias = g->bias.data_ptr<float>();
+  }
+  return n;
+}
 
 // signs (where defined): dy counts where the block's output was above zero;
 // otherwise relu says whether this layer had a ReLU of its own.
@@ -217,7 +251,7 @@ bool OwnTail(const Tensor& out, const Tensor& w, int64_t stride) {
 // a: the convolution's input; leaf: its weight as the user has it.
 TailGradients TailBackward(const Tensor& dy, const Tensor& signs, const Tensor& x, const Tensor& a,
                            const Tensor& w, const Tensor& weight, const Tensor& saved,
-                           const Tensor& leaf, bool want_a) {
+                           const Tensor& leaf, const Sums& sums, bool want_a) {
   kern::NormConvBackward n;
   const auto fp32 = x.options().dtype(at::kFloat);
   TailGradients g;
@@ -234,7 +268,6 @@ TailGradients TailBackward(const Tensor& dy, const Tensor& signs, const Tensor& 
   const Tensor partial =
       at::empty({kern::NormConvBackwardParts(n.rows), n.cout, n.cin}, fp32,
                 at::MemoryFormat::Contiguous);
-  Sums sums(x, n.cout);
   n.dy = dy.data_ptr();
   n.x = x.data_ptr();
   n.a = a.data_ptr();
@@ -246,6 +279,7 @@ TailGradients TailBackward(const Tensor& dy, const Tensor& signs, const Tensor& 
   n.dw_stride_o = g.w.stride(0);
   n.dw_stride_i = g.w.stride(1);
   n.sums = sums.p;
+  n.summed = sums.ready;
   n.gamma = FloatPtrOrNull(weight, n.cout, "weight");
   n.saved = saved.data_ptr<float>();
   n.dgamma = g.weight.data_ptr<float>();
@@ -320,16 +354,22 @@ class Bottleneck : public torch::autograd::Function<Bottleneck> {
     const auto w = Cast(weights, block.type);
     std::array<Tensor, LAYERS> out, saved;  // of the convolutions; of the batch norms
     Tensor signs;
-    auto layer = [&](int i, const Tensor& in, int64_t stride, const Tensor& residual) {
-      Sums sums(x, static_cast<int>(w[i].size(0)));
-      out[i] = ConvForward(in, w[i], stride, &sums);
-      return NormForward(out[i], residual, gammas[i], betas[i], block.norms[i], i != DOWN, sums,
-                         &saved[i], &signs);
+    std::array<kern::BatchNormForward, LAYERS> norms;
+    std::vector<Sums> sums;  // kept until the kernels are launched
+    sums.reserve(LAYERS);
+    auto convolve = [&](int i, const Tensor& in, int64_t stride) {
+      sums.emplace_back(x, static_cast<int>(w[i].size(0)));
+      out[i] = ConvForward(in, w[i], stride, &sums.back());
+      norms[i] = Describe(gammas[i], betas[i], block.norms[i], sums.back(), &saved[i]);
     };
-    const Tensor a1 = layer(0, x, 1, {});
-    const Tensor a2 = layer(1, a1, block.stride, {});
-    const Tensor skip = down ? layer(DOWN, x, block.stride, {}) : x;
-    const Tensor y = layer(2, a2, 1, skip);
+    convolve(0, x, 1);
+    const Tensor a1 = NormForward(out[0], norms[0], {}, nullptr, nullptr);
+    convolve(1, a1, block.stride);
+    const Tensor a2 = NormForward(out[1], norms[1], {}, nullptr, nullptr);
+    if (down) convolve(DOWN, x, block.stride);
+    convolve(2, a2, 1);
+    const Tensor y = NormForward(out[2], norms[2], down ? out[DOWN] : x,
+                                 down ? &norms[DOWN] : nullptr, &signs);
     // Like relu's own backward, this one refuses to run when somebody has
     // changed y in place, although it does not read it.
     variable_list keep = {x, y, a1, a2, signs};
@@ -395,25 +435,61 @@ class Bottleneck : public torch::autograd::Function<Bottleneck> {
     const bool fused = kern::Conv1x1Supported(Rows(x), Channels(out[0]), Channels(x));
     Tensor da2, da1, dx, skip, mask;
     if (!down && fused) skip = dy, mask = signs;
-    // The end of the block and its skip convolution: `in`'s gradient (where
-    // wanted), the weight's goes to dw, the batch norm's to result.
-    auto tail = [&](int i, const Tensor& in, int64_t s, bool want_in) {
-      if (OwnTail(out[i], w[i], s)) {
+    auto keep_norm = [&](int i, const NormGradients& g) {
+      if (wanted(2 + 3 * i)) result[2 + 3 * i] = g.weight;
+      if (wanted(3 + 3 * i)) result[3 + 3 * i] = g.bias;
+    };
+    // The batch norms of the end of the block and of its skip connection have dy in
+    // common. Their convolutions' gradients come from the kernel that forms theirs
+    // (OwnTail) or from what is formed here.
+    const bool tails = OwnTail(out[2], w[2], 1) && (!down || OwnTail(out[DOWN], w[DOWN], stride));
+    Sums sums2, sums3;
+    if (down || tails) sums2 = Sums(x, Channels(out[2]));
+    if (down) sums3 = Sums(x, Channels(out[2]));
+    NormGradients g2, g3;
+    if (down) {
+      const bool bf16 = x.scalar_type() == at::kBFloat16;
+      const kern::BatchNormBackward n2 = Describe(gammas[2], saved[2], sums2, &g2),
+                                    n3 = Describe(gammas[DOWN], saved[DOWN], sums3, &g3);
+      const int C = Channels(dy);
+      if (tails) {
+        Check(kern::LaunchBatchNormPairSums(dy.data_ptr(), signs.data_ptr<uint8_t>(),
+                                            out[2].data_ptr(), out[DOWN].data_ptr(), Rows(dy), C,
+                                            bf16, n2, n3, Stream()),
+              "batch norm backward");
+        sums2.ready = sums3.ready = true;
+      } else {
+        g2.x = at::empty_like(out[2], out[2].options(), CL);
+        g3.x = at::empty_like(out[2], out[2].options(), CL);
+        Check(kern::LaunchBatchNormPairBackward(
+                  dy.data_ptr(), signs.data_ptr<uint8_t>(), out[2].data_ptr(),
+                  out[DOWN].data_ptr(), g2.x.data_ptr(), g3.x.data_ptr(), Rows(dy), C, bf16, n2,
+                  n3, Stream()),
+              "batch norm backward");
+        keep_norm(2, g2);
+        keep_norm(DOWN, g3);
+      }
+    } else if (!tails) {
+      g2 = norm(2, dy, signs, want_x && !fused);
+      if (want_x && !fused) skip = g2.residual;
+    }
+    // The gradient of the convolution's input `in`, where wanted.
+    auto tail = [&](int i, const Tensor& in, int64_t s, Tensor d_out, const Sums& sums,
+                    bool want_in) {
+      Tensor d_in;
+      if (tails) {
         const TailGradients g = TailBackward(dy, signs, out[i], in, w[i], gammas[i], saved[i],
-                                             weights[i], want_in);
+                                             weights[i], sums, want_in);
         if (wanted(2 + 3 * i)) result[2 + 3 * i] = g.weight;
         if (wanted(3 + 3 * i)) result[3 + 3 * i] = g.bias;
         if (wanted(1 + 3 * i)) result[1 + 3 * i] = g.w;
         return g.a;
       }
-      const bool want_skip = i == 2 && want_x && !down && !fused;
-      const NormGradients g = norm(i, dy, signs, want_skip);
-      if (want_skip) skip = g.residual;
-      Tensor d_in;
-      std::tie(d_in, dw[i]) = ConvBackward(g.x, in, w[i], s, want_in, wanted(1 + 3 * i));
+      std::tie(d_in, dw[i]) = ConvBackward(d_out, in, w[i], s, want_in, wanted(1 + 3 * i));
       return d_in;
     };
-    da2 = tail(2, a2, 1, true);
+    da2 = tail(2, a2, 1, g2.x, sums2, true);
+    g2.x.reset();
     const Tensor d2 = norm(1, da2, {}, false).x;
     da2.reset();
     std::tie(da1, dw[1]) = ConvBackward(d2, a1, w[1], stride, true, wanted(4));
@@ -424,12 +500,11 @@ class Bottleneck : public torch::autograd::Function<Bottleneck> {
                            kern::Conv1x1Supported(Rows(dy), Channels(dy), Channels(x));
       if (want_x && scatter) {
         // Its gradient of x is zero but for every fourth pixel: added in place.
-        const Tensor dd = norm(DOWN, dy, signs, false).x;
         std::tie(dx, dw[0]) = ConvBackward(d1, x, w[0], 1, true, wanted(1));
-        ConvInputGradient(dd, w[DOWN], dx, {}, true);
-        dw[DOWN] = ConvBackward(dd, x, w[DOWN], stride, false, wanted(10)).second;
+        ConvInputGradient(g3.x, w[DOWN], dx, {}, true);
+        dw[DOWN] = ConvBackward(g3.x, x, w[DOWN], stride, false, wanted(10)).second;
       } else {
-        skip = tail(DOWN, x, stride, want_x);
+        skip = tail(DOWN, x, stride, g3.x, sums3, want_x);
       }
     }
     if (!dx.defined()) {

@@ -242,6 +242,7 @@ def _rel(a, b):
 SHAPES = [
     (256, 64, 1, False, 4, 12, 10, torch.bfloat16), (64, 64, 1, True, 4, 12, 10, torch.bfloat16),
     (256, 128, 2, True, 4, 12, 10, torch.float16),
+    (64, 64, 1, True, 16, 28, 27, torch.float16), (256, 64, 2, True, 3, 10, 10, torch.bfloat16),
     (256, 128, 2, True, 4, 11, 9, torch.bfloat16),    # odd sizes: PyTorch's strided layers
     (64, 64, 2, True, 1, 2, 260, torch.bfloat16),     # and rows of more than 128 pixels
     (1024, 256, 1, False, 9, 7, 7, torch.float16),    # the first convolution is PyTorch's
