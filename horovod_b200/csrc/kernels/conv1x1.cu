@@ -51,17 +51,16 @@ constexpr uint16_t NAN16 = 0x7fff;  // a NaN of either 16-bit type
 
 enum Epilogue : int { STORE = 0, STORE_SUMS = 1, ADD = 2, ADD_MASKED = 3 };
 
+// Shared memory: output tiles, w where it stays, and a ring of slices of the
+// operands.
+constexpr int MOST_SLOTS = 8, MOST_BYTES = 226 * 1024;
 template <int BN, int EPI>
 struct Layout {
   static constexpr int BUFFER = BN / 64 * BOX_BYTES;
   // Output tiles: one more where a tile is also loaded ahead, one where it is
   // large.
   static constexpr int BUFFERS = BN == 256 ? 1 : EPI >= ADD ? 3 : 2;
-  static constexpr int SLICE = BOX_BYTES + BN * 128;
-  static constexpr int FIT = (224 * 1024 - 1024 - BUFFERS * BUFFER) / SLICE;
-  static constexpr int SLICES = FIT < 6 ? FIT : 6;
-  static constexpr int BYTES = 1024 + BUFFERS * BUFFER + SLICES * SLICE;
-  static_assert(SLICES >= 3, "too few slices in flight");
+  static constexpr int W_SLICE = BN * 128;
 };
 
 struct Maps {
@@ -71,6 +70,8 @@ struct Maps {
 struct Shape {
   int64_t rows;
   int n, slices_k, tiles_m, tiles_n;
+  bool w_stays;
+  int slots;
   int tile_rows;       // rows of a tile that count: 128, or whole rows of pixels
   int x_step1, x_step2, y_step1, y_step2;  // coordinates of a tile per tile
   int width;           // y's pixels: see pixel_at()
@@ -118,12 +119,16 @@ conv1x1_kernel(const __grid_constant__ Maps maps, const __grid_constant__ Shape 
                const uint32_t wait_ns) {
   using L = Layout<BN, EPI>;
   extern __shared__ unsigned char raw[];
-  __shared__ __align__(8) uint64_t s_full[L::SLICES], s_empty[L::SLICES], s_acc_full[2],
+  __shared__ __align__(8) uint64_t s_full[MOST_SLOTS], s_empty[MOST_SLOTS], s_w_full,
+      s_acc_full[2],
       s_acc_empty[2], s_add_full[L::BUFFERS], s_add_empty[L::BUFFERS], s_drain;
   __shared__ uint32_t s_tmem;
   __shared__ volatile int s_stop;
   const uint32_t buffers = (smem_addr(raw) + 1023u) & ~1023u;
-  const uint32_t slices = buffers + L::BUFFERS * L::BUFFER;
+  // The slices of w are either before the ring or each behind its slice of x.
+  const uint32_t weights = buffers + L::BUFFERS * L::BUFFER;
+  const uint32_t slices = weights + (s.w_stays ? s.slices_k * L::W_SLICE : 0);
+  const uint32_t slice_bytes = BOX_BYTES + (s.w_stays ? 0 : L::W_SLICE);
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
 
   if (threadIdx.x == 0) {
@@ -131,7 +136,8 @@ conv1x1_kernel(const __grid_constant__ Maps maps, const __grid_constant__ Shape 
       asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;"
                    ::"r"(smem_addr(bar)), "r"(count) : "memory");
     };
-    for (int i = 0; i < L::SLICES; ++i) init(s_full + i, 1), init(s_empty + i, 1);
+    for (int i = 0; i < MOST_SLOTS; ++i) init(s_full + i, 1), init(s_empty + i, 1);
+    init(&s_w_full, 1);
     for (int i = 0; i < 2; ++i) init(s_acc_full + i, 1), init(s_acc_empty + i, 8);
     for (int i = 0; i < L::BUFFERS; ++i) init(s_add_full + i, 1), init(s_add_empty + i, 1);
     init(&s_drain, 1);
@@ -154,53 +160,63 @@ conv1x1_kernel(const __grid_constant__ Maps maps, const __grid_constant__ Shape 
 
   if (warp == 0) {
     if (lane == 0) {
-      uint32_t issued = 0;
+      auto load_w = [&](uint32_t to, int k, uint32_t bar) {
+        if (W_MN) {
+#pragma unroll
+          for (int j = 0; j < BN / 64; ++j)
+            load_box(to + j * 8192, &maps.w, n0 + j * 64, k * SLICE_K, 0, bar);
+        } else {
+          load_box(to, &maps.w, k * SLICE_K, n0, 0, bar);
+        }
+      };
+      if (s.w_stays) {
+        expect_bytes(smem_addr(&s_w_full), s.slices_k * L::W_SLICE);
+        for (int k = 0; k < s.slices_k; ++k)
+          load_w(weights + k * L::W_SLICE, k, smem_addr(&s_w_full));
+      }
+      uint32_t slot = 0, phase = 0, issued = 0;
       bool ok = true;
       for (int tile = first; ok && tile < s.tiles_m; tile += step)
         for (int k = 0; k < s.slices_k; ++k, ++issued) {
-          const uint32_t i = issued % L::SLICES, bar = smem_addr(&s_full[i]);
-          ok = wait_or_stop(smem_addr(&s_empty[i]), (issued / L::SLICES & 1u) ^ 1u, wait_ns,
-                            &s_stop);
+          const uint32_t bar = smem_addr(&s_full[slot]), to = slices + slot * slice_bytes;
+          ok = wait_or_stop(smem_addr(&s_empty[slot]), phase ^ 1u, wait_ns, &s_stop);
           if (!ok) break;
-          const uint32_t to = slices + i * L::SLICE;
-          expect_bytes(bar, s.tile_rows * 128 + BN * 128);
+          expect_bytes(bar, s.tile_rows * 128 + (s.w_stays ? 0 : L::W_SLICE));
           load_box(to, &maps.x, k * SLICE_K, tile * s.x_step1, tile * s.x_step2, bar);
-          if (W_MN) {
-#pragma unroll
-            for (int j = 0; j < BN / 64; ++j)
-              load_box(to + BOX_BYTES + j * 8192, &maps.w, n0 + j * 64, k * SLICE_K, 0, bar);
-          } else {
-            load_box(to + BOX_BYTES, &maps.w, k * SLICE_K, n0, 0, bar);
-          }
+          if (!s.w_stays) load_w(to + BOX_BYTES, k, bar);
+          if (++slot == s.slots) slot = 0, phase ^= 1u;
         }
       if (!ok) s_stop = 1;
       // No copy may be in flight when the CTA ends.
-      for (uint32_t u = issued < L::SLICES ? 0 : issued - L::SLICES; u < issued; ++u)
-        wait_bounded(smem_addr(&s_full[u % L::SLICES]), u / L::SLICES & 1u, STEM_WAIT_NS);
+      if (s.w_stays) wait_bounded(smem_addr(&s_w_full), 0, STEM_WAIT_NS);
+      const uint32_t slots = s.slots;
+      for (uint32_t u = issued < slots ? 0 : issued - slots; u < issued; ++u)
+        wait_bounded(smem_addr(&s_full[u % slots]), u / slots & 1u, STEM_WAIT_NS);
     }
   } else if (warp == 1) {
     if (lane == 0) {
       constexpr uint32_t idesc =
           instruction(std::is_same<T, __nv_bfloat16>::value, false, W_MN, TILE_M, BN);
-      uint32_t taken = 0, i = 0;
-      bool ok = true;
-      for (int tile = first; tile < s.tiles_m; tile += step, ++i) {
+      uint32_t slot = 0, phase = 0, i = 0;
+      bool ok = !s.w_stays || wait_or_stop(smem_addr(&s_w_full), 0, wait_ns, &s_stop);
+      for (int tile = first; ok && tile < s.tiles_m; tile += step, ++i) {
         const uint32_t acc = i & 1u;
         ok = wait_or_stop(smem_addr(&s_acc_empty[acc]), (i >> 1 & 1u) ^ 1u, wait_ns, &s_stop);
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        for (int k = 0; k < s.slices_k; ++k, ++taken) {
-          const uint32_t slot = taken % L::SLICES;
-          ok = wait_or_stop(smem_addr(&s_full[slot]), taken / L::SLICES & 1u, wait_ns, &s_stop);
+        for (int k = 0; k < s.slices_k; ++k) {
+          ok = wait_or_stop(smem_addr(&s_full[slot]), phase, wait_ns, &s_stop);
           if (!ok) break;
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          const uint32_t a = slices + slot * L::SLICE, b = a + BOX_BYTES;
+          const uint32_t a = slices + slot * slice_bytes;
+          const uint32_t b = s.w_stays ? weights + k * L::W_SLICE : a + BOX_BYTES;
 #pragma unroll
           for (int j = 0; j < SLICE_K / 16; ++j)
             mma(tmem + acc * BN, operand_swizzled(a + j * 32, 16),
                 W_MN ? operand_swizzled(b + j * 2048, 8192) : operand_swizzled(b + j * 32, 16),
                 idesc, k > 0 || j > 0);
           commit(smem_addr(&s_empty[slot]));
+          if (++slot == s.slots) slot = 0, phase ^= 1u;
         }
         if (!ok) break;
         commit(smem_addr(&s_acc_full[acc]));
@@ -419,14 +435,24 @@ cudaError_t LaunchTyped(const Conv1x1& c, Shape s, cudaStream_t stream, int* sta
                      static_cast<int64_t>(w_rows) * w_cols, W_MN ? SLICE_K : BN, 1);
   if (!ok) return cudaErrorInvalidValue;
   auto kernel = conv1x1_kernel<T, BN, W_MN, EPI>;
+  // w stays in shared memory for all tiles of a CTA where three slices of x still fit
+  // beside it: gradient of 1024 channels from 256 with the masked sum, 50176 rows, 62 to 53
+  // us; of 256 from 64, 802816 rows, 174 to 152.
+  const int fixed = 1024 + L::BUFFERS * L::BUFFER, all_of_w = s.slices_k * L::W_SLICE;
+  s.w_stays = fixed + all_of_w + 3 * BOX_BYTES <= MOST_BYTES;
+  const int slice = BOX_BYTES + (s.w_stays ? 0 : L::W_SLICE);
+  const int before = fixed + (s.w_stays ? all_of_w : 0);
+  s.slots = (MOST_BYTES - before) / slice;
+  if (s.slots > MOST_SLOTS) s.slots = MOST_SLOTS;
+  const int bytes = before + s.slots * slice;
   const cudaError_t err =
-      cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, L::BYTES);
+      cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
   if (err != cudaSuccess) return err;
   int per_column = 148 / s.tiles_n;  // CTAs of a column of tiles
   if (per_column < 1) per_column = 1;
   if (per_column > s.tiles_m) per_column = s.tiles_m;
   CountKernelLaunches(1);
-  kernel<<<per_column * s.tiles_n, THREADS, L::BYTES, stream>>>(
+  kernel<<<per_column * s.tiles_n, THREADS, bytes, stream>>>(
       maps, s, c.signs, static_cast<uint16_t*>(c.y), c.sums, status, wait_ns);
   return cudaGetLastError();
 }
@@ -477,12 +503,13 @@ cudaError_t LaunchConv1x1(const Conv1x1& c, cudaStream_t stream, uint32_t wait_n
   s.slices_k = c.k / SLICE_K;
   s.copies = c.copies;
   const int64_t tiles_m = (c.rows + TILE_M - 1) / TILE_M;
-  // The widest tile that still gives every SM one: wider tiles read x less often (64
-  // to 256 channels at 802816 rows), narrower ones spread few rows over more SMs. With
-  // a tile to add, 128 leaves room for three of them ahead.
+  // Wider tiles read x less often, which is what the loop over k waits for: 50176 rows,
+  // 256 to 1024 channels: 70, 43 and 39 us with 64, 128 and 256; 6272 rows, 1024 to 256:
+  // 18, 14 and 16. Tiles of 256 want two for every SM (6272 rows, 256 to 1024: 12 us with
+  // 128, 14 with 256). With a tile to add, 128 leaves room for three of them ahead.
   int width = 64;
-  if (c.n % 128 == 0 && tiles_m * (c.n / 128) >= 148) width = 128;
-  if (c.n % 256 == 0 && c.add == nullptr && tiles_m * (c.n / 256) >= 148) width = 256;
+  if (c.n % 128 == 0) width = 128;
+  if (c.n % 256 == 0 && c.add == nullptr && tiles_m * (c.n / 256) >= 2 * 148) width = 256;
   if (c.bf16)
     return width == 256   ? LaunchWidth<__nv_bfloat16, 256>(c, s, stream, status, wait_ns)
            : width == 128 ? LaunchWidth<__nv_bfloat16, 128>(c, s, stream, status, wait_ns)
