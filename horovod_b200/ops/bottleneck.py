@@ -60,13 +60,17 @@ def _plain_norm(norm, relu, conv, device):
 
 def _layers(block):
     """(convolution, batch norm, kernel size, stride, has a ReLU) of every layer, or
-    None when the skip connection is something else."""
+    None when one of them is something else."""
+    for conv in (block.conv1, block.conv2, block.conv3):
+        if type(conv) is not nn.Conv2d:
+            return None
     stride = block.conv2.stride[0]
     layers = [(block.conv1, block.bn1, 1, 1, True), (block.conv2, block.bn2, 3, stride, True),
               (block.conv3, block.bn3, 1, 1, True)]
     down = block.downsample
     if down is not None:
-        if type(down) is not nn.Sequential or len(down) != 2 or _observed(down):
+        if type(down) is not nn.Sequential or len(down) != 2 or _observed(down) or \
+                type(down[0]) is not nn.Conv2d:
             return None
         layers.append((down[0], down[1], 1, stride, False))
     return layers

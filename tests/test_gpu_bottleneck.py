@@ -326,6 +326,34 @@ def test_block_with_other_layouts(change, monkeypatch):
         assert a is None or (_rel(a, b) <= 4e-2 and a.dtype == b.dtype)
 
 
+class _Add(nn.Module):
+    def __init__(self, norm):
+        super().__init__()
+        self.norm = norm
+
+    def forward(self, x, residual):
+        return self.norm(x) + residual
+
+
+@pytest.mark.parametrize("inplanes,planes,stride,down", [
+    (256, 64, 1, False), (64, 64, 1, True), (256, 128, 2, True), (512, 128, 1, False)])
+def test_block_whose_input_wants_no_gradient(inplanes, planes, stride, down):
+    """The parameters' gradients are those of a block whose input does."""
+    block = _block(inplanes, planes, stride, down)
+    g = torch.Generator(device=_dev()).manual_seed(14)
+    x = _act(g, 4, inplanes, 12, 10, torch.bfloat16).relu_()
+    assert _available(block, x)
+    params = list(block.parameters())
+
+    def grads(x):
+        with torch.autocast("cuda", dtype=torch.bfloat16):
+            y = block(x)
+        return torch.autograd.grad(y, params, torch.ones_like(y))
+
+    for a, b in zip(grads(x), grads(x.detach().requires_grad_(True))):
+        assert _rel(a, b) <= 2e-2  # sums in another order
+
+
 def test_block_leaves_the_rest_to_its_layers():
     from horovod_b200.ops.bottleneck import fused_bottleneck_available
     g = torch.Generator(device=_dev()).manual_seed(6)
@@ -355,6 +383,12 @@ def test_block_leaves_the_rest_to_its_layers():
     plain(changed(lambda b: setattr(b.conv2, "dilation", (2, 2))
                   or setattr(b.conv2, "padding", (2, 2))))
     plain(changed(lambda b: nn.utils.parametrizations.weight_norm(b.conv1)))
+    # layers without a stride, channels or statistics of their own
+    plain(changed(lambda b: setattr(b, "conv1", nn.Sequential(b.conv1))))
+    plain(changed(lambda b: setattr(b, "conv2", nn.Sequential(b.conv2))))
+    plain(changed(lambda b: setattr(b, "bn3", _Add(b.bn3))))
+    plain(changed(lambda b: setattr(b, "downsample", nn.Sequential(nn.Identity(), nn.Identity()))))
+    plain(changed(lambda b: setattr(b, "downsample", nn.Identity())))
     calls = []
     plain(changed(lambda b: b.conv2.register_forward_hook(lambda *a: calls.append(1))))
     plain(changed(lambda b: b.bn3.register_full_backward_hook(lambda *a: None)))
