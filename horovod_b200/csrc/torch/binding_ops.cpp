@@ -5,6 +5,7 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/extension.h>
 
+#include <atomic>
 #include <cstdint>
 #include <map>
 #include <mutex>
@@ -44,12 +45,15 @@ const float* FloatPtrOrNull(const c10::optional<at::Tensor>& t, int64_t channels
 
 // Zero-filled scratch for the batch-norm reductions without a fill launch per
 // call: slices are handed out from a per-stream pool that is cleared with one
-// memset whenever it has been used up. Slices are consumed in stream order
-// and the memset is queued behind their consumers, so a slice is zero when
-// the kernel that was given it runs. A stream that is being captured gets memory
-// of its own, filled inside the graph (`own` keeps it until the launches are
-// queued): every replay has to start from zeros, and slices of the pool would be
-// cleared by none.
+// memset whenever it has been used up. The memset is queued behind the consumers of
+// all slices whose `own` is gone, so a slice is zero when the first kernel that was
+// given it runs. Where a slice is still held, by the caller itself (a block of layers
+// keeps the sums of one layer while it asks for the next one's) or by another thread
+// that launches to the same stream, a memset could erase sums that nobody has read or
+// come before kernels that still add to theirs: such a pool is left to its holders and
+// a new one takes its place. A stream that is being captured gets memory of its own,
+// filled inside the graph: every replay has to start from zeros, and slices of the
+// pool would be cleared by none.
 double* ZeroedDoubles(int64_t count, const at::Tensor& like, cudaStream_t stream,
                       at::Tensor* own) {
   // (The default stream cannot be captured. Asking takes 0.2 to 0.4 us on the host,
@@ -69,15 +73,24 @@ double* ZeroedDoubles(int64_t count, const at::Tensor& like, cudaStream_t stream
   TORCH_CHECK(count <= POOL_DOUBLES, "batch norm scratch request too large");
   std::lock_guard<std::mutex> lock(mu);
   Pool& p = pools[{like.get_device(), stream}];
+  const int64_t need = (count + 31) / 32 * 32;  // 256-byte slices
+  if (p.buf.defined() && p.used + need > POOL_DOUBLES) {
+    if (p.buf.use_count() == 1) {
+      // Another thread's launches came before it let go of its slice.
+      std::atomic_thread_fence(std::memory_order_acquire);
+      const cudaError_t err =
+          cudaMemsetAsync(p.buf.data_ptr(), 0, POOL_DOUBLES * sizeof(double), stream);
+      TORCH_CHECK(err == cudaSuccess, "batch norm scratch: ", cudaGetErrorString(err));
+      p.used = 0;
+    } else {
+      p.buf.reset();
+    }
+  }
   if (!p.buf.defined()) {
     p.buf = at::zeros({POOL_DOUBLES}, like.options().dtype(at::kDouble));
     p.used = 0;
   }
-  const int64_t need = (count + 31) / 32 * 32;  // 256-byte slices
-  if (p.used + need > POOL_DOUBLES) {
-    cudaMemsetAsync(p.buf.data_ptr(), 0, POOL_DOUBLES * sizeof(double), stream);
-    p.used = 0;
-  }
+  *own = p.buf;
   double* out = p.buf.data_ptr<double>() + p.used;
   p.used += need;
   return out;

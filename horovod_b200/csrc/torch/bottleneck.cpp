@@ -107,7 +107,8 @@ std::array<Tensor, LAYERS> Cast(const std::array<Tensor, LAYERS>& from, at::Scal
   return out;
 }
 
-// Sums of a batch norm's input: scratch, and whether the convolution filled it.
+// Sums of a batch norm's input: scratch, and whether they are in it already. Has to
+// live until the kernels that read them are launched.
 struct Sums {
   double* p = nullptr;
   Tensor own;

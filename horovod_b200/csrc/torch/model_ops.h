@@ -15,8 +15,9 @@ void CheckActivations(const at::Tensor& t, const char* what);
 at::Tensor Activations(const at::Tensor& t, const char* what);
 const float* FloatPtrOrNull(const c10::optional<at::Tensor>& t, int64_t channels,
                             const char* what);
-// `count` doubles that are zero when the next kernel of the stream runs; `own` has
-// to live until that kernel is launched.
+// `count` doubles that are zero when the next kernel of the stream runs. `own` has to
+// live until the last kernel that uses them is launched; until then no other request
+// clears them.
 double* ZeroedDoubles(int64_t count, const at::Tensor& like, cudaStream_t stream,
                       at::Tensor* own);
 

@@ -501,3 +501,71 @@ def test_block_on_two_streams():
     torch.cuda.synchronize()
     for a, b in zip(alone, together):
         assert max(_rel(b[k], a[k]) for k in a if a[k].is_floating_point()) <= 2e-2
+
+
+@pytest.mark.parametrize("inplanes,planes,stride", [(64, 64, 1), (256, 128, 2), (1024, 256, 2)])
+def test_block_holds_its_sums_while_others_ask_for_scratch(inplanes, planes, stride):
+    """The zeroed scratch of the batch norms is cleared whenever it has been handed out
+    once. Wherever in a step of a block that happens, and for whatever was written
+    before, every step has the results of the first."""
+    from horovod_b200 import _C
+    import random
+    block = _block(inplanes, planes, stride, True)
+    for m in block.modules():
+        if isinstance(m, nn.BatchNorm2d):
+            m.momentum = 1.0  # the running statistics are those of the step
+    g = torch.Generator(device=_dev()).manual_seed(21)
+    x = _act(g, 2, inplanes, 8, 6, torch.bfloat16).relu_()
+    dy = _act(g, 2, planes * 4, 8 // stride, 6 // stride, torch.bfloat16)
+    assert _available(block, x)
+    other = _act(g, 1, 64, 2, 2, torch.bfloat16)
+    rng = random.Random(22)  # where in a step the scratch is used up: all over it
+    want, worst = None, None
+    for _ in range(1200):
+        for _ in range(rng.randrange(8)):
+            _C.bn_forward(other, None, None, None, None, None, 0.1, 1e-5, False, None)
+        got = [t.double() for t in _step(block, x, dy).values() if t.is_floating_point()]
+        if want is None:
+            want, worst = got, torch.zeros(len(got), device=_dev(), dtype=torch.float64)
+        worst = torch.maximum(worst, torch.stack(
+            [(a - b).norm() / (b.norm() + 1e-30) for a, b in zip(got, want)]))
+    # Sums in another order: a value in a few thousand rounds the other way or passes
+    # a ReLU (2^-8 and 1 of its size). Sums that are lost change all values of a layer.
+    assert bool((worst <= 5e-2).all()), worst.tolist()
+
+
+def test_blocks_of_two_threads_on_one_stream():
+    """Each thread has the results of one alone."""
+    import threading
+    g = torch.Generator(device=_dev()).manual_seed(23)
+    blocks = [_block(64, 64, 1, True, seed) for seed in (1, 2)]
+    x = _act(g, 2, 64, 8, 6, torch.bfloat16)
+    dy = _act(g, 2, 256, 8, 6, torch.bfloat16)
+    worst = {}
+
+    def work(i):
+        params = list(blocks[i].parameters())
+
+        def step():
+            with torch.autocast("cuda", dtype=torch.bfloat16):
+                y = blocks[i](x)
+            return [y.detach()] + list(torch.autograd.grad(y, params, dy))
+        want = first[i]
+        worst[i] = torch.zeros(len(want), device=_dev(), dtype=torch.float64)
+        for _ in range(300):
+            worst[i] = torch.maximum(worst[i], torch.stack(
+                [(a.double() - b.double()).norm() / (b.double().norm() + 1e-30)
+                 for a, b in zip(step(), want)]))
+
+    first = []
+    for b in blocks:
+        with torch.autocast("cuda", dtype=torch.bfloat16):
+            y = b(x)
+        first.append([y.detach()] + list(torch.autograd.grad(y, list(b.parameters()), dy)))
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for i in range(2):
+        assert bool((worst[i] <= 5e-2).all()), worst[i].tolist()
