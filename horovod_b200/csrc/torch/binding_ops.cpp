@@ -178,7 +178,7 @@ struct NormGradients {
 };
 
 NormGradients NormBackward(at::Tensor dy, at::Tensor x, const c10::optional<at::Tensor>& weight,
-                           const at::Tensor& saved, const c10::optional<at::Tensor>& signs,
+                           at::Tensor saved, const c10::optional<at::Tensor>& signs,
                            bool relu, bool want_dresidual) {
   x = Activations(x, "x");
   dy = Activations(dy, "dy");
@@ -187,6 +187,8 @@ NormGradients NormBackward(at::Tensor dy, at::Tensor x, const c10::optional<at::
   TORCH_CHECK(saved.is_cuda() && saved.scalar_type() == at::kFloat && saved.is_contiguous() &&
                   saved.numel() == 3 * C,
               "saved must be the tensor returned by bn_forward");
+  // (A saved-tensor hook may have moved it.)
+  if (reinterpret_cast<uintptr_t>(saved.data_ptr()) % 16 != 0) saved = saved.clone();
   const uint8_t* sign_bits = nullptr;
   if (signs.has_value() && signs->defined()) {
     TORCH_CHECK(signs->is_cuda() && signs->scalar_type() == at::kByte &&

@@ -57,6 +57,12 @@ void Check(cudaError_t err, const char* what) {
   TORCH_CHECK(err == cudaSuccess, what, ": ", cudaGetErrorString(err));
 }
 
+// t in a memory format and on a 16-byte boundary, which is how the kernels read it.
+Tensor Dense(const Tensor& t, at::MemoryFormat format) {
+  const Tensor c = t.contiguous(format);
+  return reinterpret_cast<uintptr_t>(c.data_ptr()) % 16 == 0 ? c : c.clone(format);
+}
+
 int64_t Rows(const Tensor& t) { return t.numel() / t.size(1); }
 int Channels(const Tensor& t) { return static_cast<int>(t.size(1)); }
 
@@ -337,6 +343,47 @@ Tensor Composition(const Tensor& x, const std::array<Tensor, LAYERS>& w,
   return at::relu(layer(2, a2, 1) + skip);
 }
 
+// What a backward has saved, by layer.
+struct Kept {
+  Tensor x, a1, a2, signs;
+  std::array<Tensor, LAYERS> w, gammas, betas, out, saved;
+};
+
+// Saved tensors went through the user's hooks, if there are any. Their values and
+// shapes are the forward's; the kernels read them by pointer, so that is looked at.
+void CheckKept(const Kept& k, int layers, const Tensor& dy, int64_t stride) {
+  bool ok = k.x.defined() && k.x.dim() == 4;
+  auto is = [&](const Tensor& t, at::ScalarType type, at::IntArrayRef sizes) {
+    ok = ok && t.defined() && t.layout() == at::kStrided && t.device() == dy.device() &&
+         t.scalar_type() == type && t.sizes() == sizes;
+  };
+  std::array<int64_t, LAYERS> c;
+  for (int i = 0; i < layers; ++i) c[i] = k.gammas[i].defined() ? k.gammas[i].numel() : 0;
+  if (ok) {
+    const at::ScalarType type = k.x.scalar_type();
+    const int64_t n = dy.size(0), h = k.x.size(2), w = k.x.size(3), ho = dy.size(2),
+                  wo = dy.size(3), cx = k.x.size(1);
+    ok = (type == at::kBFloat16 || type == at::kHalf) && (h - 1) / stride + 1 == ho &&
+         (w - 1) / stride + 1 == wo && c[2] == dy.size(1);
+    is(k.x, type, {n, cx, h, w});
+    is(k.a1, type, {n, c[0], h, w});
+    is(k.a2, type, {n, c[1], ho, wo});
+    is(k.signs, at::kByte, {n * ho * wo, c[2] / 8});
+    is(k.w[0], type, {c[0], cx, 1, 1});
+    is(k.w[1], type, {c[1], c[0], 3, 3});
+    is(k.w[2], type, {c[2], c[1], 1, 1});
+    if (layers > DOWN) is(k.w[DOWN], type, {c[2], cx, 1, 1});
+    is(k.out[0], type, {n, c[0], h, w});
+    is(k.out[1], type, {n, c[1], ho, wo});
+    for (int i = 2; i < layers; ++i) is(k.out[i], type, {n, c[2], ho, wo});
+    for (int i = 0; i < layers; ++i) {
+      is(k.gammas[i], at::kFloat, k.gammas[i].sizes());
+      is(k.saved[i], at::kFloat, {3, c[i]});
+    }
+  }
+  TORCH_CHECK(ok, "bottleneck: a saved tensor has come back with another shape, type or device");
+}
+
 class Bottleneck : public torch::autograd::Function<Bottleneck> {
  public:
   static Variable forward(AutogradContext* ctx, const Variable& x, const Variable& w0,
@@ -389,20 +436,25 @@ class Bottleneck : public torch::autograd::Function<Bottleneck> {
   }
 
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    // Inputs: x, then weight, gamma and beta of each layer.
+    variable_list result(1 + 3 * LAYERS + 1);
+    if (!grads[0].defined()) return result;
     const variable_list keep = ctx->get_saved_variables();
-    const Tensor &x = keep[0], &a1 = keep[2], &a2 = keep[3], &signs = keep[4];
     const bool down = keep.size() > 5 + 5 * DOWN;
+    const int layers = down ? LAYERS : DOWN;
     const int64_t stride = ctx->saved_data["stride"].toInt();
     const std::vector<Tensor> leaves = ctx->saved_data["weights"].toTensorVector();
-    std::array<Tensor, LAYERS> w, gammas, betas, out, saved, weights;
-    for (int i = 0; i < (down ? LAYERS : DOWN); ++i) {
+    Kept k;
+    Tensor &x = k.x, &a1 = k.a1, &a2 = k.a2, &signs = k.signs;
+    auto &w = k.w, &gammas = k.gammas, &betas = k.betas, &out = k.out, &saved = k.saved;
+    std::array<Tensor, LAYERS> weights;
+    x = keep[0], a1 = keep[2], a2 = keep[3], signs = keep[4];
+    for (int i = 0; i < layers; ++i) {
       const size_t at = 5 + 5 * static_cast<size_t>(i);
       w[i] = keep[at], gammas[i] = keep[at + 1], betas[i] = keep[at + 2], out[i] = keep[at + 3],
       saved[i] = keep[at + 4], weights[i] = leaves[i];
     }
-    // Inputs: x, then weight, gamma and beta of each layer.
-    variable_list result(1 + 3 * LAYERS + 1);
-    if (!grads[0].defined()) return result;
+    CheckKept(k, layers, grads[0], stride);
     auto wanted = [&](int input) { return ctx->needs_input_grad(input); };
     if (at::GradMode::is_enabled()) {
       variable_list inputs;
@@ -420,6 +472,14 @@ class Bottleneck : public torch::autograd::Function<Bottleneck> {
       return result;
     }
     c10::cuda::CUDAGuard guard(x.device());
+    x = Dense(x, CL), a1 = Dense(a1, CL), a2 = Dense(a2, CL);
+    signs = Dense(signs, at::MemoryFormat::Contiguous);
+    for (int i = 0; i < layers; ++i) {
+      out[i] = Dense(out[i], CL);
+      if (i != 1) w[i] = Dense(w[i], at::MemoryFormat::Contiguous);  // (the 3x3 is PyTorch's)
+      gammas[i] = Dense(gammas[i], at::MemoryFormat::Contiguous);
+      saved[i] = Dense(saved[i], at::MemoryFormat::Contiguous);
+    }
     Tensor dy = grads[0];
     if (dy.scalar_type() != x.scalar_type()) dy = dy.to(x.scalar_type());
     dy = Activations(dy.contiguous(CL), "dy");

@@ -569,3 +569,51 @@ def test_blocks_of_two_threads_on_one_stream():
         t.join()
     for i in range(2):
         assert bool((worst[i] <= 5e-2).all()), worst[i].tolist()
+
+
+@pytest.mark.parametrize("inplanes,planes,stride,down", [
+    (256, 64, 1, False), (64, 64, 1, True), (256, 128, 2, True), (32, 16, 2, True)])
+def test_block_whose_saved_tensors_come_back_in_another_layout(inplanes, planes, stride, down):
+    """save_on_cpu(pin_memory=True) packs into contiguous memory: what comes back is NCHW."""
+    block = _block(inplanes, planes, stride, down)
+    g = torch.Generator(device=_dev()).manual_seed(24)
+    x = _act(g, 4, inplanes, 12, 10, torch.bfloat16).relu_().requires_grad_(True)
+    inputs = [x] + list(block.parameters())
+    assert _available(block, x)
+
+    def grads():
+        with torch.autocast("cuda", dtype=torch.bfloat16):
+            y = block(x)
+        return y
+
+    y = grads()
+    want = torch.autograd.grad(y, inputs, torch.ones_like(y))
+    with torch.autograd.graph.save_on_cpu(pin_memory=True):
+        y = grads()
+    for a, b in zip(torch.autograd.grad(y, inputs, torch.ones_like(y)), want):
+        assert _rel(a, b) <= 2e-2  # sums in another order
+
+
+def test_block_whose_saved_tensors_come_back_off_a_boundary():
+    """And with what does not fit the forward's, the backward raises."""
+    block = _block(64, 64, 1, True)
+    g = torch.Generator(device=_dev()).manual_seed(25)
+    x = _act(g, 4, 64, 12, 10, torch.bfloat16).relu_().requires_grad_(True)
+    inputs = [x] + list(block.parameters())
+
+    def off(t):
+        flat = torch.empty(t.numel() + 1, device=t.device, dtype=t.dtype)
+        return torch.as_strided(flat, t.shape, t.stride(), 1).copy_(t)
+
+    def run(unpack):
+        with torch.autograd.graph.saved_tensors_hooks(lambda t: t, unpack):
+            with torch.autocast("cuda", dtype=torch.bfloat16):
+                y = block(x)
+        return torch.autograd.grad(y, inputs, torch.ones_like(y))
+
+    for a, b in zip(run(off), run(lambda t: t)):
+        assert _rel(a, b) <= 2e-2  # sums in another order
+    for spoil in (lambda t: t[:1], lambda t: t.cpu(),
+                  lambda t: t.float() if t.dtype == torch.bfloat16 else t):
+        with pytest.raises(RuntimeError, match="saved"):
+            run(spoil)
