@@ -596,6 +596,9 @@ void BindBottleneck(py::module_& m) {
     TORCH_CHECK(layers.size() >= DOWN && layers.size() <= LAYERS && rates.size() == layers.size(),
                 "bottleneck: three or four layers");
     CheckActivations(x, "x");
+    TORCH_CHECK(x.numel() > 0 && reinterpret_cast<uintptr_t>(x.data_ptr()) % 16 == 0,
+                "bottleneck: x must have elements and start on a 16-byte boundary");
+    TORCH_CHECK(stride == 1 || stride == 2, "bottleneck: a stride of 1 or 2");
     Block block;
     block.stride = stride;
     block.type = x.scalar_type();
@@ -603,10 +606,12 @@ void BindBottleneck(py::module_& m) {
     for (size_t i = 0; i < layers.size(); ++i) {
       TORCH_CHECK(layers[i].size() == 6, "bottleneck: six tensors per layer");
       for (int k = 0; k < 5; ++k)
-        TORCH_CHECK(layers[i][k].has_value() && layers[i][k]->is_cuda(),
-                    "bottleneck: tensors of a layer must be on the GPU");
+        TORCH_CHECK(layers[i][k].has_value() && layers[i][k]->device() == x.device(),
+                    "bottleneck: tensors of a layer must be on the device of x");
       for (int k = 0; k < 3; ++k) p[3 * i + k] = *layers[i][k];
       TORCH_CHECK(p[3 * i].dim() == 4, "bottleneck: weights of convolutions are 4-D");
+      TORCH_CHECK(p[3 * i].scalar_type() == at::kFloat || p[3 * i].scalar_type() == block.type,
+                  "bottleneck: weights of convolutions are float32 or of the type of x");
       const int64_t C = p[3 * i].size(0);
       for (int k = 1; k < 5; ++k) FloatPtrOrNull(layers[i][k], C, "a batch norm's tensor");
       Norm& n = block.norms[i];
@@ -618,7 +623,16 @@ void BindBottleneck(py::module_& m) {
                   "num_batches_tracked must be one int64 on the GPU");
       n.momentum = rates[i].first;
       n.eps = rates[i].second;
+      TORCH_CHECK(kern::BatchNormSupported(1, static_cast<int>(C)), "bottleneck does not support ",
+                  C, " channels");
     }
+    // The kernels take the sizes of a weight from its neighbours.
+    const bool down = layers.size() > DOWN;
+    const int64_t c0 = p[0].size(0), c1 = p[3].size(0), c2 = p[6].size(0), cx = x.size(1);
+    const auto is = [&](int k, at::IntArrayRef sizes) { return p[k].sizes() == sizes; };
+    TORCH_CHECK(is(0, {c0, cx, 1, 1}) && is(3, {c1, c0, 3, 3}) && is(6, {c2, c1, 1, 1}) &&
+                    (down ? is(9, {c2, cx, 1, 1}) : c2 == cx && stride == 1),
+                "bottleneck: the weights' shapes do not match x and one another");
     py::gil_scoped_release unlocked;
     auto skip = [&](int k) {
       return p[k].defined() ? c10::optional<Tensor>(p[k]) : c10::nullopt;

@@ -40,6 +40,8 @@ def _plain_conv(conv, kernel, stride, dtypes, device):
             and conv.padding == (kernel // 2, kernel // 2) and conv.dilation == (1, 1)
             and conv.groups == 1 and conv.bias is None and conv.padding_mode == "zeros"
             and type(weight) in PLAIN and weight.dtype in dtypes and weight.device == device
+            # (A weight may have been replaced without the layer's attributes.)
+            and weight.shape == (conv.out_channels, conv.in_channels, kernel, kernel)
             and not _observed(conv))
 
 

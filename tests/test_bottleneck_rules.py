@@ -1,0 +1,25 @@
+"""Which layers a residual block hands to its native node, as far as that is decided
+by the layers alone."""
+import torch
+import torch.nn as nn
+
+from horovod_b200.ops import bottleneck
+
+CPU = torch.device("cpu")
+
+
+def _plain_conv(weight=None, cin=64, cout=32, kernel=1):
+    conv = nn.Conv2d(cin, cout, kernel, padding=kernel // 2, bias=False)
+    if weight is not None:
+        conv.weight = nn.Parameter(torch.randn(weight))
+    return bottleneck._plain_conv(conv, kernel, 1, (torch.float32,), CPU)
+
+
+def test_weights_that_do_not_fit_their_layer():
+    """Replaced without the layer's attributes: PyTorch's convolution says what is wrong."""
+    assert _plain_conv() and _plain_conv((32, 64, 1, 1)) and _plain_conv(kernel=3)
+    assert not _plain_conv((32, 48, 1, 1))       # fewer inputs
+    assert not _plain_conv((24, 64, 1, 1))       # fewer outputs
+    assert not _plain_conv((32, 64, 3, 3))       # another size
+    assert not _plain_conv((32, 64, 1, 1), kernel=3)
+    assert not _plain_conv((32, 64, 1))          # not even four dimensions

@@ -617,3 +617,27 @@ def test_block_whose_saved_tensors_come_back_off_a_boundary():
                   lambda t: t.float() if t.dtype == torch.bfloat16 else t):
         with pytest.raises(RuntimeError, match="saved"):
             run(spoil)
+
+
+@pytest.mark.parametrize("name,shape", [
+    ("conv1", (64, 128, 1, 1)), ("conv2", (64, 32, 3, 3)), ("conv2", (64, 64, 1, 1)),
+    ("conv3", (256, 32, 1, 1)), ("downsample", (256, 128, 1, 1))])
+def test_block_with_a_weight_of_another_shape(name, shape):
+    """One that was replaced without the layer's attributes raises, as in the layers."""
+    from horovod_b200.ops.bottleneck import fused_bottleneck, fused_bottleneck_available
+    block = _block(256, 64, 2, True)
+    g = torch.Generator(device=_dev()).manual_seed(32)
+    x = _act(g, 2, 256, 8, 8, torch.bfloat16)
+    with torch.autocast("cuda", dtype=torch.bfloat16):
+        layers = fused_bottleneck_available(block, x)
+        assert layers is not None
+        conv = block.downsample[0] if name == "downsample" else getattr(block, name)
+        conv.weight = nn.Parameter(torch.randn(shape, device=_dev()))
+        assert fused_bottleneck_available(block, x) is None
+        with pytest.raises(RuntimeError, match="shapes do not match"):
+            fused_bottleneck(x, layers)
+        with pytest.raises(RuntimeError):
+            block(x)
+    with pytest.raises(RuntimeError, match="16-byte"):
+        flat = torch.empty(x.numel() + 1, device=_dev(), dtype=x.dtype)
+        fused_bottleneck(torch.as_strided(flat, x.shape, x.stride(), 1), layers)
