@@ -502,8 +502,10 @@ class Bottleneck : public torch::autograd::Function<Bottleneck> {
     };
     // The batch norms of the end of the block and of its skip connection have dy in
     // common. Their convolutions' gradients come from the kernel that forms theirs
-    // (OwnTail) or from what is formed here.
-    const bool tails = OwnTail(out[2], w[2], 1) && (!down || OwnTail(out[DOWN], w[DOWN], stride));
+    // (OwnTail) or from what is formed here. The kernel stores no gradient of the skip
+    // connection: where x itself is that, another kernel (`fused`) has to add it.
+    const bool tails = OwnTail(out[2], w[2], 1) &&
+                       (down ? OwnTail(out[DOWN], w[DOWN], stride) : fused || !want_x);
     Sums sums2, sums3;
     if (down || tails) sums2 = Sums(x, Channels(out[2]));
     if (down) sums3 = Sums(x, Channels(out[2]));

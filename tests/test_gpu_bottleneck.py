@@ -641,3 +641,45 @@ def test_block_with_a_weight_of_another_shape(name, shape):
     with pytest.raises(RuntimeError, match="16-byte"):
         flat = torch.empty(x.numel() + 1, device=_dev(), dtype=x.dtype)
         fused_bottleneck(torch.as_strided(flat, x.shape, x.stride(), 1), layers)
+
+
+def _block_of(widths):
+    """A block without a convolution in its skip connection whose convolutions have
+    widths of their own, as after the pruning of channels."""
+    block = _block(widths[0], 64, 1, False)
+    convs, norms = ("conv1", "conv2", "conv3"), ("bn1", "bn2", "bn3")
+    from horovod_b200.ops.batch_norm import BatchNormAct2d
+    for i, (conv, norm) in enumerate(zip(convs, norms)):
+        kernel = 3 if i == 1 else 1
+        setattr(block, conv, nn.Conv2d(widths[i], widths[i + 1], kernel, padding=kernel // 2,
+                                       bias=False))
+        setattr(block, norm, BatchNormAct2d(widths[i + 1], relu=True))
+    return block.to(_dev()).to(memory_format=CL)
+
+
+@pytest.mark.parametrize("widths", [
+    (256, 32, 64, 256),   # the end of the block is this library's, its first convolution is not
+    (128, 32, 64, 128), (128, 64, 64, 128),
+    (256, 64, 32, 256),   # the other way round
+    (256, 32, 32, 256), (512, 128, 64, 512)])
+@pytest.mark.parametrize("want_x", [True, False])
+def test_block_with_widths_of_its_own(widths, want_x, monkeypatch):
+    block = _block_of(widths)
+    g = torch.Generator(device=_dev()).manual_seed(26)
+    x = _act(g, 4, widths[0], 12, 10, torch.bfloat16).relu_()
+    dy = _act(g, 4, widths[0], 12, 10, torch.bfloat16)
+    assert _available(block, x)
+
+    def step(block):
+        xx = x.detach().clone(memory_format=CL).requires_grad_(want_x)
+        with torch.autocast("cuda", dtype=torch.bfloat16):
+            y = block(xx)
+        y.backward(dy)
+        return [y.detach()] + ([xx.grad] if want_x else []) + [p.grad for p in block.parameters()]
+
+    fused = step(copy.deepcopy(block))
+    monkeypatch.setenv("HOROVOD_B200_FUSED_BLOCK", "0")
+    layers = step(copy.deepcopy(block))
+    for a, b in zip(fused, layers):
+        # the two round the same values in the same places but for a few
+        assert _rel(a, b) <= 4e-2
