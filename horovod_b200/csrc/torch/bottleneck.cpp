@@ -328,14 +328,29 @@ Tensor ConvInputGradient(const Tensor& dy, const Tensor& w, const Tensor& add, c
   return dx;
 }
 
-// The block by PyTorch's operations, for gradients of its gradients.
+// A weight with the value that a forward worked on, for gradients of gradients: the
+// leaf may have changed since, and its gradients are those of the cast.
+class AsOfForward : public torch::autograd::Function<AsOfForward> {
+ public:
+  static Variable forward(AutogradContext* ctx, const Variable& leaf, const Variable& value) {
+    ctx->saved_data["type"] = static_cast<int64_t>(leaf.scalar_type());
+    return value.clone();
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    if (!grads[0].defined()) return {Tensor(), Tensor()};
+    const auto type = static_cast<at::ScalarType>(ctx->saved_data["type"].toInt());
+    return {grads[0].to(type), Tensor()};
+  }
+};
+
+// The block by PyTorch's operations, for gradients of its gradients. w: in the type of x.
 Tensor Composition(const Tensor& x, const std::array<Tensor, LAYERS>& w,
                    const std::array<Tensor, LAYERS>& g, const std::array<Tensor, LAYERS>& b,
                    const std::vector<double>& eps, int64_t stride) {
   auto layer = [&](int i, const Tensor& in, int64_t s) {
     const int64_t pad = w[i].size(2) / 2;
-    const Tensor out = at::convolution(in, w[i].to(in.scalar_type()), {}, {s, s}, {pad, pad},
-                                       {1, 1}, false, {0, 0}, 1);
+    const Tensor out =
+        at::convolution(in, w[i], {}, {s, s}, {pad, pad}, {1, 1}, false, {0, 0}, 1);
     return at::batch_norm(out, g[i], b[i], {}, {}, true, 0.0, eps[i], true);
   };
   const Tensor a1 = at::relu(layer(0, x, 1)), a2 = at::relu(layer(1, a1, stride));
@@ -428,8 +443,8 @@ class Bottleneck : public torch::autograd::Function<Bottleneck> {
     for (const Norm& norm : block.norms) eps.push_back(norm.eps);
     ctx->saved_data["eps"] = eps;
     ctx->saved_data["stride"] = block.stride;
-    // For gradients of gradients only; a backward of the usual kind works on the
-    // casts, and the weights may have changed since.
+    // For the edges of gradients of gradients. Every backward works on the casts: the
+    // weights may have changed since.
     ctx->saved_data["weights"] =
         std::vector<Tensor>(weights.begin(), weights.begin() + (down ? LAYERS : DOWN));
     return y;
@@ -465,8 +480,10 @@ class Bottleneck : public torch::autograd::Function<Bottleneck> {
       add(0, x);
       for (int i = 0; i < LAYERS; ++i)
         add(1 + 3 * i, weights[i]), add(2 + 3 * i, gammas[i]), add(3 + 3 * i, betas[i]);
+      std::array<Tensor, LAYERS> then;
+      for (int i = 0; i < layers; ++i) then[i] = AsOfForward::apply(weights[i], w[i].detach());
       const Tensor y =
-          Composition(x, weights, gammas, betas, ctx->saved_data["eps"].toDoubleVector(), stride);
+          Composition(x, then, gammas, betas, ctx->saved_data["eps"].toDoubleVector(), stride);
       const variable_list g = torch::autograd::grad({y}, inputs, {grads[0]}, true, true, true);
       for (size_t i = 0; i < to.size(); ++i) result[to[i]] = g[i];
       return result;

@@ -683,3 +683,51 @@ def test_block_with_widths_of_its_own(widths, want_x, monkeypatch):
     for a, b in zip(fused, layers):
         # the two round the same values in the same places but for a few
         assert _rel(a, b) <= 4e-2
+
+
+def _composed(block, x):
+    """The block by PyTorch's operations under bf16 autocast."""
+    import torch.nn.functional as F
+
+    def layer(conv, norm, x):
+        out = F.conv2d(x, conv.weight.to(x.dtype), None, conv.stride, conv.padding)
+        return F.batch_norm(out, None, None, norm.weight, norm.bias, True, 0.0, norm.eps)
+
+    out = F.relu(layer(block.conv2, block.bn2, F.relu(layer(block.conv1, block.bn1, x))))
+    skip = layer(*block.downsample, x) if block.downsample is not None else x
+    return F.relu(layer(block.conv3, block.bn3, out) + skip)
+
+
+@pytest.mark.parametrize("inplanes,planes,stride,down", [(256, 64, 1, False), (64, 64, 1, True),
+                                                         (256, 128, 2, True)])
+def test_block_gradients_of_gradients(inplanes, planes, stride, down):
+    """Those of PyTorch's operations, also of weights as they were in the forward."""
+    block = _block(inplanes, planes, stride, down)
+    g = torch.Generator(device=_dev()).manual_seed(27)
+    x = _act(g, 4, inplanes, 12, 10, torch.bfloat16).relu_().requires_grad_(True)
+    dy = _act(g, 4, planes * 4, 12 // stride, 10 // stride, torch.bfloat16)
+    inputs = [x] + list(block.parameters())
+    assert _available(block, x)
+
+    def second(first):
+        return torch.autograd.grad(sum(t.float().square().sum() for t in first), inputs)
+
+    first = torch.autograd.grad(_composed(block, x), inputs, dy, create_graph=True)
+    want = [t.detach() for t in first] + list(second(first))
+    for change in (False, True):
+        with torch.autocast("cuda", dtype=torch.bfloat16):
+            y = block(x)
+        weights = [m.weight for m in block.modules() if isinstance(m, nn.Conv2d)]
+        before = [w.detach().clone() for w in weights]
+        if change:
+            with torch.no_grad():
+                for w in weights:
+                    w.mul_(-2.0)
+        first = torch.autograd.grad(y, inputs, dy, create_graph=True)
+        got = [t.detach() for t in first] + list(second(first))
+        with torch.no_grad():
+            for w, b in zip(weights, before):
+                w.copy_(b)
+        for i, (a, b) in enumerate(zip(got, want)):
+            # the same operations, whose convolutions' sums may have another order
+            assert _rel(a, b) <= 2e-2, (change, i)
