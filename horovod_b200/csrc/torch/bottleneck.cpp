@@ -361,7 +361,7 @@ Tensor Composition(const Tensor& x, const std::array<Tensor, LAYERS>& w,
 // What a backward has saved, by layer.
 struct Kept {
   Tensor x, a1, a2, signs;
-  std::array<Tensor, LAYERS> w, gammas, betas, out, saved;
+  std::array<Tensor, LAYERS> w, gammas, out, saved;
 };
 
 // Saved tensors went through the user's hooks, if there are any. Their values and
@@ -437,7 +437,7 @@ class Bottleneck : public torch::autograd::Function<Bottleneck> {
     // changed y in place, although it does not read it.
     variable_list keep = {x, y, a1, a2, signs};
     for (int i = 0; i < (down ? LAYERS : DOWN); ++i)
-      for (const Tensor& t : {w[i], gammas[i], betas[i], out[i], saved[i]}) keep.push_back(t);
+      for (const Tensor& t : {w[i], gammas[i], out[i], saved[i]}) keep.push_back(t);
     ctx->save_for_backward(keep);
     std::vector<double> eps;
     for (const Norm& norm : block.norms) eps.push_back(norm.eps);
@@ -445,8 +445,15 @@ class Bottleneck : public torch::autograd::Function<Bottleneck> {
     ctx->saved_data["stride"] = block.stride;
     // For the edges of gradients of gradients. Every backward works on the casts: the
     // weights may have changed since.
-    ctx->saved_data["weights"] =
-        std::vector<Tensor>(weights.begin(), weights.begin() + (down ? LAYERS : DOWN));
+    const int layers = down ? LAYERS : DOWN;
+    ctx->saved_data["weights"] = std::vector<Tensor>(weights.begin(), weights.begin() + layers);
+    // A gradient needs no betas, a gradient of a gradient does: changes are noticed
+    // there alone.
+    ctx->saved_data["betas"] = std::vector<Tensor>(betas.begin(), betas.begin() + layers);
+    std::vector<int64_t> versions;
+    for (int i = 0; i < layers; ++i)
+      versions.push_back(betas[i].is_inference() ? 0 : betas[i]._version());
+    ctx->saved_data["versions"] = versions;
     return y;
   }
 
@@ -455,23 +462,32 @@ class Bottleneck : public torch::autograd::Function<Bottleneck> {
     variable_list result(1 + 3 * LAYERS + 1);
     if (!grads[0].defined()) return result;
     const variable_list keep = ctx->get_saved_variables();
-    const bool down = keep.size() > 5 + 5 * DOWN;
+    const bool down = keep.size() > 5 + 4 * DOWN;
     const int layers = down ? LAYERS : DOWN;
     const int64_t stride = ctx->saved_data["stride"].toInt();
     const std::vector<Tensor> leaves = ctx->saved_data["weights"].toTensorVector();
     Kept k;
     Tensor &x = k.x, &a1 = k.a1, &a2 = k.a2, &signs = k.signs;
-    auto &w = k.w, &gammas = k.gammas, &betas = k.betas, &out = k.out, &saved = k.saved;
+    auto &w = k.w, &gammas = k.gammas, &out = k.out, &saved = k.saved;
     std::array<Tensor, LAYERS> weights;
     x = keep[0], a1 = keep[2], a2 = keep[3], signs = keep[4];
     for (int i = 0; i < layers; ++i) {
-      const size_t at = 5 + 5 * static_cast<size_t>(i);
-      w[i] = keep[at], gammas[i] = keep[at + 1], betas[i] = keep[at + 2], out[i] = keep[at + 3],
-      saved[i] = keep[at + 4], weights[i] = leaves[i];
+      const size_t at = 5 + 4 * static_cast<size_t>(i);
+      w[i] = keep[at], gammas[i] = keep[at + 1], out[i] = keep[at + 2], saved[i] = keep[at + 3];
+      weights[i] = leaves[i];
     }
     CheckKept(k, layers, grads[0], stride);
     auto wanted = [&](int input) { return ctx->needs_input_grad(input); };
     if (at::GradMode::is_enabled()) {
+      const auto kept_betas = ctx->saved_data["betas"].toTensorVector();
+      const auto versions = ctx->saved_data["versions"].toIntVector();
+      std::array<Tensor, LAYERS> betas;
+      for (int i = 0; i < layers; ++i) {
+        betas[i] = kept_betas[i];
+        TORCH_CHECK(betas[i].is_inference() || betas[i]._version() == versions[i],
+                    "one of the variables needed for gradient computation has been modified by an "
+                    "inplace operation: the bias of a block's batch norm");
+      }
       variable_list inputs;
       std::vector<size_t> to;
       auto add = [&](size_t i, const Tensor& t) {

@@ -731,3 +731,31 @@ def test_block_gradients_of_gradients(inplanes, planes, stride, down):
         for i, (a, b) in enumerate(zip(got, want)):
             # the same operations, whose convolutions' sums may have another order
             assert _rel(a, b) <= 2e-2, (change, i)
+
+
+def test_block_whose_batch_norms_change_after_the_forward():
+    """A bias is not needed for the backward, a weight is; both for a gradient's."""
+    block = _block(256, 64, 1, False)
+    g = torch.Generator(device=_dev()).manual_seed(28)
+    x = _act(g, 4, 256, 8, 8, torch.bfloat16).relu_().requires_grad_(True)
+    inputs = [x] + list(block.parameters())
+
+    def forward():
+        with torch.autocast("cuda", dtype=torch.bfloat16):
+            return block(x)
+
+    y = forward()
+    want = torch.autograd.grad(y, inputs, torch.ones_like(y))
+    y = forward()
+    with torch.no_grad():
+        block.bn2.bias.add_(0.0)
+    got = torch.autograd.grad(y, inputs, torch.ones_like(y), retain_graph=True)
+    for a, b in zip(got, want):
+        assert _rel(a, b) <= 2e-2  # sums in another order
+    with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+        torch.autograd.grad(y, inputs, torch.ones_like(y), create_graph=True)
+    y = forward()
+    with torch.no_grad():
+        block.bn2.weight.add_(0.0)
+    with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+        torch.autograd.grad(y, inputs, torch.ones_like(y))
