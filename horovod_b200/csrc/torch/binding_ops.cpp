@@ -301,14 +301,17 @@ void BindModelOps(py::module_& m) {
     return std::make_tuple(g.x, OrNone(g.residual), g.weight, g.bias);
   });
   // The whole layer, differentiable: y, or None where the kernels cannot take the
-  // call (the caller then composes PyTorch's operations).
-  m.def("bn_act", [](const at::Tensor& x, const c10::optional<at::Tensor>& residual,
-                     const c10::optional<at::Tensor>& weight,
-                     const c10::optional<at::Tensor>& bias,
-                     const c10::optional<at::Tensor>& running_mean,
-                     const c10::optional<at::Tensor>& running_var, double momentum, double eps,
-                     bool relu,
-                     const c10::optional<at::Tensor>& batches) -> c10::optional<at::Tensor> {
+  // call (the caller then composes PyTorch's operations). Wrapped, so that what a
+  // saved-tensor hook raises arrives as what it is: a checkpointed region ends its second
+  // forward that way.
+  m.def("bn_act", torch::wrap_pybind_function([](
+                      const at::Tensor& x, const c10::optional<at::Tensor>& residual,
+                      const c10::optional<at::Tensor>& weight,
+                      const c10::optional<at::Tensor>& bias,
+                      const c10::optional<at::Tensor>& running_mean,
+                      const c10::optional<at::Tensor>& running_var, double momentum, double eps,
+                      bool relu,
+                      const c10::optional<at::Tensor>& batches) -> c10::optional<at::Tensor> {
     if (!x.is_cuda() || x.dim() != 4 ||
         (x.scalar_type() != at::kBFloat16 && x.scalar_type() != at::kHalf) ||
         !x.is_contiguous(at::MemoryFormat::ChannelsLast) || x.numel() == 0 ||
@@ -319,7 +322,7 @@ void BindModelOps(py::module_& m) {
       return c10::nullopt;
     return NormNode::apply(x, residual, weight, bias, running_mean, running_var, momentum, eps,
                            relu, batches);
-  });
+  }));
 
   // ---- max pooling 3x3 / stride 2 / padding 1 (channels-last, 16-bit) -------
   m.def("maxpool3s2_supported", [](int64_t channels) {

@@ -626,8 +626,12 @@ class Bottleneck : public torch::autograd::Function<Bottleneck> {
 void BindBottleneck(py::module_& m) {
   // (x, [weight, gamma, beta, running mean, running variance, count of batches or
   //  None] per layer, [(momentum, eps)] per layer, stride)
-  m.def("bottleneck", [](const Tensor& x, const std::vector<std::vector<c10::optional<Tensor>>>& layers,
-                         const std::vector<std::pair<double, double>>& rates, int64_t stride) {
+  // Wrapped, so that what a saved-tensor hook raises arrives as what it is (a
+  // checkpointed region ends its second forward that way), and so do PyTorch's errors.
+  m.def("bottleneck", torch::wrap_pybind_function([](
+                          const Tensor& x,
+                          const std::vector<std::vector<c10::optional<Tensor>>>& layers,
+                          const std::vector<std::pair<double, double>>& rates, int64_t stride) {
     TORCH_CHECK(layers.size() >= DOWN && layers.size() <= LAYERS && rates.size() == layers.size(),
                 "bottleneck: three or four layers");
     CheckActivations(x, "x");
@@ -674,7 +678,7 @@ void BindBottleneck(py::module_& m) {
     };
     return Bottleneck::apply(x, p[0], p[1], p[2], p[3], p[4], p[5], p[6], p[7], p[8], skip(9),
                              skip(10), skip(11), block);
-  });
+  }));
 }
 
 }  // namespace hvd

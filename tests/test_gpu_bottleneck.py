@@ -759,3 +759,32 @@ def test_block_whose_batch_norms_change_after_the_forward():
         block.bn2.weight.add_(0.0)
     with pytest.raises(RuntimeError, match="modified by an inplace operation"):
         torch.autograd.grad(y, inputs, torch.ones_like(y))
+
+
+@pytest.mark.parametrize("what", ["block", "norm"])
+def test_recomputed_activations(what):
+    """A checkpointed region ends its second forward with an exception out of a
+    saved-tensor hook, which has to arrive as what it is."""
+    from torch.utils.checkpoint import checkpoint
+    block = _block(256, 64, 1, False)
+    layer = block if what == "block" else block.bn3
+    g = torch.Generator(device=_dev()).manual_seed(30)
+    x = _act(g, 2, 256, 8, 8, torch.bfloat16).requires_grad_(True)
+    inputs = [x] + list(layer.parameters())
+
+    def grads(f):
+        with torch.autocast("cuda", dtype=torch.bfloat16):
+            y = f(x)
+        return torch.autograd.grad(y, inputs, torch.ones_like(y))
+
+    for a, b in zip(grads(lambda x: checkpoint(layer, x, use_reentrant=False)), grads(layer)):
+        assert _rel(a, b) <= 2e-2  # sums in another order
+
+    class Stop(Exception):
+        pass
+
+    def stop(t):
+        raise Stop()
+
+    with torch.autograd.graph.saved_tensors_hooks(stop, lambda t: t), pytest.raises(Stop):
+        grads(layer)
