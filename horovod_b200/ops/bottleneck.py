@@ -6,7 +6,8 @@ the gradient of the skip connection is added inside one.
 ``fused_bottleneck_available`` says whether a block and its input can take it. What
 it cannot represent is left to the sequence of layers: evaluation mode, other
 memory formats and types, layers of other classes, hooks on a layer, tracing,
-transforms. ``HOROVOD_B200_FUSED_BLOCK=0`` leaves every block to its layers.
+transforms, modes that watch functions. ``HOROVOD_B200_FUSED_BLOCK=0`` leaves every
+block to its layers.
 
 The reference has no counterpart (it takes convolutions and batch normalisation from
 the framework).
@@ -17,7 +18,7 @@ import torch
 import torch.nn as nn
 from torch.nn.modules.module import _has_any_global_hook
 
-from horovod_b200.ops._native import PLAIN, plain_autograd
+from horovod_b200.ops._native import PLAIN, functions_watched, plain_autograd
 from horovod_b200.ops.batch_norm import BatchNormAct2d, fused_batch_norm_available
 from horovod_b200.ops.stem_conv import tensor_core_kernels_enabled
 
@@ -84,7 +85,7 @@ def fused_bottleneck_available(block, x):
             and x.dtype in (torch.bfloat16, torch.float16)):
         return None
     if os.environ.get("HOROVOD_B200_FUSED_BLOCK", "1") != "1" or _has_any_global_hook() or \
-            not plain_autograd():
+            not plain_autograd() or functions_watched():
         return None
     if not x.is_contiguous(memory_format=torch.channels_last) or x.data_ptr() % 16 != 0:
         return None

@@ -23,3 +23,22 @@ def test_weights_that_do_not_fit_their_layer():
     assert not _plain_conv((32, 64, 3, 3))       # another size
     assert not _plain_conv((32, 64, 1, 1), kernel=3)
     assert not _plain_conv((32, 64, 1))          # not even four dimensions
+
+
+def test_modes_that_watch_functions():
+    from torch.overrides import TorchFunctionMode
+
+    from horovod_b200.ops._native import functions_watched
+
+    class Watch(TorchFunctionMode):
+        def __torch_function__(self, func, types, args=(), kwargs=None):
+            return func(*args, **(kwargs or {}))
+
+    assert not functions_watched()
+    with torch.device("cpu"):
+        assert not functions_watched()
+        with Watch():
+            assert functions_watched()
+            with torch.device("cpu"):  # the one below it still watches
+                assert functions_watched()
+    assert not functions_watched()

@@ -788,3 +788,25 @@ def test_recomputed_activations(what):
 
     with torch.autograd.graph.saved_tensors_hooks(stop, lambda t: t), pytest.raises(Stop):
         grads(layer)
+
+
+def test_block_under_function_modes():
+    """A mode that watches functions sees the layers' convolutions; a default device
+    is no such mode."""
+    from torch.overrides import TorchFunctionMode
+
+    class Watch(TorchFunctionMode):
+        seen = 0
+
+        def __torch_function__(self, func, types, args=(), kwargs=None):
+            Watch.seen += func in (torch.conv2d, nn.functional.conv2d)
+            return func(*args, **(kwargs or {}))
+
+    block = _block(256, 64, 1, False)
+    g = torch.Generator(device=_dev()).manual_seed(29)
+    x = _act(g, 2, 256, 8, 8, torch.bfloat16)
+    with torch.device("cuda"):
+        assert _available(block, x)
+        with Watch(), torch.autocast("cuda", dtype=torch.bfloat16):
+            block(x)
+    assert Watch.seen == 3
