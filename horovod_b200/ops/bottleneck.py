@@ -51,9 +51,10 @@ def _plain_norm(norm, relu, conv, device):
             and norm.track_running_stats and norm.momentum is not None and norm.affine
             and norm.num_features == conv.out_channels and not _observed(norm)):
         return False
-    weight, bias = norm._parameters["weight"], norm._parameters["bias"]
-    mean, var = norm._buffers["running_mean"], norm._buffers["running_var"]
-    batches = norm._buffers["num_batches_tracked"]
+    # (Some of them may be attributes of another kind.)
+    weight, bias = norm._parameters.get("weight"), norm._parameters.get("bias")
+    mean, var = norm._buffers.get("running_mean"), norm._buffers.get("running_var")
+    batches = norm._buffers.get("num_batches_tracked")
     for t in (weight, bias, mean, var):
         if not (type(t) in PLAIN and t.dtype == torch.float32 and t.device == device
                 and t.is_contiguous()):

@@ -42,3 +42,20 @@ def test_modes_that_watch_functions():
             with torch.device("cpu"):  # the one below it still watches
                 assert functions_watched()
     assert not functions_watched()
+
+
+def test_batch_norms_whose_tensors_are_plain_attributes():
+    """As after some functional rewrites: left to the layer, which reads attributes."""
+    from horovod_b200.ops.batch_norm import BatchNormAct2d
+
+    def plain(name=None):
+        norm, conv = BatchNormAct2d(32), nn.Conv2d(64, 32, 1, bias=False)
+        if name is not None:
+            value = getattr(norm, name).detach()
+            delattr(norm, name)
+            norm.__dict__[name] = value
+        return bottleneck._plain_norm(norm, True, conv, CPU)
+
+    assert plain()
+    for name in ("weight", "bias", "running_mean", "running_var", "num_batches_tracked"):
+        assert not plain(name)
