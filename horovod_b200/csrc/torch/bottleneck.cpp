@@ -524,6 +524,10 @@ class Bottleneck : public torch::autograd::Function<Bottleneck> {
       return g;
     };
     const bool want_x = wanted(0);
+    // Whether anything before the first (the second) ReLU wants a gradient: the input and
+    // the first layers of a network are often frozen.
+    const bool need_a1 = want_x || wanted(1) || wanted(2) || wanted(3);
+    const bool need_a2 = need_a1 || wanted(4) || wanted(5) || wanted(6);
     // The gradients of x through the first convolution and through the skip
     // connection meet in a kernel of this library where it takes the shapes.
     const bool fused = kern::Conv1x1Supported(Rows(x), Channels(out[0]), Channels(x));
@@ -573,6 +577,7 @@ class Bottleneck : public torch::autograd::Function<Bottleneck> {
     auto tail = [&](int i, const Tensor& in, int64_t s, Tensor d_out, const Sums& sums,
                     bool want_in) {
       Tensor d_in;
+      if (!want_in && !wanted(1 + 3 * i) && !wanted(2 + 3 * i) && !wanted(3 + 3 * i)) return d_in;
       if (tails) {
         const TailGradients g = TailBackward(dy, signs, out[i], in, w[i], gammas[i], saved[i],
                                              weights[i], sums, want_in);
@@ -584,12 +589,13 @@ class Bottleneck : public torch::autograd::Function<Bottleneck> {
       std::tie(d_in, dw[i]) = ConvBackward(d_out, in, w[i], s, want_in, wanted(1 + 3 * i));
       return d_in;
     };
-    da2 = tail(2, a2, 1, g2.x, sums2, true);
+    da2 = tail(2, a2, 1, g2.x, sums2, need_a2);
     g2.x.reset();
-    const Tensor d2 = norm(1, da2, {}, false).x;
+    Tensor d2, d1;
+    if (need_a2) d2 = norm(1, da2, {}, false).x;
     da2.reset();
-    std::tie(da1, dw[1]) = ConvBackward(d2, a1, w[1], stride, true, wanted(4));
-    const Tensor d1 = norm(0, da1, {}, false).x;
+    std::tie(da1, dw[1]) = ConvBackward(d2, a1, w[1], stride, need_a1, wanted(4));
+    if (need_a1) d1 = norm(0, da1, {}, false).x;
     da1.reset();
     if (down) {
       const bool scatter = stride == 2 && EveryOther(x) &&

@@ -810,3 +810,36 @@ def test_block_under_function_modes():
         with Watch(), torch.autocast("cuda", dtype=torch.bfloat16):
             block(x)
     assert Watch.seen == 3
+
+
+@pytest.mark.parametrize("down", [False, True])
+def test_block_does_not_compute_gradients_that_nobody_wants(down):
+    """With the first layers frozen and an input without a gradient, the backward ends
+    at the layers that are trained: fewer launches, the same gradients."""
+    from horovod_b200 import _C
+    block = _block(64 if down else 256, 64, 1, down)
+    g = torch.Generator(device=_dev()).manual_seed(31)
+    x = _act(g, 2, 64 if down else 256, 8, 8, torch.bfloat16)
+    dy = _act(g, 2, 256, 8, 8, torch.bfloat16)
+
+    def step():
+        with torch.autocast("cuda", dtype=torch.bfloat16):
+            y = block(x)
+        before = _C.kernel_launch_count()
+        y.backward(dy)
+        torch.cuda.synchronize()
+        grads = {n: p.grad for n, p in block.named_parameters() if p.requires_grad}
+        block.zero_grad()
+        return _C.kernel_launch_count() - before, grads
+
+    every, want = step()
+    last = every
+    for frozen in ("conv1", "bn1", "conv2", "bn2") + (("downsample",) if down else ()):
+        for p in getattr(block, frozen).parameters():
+            p.requires_grad_(False)
+        launches, got = step()
+        for n, t in got.items():
+            assert _rel(t, want[n]) <= 2e-2, n  # sums in another order
+        if not frozen.startswith("conv"):
+            assert launches < last  # the batch norm's two kernels and more
+            last = launches
