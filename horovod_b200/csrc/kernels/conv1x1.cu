@@ -492,6 +492,8 @@ cudaError_t LaunchConv1x1(const Conv1x1& c, cudaStream_t stream, uint32_t wait_n
   if ((c.strided_x && c.strided_y) || (c.signs != nullptr && (c.add == nullptr || c.strided_y)) ||
       (c.sums != nullptr && c.copies < 1) || !TmaAvailable())
     return cudaErrorInvalidValue;
+  // (The maps refuse what else is off its boundary.)
+  if (reinterpret_cast<uintptr_t>(c.signs) % 4 != 0) return cudaErrorInvalidValue;
   int device = 0;
   const cudaError_t err = cudaGetDevice(&device);
   if (err != cudaSuccess) return err;

@@ -465,6 +465,11 @@ int NormConvBackwardParts(int64_t rows) {
 cudaError_t LaunchNormConvBackward(const NormConvBackward& n, cudaStream_t stream,
                                    uint32_t wait_ns) {
   if (!NormConvBackwardSupported(n.rows, n.cout, n.cin)) return cudaErrorInvalidValue;
+  // What is copied, loaded and stored in 16 (da: 32) bytes at a time.
+  for (const void* p : {n.dy, n.x, n.a, n.w, static_cast<const void*>(n.signs),
+                        static_cast<const void*>(n.saved), static_cast<const void*>(n.partial)})
+    if (reinterpret_cast<uintptr_t>(p) % 16 != 0) return cudaErrorInvalidValue;
+  if (reinterpret_cast<uintptr_t>(n.da) % 32 != 0) return cudaErrorInvalidValue;
   int device = 0;
   cudaError_t err = cudaGetDevice(&device);
   if (err != cudaSuccess) return err;

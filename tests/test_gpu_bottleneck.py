@@ -843,3 +843,26 @@ def test_block_does_not_compute_gradients_that_nobody_wants(down):
         if not frozen.startswith("conv"):
             assert launches < last  # the batch norm's two kernels and more
             last = launches
+
+
+def test_kernels_refuse_what_starts_off_a_boundary():
+    from horovod_b200 import _C
+    g = torch.Generator(device=_dev()).manual_seed(33)
+
+    def off(t):
+        flat = torch.empty(t.numel() + 1, device=t.device, dtype=t.dtype)
+        return torch.as_strided(flat, t.shape, t.stride(), 1).copy_(t)
+
+    args = _tail(g, 3, 256, 9, 11, torch.bfloat16)
+    for i in (0, 1, 2, 3, 4, 6):  # gamma is read value by value
+        with pytest.raises(RuntimeError, match="invalid argument"):
+            _C.norm_conv_backward(*[off(t) if i == k else t for k, t in enumerate(args)])
+    da, dw, _, _ = _C.norm_conv_backward(*args)
+    args = tuple(off(t) if k == 5 else t for k, t in enumerate(args))
+    assert torch.equal(_C.norm_conv_backward(*args)[0], da)
+    x, add = _act(g, 2, 64, 9, 9, torch.bfloat16), _act(g, 2, 64, 9, 9, torch.bfloat16)
+    weight = torch.randn(64, 64, device=_dev(), generator=g).bfloat16()
+    signs = _signs(add > 0)
+    for kw in (dict(x=off(x)), dict(w=off(weight)), dict(add=off(add)), dict(signs=off(signs))):
+        with pytest.raises(RuntimeError, match="invalid argument"):
+            _C.conv1x1(**{**dict(x=x, w=weight, w_transposed=True, add=add, signs=signs), **kw})
