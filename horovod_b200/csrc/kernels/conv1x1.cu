@@ -49,7 +49,7 @@ constexpr int EPILOGUE_WARP = 4, EPILOGUE_THREADS = 256;
 constexpr int SLICE_K = 64;
 constexpr uint16_t NAN16 = 0x7fff;  // a NaN of either 16-bit type
 
-enum Epilogue : int { STORE = 0, STORE_SUMS = 1, ADD = 2, ADD_MASKED = 3 };
+enum Epilogue : int { STORE_SUMS = 0, ADD = 1, ADD_MASKED = 2 };
 
 // Shared memory: output tiles, w where it stays, and a ring of slices of the
 // operands.
@@ -460,18 +460,12 @@ cudaError_t LaunchTyped(const Conv1x1& c, Shape s, cudaStream_t stream, int* sta
 template <typename T, int BN>
 cudaError_t LaunchWidth(const Conv1x1& c, const Shape& s, cudaStream_t stream, int* status,
                         uint32_t wait_ns) {
-  if (c.w_transposed) {
-    if (c.sums != nullptr) return cudaErrorInvalidValue;
-    if (c.add == nullptr) return LaunchTyped<T, BN, true, STORE>(c, s, stream, status, wait_ns);
-    if constexpr (BN <= 128) {
-      if (c.signs == nullptr) return LaunchTyped<T, BN, true, ADD>(c, s, stream, status, wait_ns);
-      return LaunchTyped<T, BN, true, ADD_MASKED>(c, s, stream, status, wait_ns);
-    }
-    return cudaErrorInvalidValue;
+  if (!c.w_transposed) return LaunchTyped<T, BN, false, STORE_SUMS>(c, s, stream, status, wait_ns);
+  if constexpr (BN <= 128) {
+    if (c.signs == nullptr) return LaunchTyped<T, BN, true, ADD>(c, s, stream, status, wait_ns);
+    return LaunchTyped<T, BN, true, ADD_MASKED>(c, s, stream, status, wait_ns);
   }
-  if (c.add != nullptr) return cudaErrorInvalidValue;
-  if (c.sums == nullptr) return LaunchTyped<T, BN, false, STORE>(c, s, stream, status, wait_ns);
-  return LaunchTyped<T, BN, false, STORE_SUMS>(c, s, stream, status, wait_ns);
+  return cudaErrorInvalidValue;
 }
 
 }  // namespace
@@ -489,8 +483,12 @@ cudaError_t LaunchConv1x1(const Conv1x1& c, cudaStream_t stream, uint32_t wait_n
   if (!Conv1x1Supported(c.rows, c.k, c.n)) return cudaErrorInvalidValue;
   if ((c.strided_x || c.strided_y) && !Conv1x1StrideSupported(c.rows, c.width))
     return cudaErrorInvalidValue;
-  if ((c.strided_x && c.strided_y) || (c.signs != nullptr && (c.add == nullptr || c.strided_y)) ||
-      (c.sums != nullptr && c.copies < 1) || !TmaAvailable())
+  // The forward has a batch norm behind it, the gradient something to add: PyTorch's
+  // kernels cost less where they do not.
+  if (c.w_transposed ? c.add == nullptr || c.sums != nullptr
+                     : c.add != nullptr || c.signs != nullptr || c.sums == nullptr || c.copies < 1)
+    return cudaErrorInvalidValue;
+  if ((c.strided_x && c.strided_y) || (c.signs != nullptr && c.strided_y) || !TmaAvailable())
     return cudaErrorInvalidValue;
   // (The maps refuse what else is off its boundary.)
   if (reinterpret_cast<uintptr_t>(c.signs) % 4 != 0) return cudaErrorInvalidValue;

@@ -455,10 +455,11 @@ cudaError_t LaunchStemConvWgrad(const void* x, const void* dy, float* partial, v
 // 1x1 convolution of channels-last 16-bit activations, as the product
 //   y[rows, n] = x[rows, k] * w (+ add, where signs say so)
 // with w [n, k] (forward) or [k, n] (w_transposed: gradient of the input).
-// sums: also adds up sum(y) and sum(y * y) per channel, as LaunchBatchNormForward
-// does for itself, in `copies` copies of [2][n].
-// add: [rows, n], added in fp32 before y is rounded (y may be the same memory);
-// signs: a byte per 8 channels of it in bn_forward's order, which values count.
+// sums (forward): sum(y) and sum(y * y) per channel are added to them, as
+// LaunchBatchNormForward does for itself, in `copies` copies of [2][n].
+// add (gradient): [rows, n], added in fp32 before y is rounded (y may be the same
+// memory); signs (optional): a byte per 8 channels of it in bn_forward's order, which
+// values count.
 // With a stride of 2, the rows are output pixels [images * height][width], and
 // x (strided_x) or y and add (strided_y) are the pixels of twice the height and
 // width, of which every other one in each direction takes part.

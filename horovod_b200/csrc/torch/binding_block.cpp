@@ -15,8 +15,9 @@ namespace hvd {
 void BindBlockOps(py::module_& m) {
   m.def("conv1x1_supported", &kern::Conv1x1Supported);  // (rows, k, n)
   // The kernel alone. x: channels-last activations; w: [n, k], or [k, n] with
-  // w_transposed; add, signs: see kernels.h. With scatter, y is written to (and add
-  // read from) every other pixel of `y`; with gather, x is read that way.
+  // w_transposed; add (zeros where there is none), signs: see kernels.h. With scatter, y
+  // is written to (and add read from) every other pixel of `y`; with gather, x is read
+  // that way.
   //   -> (y, sums of [2, n] in fp64 or None)
   m.def("conv1x1", [](const at::Tensor& x, const at::Tensor& w, bool w_transposed,
                       const c10::optional<at::Tensor>& add,
@@ -53,6 +54,11 @@ void BindBlockOps(py::module_& m) {
                   "conv1x1: add does not match");
       c.add = scatter ? y.data_ptr() : add->data_ptr();
     }
+    at::Tensor zeros;
+    if (w_transposed && !add.has_value()) {
+      zeros = at::zeros_like(y);
+      c.add = zeros.data_ptr();
+    }
     if (signs.has_value()) {
       TORCH_CHECK(signs->is_cuda() && signs->scalar_type() == at::kByte &&
                       signs->is_contiguous() && signs->numel() * 8 == y.numel(),
@@ -60,7 +66,7 @@ void BindBlockOps(py::module_& m) {
       c.signs = signs->data_ptr<uint8_t>();
     }
     at::Tensor sums;
-    if (want_sums) {
+    if (!w_transposed || want_sums) {
       c.copies = kern::BatchNormCopies(c.n);
       sums = at::zeros({c.copies, 2, n}, x.options().dtype(at::kDouble));
       c.sums = sums.data_ptr<double>();
