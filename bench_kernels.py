@@ -24,6 +24,21 @@ Cases
   stem_conv     7x7 / stride 2 / padding 3 convolution of 256 images of 224 x 224
                 x 3 to 64 channels in bf16: forward reads x and writes y (488 MB),
                 the weights' gradient reads x and dy. Next to PyTorch's.
+  conv1x1       1x1 convolutions of ResNet-50's first and third stage (256 images of
+                56 x 56 and 14 x 14) in bf16: forward, which reads x and writes y
+                and the sums of a batch norm (the call clears them too), and the
+                gradient of the input, which reads dy, the skip connection's
+                gradient and a bit per element of it and writes dx.
+  norm_conv     backward of a batch norm over 256 channels and of the 1x1
+                convolution from 64 before it, 256 images of 56 x 56: the sums
+                read dy, x and a bit per element; the fused kernel reads them
+                again, and a, and writes da. Next to the same as kernels of
+                their own (bn_backward, then PyTorch's convolution_backward).
+  residual_block
+                forward and backward of the first block of ResNet-50's first two
+                stages, 256 images of 56 x 56 in bf16, as one node and (which moves
+                other bytes) layer by layer. No bytes are given: PyTorch's 3x3
+                convolutions and weight gradients are among it.
   max_pool      3x3 / stride 2 / padding 1 max pooling on the ResNet stem
                 activation 256 x 64 x 112 x 112 bf16 (411 MB): forward reads x,
                 writes y (1/4 of x) and half an index byte per output element
@@ -114,7 +129,8 @@ def main():
                           "clocks": clock_log.window(t_begin, t_end)}), flush=True)
 
     cases = ["fused_local", "fused_fp16", "reducescatter", "exchange", "batch_norm", "stem_conv",
-             "max_pool", "fused_sgd"] if args.case == "all" else [args.case]
+             "conv1x1", "norm_conv", "residual_block", "max_pool",
+             "fused_sgd"] if args.case == "all" else [args.case]
 
     def timed_events(fn, reps):
         for _ in range(args.warmup):
@@ -212,6 +228,81 @@ def main():
                 us = timed_events(fn, args.iters)
                 report_line(name + which, us, moved if name == "stem_conv_fused" else None,
                             {"shape": list(x.shape)})
+
+    def activations(n, channels, size):
+        return torch.randn(n, size, size, channels, device=dev).bfloat16().permute(0, 3, 1, 2)
+
+    if "conv1x1" in cases:
+        n = 256 if args.mb >= 512 else 64
+
+        def forward(size, k, co):
+            x = activations(n, k, size)
+            w = torch.randn(co, k, device=dev).bfloat16()
+            rows = n * size * size
+            us = timed_events(lambda: _C.conv1x1(x, w), args.iters)
+            report_line("conv1x1_forward", us, 2 * rows * (k + co), {"rows": rows, "k": k, "n": co})
+
+        def gradient(size, k, co, masked):
+            dy, add = activations(n, k, size), activations(n, co, size)
+            w = torch.randn(k, co, device=dev).bfloat16()
+            rows = n * size * size
+            signs = torch.randint(0, 256, (rows, co // 8), device=dev, dtype=torch.uint8) \
+                if masked else None
+            us = timed_events(lambda: _C.conv1x1(dy, w, w_transposed=True, add=add, signs=signs),
+                              args.iters)
+            report_line("conv1x1_gradient" + ("_masked_sum" if masked else "_sum"), us,
+                        2 * rows * (k + 2 * co) + (rows * co // 8 if masked else 0),
+                        {"rows": rows, "k": k, "n": co})
+        forward(56, 64, 256)
+        gradient(56, 64, 256, True)
+        gradient(14, 256, 1024, True)
+        gradient(14, 256, 1024, False)
+        forward(14, 256, 1024)
+        forward(56, 256, 64)
+    if "norm_conv" in cases:
+        n = 256 if args.mb >= 512 else 64
+        x, res, dy, a = (activations(n, c, 56) for c in (256, 256, 256, 64))
+        w = torch.randn(256, 64, device=dev).bfloat16() / 8
+        gamma = torch.ones(256, device=dev)
+        _, saved, signs = _C.bn_forward(x, res, gamma, gamma, None, None, 0.1, 1e-5, True, None)
+        del res
+        rows = n * 56 * 56
+
+        def apart():
+            dx = _C.bn_backward(dy, x, gamma, saved, signs, True, False)[0]
+            torch.ops.aten.convolution_backward(dx, a, w[:, :, None, None], None, [1, 1], [0, 0],
+                                                [1, 1], False, [0, 0], 1, [True, True, False])
+        moved = rows * (2 * (2 * 512 + 32) + 2 * 128)
+        us = timed_events(lambda: _C.norm_conv_backward(dy, signs, x, a, w, gamma, saved),
+                          args.iters)
+        report_line("norm_conv_backward_fused", us, moved, {"rows": rows})
+        report_line("norm_conv_backward_apart", timed_events(apart, args.iters), None,
+                    {"rows": rows})
+        del x, dy, a, saved, signs
+    if "residual_block" in cases:
+        from horovod_b200.models.resnet import ResNet
+        n = 256 if args.mb >= 512 else 64
+        model = ResNet().to(dev).to(memory_format=torch.channels_last)
+        for which, block, channels in (("stage1", model.layer1[0], 64),
+                                       ("stage2", model.layer2[0], 256)):
+            x = activations(n, channels, 56).requires_grad_(True)
+            wanted = [x] + list(block.parameters())
+
+            def fwd():
+                with torch.autocast("cuda", dtype=torch.bfloat16):
+                    return block(x)
+            dy = torch.randn_like(fwd())
+            for kind, switch in (("node", "1"), ("layers", "0")):
+                os.environ["HOROVOD_B200_FUSED_BLOCK"] = switch
+                t_f = timed_events(fwd, args.iters)
+                y = fwd()
+                t_b = timed_events(lambda: torch.autograd.grad(y, wanted, dy, retain_graph=True),
+                                   args.iters)
+                for name, us in (("forward", t_f), ("backward", t_b)):
+                    report_line("residual_block_%s_%s_%s" % (which, kind, name), us, None,
+                                {"shape": list(x.shape)})
+                del y
+            os.environ.pop("HOROVOD_B200_FUSED_BLOCK")
     if "max_pool" in cases:
         import torch.nn.functional as F
         from horovod_b200.ops.pooling import max_pool_3x3_s2
