@@ -40,6 +40,11 @@ constexpr auto CL = at::MemoryFormat::ChannelsLast;
 // skip connection (its weights are undefined tensors where there is none).
 constexpr int LAYERS = 4, DOWN = 3;
 
+// Names of what a node keeps beside its saved tensors. (Compiled autograd finds tensors
+// there, but not lists of them.)
+constexpr const char* WEIGHT[LAYERS] = {"w0", "w1", "w2", "w3"};
+constexpr const char* BETA[LAYERS] = {"b0", "b1", "b2", "b3"};
+
 struct Norm {
   Tensor mean, var, batches;
   double momentum = 0.0, eps = 0.0;
@@ -446,13 +451,14 @@ class Bottleneck : public torch::autograd::Function<Bottleneck> {
     // For the edges of gradients of gradients. Every backward works on the casts: the
     // weights may have changed since.
     const int layers = down ? LAYERS : DOWN;
-    ctx->saved_data["weights"] = std::vector<Tensor>(weights.begin(), weights.begin() + layers);
+    for (int i = 0; i < layers; ++i) ctx->saved_data[WEIGHT[i]] = weights[i];
     // A gradient needs no betas, a gradient of a gradient does: changes are noticed
     // there alone.
-    ctx->saved_data["betas"] = std::vector<Tensor>(betas.begin(), betas.begin() + layers);
     std::vector<int64_t> versions;
-    for (int i = 0; i < layers; ++i)
+    for (int i = 0; i < layers; ++i) {
+      ctx->saved_data[BETA[i]] = betas[i];
       versions.push_back(betas[i].is_inference() ? 0 : betas[i]._version());
+    }
     ctx->saved_data["versions"] = versions;
     return y;
   }
@@ -465,7 +471,6 @@ class Bottleneck : public torch::autograd::Function<Bottleneck> {
     const bool down = keep.size() > 5 + 4 * DOWN;
     const int layers = down ? LAYERS : DOWN;
     const int64_t stride = ctx->saved_data["stride"].toInt();
-    const std::vector<Tensor> leaves = ctx->saved_data["weights"].toTensorVector();
     Kept k;
     Tensor &x = k.x, &a1 = k.a1, &a2 = k.a2, &signs = k.signs;
     auto &w = k.w, &gammas = k.gammas, &out = k.out, &saved = k.saved;
@@ -474,16 +479,15 @@ class Bottleneck : public torch::autograd::Function<Bottleneck> {
     for (int i = 0; i < layers; ++i) {
       const size_t at = 5 + 4 * static_cast<size_t>(i);
       w[i] = keep[at], gammas[i] = keep[at + 1], out[i] = keep[at + 2], saved[i] = keep[at + 3];
-      weights[i] = leaves[i];
+      weights[i] = ctx->saved_data[WEIGHT[i]].toTensor();
     }
     CheckKept(k, layers, grads[0], stride);
     auto wanted = [&](int input) { return ctx->needs_input_grad(input); };
     if (at::GradMode::is_enabled()) {
-      const auto kept_betas = ctx->saved_data["betas"].toTensorVector();
       const auto versions = ctx->saved_data["versions"].toIntVector();
       std::array<Tensor, LAYERS> betas;
       for (int i = 0; i < layers; ++i) {
-        betas[i] = kept_betas[i];
+        betas[i] = ctx->saved_data[BETA[i]].toTensor();
         TORCH_CHECK(betas[i].is_inference() || betas[i]._version() == versions[i],
                     "one of the variables needed for gradient computation has been modified by an "
                     "inplace operation: the bias of a block's batch norm");

@@ -866,3 +866,20 @@ def test_kernels_refuse_what_starts_off_a_boundary():
     for kw in (dict(x=off(x)), dict(w=off(weight)), dict(add=off(add)), dict(signs=off(signs))):
         with pytest.raises(RuntimeError, match="invalid argument"):
             _C.conv1x1(**{**dict(x=x, w=weight, w_transposed=True, add=add, signs=signs), **kw})
+
+
+@pytest.mark.parametrize("down", [False, True])
+def test_block_under_compiled_autograd(down):
+    """A backward that is traced runs the node as it is."""
+    from torch._dynamo import compiled_autograd
+    block = _block(64 if down else 256, 64, 1, down)
+    g = torch.Generator(device=_dev()).manual_seed(34)
+    x = _act(g, 2, 64 if down else 256, 8, 8, torch.bfloat16).requires_grad_(True)
+    inputs = [x] + list(block.parameters())
+    with torch.autocast("cuda", dtype=torch.bfloat16):
+        y = block(x)
+    want = torch.autograd.grad(y, inputs, torch.ones_like(y), retain_graph=True)
+    with compiled_autograd._enable(lambda graph: graph):
+        y.backward(torch.ones_like(y))
+    for t, b in zip(inputs, want):
+        assert _rel(t.grad, b) <= 2e-2  # sums in another order
