@@ -10,21 +10,24 @@
 //
 // A persistent CTA computes tiles of 128 rows x BN channels of one column of
 // tiles: a thread's sums then belong to the same channels in every tile and stay
-// in registers. Warp 0 brings 64-deep slices of both operands into shared memory
-// by TMA, one thread of warp 1 issues the products into one of two accumulators
-// in tensor memory, warp 2 brings the tile that is added, and eight warps take
-// the other accumulator to registers, round it, store it to shared memory and
-// from there by TMA. The kernels are bound by the bytes of x, y and add where k or n
-// is small (the first two stages of a ResNet), else by what the SMs read of the
-// operands from L2 (9 to 11 TB/s).
+// in registers. Warp 0 brings 64-deep slices of x into shared memory by TMA, and those
+// of w (once for all tiles where they fit, else with every tile), one thread of
+// warp 1 issues the products into one of two accumulators in tensor memory, warp 2
+// brings the tile that is added, and eight warps take the other accumulator to
+// registers, round it, store it to shared memory and from there by TMA. Where k and n
+// are small (the first stages of a ResNet) the bytes of x, y and add are the bound, else
+// what the SMs move between L2 and shared memory: 308 MB at 8.0 TB/s in the forward of
+// 50176 rows from 256 to 1024 channels, whose w is read with every tile.
 //
-// On a B200, bf16, k to n channels, in us (launch of 5 us included):
-//   802816 rows, 64 to 256: forward with sums 91 (the convolution 83 and the
-//     statistics 70 before); 256 to 64, 91 (87 and 17)
-//   802816 rows, gradient of 256 channels from 64 and the masked sum: 150 (87, a sum
-//     of 191 and 64 for storing the masked gradient before)
-//   50176 rows, 256 to 1024: 42 (40 and 18); gradient of 1024 from 256, with the sum, 66
-//     (40, 42 and 16)
+// The kernel alone on a B200, bf16, in us (in brackets: PyTorch's kernel for the product,
+// then the pass or passes that are gone; floor: the bytes at a copy's rate):
+//   802816 rows, 64 to 256 channels, forward with sums      88 (78, 69)    floor 78
+//   802816 rows, 256 to 64                                  79 (77, 22)          78
+//   50176 rows, 256 to 1024                                 39 (35, 22)          20
+//   802816 rows, gradient of 256 from 64 and the masked sum 147 (79, 140 and 64)  145
+//   50176 rows, gradient of 1024 from 256, masked sum       53 (35, 37 and 16)   36
+//     with a sum that is not masked                         51 (35, 37)          36
+// bench_kernels.py --case conv1x1 measures the calls.
 //
 // Waits are bounded. When one runs out, what the CTA had not finished becomes
 // NaN, its sums too, and TensorCoreStatusWord() of the device is set.
@@ -436,8 +439,8 @@ cudaError_t LaunchTyped(const Conv1x1& c, Shape s, cudaStream_t stream, int* sta
   if (!ok) return cudaErrorInvalidValue;
   auto kernel = conv1x1_kernel<T, BN, W_MN, EPI>;
   // w stays in shared memory for all tiles of a CTA where three slices of x still fit
-  // beside it: gradient of 1024 channels from 256 with the masked sum, 50176 rows, 62 to 53
-  // us; of 256 from 64, 802816 rows, 174 to 152.
+  // beside it: gradient of 1024 channels from 256 with the masked sum, 50176 rows, 53 us,
+  // 62 with w read for every tile; of 256 from 64, 802816 rows, 147 to 152, 174 without.
   const int fixed = 1024 + L::BUFFERS * L::BUFFER, all_of_w = s.slices_k * L::W_SLICE;
   s.w_stays = fixed + all_of_w + 3 * BOX_BYTES <= MOST_BYTES;
   const int slice = BOX_BYTES + (s.w_stays ? 0 : L::W_SLICE);

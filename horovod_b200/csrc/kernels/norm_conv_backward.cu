@@ -17,7 +17,8 @@
 // limits the kernel to 256 wide and 64 narrow channels.
 //
 // Bound by the bytes of dy, x, a and da. 802816 rows, 256 and 64 channels, bf16, with
-// the batch norm's sums: 361 us (287 for the bytes); the kernels apart 345 and 180. 2304
+// the batch norm's sums: 359 to 361 us (290 for the bytes), of which this kernel takes 215;
+// the kernels apart 345 and 167 to 180 (bench_kernels.py --case norm_conv). 2304
 // rows: 24 us, apart 28. The copies alone take 320 us, with the forming of dx, but no
 // products, 333. A tile of dx of its own for the products to work on while the
 // next is formed leaves no room for the ring: with loads into registers instead, which

@@ -1,4 +1,4 @@
-// Python entry points of the model-side kernels (fused batch normalisation).
+// Python entry points of the model-side kernels but those of the residual block.
 // They run on the caller's current CUDA stream like any torch op.
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAGraphsC10Utils.h>
