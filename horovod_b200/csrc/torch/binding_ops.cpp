@@ -71,29 +71,39 @@ double* ZeroedDoubles(int64_t count, const at::Tensor& like, cudaStream_t stream
   static std::mutex mu;
   static std::map<std::pair<int, cudaStream_t>, Pool> pools;
   TORCH_CHECK(count <= POOL_DOUBLES, "batch norm scratch request too large");
-  std::lock_guard<std::mutex> lock(mu);
-  Pool& p = pools[{like.get_device(), stream}];
   const int64_t need = (count + 31) / 32 * 32;  // 256-byte slices
-  if (p.buf.defined() && p.used + need > POOL_DOUBLES) {
-    if (p.buf.use_count() == 1) {
-      // Another thread's launches came before it let go of its slice.
-      std::atomic_thread_fence(std::memory_order_acquire);
-      const cudaError_t err =
-          cudaMemsetAsync(p.buf.data_ptr(), 0, POOL_DOUBLES * sizeof(double), stream);
-      TORCH_CHECK(err == cudaSuccess, "batch norm scratch: ", cudaGetErrorString(err));
-      p.used = 0;
-    } else {
-      p.buf.reset();
+  // Memory is allocated and given back outside the lock: the allocator may ask for the
+  // interpreter's lock (to note a stack), which a thread that waits for this one can hold.
+  at::Tensor fresh, old;
+  for (;;) {
+    {
+      std::lock_guard<std::mutex> lock(mu);
+      Pool& p = pools[{like.get_device(), stream}];
+      bool room = p.buf.defined() && p.used + need <= POOL_DOUBLES;
+      if (!room && p.buf.defined() && p.buf.use_count() == 1) {
+        // Another thread's launches came before it let go of its slice.
+        std::atomic_thread_fence(std::memory_order_acquire);
+        const cudaError_t err =
+            cudaMemsetAsync(p.buf.data_ptr(), 0, POOL_DOUBLES * sizeof(double), stream);
+        TORCH_CHECK(err == cudaSuccess, "batch norm scratch: ", cudaGetErrorString(err));
+        p.used = 0;
+        room = true;
+      }
+      if (!room && fresh.defined()) {
+        old = std::move(p.buf);
+        p.buf = std::move(fresh);
+        p.used = 0;
+        room = true;
+      }
+      if (room) {
+        *own = p.buf;
+        double* out = p.buf.data_ptr<double>() + p.used;
+        p.used += need;
+        return out;
+      }
     }
+    fresh = at::zeros({POOL_DOUBLES}, like.options().dtype(at::kDouble));
   }
-  if (!p.buf.defined()) {
-    p.buf = at::zeros({POOL_DOUBLES}, like.options().dtype(at::kDouble));
-    p.used = 0;
-  }
-  *own = p.buf;
-  double* out = p.buf.data_ptr<double>() + p.used;
-  p.used += need;
-  return out;
 }
 
 namespace {

@@ -883,3 +883,43 @@ def test_block_under_compiled_autograd(down):
         y.backward(torch.ones_like(y))
     for t, b in zip(inputs, want):
         assert _rel(t.grad, b) <= 2e-2  # sums in another order
+
+
+_RECORDED = """
+import threading, torch
+from horovod_b200.models.resnet import Bottleneck
+from horovod_b200.ops.batch_norm import BatchNormAct2d
+torch.cuda.memory._record_memory_history(enabled="all", stacks="python")
+down = torch.nn.Sequential(torch.nn.Conv2d(64, 256, 1, bias=False), BatchNormAct2d(256, relu=False))
+block = Bottleneck(64, 64, 1, down).cuda().to(memory_format=torch.channels_last)
+norm = BatchNormAct2d(256).cuda()
+
+def blocks():
+    x = torch.randn(2, 8, 6, 64, device="cuda").bfloat16().permute(0, 3, 1, 2)
+    for _ in range(400):
+        with torch.autocast("cuda", dtype=torch.bfloat16):
+            block(x).sum().backward()
+
+def norms():
+    x = torch.randn(2, 8, 6, 256, device="cuda").bfloat16().permute(0, 3, 1, 2)
+    for _ in range(4000):
+        norm(x)
+
+threads = [threading.Thread(target=f) for f in (blocks, norms)]
+[t.start() for t in threads]
+[t.join() for t in threads]
+torch.cuda.synchronize()
+print("done")
+"""
+
+
+def test_two_threads_while_allocations_are_recorded():
+    """The allocator then takes the interpreter's lock, which one thread holds while it
+    waits for the scratch that the other one is given: nobody waits for both."""
+    import os
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    run = subprocess.run([sys.executable, "-c", _RECORDED], cwd=root, capture_output=True,
+                         text=True, timeout=200)
+    assert run.returncode == 0 and "done" in run.stdout, run.stderr[-2000:]
