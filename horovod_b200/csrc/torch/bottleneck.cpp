@@ -446,6 +446,7 @@ class Bottleneck : public torch::autograd::Function<Bottleneck> {
     ctx->save_for_backward(keep);
     std::vector<double> eps;
     for (const Norm& norm : block.norms) eps.push_back(norm.eps);
+    ctx->saved_data.reserve(3 + 2 * LAYERS);
     ctx->saved_data["eps"] = eps;
     ctx->saved_data["stride"] = block.stride;
     // For the edges of gradients of gradients. Every backward works on the casts: the

@@ -22,4 +22,5 @@ def functions_watched():
     """Whether a mode is to see the calls of torch's functions, those that a native node
     has no calls of among them. A device as a context is a mode too, one that changes
     where tensors are made and nothing else."""
-    return any(type(mode) is not DeviceContext for mode in _get_current_function_mode_stack())
+    return torch._C._len_torch_function_stack() > 0 and \
+        any(type(mode) is not DeviceContext for mode in _get_current_function_mode_stack())

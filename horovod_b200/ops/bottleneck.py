@@ -101,11 +101,12 @@ def fused_bottleneck_available(block, x):
         return None
     device, channels = x.device, x.size(1)
     into = (channels, block.conv1.out_channels, block.conv2.out_channels, channels)
+    norm_supported = _extension().bn_supported
     for (conv, norm, kernel, stride, relu), inputs in zip(layers, into):
         if stride not in (1, 2) or conv.in_channels != inputs or \
                 not _plain_conv(conv, kernel, stride, dtypes, device) or \
                 not _plain_norm(norm, relu, conv, device) or \
-                not _extension().bn_supported(1, conv.out_channels):
+                not norm_supported(1, conv.out_channels):
             return None
     if len(layers) == 3 and (layers[1][3] != 1 or block.conv3.out_channels != channels):
         return None
