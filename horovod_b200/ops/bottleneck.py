@@ -19,7 +19,7 @@ import torch.nn as nn
 from torch.nn.modules.module import _has_any_global_hook
 
 from horovod_b200.ops._native import PLAIN, functions_watched, plain_autograd
-from horovod_b200.ops.batch_norm import BatchNormAct2d, fused_batch_norm_available
+from horovod_b200.ops.batch_norm import BatchNormAct2d
 from horovod_b200.ops.stem_conv import tensor_core_kernels_enabled
 
 
@@ -85,7 +85,8 @@ def fused_bottleneck_available(block, x):
     if not (type(x) in PLAIN and x.is_cuda and x.dim() == 4 and x.numel() > 0
             and x.dtype in (torch.bfloat16, torch.float16)):
         return None
-    if os.environ.get("HOROVOD_B200_FUSED_BLOCK", "1") != "1" or _has_any_global_hook() or \
+    if os.environ.get("HOROVOD_B200_FUSED_BLOCK", "1") != "1" or \
+            os.environ.get("HOROVOD_B200_FUSED_BN", "1") != "1" or _has_any_global_hook() or \
             not plain_autograd() or functions_watched():
         return None
     if not x.is_contiguous(memory_format=torch.channels_last) or x.data_ptr() % 16 != 0:
@@ -112,7 +113,7 @@ def fused_bottleneck_available(block, x):
         return None
     if len(layers) == 4 and layers[3][0].out_channels != block.conv3.out_channels:
         return None
-    if not fused_batch_norm_available(x, 0.1) or not tensor_core_kernels_enabled(device):
+    if not norm_supported(1, channels) or not tensor_core_kernels_enabled(device):
         return None
     return layers
 
